@@ -666,81 +666,6 @@ __global__ void __launch_bounds__(256)
   reduce_finish<1>(acc, mx, rb, [=](const Sums<1>& s) { lsc->sb = zm ? s.v[0] / n : 0.0; });
 }
 
-// direct_coarse_solve (linsolve/poisson_solver.cpp:530-567) with the
-// elimination precomputed on the host: row swaps, multipliers and the upper
-// factor are applied to the right-hand side in the reference's order.
-template <typename T, typename B>
-__global__ void k_coarse_solve(int n, const int* __restrict__ swaps, const double* __restrict__ f,
-                               const B* __restrict__ b, const double* sb_ptr, T* __restrict__ out,
-                               LevelScalars* ls, int zm, SolveScalars* sc) {
-  pdl_enter();
-  __shared__ double y[kMaxCoarse];
-  __shared__ double red[32];
-  const int t = threadIdx.x;
-  const double sb = *sb_ptr;
-  for(int q = t; q < n; q += blockDim.x) y[q] = double(b[q]) - sb;
-  __syncthreads();
-  if(zm && t == 0) y[n - 1] = 0.0;
-  __syncthreads();
-  for(int p = 0; p < n; ++p) {
-    if(t == 0 && swaps[p] != p) {
-      const double tmp = y[p];
-      y[p] = y[swaps[p]];
-      y[swaps[p]] = tmp;
-    }
-    __syncthreads();
-    const double yp = y[p];
-    for(int r = p + 1 + t; r < n; r += blockDim.x) {
-      const double factor = f[static_cast<size_t>(r) * n + p];
-      if(factor != 0.0) y[r] -= factor * yp;
-    }
-    __syncthreads();
-  }
-  for(int row = n - 1; row >= 0; --row) {
-    if(t == 0) y[row] = y[row] / f[static_cast<size_t>(row) * n + row];
-    __syncthreads();
-    const double yr = y[row];
-    for(int r = t; r < row; r += blockDim.x) y[r] -= f[static_cast<size_t>(r) * n + row] * yr;
-    __syncthreads();
-  }
-  // subtract_active_mean on the coarse correction
-  double part = 0.0;
-  for(int q = t; q < n; q += blockDim.x) part += y[q];
-  part = warp_sum(part);
-  if((t & 31) == 0) red[t >> 5] = part;
-  __syncthreads();
-  double mean = 0.0;
-  if(zm) {
-    double s = 0.0;
-    for(int w = 0; w < (int(blockDim.x) + 31) / 32; ++w) s += red[w];
-    mean = s / n;
-  }
-  double rzp = 0.0;
-  for(int q = t; q < n; q += blockDim.x) {
-    const double v = y[q] - mean;
-    out[q] = T(v);
-    rzp += (double(b[q]) - sb) * v;
-  }
-  __syncthreads();
-  rzp = warp_sum(rzp);
-  if((t & 31) == 0) red[t >> 5] = rzp;
-  __syncthreads();
-  if(t == 0) {
-    ls->sx = 0.0;
-    ls->sum_x = 0.0;
-    if(sc != nullptr) {
-      double s = 0.0;
-      for(int w = 0; w < (int(blockDim.x) + 31) / 32; ++w) s += red[w];
-      if(sc->first) {
-        sc->rz = s;
-      } else {
-        sc->beta = s / sc->rz;
-        sc->rz = s;
-      }
-    }
-  }
-}
-
 // ---------------------------------------------------------------------------
 // Plane-pipelined stencil kernels.  A block owns a tile of whole rows (all nx
 // cells, TY = 1024 / nx rows) and a chunk of k planes.  One thread stages each
@@ -2060,24 +1985,26 @@ __global__ void __launch_bounds__(256)
 }
 
 // ---------------------------------------------------------------------------
-// The small end of the hierarchy in one block.  From the first level of at
-// most kTailMaxCells cells down to the coarsest, v_cycle (:597-633) runs in
-// one block with every level's rhs, correction and scratch in shared memory.
-// Each phase ends with one barrier that also publishes the warp partials of
-// the vector it produced; every thread then adds the partials itself (same
-// order in every thread), so the mean of the reference's subtract_active_mean
-// (after every sweep, on the residual, on the coarse rhs, after the
-// prolongation) is known without a second barrier and is subtracted as the
-// next phase loads the vector (a pending shift), as in the per-level kernels.
-// The two pre-sweeps from zero are one phase (k_vsmooth_pre), the
-// prolongation and the first post-sweep another (k_vprolong_smooth).
+// The small end of the hierarchy as one matrix.  From the first level of at
+// most kDenseCells cells down to the coarsest, v_cycle (:597-633) is a fixed
+// linear map of that level's rhs (sweeps, restriction, elimination and mean
+// removals are all linear), so its matrix G is formed once per plan -- column
+// c is the V-cycle of the unit vector e_c, one block each (k_dense_columns) --
+// and a solve applies it with one matrix-vector product (k_dense_apply).
+//
+// Replaying the V-cycle instead costs one block ~45 barrier-separated phases,
+// and above 32 coarse unknowns an elimination of two barriers per unknown:
+// 27 us per V-cycle from 16^3 down, 207 us with 135 coarse unknowns (96 x 80 x
+// 72), 578 us with 315 (144 x 80 x 112).  G of 512 cells is 2 MB and of 1024
+// cells 8 MB, read from L2 by a block per kDenseRows rows in a few us; above
+// 1024 cells it would leave L2 no room (4096 cells: 134 MB).
 // ---------------------------------------------------------------------------
-constexpr int kTailMaxCells = 4096;
+constexpr int kDenseCells = 1024;
 constexpr int kTailMaxLevels = 12;
 constexpr int kTailThreads = 512;
 
 // Per tail level (all but the coarsest), built on the host when the plan is
-// made and staged into shared memory by every tail launch:
+// made and staged into shared memory by every block of k_dense_columns:
 //   nbr[6][n]   the six operand positions of each cell under the boundary
 //               rules (nb_lo / nb_hi: neighbour, periodic image, or the cell
 //               itself), as +-(index + 1), minus for a homogeneous-Dirichlet
@@ -2094,7 +2021,6 @@ struct TailLevel {
   int off;         // offset of the level's b, x, s arrays in shared memory (elements)
   int tab;         // byte offset of the level's tables in the table region
   int nch;         // children per coarser cell
-  double d0;       // the inverse diagonal, where every class has the same one
 };
 
 struct TailArgs {
@@ -2109,10 +2035,6 @@ struct TailArgs {
   const int* swaps;
   const double* factors;
   int zm;
-  // every tail level fully periodic with power-of-two extents and one
-  // inverse diagonal: neighbours, parents and children by bit arithmetic
-  // (PerGeom), no tables staged
-  int per;
 };
 
 // Byte layout of one tail level's tables (see TailLevel).
@@ -2186,38 +2108,13 @@ __device__ __forceinline__ A tab_apply(const short* nbr, int n, int q, A ix, A i
   return -(r - two_c + l) * ix - (u - two_c + d) * iy - (f - two_c + b) * iz;
 }
 
-// Index arithmetic of a periodic level with power-of-two extents: the same
-// operand positions, parents and children (dz, dy, dx order) as the tables.
-struct PerGeom {
-  int lx, ly, mx, my, mz;  // log2 nx, log2 ny, nx - 1, ny - 1, nz - 1
-};
-
-__device__ __forceinline__ PerGeom per_geom(const CLay& L) {
-  return PerGeom{__ffs(L.nx) - 1, __ffs(L.ny) - 1, L.nx - 1, L.ny - 1, L.nz - 1};
-}
-
-// A u at cell q (same operand order and arithmetic as tab_apply).
-template <typename A, typename Op>
-__device__ __forceinline__ A per_apply(const PerGeom& g, int q, A ix, A iy, A iz, Op op, A& c) {
-  const int i = q & g.mx, j = (q >> g.lx) & g.my, sh = g.lx + g.ly, k = q >> sh;
-  const int qi = q - i, qj = q - (j << g.lx), qk = q - (k << sh);
-  c = op(q);
-  const A l = op(qi + ((i - 1) & g.mx));
-  const A r = op(qi + ((i + 1) & g.mx));
-  const A d = op(qj + (((j - 1) & g.my) << g.lx));
-  const A u = op(qj + (((j + 1) & g.my) << g.lx));
-  const A b = op(qk + (((k - 1) & g.mz) << sh));
-  const A f = op(qk + (((k + 1) & g.mz) << sh));
-  const A two_c = A(2) * c;
-  return -(r - two_c + l) * ix - (u - two_c + d) * iy - (f - two_c + b) * iz;
-}
-
-// The whole tail V-cycle in the calling block: b_in (shift sb) in, x_out
-// (mean removed) out; sm is the tail's shared-memory layout (TailArgs).
-template <typename T, bool PER>
-__device__ void vcycle_tail_body(const TailArgs& a, const T* __restrict__ b_in, double sb,
-                                 T* __restrict__ x_out, T* sm) {
-  using A = T;
+// The tail V-cycle of the unit vector e_c (its mean removed on singular
+// problems, as the rhs of every level has it removed) in the calling block;
+// x_out gets the result, its mean removed.  sm is the tail's shared-memory
+// layout (TailArgs).
+template <typename T>
+__device__ void vcycle_tail_column(const TailArgs& a, int c, T* __restrict__ x_out, double* sm) {
+  using A = double;
   __shared__ double red[2][32];
   int par = 0;
   const int tid = threadIdx.x, bd = blockDim.x;
@@ -2237,13 +2134,12 @@ __device__ void vcycle_tail_body(const TailArgs& a, const T* __restrict__ b_in, 
     for(int q = tid; q < nco; q += bd) swp[q] = a.swaps[q];
   }
   {
-    if constexpr(!PER) {
-      const uint4* src = reinterpret_cast<const uint4*>(a.tabs);
-      uint4* dst = reinterpret_cast<uint4*>(tabs);
-      for(int q = tid; q < a.tab_bytes / 16; q += bd) dst[q] = __ldg(&src[q]);
-    }
+    const uint4* src = reinterpret_cast<const uint4*>(a.tabs);
+    uint4* dst = reinterpret_cast<uint4*>(tabs);
+    for(int q = tid; q < a.tab_bytes / 16; q += bd) dst[q] = __ldg(&src[q]);
     const int n0 = a.lv[0].op.L.count();
-    for(int q = tid; q < n0; q += bd) B(0)[q] = A(double(b_in[q]) - sb);
+    const double mean = zm ? 1.0 / n0 : 0.0;
+    for(int q = tid; q < n0; q += bd) B(0)[q] = (q == c ? 1.0 : 0.0) - mean;
   }
   __syncthreads();
   double sbs[kTailMaxLevels], sxs[kTailMaxLevels];
@@ -2253,22 +2149,14 @@ __device__ void vcycle_tail_body(const TailArgs& a, const T* __restrict__ b_in, 
     const TailLevel& tl = a.lv[l];
     const int n = tl.op.L.count();
     const int nc = a.lv[l + 1].op.L.count();
-    const TailTabLayout lay = tail_tab_layout(n, nc, tl.nch, sizeof(T));
+    const TailTabLayout lay = tail_tab_layout(n, nc, tl.nch, sizeof(double));
     const short* nbr = reinterpret_cast<const short*>(tabs + tl.tab + lay.nbr);
     const short* child = reinterpret_cast<const short*>(tabs + tl.tab + lay.child);
     const unsigned char* cls = tabs + tl.tab + lay.cls;
     const A* itab = reinterpret_cast<const A*>(tabs + tl.tab + lay.itab);
-    const A d0 = A(tl.d0);
-    auto dinv = [&](int p) {
-      if constexpr(PER) return d0;
-      else return itab[cls[p]];
-    };
-    const PerGeom pg = per_geom(tl.op.L);
+    auto dinv = [&](int p) { return itab[cls[p]]; };
     const A ix = A(tl.op.inv2[0]), iy = A(tl.op.inv2[1]), iz = A(tl.op.inv2[2]);
-    auto apply = [&](int q, auto op, A& c) {
-      if constexpr(PER) return per_apply<A>(pg, q, ix, iy, iz, op, c);
-      else return tab_apply<A>(nbr, n, q, ix, iy, iz, op, c);
-    };
+    auto apply = [&](int q, auto op, A& c) { return tab_apply<A>(nbr, n, q, ix, iy, iz, op, c); };
     const A* b = B(l);
     A* x = X(l);
     A* s = S(l);
@@ -2299,19 +2187,9 @@ __device__ void vcycle_tail_body(const TailArgs& a, const T* __restrict__ b_in, 
     const A inv_children = A(1.0 / double(nch));
     A* bc = B(l + 1);
     part = 0.0;
-    const PerGeom cg = per_geom(a.lv[l + 1].op.L);
     for(int Q = tid; Q < nc; Q += bd) {
       A sum = A(0);
-      if constexpr(PER) {
-        const int I = Q & cg.mx, J = (Q >> cg.lx) & cg.my, K = Q >> (cg.lx + cg.ly);
-        for(int dz = 0; dz < (1 << tl.sz); ++dz)
-          for(int dy = 0; dy < (1 << tl.sy); ++dy)
-            for(int dx = 0; dx < (1 << tl.sx); ++dx)
-              sum += s[((I << tl.sx) + dx) + (((J << tl.sy) + dy) << pg.lx) +
-                       (((K << tl.sz) + dz) << (pg.lx + pg.ly))];
-      } else {
-        for(int t = 0; t < nch; ++t) sum += s[child[Q * nch + t]];
-      }
+      for(int t = 0; t < nch; ++t) sum += s[child[Q * nch + t]];
       const A v = inv_children * sum;
       bc[Q] = v;
       part += double(v);
@@ -2401,31 +2279,15 @@ __device__ void vcycle_tail_body(const TailArgs& a, const T* __restrict__ b_in, 
     const TailLevel& tl = a.lv[l];
     const int n = tl.op.L.count();
     const int nc = a.lv[l + 1].op.L.count();
-    const TailTabLayout lay = tail_tab_layout(n, nc, tl.nch, sizeof(T));
+    const TailTabLayout lay = tail_tab_layout(n, nc, tl.nch, sizeof(double));
     const short* nbr = reinterpret_cast<const short*>(tabs + tl.tab + lay.nbr);
     const short* parent = reinterpret_cast<const short*>(tabs + tl.tab + lay.parent);
     const unsigned char* cls = tabs + tl.tab + lay.cls;
     const A* itab = reinterpret_cast<const A*>(tabs + tl.tab + lay.itab);
-    const A d0 = A(tl.d0);
-    auto dinv = [&](int p) {
-      if constexpr(PER) return d0;
-      else return itab[cls[p]];
-    };
-    const PerGeom pg = per_geom(tl.op.L);
-    const PerGeom cg = per_geom(a.lv[l + 1].op.L);
-    auto parent_of = [&](int p) {
-      if constexpr(PER) {
-        const int i = p & pg.mx, j = (p >> pg.lx) & pg.my, k = p >> (pg.lx + pg.ly);
-        return (i >> tl.sx) + ((j >> tl.sy) << cg.lx) + ((k >> tl.sz) << (cg.lx + cg.ly));
-      } else {
-        return static_cast<int>(parent[p]);
-      }
-    };
+    auto dinv = [&](int p) { return itab[cls[p]]; };
+    auto parent_of = [&](int p) { return static_cast<int>(parent[p]); };
     const A ix = A(tl.op.inv2[0]), iy = A(tl.op.inv2[1]), iz = A(tl.op.inv2[2]);
-    auto apply = [&](int q, auto op, A& c) {
-      if constexpr(PER) return per_apply<A>(pg, q, ix, iy, iz, op, c);
-      else return tab_apply<A>(nbr, n, q, ix, iy, iz, op, c);
-    };
+    auto apply = [&](int q, auto op, A& c) { return tab_apply<A>(nbr, n, q, ix, iy, iz, op, c); };
     const A* b = B(l);
     A* x = X(l);
     A* s = S(l);
@@ -2460,20 +2322,74 @@ __device__ void vcycle_tail_body(const TailArgs& a, const T* __restrict__ b_in, 
   }
   const int n0 = a.lv[0].op.L.count();
   const A s0 = A(sxc);
-  for(int q = tid; q < n0; q += bd) x_out[q] = X(0)[q] - s0;
+  for(int q = tid; q < n0; q += bd) x_out[q] = T(X(0)[q] - s0);
 }
 
-template <typename T, bool PER>
-__global__ void __launch_bounds__(kTailThreads)
-    k_vcycle_tail(TailArgs a, const T* __restrict__ b_in, const double* sb_ptr, T* __restrict__ x_out,
-                  LevelScalars* ls_out) {
-  pdl_enter();
+// Column c of G, one block per column: G[c * n + row] (FP32 on the mixed path,
+// formed in FP64).
+template <typename T>
+__global__ void __launch_bounds__(kTailThreads) k_dense_columns(TailArgs a, T* __restrict__ G) {
   extern __shared__ __align__(16) unsigned char tail_smem[];
-  vcycle_tail_body<T, PER>(a, b_in, *sb_ptr, x_out, reinterpret_cast<T*>(tail_smem));
-  if(threadIdx.x == 0) {
-    ls_out->sx = 0.0;  // the mean is already removed
-    ls_out->sum_x = 0.0;
+  const int n = a.lv[0].op.L.count();
+  vcycle_tail_column<T>(a, blockIdx.x, G + static_cast<size_t>(blockIdx.x) * n,
+                        reinterpret_cast<double*>(tail_smem));
+}
+
+// x = G b, sums in FP64.  A block owns kDenseRows rows; its threads split the
+// columns into groups, so that a warp reads runs of kDenseRows consecutive
+// entries of a column (128 bytes in FP64) and every thread has the loads of
+// its n / 16 columns in flight at once; the groups' partial sums meet in shared
+// memory in a fixed order.  Bound by the read of G from L2 (n = 512: 2 MB over
+// 32 blocks).  G removes the rhs's and the result's mean, so no shift is read
+// or left.  With sc (the dense level is the finest) it also forms r.z.
+constexpr int kDenseRows = 16;
+constexpr int kDenseThreads = 256;
+
+template <typename T, typename B>
+__global__ void __launch_bounds__(kDenseThreads)
+    k_dense_apply(int n, const T* __restrict__ G, const B* __restrict__ b, T* __restrict__ x,
+                  LevelScalars* ls, SolveScalars* sc, RedBuf rb) {
+  pdl_enter();
+  constexpr int kGroups = kDenseThreads / kDenseRows;
+  __shared__ double part[kGroups][kDenseRows + 1];
+  __shared__ double bs[kDenseCells];
+  const int r = threadIdx.x % kDenseRows, grp = threadIdx.x / kDenseRows;
+  const int row = blockIdx.x * kDenseRows + r;
+  for(int q = threadIdx.x; q < n; q += kDenseThreads) bs[q] = double(b[q]);
+  __syncthreads();
+  double sum = 0.0;
+  if(row < n) {
+#pragma unroll 8
+    for(int c = grp; c < n; c += kGroups) sum += double(__ldg(&G[static_cast<size_t>(c) * n + row])) * bs[c];
   }
+  part[grp][r] = sum;
+  __syncthreads();
+  double acc[2] = {0.0, 0.0};
+  if(grp == 0 && row < n) {
+    double v = 0.0;
+#pragma unroll
+    for(int k = 0; k < kGroups; ++k) v += part[k][r];
+    x[row] = T(v);
+    acc[0] = double(T(v));
+    acc[1] = bs[row] * double(T(v));
+  }
+  if(sc == nullptr) {
+    if(blockIdx.x == 0 && threadIdx.x == 0) {
+      ls->sx = 0.0;  // the mean is already removed
+      ls->sum_x = 0.0;
+    }
+    return;
+  }
+  const bool mx[2] = {false, false};
+  reduce_finish<2>(acc, mx, rb, [=](const Sums<2>& s) {
+    const double mean = sc->zero_mean ? s.v[0] / n : 0.0;
+    ls->sx = mean;
+    ls->sum_x = s.v[0];
+    // r.z with z = x - mean, r = b - sr (linsolve/poisson_solver.cpp:749, :791)
+    const double rz_new = s.v[1] - mean * (sc->sum_r - sc->n * sc->sr) - sc->sr * s.v[0];
+    if(!sc->first) sc->beta = rz_new / sc->rz;
+    sc->rz = rz_new;
+  });
 }
 
 // ---------------------------------------------------------------------------
@@ -2814,8 +2730,6 @@ struct PoissonPlan {
   int zero_mean = 1;
   std::vector<Level> levels;
   int coarse_n = 0;
-  int* swaps = nullptr;
-  double* factors = nullptr;
   LevelScalars* ls = nullptr;  // device, one per level
   double *b = nullptr, *x = nullptr, *r = nullptr, *p = nullptr, *ap = nullptr;
   double* hist = nullptr;
@@ -2837,11 +2751,9 @@ struct PoissonPlan {
   CUtensorMap tm_pm, tm_ph, tm_pm2, tm_ph2;
   double* p2 = nullptr;     // second p buffer of the fused CG step
   float* p32b = nullptr;
-  // levels tail_first.. run as one single-block launch (k_vcycle_tail)
+  // levels tail_first.. run as one matrix-vector product (k_dense_apply)
   int tail_first = -1;
-  TailArgs tail{};
-  size_t tail_smem = 0;
-  unsigned char* tail_tabs = nullptr;  // the tail's staged tables (TailLevel)
+  void* dense = nullptr;  // their V-cycle's matrix, column by column
 };
 
 namespace {
@@ -2888,6 +2800,17 @@ std::vector<double> inverse_diagonal_table(const Grid& g, const PBC& pbc) {
   return t;
 }
 
+// Device memory of the plan's setup, freed with its scope.
+struct DeviceBytes {
+  void* p = nullptr;
+  explicit DeviceBytes(size_t n) {
+    if(n > 0) OFB_CHECK(cudaMalloc(&p, n));
+  }
+  ~DeviceBytes() { cudaFree(p); }
+  DeviceBytes(const DeviceBytes&) = delete;
+  DeviceBytes& operator=(const DeviceBytes&) = delete;
+};
+
 // Host copy of apply_poisson_operator with homogeneous rules, for assembling
 // the coarse matrix column by column as direct_coarse_solve does.
 void host_apply(const Grid& g, const PBC& pbc, const std::vector<double>& in,
@@ -2931,34 +2854,16 @@ void host_apply(const Grid& g, const PBC& pbc, const std::vector<double>& in,
 
 namespace {
 
-// Chooses the first level (below the finest) whose cells fit the single-block
-// tail and lays out its shared memory: per level b, x, s (T), then the
-// coarsest solve's FP64 vector.  ORCHARD_B200_NO_TAIL=1 keeps every level on
-// the per-level kernels (for comparisons).
-// Whether the tail from level `first` can run on index arithmetic: every
-// axis periodic, every extent a power of two, and one inverse diagonal for
-// all 64 boundary classes of each level.
-bool tail_periodic(const PoissonPlan* P, int first) {
-  for(int l = first; l < static_cast<int>(P->levels.size()); ++l) {
-    const Level& lv = P->levels[l];
-    for(int a = 0; a < 3; ++a) {
-      const int n = lv.L.n(a);
-      if(!lv.op.periodic[a] || (n & (n - 1)) != 0) return false;
-    }
-    const std::vector<double> t = inverse_diagonal_table(lv.g, P->pbc);
-    for(int c = 1; c < 64; ++c)
-      if(t[c] != t[0]) return false;
-  }
-  return true;
-}
-
-void setup_tail(PoissonPlan* P, size_t tsz) {
-  const char* e = std::getenv("ORCHARD_B200_NO_TAIL");
-  if(e != nullptr && e[0] == '1') return;
+// Chooses the first level of at most kDenseCells cells (the coarsest has no
+// more, so there is one), lays out the shared memory of its V-cycle -- per
+// level b, x, s, then the coarsest solve's vector, factors and the levels'
+// tables -- and forms the V-cycle's matrix.
+void setup_dense(PoissonPlan* P, const int* swaps, const double* factors) {
   const int nl = static_cast<int>(P->levels.size());
+  constexpr size_t tsz = sizeof(double);
   constexpr size_t kSmemLimit = 200 * 1024;
-  for(int first = 1; first < nl; ++first) {
-    if(P->levels[first].L.count() > kTailMaxCells || nl - first > kTailMaxLevels) continue;
+  for(int first = 0; first < nl; ++first) {
+    if(P->levels[first].L.count() > kDenseCells || nl - first > kTailMaxLevels) continue;
     TailArgs t{};
     t.count = nl - first;
     size_t cursor = 0;  // elements of T
@@ -3034,10 +2939,7 @@ void setup_tail(PoissonPlan* P, size_t tsz) {
             base[lay.cls + q] =
                 static_cast<unsigned char>(cls(i, lv.L.nx) + 4 * cls(j, lv.L.ny) + 16 * cls(k, lv.L.nz));
           }
-      for(int c = 0; c < 64; ++c) {
-        if(tsz == sizeof(float)) reinterpret_cast<float*>(base + lay.itab)[c] = static_cast<float>(tinv[c]);
-        else reinterpret_cast<double*>(base + lay.itab)[c] = tinv[c];
-      }
+      for(int c = 0; c < 64; ++c) reinterpret_cast<double*>(base + lay.itab)[c] = tinv[c];
       for(int K = 0; K < cv.L.nz; ++K)
         for(int J = 0; J < cv.L.ny; ++J)
           for(int I = 0; I < cv.L.nx; ++I) {
@@ -3054,31 +2956,29 @@ void setup_tail(PoissonPlan* P, size_t tsz) {
     t.tab_bytes = static_cast<int>(blob.size());
     const size_t bytes = tab_off + blob.size();
     if(bytes > kSmemLimit) continue;
-    if(!blob.empty()) {
-      OFB_CHECK(cudaMalloc(&P->tail_tabs, blob.size()));
-      OFB_CHECK(cudaMemcpy(P->tail_tabs, blob.data(), blob.size(), cudaMemcpyHostToDevice));
-    }
-    t.tabs = P->tail_tabs;
-    t.swaps = P->swaps;
-    t.factors = P->factors;
+    DeviceBytes tabs(blob.size());
+    if(!blob.empty())
+      OFB_CHECK(cudaMemcpy(tabs.p, blob.data(), blob.size(), cudaMemcpyHostToDevice));
+    t.tabs = static_cast<const unsigned char*>(tabs.p);
+    t.swaps = swaps;
+    t.factors = factors;
     t.zm = P->zero_mean;
-    t.per = tail_periodic(P, first) ? 1 : 0;
-    for(int l = first; l < nl; ++l) t.lv[l - first].d0 = inverse_diagonal_table(P->levels[l].g, P->pbc)[0];
-    auto smem_attr = [&](const void* k) {
-      OFB_CHECK(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(bytes)));
+    const int n = P->levels[first].L.count();
+    auto columns = [&](auto* G, auto kern) {
+      OFB_CHECK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(bytes)));
+      kern<<<n, kTailThreads, bytes>>>(t, G);
+      OFB_LAUNCH_CHECK("k_dense_columns");
     };
-    if(tsz == sizeof(float)) {
-      smem_attr(reinterpret_cast<const void*>(k_vcycle_tail<float, false>));
-      smem_attr(reinterpret_cast<const void*>(k_vcycle_tail<float, true>));
-    } else {
-      smem_attr(reinterpret_cast<const void*>(k_vcycle_tail<double, false>));
-      smem_attr(reinterpret_cast<const void*>(k_vcycle_tail<double, true>));
-    }
-    P->tail = t;
+    const size_t gbytes = static_cast<size_t>(n) * n * (P->precision == 1 ? sizeof(float) : sizeof(double));
+    OFB_CHECK(cudaMalloc(&P->dense, gbytes));
+    P->bytes += gbytes;
+    if(P->precision == 1) columns(static_cast<float*>(P->dense), k_dense_columns<float>);
+    else columns(static_cast<double*>(P->dense), k_dense_columns<double>);
+    OFB_CHECK(cudaStreamSynchronize(nullptr));  // the tables and factors are freed on return
     P->tail_first = first;
-    P->tail_smem = bytes;
     return;
   }
+  throw std::invalid_argument("the coarsest multigrid level does not fit the dense solve");
 }
 
 // Tensor maps of the plane-pipelined kernels for every level above the
@@ -3276,13 +3176,12 @@ PoissonPlan* poisson_plan_create(const Grid& g, const PBC& pbc_in, int precision
       m[static_cast<size_t>(row) * n + piv] = factor;  // keep the multiplier
     }
   }
-  OFB_CHECK(cudaMalloc(&P->swaps, n * sizeof(int)));
-  OFB_CHECK(cudaMalloc(&P->factors, static_cast<size_t>(n) * n * sizeof(double)));
-  OFB_CHECK(cudaMemcpy(P->swaps, swaps.data(), n * sizeof(int), cudaMemcpyHostToDevice));
-  OFB_CHECK(cudaMemcpy(P->factors, m.data(), static_cast<size_t>(n) * n * sizeof(double),
-                       cudaMemcpyHostToDevice));
-
-  setup_tail(P, tsz);
+  {
+    DeviceBytes dswaps(n * sizeof(int)), dfact(static_cast<size_t>(n) * n * sizeof(double));
+    OFB_CHECK(cudaMemcpy(dswaps.p, swaps.data(), n * sizeof(int), cudaMemcpyHostToDevice));
+    OFB_CHECK(cudaMemcpy(dfact.p, m.data(), static_cast<size_t>(n) * n * sizeof(double), cudaMemcpyHostToDevice));
+    setup_dense(P, static_cast<const int*>(dswaps.p), static_cast<const double*>(dfact.p));
+  }
 
   const size_t nf = P->levels[0].L.count();
   OFB_CHECK(cudaMalloc(&P->b, nf * sizeof(double)));
@@ -3331,8 +3230,6 @@ void poisson_plan_destroy(PoissonPlan* P) {
   if(P->graph) cudaGraphDestroy(P->graph);
   cudaFree(P->hist);
   cudaFree(P->ls);
-  cudaFree(P->swaps);
-  cudaFree(P->factors);
   cudaFree(P->b);
   cudaFree(P->x);
   cudaFree(P->r);
@@ -3346,7 +3243,7 @@ void poisson_plan_destroy(PoissonPlan* P) {
   cudaFree(P->p32b);
   cudaFree(P->sc_in);
   cudaFree(P->fault);
-  cudaFree(P->tail_tabs);
+  cudaFree(P->dense);
   delete P;
 }
 
@@ -3445,21 +3342,16 @@ void v_cycle(PoissonPlan* P, int l, const V* r0, SolveScalars* sc, RedBuf rb, cu
   T* a = static_cast<T*>(lv.a);
   T* x = static_cast<T*>(lv.x);
   if(l == P->tail_first) {
-    ProfScope ps(kKCoarseLevels, s);
-    launch_pdl(P->tail.per ? k_vcycle_tail<T, true> : k_vcycle_tail<T, false>, 1, kTailThreads, P->tail_smem,
-               s, P->tail, static_cast<const T*>(lv.b), &ls->sb, x, ls);
-    OFB_LAUNCH_CHECK("k_vcycle_tail");
-    return;
-  }
-  if(l + 1 == nl) {
-    ProfScope ps(kKCoarseSolve, s);
+    ProfScope ps(l == 0 ? kKCoarseSolve : kKCoarseLevels, s);
+    const int n = lv.L.count();
+    const dim3 grid((n + kDenseRows - 1) / kDenseRows);
+    const T* G = static_cast<const T*>(P->dense);
     if(l == 0)
-      launch_pdl(k_coarse_solve<T, V>, 1, 256, 0, s, P->coarse_n, P->swaps, P->factors, r0, sb_ptr, x, ls, zm,
-                 rz_sc);
+      launch_pdl(k_dense_apply<T, V>, grid, kDenseThreads, 0, s, n, G, r0, x, ls, sc, rb);
     else
-      launch_pdl(k_coarse_solve<T, T>, 1, 256, 0, s, P->coarse_n, P->swaps, P->factors,
-                 static_cast<const T*>(lv.b), sb_ptr, x, ls, zm, rz_sc);
-    OFB_LAUNCH_CHECK("k_coarse_solve");
+      launch_pdl(k_dense_apply<T, T>, grid, kDenseThreads, 0, s, n, G, static_cast<const T*>(lv.b), x, ls,
+                 static_cast<SolveScalars*>(nullptr), rb);
+    OFB_LAUNCH_CHECK("k_dense_apply");
     return;
   }
   const Launch3 ln = launch3(lv.L.nx, lv.L.ny, lv.L.nz);
