@@ -1,0 +1,713 @@
+// Fused multigrid and CG kernels that march the k planes of a tile.
+//
+// A block owns an interior tile of ix x iy cells and a chunk of k planes, plus
+// a halo of one patch on either x side and two rows on either y side.  A thread
+// owns a patch of two rows of W cells (16 bytes: W = 2 in FP64, 4 in FP32;
+// whole footprints of coarse cells, so restriction and prolongation are local
+// to it) and walks k with its z neighbours in registers; per plane the block
+// publishes the fields whose in-plane neighbours it needs in shared memory,
+// passes one barrier (the planes alternate between two buffers) and computes.
+// Several sweeps are pipelined in one pass, each a plane behind the one it
+// reads: the halo shrinks by one cell per sweep, so intermediate vectors are
+// never written to memory.
+//
+// Cells outside the domain are images: the load maps an index to the cell
+// whose value it repeats (periodic wrap, or the mirror cell of a
+// homogeneous-Neumann wall) and, for a homogeneous-Dirichlet wall, the sign -1
+// (neighbor_value, linsolve/poisson_solver.cpp:195-242).  The operator, the
+// Jacobi diagonal and the sweeps commute with these reflections, so a sweep on
+// image cells gives the images of the sweep's result and the stencils need no
+// boundary cases.
+//
+// Shared memory holds a row's cells by their position in the patch (all first
+// cells, then all second ones, ...): a warp's accesses are then consecutive
+// words (no bank conflicts).  Rows
+// have a fixed stride and the k loop is unrolled by four with every field's
+// planes in a ring of four register slots, so that shared-memory addresses are
+// immediates and no plane is ever moved between registers: at one patch per
+// thread the loop is bound by its instruction count (rotating registers and
+// run-time strides took 359 instructions per patch and plane, 75 of them FP64).
+#pragma once
+
+#include "kernels.hpp"
+
+#include <type_traits>
+
+namespace ofb {
+
+struct OpInfo {
+  CLay L;
+  double inv2[3];  // 1 / h^2
+  int periodic[3];
+  int dir_lo[3], dir_hi[3];  // homogeneous Dirichlet (else Neumann) at each end
+  const double* invd;        // 64-entry inverse-diagonal table
+};
+
+__device__ __forceinline__ int axis_class(int c, int n) {
+  return n == 1 ? 3 : (c == 0 ? 1 : (c == n - 1 ? 2 : 0));
+}
+
+namespace march {
+
+// Patches per shared-memory row: tiles are at most 64 (FP64) or 128 cells wide.
+constexpr int kPX = 34;
+
+// Cells of a patch row: 16 bytes.
+template <typename T>
+constexpr int kW = 16 / static_cast<int>(sizeof(T));
+
+// Tile of one launch (host-chosen, see plan_tile in poisson.cu).
+struct Tile {
+  int ix, iy;    // interior cells: ix a multiple of W up to W (kPX - 2), iy even
+  int px, ey;    // extended tile: patches per row (ix / W + 2), rows
+  int tx;        // tiles along x
+  int chunk;     // k planes per block
+};
+
+// The cell that index c repeats, with the sign of a homogeneous-Dirichlet
+// reflection.
+__device__ __forceinline__ int image(int c, int n, int per, int dlo, int dhi, bool& neg) {
+  neg = false;
+  while(c < 0 || c >= n) {
+    if(per) {
+      c += c < 0 ? n : -n;
+    } else if(c < 0) {
+      c = -1 - c;
+      neg ^= dlo != 0;
+    } else {
+      c = 2 * n - 1 - c;
+      neg ^= dhi != 0;
+    }
+  }
+  return c;
+}
+
+template <typename T>
+struct Patch {
+  T v[2][kW<T>];  // [row][x cell]
+};
+
+// The 16-byte vector of a patch row.
+template <typename T>
+using Vec = std::conditional_t<std::is_same_v<T, double>, double2, float4>;
+
+template <typename T>
+__device__ __forceinline__ void unpack(const Vec<T>& d, T (&v)[kW<T>]) {
+  v[0] = d.x;
+  v[1] = d.y;
+  if constexpr(kW<T> == 4) {
+    v[2] = d.z;
+    v[3] = d.w;
+  }
+}
+
+template <typename T>
+__device__ __forceinline__ Vec<T> pack(const T (&v)[kW<T>]) {
+  if constexpr(kW<T> == 4) return make_float4(v[0], v[1], v[2], v[3]);
+  else return make_double2(v[0], v[1]);
+}
+
+// One thread's patch: image cells, signs, diagonal classes, interior flags
+// (bit W r + c for cell c of row r).
+template <typename T, bool SGN>
+struct Place {
+  static constexpr int W = kW<T>;
+  static constexpr unsigned kAll = (1u << (2 * W)) - 1u;
+  int p, row0;    // patch in its row, first extended row
+  int xi[W];      // image columns
+  int yj[2];      // image rows
+  int off[2];     // offsets of the rows' first cells in a plane
+  int yo[2];      // image rows times nx
+  unsigned cls;   // diagonal classes of the cells (x + 4 y), four bits each
+  unsigned neg;   // negated images
+  unsigned in;    // interior cells of the domain
+  int x0, y0;     // unmapped coordinates of the first cell
+  bool vec;       // the row's cells are contiguous and 16-byte aligned
+
+  __device__ __forceinline__ Place(const OpInfo& o, const Tile& t, int halo_rows) {
+    p = threadIdx.x % t.px;
+    row0 = 2 * (threadIdx.x / t.px);
+    x0 = (blockIdx.x % t.tx) * t.ix + W * (p - 1);
+    y0 = (blockIdx.x / t.tx) * t.iy + row0 - halo_rows;
+    cls = 0;
+    neg = 0;
+    in = 0;
+    bool nx_[W], ny_[2];
+    vec = o.L.nx % W == 0;
+#pragma unroll
+    for(int c = 0; c < W; ++c) {
+      xi[c] = image(x0 + c, o.L.nx, o.periodic[0], o.dir_lo[0], o.dir_hi[0], nx_[c]);
+      vec = vec && xi[c] == xi[0] + c;
+    }
+    vec = vec && xi[0] % W == 0;
+#pragma unroll
+    for(int r = 0; r < 2; ++r) {
+      yj[r] = image(y0 + r, o.L.ny, o.periodic[1], o.dir_lo[1], o.dir_hi[1], ny_[r]);
+      yo[r] = yj[r] * o.L.nx;
+      off[r] = yo[r] + xi[0];
+    }
+    const bool own = p > 0 && p < t.px - 1;
+#pragma unroll
+    for(int r = 0; r < 2; ++r)
+#pragma unroll
+      for(int c = 0; c < W; ++c) {
+        const int e = row0 + r, bit = W * r + c;
+        if(own && e >= halo_rows && e < t.ey - halo_rows && x0 + c < o.L.nx && y0 + r < o.L.ny)
+          in |= 1u << bit;
+        if(nx_[c] != ny_[r]) neg |= 1u << bit;
+        cls |= static_cast<unsigned>(axis_class(xi[c], o.L.nx) + 4 * axis_class(yj[r], o.L.ny)) << (4 * bit);
+      }
+  }
+  __device__ __forceinline__ bool interior(int r, int c) const { return (in >> (W * r + c)) & 1u; }
+
+  // The patch of f's plane that starts at cell zo.
+  __device__ __forceinline__ Patch<T> load(const T* __restrict__ f, int zo) const {
+    Patch<T> q;
+#pragma unroll
+    for(int r = 0; r < 2; ++r) {
+      if(vec) {
+        unpack<T>(*reinterpret_cast<const Vec<T>*>(f + (zo + off[r])), q.v[r]);
+      } else {
+#pragma unroll
+        for(int c = 0; c < W; ++c) q.v[r][c] = f[zo + yo[r] + xi[c]];
+      }
+    }
+    return q;
+  }
+
+  // The same into the thread's own words of a ring slot (the block's threads
+  // side by side, row by row), without waiting: take() reads them back.
+  __device__ __forceinline__ void fetch(T* slot, const T* __restrict__ f, int zo) const {
+    const unsigned d = static_cast<unsigned>(__cvta_generic_to_shared(slot)) + 16 * threadIdx.x;
+    const unsigned dr = 16 * blockDim.x;
+    if(vec) {
+      asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(d), "l"(f + (zo + off[0])) : "memory");
+      asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(d + dr), "l"(f + (zo + off[1])) : "memory");
+    } else {
+      constexpr int w = sizeof(T);
+#pragma unroll
+      for(int c = 0; c < W; ++c) {
+        asm volatile("cp.async.ca.shared.global [%0], [%1], %2;" ::"r"(d + w * c), "l"(f + (zo + yo[0] + xi[c])), "n"(w) : "memory");
+        asm volatile("cp.async.ca.shared.global [%0], [%1], %2;" ::"r"(d + dr + w * c), "l"(f + (zo + yo[1] + xi[c])), "n"(w) : "memory");
+      }
+    }
+  }
+
+  __device__ __forceinline__ Patch<T> take(const T* slot) const {
+    Patch<T> q;
+    unpack<T>(*reinterpret_cast<const Vec<T>*>(slot + W * threadIdx.x), q.v[0]);
+    unpack<T>(*reinterpret_cast<const Vec<T>*>(slot + W * (blockDim.x + threadIdx.x)), q.v[1]);
+    return q;
+  }
+
+  // A loaded patch less the vector's pending mean (only problems without
+  // Dirichlet faces have one) and with the signs of Dirichlet images.
+  __device__ __forceinline__ void settle(Patch<T>& q, T shift, bool zneg) const {
+#pragma unroll
+    for(int r = 0; r < 2; ++r)
+#pragma unroll
+      for(int c = 0; c < W; ++c) {
+        if constexpr(!SGN) q.v[r][c] -= shift;
+        else if((((neg >> (W * r + c)) & 1u) != 0) != zneg) q.v[r][c] = -q.v[r][c];
+      }
+  }
+
+  // Stores the interior cells into the plane that starts at cell zo.
+  __device__ __forceinline__ void store(T* __restrict__ f, int zo, const Patch<T>& q) const {
+    if(in == kAll && vec) {
+      *reinterpret_cast<Vec<T>*>(f + (zo + off[0])) = pack<T>(q.v[0]);
+      *reinterpret_cast<Vec<T>*>(f + (zo + off[1])) = pack<T>(q.v[1]);
+    } else if(in != 0) {
+#pragma unroll
+      for(int c = 0; c < W; ++c) {
+        if(interior(0, c)) f[zo + yo[0] + xi[c]] = q.v[0][c];
+        if(interior(1, c)) f[zo + yo[1] + xi[c]] = q.v[1][c];
+      }
+    }
+  }
+};
+
+// A field's plane in shared memory: ey rows of W runs of kPX cells, with a
+// guard row before and after.  `me` is the thread's first cell.
+template <typename T>
+constexpr int kRow = kW<T> * kPX;
+
+template <typename T>
+__device__ __forceinline__ void publish(T* me, const Patch<T>& q) {
+#pragma unroll
+  for(int r = 0; r < 2; ++r)
+#pragma unroll
+    for(int c = 0; c < kW<T>; ++c) me[r * kRow<T> + c * kPX] = q.v[r][c];
+}
+
+// Sums of the x and of the y neighbours of a published patch.  At the rim of
+// the extended tile the words read are not the true neighbours (another run's
+// end, a guard row); the cells they spoil are never used: the halo shrinks by
+// one cell per sweep.
+template <typename T>
+__device__ __forceinline__ void neighbour_sums(const T* me, const Patch<T>& q, Patch<T>& xs, Patch<T>& ys) {
+  constexpr int W = kW<T>;
+#pragma unroll
+  for(int r = 0; r < 2; ++r)
+#pragma unroll
+    for(int c = 0; c < W; ++c) {
+      const T l = c > 0 ? q.v[r][c > 0 ? c - 1 : 0] : me[r * kRow<T> + (W - 1) * kPX - 1];
+      const T h = c < W - 1 ? q.v[r][c < W - 1 ? c + 1 : 0] : me[r * kRow<T> + 1];
+      xs.v[r][c] = l + h;
+    }
+#pragma unroll
+  for(int c = 0; c < W; ++c) {
+    ys.v[0][c] = me[c * kPX - kRow<T>] + q.v[1][c];
+    ys.v[1][c] = q.v[0][c] + me[c * kPX + 2 * kRow<T>];
+  }
+}
+
+// Operator coefficients: A u = dd u - ix (x neighbours) - iy (y) - iz (z).  A
+// grid one cell deep (FLAT) folds its z images into dd.
+template <typename T>
+struct Coef {
+  T ix, iy, iz, dd;
+  __device__ __forceinline__ Coef(const OpInfo& o, bool flat) {
+    double d = 2.0 * (o.inv2[0] + o.inv2[1]);
+    if(!flat) d += 2.0 * o.inv2[2];
+    else if(!o.periodic[2]) d += (o.dir_lo[2] ? 2.0 * o.inv2[2] : 0.0) + (o.dir_hi[2] ? 2.0 * o.inv2[2] : 0.0);
+    ix = T(o.inv2[0]);
+    iy = T(o.inv2[1]);
+    iz = T(o.inv2[2]);
+    dd = T(d);
+  }
+};
+
+// b - A u on a patch.
+template <typename T, bool FLAT>
+__device__ __forceinline__ Patch<T> residual(const Coef<T>& a, const Patch<T>& b, const Patch<T>& u,
+                                             const Patch<T>& xs, const Patch<T>& ys, const Patch<T>& below,
+                                             const Patch<T>& above) {
+  Patch<T> o;
+#pragma unroll
+  for(int r = 0; r < 2; ++r)
+#pragma unroll
+    for(int c = 0; c < kW<T>; ++c) {
+      T t = b.v[r][c] - a.dd * u.v[r][c];
+      t += a.ix * xs.v[r][c];
+      t += a.iy * ys.v[r][c];
+      if constexpr(!FLAT) t += a.iz * (below.v[r][c] + above.v[r][c]);
+      o.v[r][c] = t;
+    }
+  return o;
+}
+
+// Threads of a march block: 512 at 128 registers fill an SM.
+constexpr int kMaxThreads = 512;
+
+// Planes streamed from memory pass through a ring of four slots per vector,
+// copied asynchronously ahead of their use: with the loads in registers one
+// plane ahead, waiting for them was the largest stall (28 % of the issue
+// slots at 256^3), and registers for more there are none.
+constexpr int kRing = 4;
+__device__ __forceinline__ void fetch_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+template <int N>
+__device__ __forceinline__ void fetch_wait() {
+  asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory");
+}
+
+// Words of one published plane, its guard rows included, and of one ring
+// slot; the shared memory of a kernel that publishes two fields (two planes
+// each) and streams `streams` vectors: rings, planes, diagonal table.
+template <typename T>
+__host__ __device__ inline int plane_words(const Tile& t) {
+  return (t.ey + 2) * kRow<T>;
+}
+template <typename T>
+__host__ __device__ inline int slot_words(const Tile& t) {
+  return kW<T> * t.px * t.ey;
+}
+template <typename T>
+inline size_t smem_bytes(const Tile& t, int streams) {
+  return (static_cast<size_t>(kRing) * streams * slot_words<T>(t) + static_cast<size_t>(4) * plane_words<T>(t) + 64) *
+         sizeof(T);
+}
+
+// The image plane of k, -2 <= k <= nz + 1 with nz >= 2, and whether it is a
+// negated image.
+__device__ __forceinline__ int zplane(const OpInfo& o, int k, bool& neg) {
+  const int nz = o.L.nz;
+  const bool lo = k < 0, hi = k >= nz;
+  neg = (lo && o.dir_lo[2]) || (hi && o.dir_hi[2]);
+  if(o.periodic[2]) return lo ? k + nz : hi ? k - nz : k;
+  return lo ? -1 - k : hi ? 2 * nz - 1 - k : k;
+}
+
+// The image planes of consecutive k (from k >= 0), advanced without the case
+// distinctions of zplane: the marching threads have no scalar unit to spare.
+struct Walk {
+  int k, kz, dk;
+  __device__ __forceinline__ Walk(const OpInfo& o, int k_) : k(k_), dk(1) {
+    bool neg;
+    kz = zplane(o, k, neg);
+    if(k >= o.L.nz && !o.periodic[2]) dk = -1;
+  }
+  __device__ __forceinline__ void next(const OpInfo& o) {
+    ++k;
+    kz += dk;
+    if(k == o.L.nz) {
+      if(o.periodic[2]) {
+        kz = 0;
+      } else {
+        kz -= 1;
+        dk = -1;
+      }
+    }
+  }
+};
+
+__device__ __forceinline__ bool zneg(const OpInfo& o, int k) {
+  return (k < 0 && o.dir_lo[2]) || (k >= o.L.nz && o.dir_hi[2]);
+}
+
+// omega / D on the planes of a march: the table is read again only when the z
+// class changes.
+template <typename T, bool CD>
+struct Weights {
+  const T* tab;
+  Patch<T> w;
+  int cz;
+  __device__ __forceinline__ Weights(const T* t, T d0) : tab(t), cz(-1) {
+#pragma unroll
+    for(int r = 0; r < 2; ++r)
+#pragma unroll
+      for(int c = 0; c < kW<T>; ++c) w.v[r][c] = d0;
+  }
+  __device__ __forceinline__ void at(const OpInfo& o, unsigned cls, int k) {
+    if constexpr(!CD) {
+      bool zn;
+      const int z = axis_class(zplane(o, k, zn), o.L.nz);
+      if(z == cz) return;
+      cz = z;
+#pragma unroll
+      for(int r = 0; r < 2; ++r)
+#pragma unroll
+        for(int c = 0; c < kW<T>; ++c) w.v[r][c] = tab[((cls >> (4 * (kW<T> * r + c))) & 15u) + 16 * z];
+    }
+  }
+};
+
+template <typename T>
+__device__ __forceinline__ Patch<T> times(const Patch<T>& w, const Patch<T>& u) {
+  Patch<T> q;
+#pragma unroll
+  for(int r = 0; r < 2; ++r)
+#pragma unroll
+    for(int c = 0; c < kW<T>; ++c) q.v[r][c] = w.v[r][c] * u.v[r][c];
+  return q;
+}
+
+// u + w res: a damped Jacobi sweep from its residual.
+template <typename T>
+__device__ __forceinline__ Patch<T> relax(const Patch<T>& u, const Patch<T>& w, const Patch<T>& res) {
+  Patch<T> q;
+#pragma unroll
+  for(int r = 0; r < 2; ++r)
+#pragma unroll
+    for(int c = 0; c < kW<T>; ++c) q.v[r][c] = u.v[r][c] + w.v[r][c] * res.v[r][c];
+  return q;
+}
+
+// Runs step(J, s) for s = s0 .. s1 with J = (s - s0) mod 4 a compile-time
+// constant (the register slot of plane s).
+template <typename Step>
+__device__ __forceinline__ void ring4(int s0, int s1, Step step) {
+  for(int s = s0; s <= s1; s += 4) {
+    step(std::integral_constant<int, 0>(), s);
+    if(s + 1 > s1) break;
+    step(std::integral_constant<int, 1>(), s + 1);
+    if(s + 2 > s1) break;
+    step(std::integral_constant<int, 2>(), s + 2);
+    if(s + 3 > s1) break;
+    step(std::integral_constant<int, 3>(), s + 3);
+  }
+}
+
+// Descent of one V-cycle level (v_cycle, linsolve/poisson_solver.cpp:597-624):
+// both pre-sweeps from a zero correction, the residual and its restriction, in
+// one pass over b:  a = omega b / D (pointwise), x = a + omega (b - A a) / D,
+// bc = R (b - A x).  b carries the pending shift *sb_ptr (its mean, finest
+// level).  The means the reference removes between these steps are constants
+// (of a and x: A annihilates them, and the prolonged sum's constant is removed
+// with mean(z)) or zero up to rounding (of bc: the residual of a zero-mean rhs
+// has zero mean), so no sum is formed here.
+//
+// Bound: one read of b, one write of x and of bc (2.125 vectors); in FP64 at
+// 256^3 the arithmetic and the shared-memory traffic are each near the DRAM time.
+template <typename T, bool SGN, bool CD, bool FLAT>
+__global__ void __launch_bounds__(kMaxThreads, 1)
+    k_descend(OpInfo o, CLay oc, Tile t, const T* __restrict__ b, const double* sb_ptr, T* __restrict__ x,
+              T* __restrict__ bc, int rx, int ry, int rz) {
+  extern __shared__ __align__(16) unsigned char march_sm[];
+  T* ring = reinterpret_cast<T*>(march_sm);
+  const int sw = slot_words<T>(t), pw = plane_words<T>(t);
+  T* planes = ring + kRing * 1 * sw;
+  T* tab = planes + 4 * pw;
+  if constexpr(!CD) {
+    for(int q = threadIdx.x; q < 64; q += blockDim.x) tab[q] = T(2.0 / 3.0 * o.invd[q]);
+    __syncthreads();
+  }
+  Weights<T, CD> W(tab, T(2.0 / 3.0 * o.invd[0]));
+  const Place<T, SGN> pl(o, t, 2);
+  const Coef<T> co(o, FLAT);
+  const T inv_children = T(1.0 / double(rx * ry * rz));
+  const int nxy = o.L.nxy;
+  const int k0 = blockIdx.y * t.chunk, k1 = min(k0 + t.chunk, o.L.nz);
+  T* me = planes + (pl.row0 + 1) * kRow<T> + pl.p;  // field 0 of the even planes
+  pdl_enter();
+  const T sb = SGN ? T(0) : T(*sb_ptr);
+  bool zn;
+  Patch<T> racc;
+  constexpr int PW = kW<T>;
+  auto restrict_out = [&](int K) {
+    if(pl.in == 0) return;
+    if(rx == 2 && ry == 2) {
+      T* out = bc + oc.idx(pl.x0 >> 1, pl.y0 >> 1, K);
+#pragma unroll
+      for(int c = 0; c < PW; c += 2)
+        if(pl.interior(0, c))
+          out[c / 2] = inv_children * ((racc.v[0][c] + racc.v[0][c + 1]) + (racc.v[1][c] + racc.v[1][c + 1]));
+      return;
+    }
+#pragma unroll
+    for(int r = 0; r < 2; ++r)
+#pragma unroll
+      for(int c = 0; c < PW; ++c) {
+        if((ry == 2 && r == 1) || (rx == 2 && (c & 1)) || !pl.interior(r, c)) continue;
+        T v = racc.v[r][c];
+        if(rx == 2) v += racc.v[r][c | 1];
+        if(ry == 2) v += racc.v[1][c];
+        bc[oc.idx((pl.x0 + c) >> (rx - 1), (pl.y0 + r) >> (ry - 1), K)] = inv_children * v;
+      }
+  };
+  Patch<T> xs, ys;
+  if constexpr(FLAT) {
+    Patch<T> bq = pl.load(b, 0);
+    pl.settle(bq, sb, false);
+    W.at(o, pl.cls, 0);
+    const Patch<T> a = times(W.w, bq);
+    publish(me, a);
+    __syncthreads();
+    neighbour_sums(me, a, xs, ys);
+    const Patch<T> xq = relax(a, W.w, residual<T, true>(co, bq, a, xs, ys, a, a));
+    pl.store(x, 0, xq);
+    publish(me + pw, xq);
+    __syncthreads();
+    neighbour_sums(me + pw, xq, xs, ys);
+    racc = residual<T, true>(co, bq, xq, xs, ys, xq, xq);
+    restrict_out(0);
+  } else {
+    // step s: x(s) from a(s - 1 .. s + 1), then the residual of plane s - 1
+    Patch<T> A[4], B[4], X[4];
+    Walk f(o, k0);  // the next plane to fetch
+    for(int q = 1; q <= 3; ++q) {
+      if(f.k <= k1 + 1) pl.fetch(ring + (q & 3) * sw, b, f.kz * nxy);
+      fetch_commit();
+      f.next(o);
+    }
+    B[3] = pl.load(b, zplane(o, k0 - 2, zn) * nxy);
+    pl.settle(B[3], sb, zn);
+    W.at(o, pl.cls, k0 - 2);
+    A[3] = times(W.w, B[3]);
+    B[0] = pl.load(b, zplane(o, k0 - 1, zn) * nxy);
+    pl.settle(B[0], sb, zn);
+    W.at(o, pl.cls, k0 - 1);
+    A[0] = times(W.w, B[0]);
+    X[2] = X[3] = A[0];
+    ring4(k0 - 1, k1, [&](auto jc, int s) {
+      constexpr int J = jc, M = (J + 3) & 3, N = (J + 1) & 3, F = (J + 2) & 3;
+      fetch_wait<2>();
+      B[N] = pl.take(ring + N * sw);
+      if(f.k <= k1 + 1) pl.fetch(ring + J * sw, b, f.kz * nxy);
+      __syncwarp();
+      fetch_commit();
+      f.next(o);
+      T* pa = me + (J & 1) * 2 * pw;
+      publish(pa, A[J]);
+      publish(pa + pw, X[M]);
+      pl.settle(B[N], sb, SGN && zneg(o, s + 1));
+      W.at(o, pl.cls, s + 1);
+      A[N] = times(W.w, B[N]);
+      __syncthreads();
+      W.at(o, pl.cls, s);
+      neighbour_sums(pa, A[J], xs, ys);
+      const Patch<T> xc = relax(A[J], W.w, residual<T, false>(co, B[J], A[J], xs, ys, A[M], A[N]));
+      if(s >= k0 && s < k1) pl.store(x, s * nxy, xc);
+      if(s > k0) {
+        neighbour_sums(pa + pw, X[M], xs, ys);
+        const Patch<T> res = residual<T, false>(co, B[M], X[M], xs, ys, X[F], xc);
+        const bool first = rz == 1 || ((s - 1) & 1) == 0;
+#pragma unroll
+        for(int r = 0; r < 2; ++r)
+#pragma unroll
+          for(int c = 0; c < kW<T>; ++c) racc.v[r][c] = first ? res.v[r][c] : racc.v[r][c] + res.v[r][c];
+        if(rz == 1 || !first) restrict_out((s - 1) >> (rz - 1));
+      }
+      X[J] = xc;
+      __syncwarp();
+    });
+  }
+}
+
+// Ascent of one V-cycle level (linsolve/poisson_solver.cpp:625-633): the
+// coarse correction added and both post-sweeps, in one pass:  y = x + P e,
+// y' = y + omega (b - A y) / D, out = y' + omega (b - A y') / D.  On the finest
+// level (FINE) it also forms mean(out) and r.z for the CG; on the others no
+// mean is needed (see k_descend).  sx, sy, sz: log2 of the coarsening ratios.
+//
+// Bound: reads x, b and e, writes out (3.125 vectors).
+template <typename T, bool SGN, bool CD, bool FLAT, bool FINE, bool PAIRS>
+__global__ void __launch_bounds__(kMaxThreads, 1)
+    k_ascend(OpInfo o, CLay lc, Tile t, const T* __restrict__ b, const double* sb_ptr, const T* __restrict__ x,
+             const T* __restrict__ e, T* __restrict__ out, int sx, int sy, int sz, LevelScalars* ls,
+             SolveScalars* sc, RedBuf rb) {
+  extern __shared__ __align__(16) unsigned char march_sm[];
+  T* ring = reinterpret_cast<T*>(march_sm);
+  const int sw = slot_words<T>(t), pw = plane_words<T>(t);
+  T* planes = ring + kRing * 2 * sw;
+  T* tab = planes + 4 * pw;
+  if constexpr(!CD) {
+    for(int q = threadIdx.x; q < 64; q += blockDim.x) tab[q] = T(2.0 / 3.0 * o.invd[q]);
+    __syncthreads();
+  }
+  Weights<T, CD> W(tab, T(2.0 / 3.0 * o.invd[0]));
+  const Place<T, SGN> pl(o, t, 2);
+  const Coef<T> co(o, FLAT);
+  const int nxy = o.L.nxy;
+  const int k0 = blockIdx.y * t.chunk, k1 = min(k0 + t.chunk, o.L.nz);
+  T* me = planes + (pl.row0 + 1) * kRow<T> + pl.p;
+  pdl_enter();
+  const T sb = SGN ? T(0) : T(*sb_ptr);
+  bool zn;
+  // the coarse correction of the patch: W / 2 parents where both x and y
+  // coarsen (PAIRS), else one per cell; loaded two planes ahead, always from
+  // valid cells (under a condition the merge would wait for the load)
+  constexpr int NR = PAIRS ? 1 : 2, NE = PAIRS ? kW<T> / 2 : kW<T>;
+  struct Parents {
+    T v[NR][NE];
+  };
+  auto lde = [&](int kz) {
+    Parents q;
+    const T* ep = e + lc.nxy * (kz >> sz);
+#pragma unroll
+    for(int r = 0; r < NR; ++r)
+#pragma unroll
+      for(int c = 0; c < NE; ++c)
+        q.v[r][c] = PAIRS ? ep[lc.nx * (pl.yj[0] >> 1) + (pl.xi[2 * c] >> 1)]
+                          : ep[lc.nx * (pl.yj[r] >> sy) + (pl.xi[c] >> sx)];
+    return q;
+  };
+  // y = x + P e with the signs of Dirichlet images
+  auto join = [&](Patch<T>& q, const Parents& ev, int k) {
+#pragma unroll
+    for(int r = 0; r < 2; ++r)
+#pragma unroll
+      for(int c = 0; c < kW<T>; ++c) q.v[r][c] += PAIRS ? ev.v[0][c / 2] : ev.v[r % NR][c % NE];
+    if constexpr(SGN) pl.settle(q, T(0), !FLAT && zneg(o, k));
+  };
+  double acc[2] = {0.0, 0.0};
+  auto finish = [&](int k, const Patch<T>& v, const Patch<T>& bq) {
+    pl.store(out, k * nxy, v);
+    if constexpr(FINE) {
+#pragma unroll
+      for(int r = 0; r < 2; ++r)
+#pragma unroll
+        for(int c = 0; c < kW<T>; ++c)
+          if(pl.interior(r, c)) {
+            acc[0] += double(v.v[r][c]);
+            acc[1] += double(bq.v[r][c]) * double(v.v[r][c]);
+          }
+    }
+  };
+  Patch<T> xs, ys;
+  if constexpr(FLAT) {
+    Patch<T> bq = pl.load(b, 0), y = pl.load(x, 0);
+    pl.settle(bq, sb, false);
+    join(y, lde(0), 0);
+    W.at(o, pl.cls, 0);
+    publish(me, y);
+    __syncthreads();
+    neighbour_sums(me, y, xs, ys);
+    const Patch<T> y1 = relax(y, W.w, residual<T, true>(co, bq, y, xs, ys, y, y));
+    publish(me + pw, y1);
+    __syncthreads();
+    neighbour_sums(me + pw, y1, xs, ys);
+    finish(0, relax(y1, W.w, residual<T, true>(co, bq, y1, xs, ys, y1, y1)), bq);
+  } else {
+    // step s: y'(s) from y(s - 1 .. s + 1), then out(s - 1)
+    Patch<T> Y[4], B[4], V[4];
+    T* bring = ring + kRing * sw;
+    // b is fetched a plane behind x: both are three steps ahead of their use
+    int zb = zplane(o, k0 - 1, zn) * nxy;
+    Walk f(o, k0);
+    Parents E[4];
+    for(int q = 1; q <= 3; ++q) {
+      const int zx = f.kz * nxy;
+      if(f.k <= k1 + 1) pl.fetch(ring + (q & 3) * sw, x, zx);
+      if(f.k <= k1 + 1) pl.fetch(bring + (q - 1) * sw, b, zb);
+      fetch_commit();
+      if(q == 1) E[1] = lde(f.kz);
+      if(q == 2) E[2] = lde(f.kz);
+      zb = zx;
+      f.next(o);
+    }
+    int ke = zplane(o, k0 + 2, zn);
+    Y[3] = pl.load(x, zplane(o, k0 - 2, zn) * nxy);
+    join(Y[3], lde(zplane(o, k0 - 2, zn)), k0 - 2);
+    Y[0] = pl.load(x, zplane(o, k0 - 1, zn) * nxy);
+    join(Y[0], lde(zplane(o, k0 - 1, zn)), k0 - 1);
+    V[2] = V[3] = Y[0];
+    B[3] = Y[0];
+    ring4(k0 - 1, k1, [&](auto jc, int s) {
+      constexpr int J = jc, M = (J + 3) & 3, N = (J + 1) & 3, F = (J + 2) & 3;
+      fetch_wait<2>();
+      Y[N] = pl.take(ring + N * sw);
+      B[J] = pl.take(bring + J * sw);
+      const int zx = f.kz * nxy;
+      if(f.k <= k1 + 1) pl.fetch(ring + J * sw, x, zx);       // plane s + 4
+      if(f.k <= k1 + 2) pl.fetch(bring + M * sw, b, zb);      // plane s + 3
+      __syncwarp();
+      fetch_commit();
+      join(Y[N], E[N], s + 1);
+      E[M] = lde(ke);
+      zb = zx;
+      ke = max(0, min(f.kz, o.L.nz - 1));
+      f.next(o);
+      T* pa = me + (J & 1) * 2 * pw;
+      publish(pa, Y[J]);
+      publish(pa + pw, V[M]);
+      pl.settle(B[J], sb, SGN && zneg(o, s));
+      __syncthreads();
+      W.at(o, pl.cls, s);
+      neighbour_sums(pa, Y[J], xs, ys);
+      const Patch<T> vc = relax(Y[J], W.w, residual<T, false>(co, B[J], Y[J], xs, ys, Y[M], Y[N]));
+      if(s > k0) {
+        W.at(o, pl.cls, s - 1);
+        neighbour_sums(pa + pw, V[M], xs, ys);
+        finish(s - 1, relax(V[M], W.w, residual<T, false>(co, B[M], V[M], xs, ys, V[F], vc)), B[M]);
+      }
+      V[J] = vc;
+      __syncwarp();
+    });
+  }
+  if constexpr(FINE) {
+    const bool mx[2] = {false, false};
+    reduce_finish<2>(acc, mx, rb, [=](const Sums<2>& s) {
+      const double mean = sc->zero_mean ? s.v[0] / sc->n : 0.0;
+      ls->sx = mean;
+      ls->sum_x = s.v[0];
+      // r.z with z = out - mean (linsolve/poisson_solver.cpp:749, :791)
+      const double rz_new = s.v[1] - mean * (sc->sum_r - sc->n * sc->sr);
+      if(!sc->first) sc->beta = rz_new / sc->rz;
+      sc->rz = rz_new;
+    });
+  }
+}
+
+}  // namespace march
+}  // namespace ofb

@@ -22,6 +22,7 @@
 #include "kernels.hpp"
 #include "vstencil.cuh"
 #include "tma.cuh"
+#include "march.cuh"
 
 #include <cmath>
 #include <cstdint>
@@ -38,18 +39,6 @@ namespace {
 constexpr double kSmallNumber = 1.0e-30;
 constexpr double kOmega = 2.0 / 3.0;
 constexpr int kMaxCoarse = 1024;
-
-struct OpInfo {
-  CLay L;
-  double inv2[3];  // 1 / h^2
-  int periodic[3];
-  int dir_lo[3], dir_hi[3];  // homogeneous Dirichlet (else Neumann) at each end
-  const double* invd;        // 64-entry inverse-diagonal table
-};
-
-__device__ __forceinline__ int axis_class(int c, int n) {
-  return n == 1 ? 3 : (c == 0 ? 1 : (c == n - 1 ? 2 : 0));
-}
 
 __device__ __forceinline__ double inv_diag(const OpInfo& o, int i, int j, int k) {
   const int t = axis_class(i, o.L.nx) + 4 * axis_class(j, o.L.ny) + 16 * axis_class(k, o.L.nz);
@@ -2716,6 +2705,8 @@ struct Level {
   void* b = nullptr;   // rhs (levels >= 1)
   double* invd = nullptr;
   int rx = 1, ry = 1, rz = 1;  // refinement ratio to the next coarser level
+  march::Tile tile{};          // of k_descend and k_ascend
+  dim3 tgrid;
   // plane-pipeline (TMA) maps: a (main rows, one halo row) and the rhs
   bool tma = false;
   CUtensorMap tm_am, tm_ah, tm_bm, tm_bh;
@@ -3066,6 +3057,111 @@ void setup_tma(PoissonPlan* P, size_t tsz) {
 
 }
 
+// The instantiation for the plan's boundary conditions: sign images where a
+// face is Dirichlet, one diagonal value where every face is periodic.
+template <typename T>
+auto descend_kernel(const PoissonPlan* P, bool flat) {
+  using namespace march;
+  if(!P->zero_mean) return flat ? k_descend<T, true, false, true> : k_descend<T, true, false, false>;
+  if(P->all_periodic) return flat ? k_descend<T, false, true, true> : k_descend<T, false, true, false>;
+  return flat ? k_descend<T, false, false, true> : k_descend<T, false, false, false>;
+}
+
+template <typename T, bool FINE, bool PAIRS>
+auto ascend_kernel_of(const PoissonPlan* P, bool flat) {
+  using namespace march;
+  if(!P->zero_mean)
+    return flat ? k_ascend<T, true, false, true, FINE, PAIRS> : k_ascend<T, true, false, false, FINE, PAIRS>;
+  if(P->all_periodic)
+    return flat ? k_ascend<T, false, true, true, FINE, PAIRS> : k_ascend<T, false, true, false, FINE, PAIRS>;
+  return flat ? k_ascend<T, false, false, true, FINE, PAIRS> : k_ascend<T, false, false, false, FINE, PAIRS>;
+}
+
+template <typename T>
+auto ascend_kernel(const PoissonPlan* P, bool flat, bool fine, bool pairs) {
+  if(fine) return pairs ? ascend_kernel_of<T, true, true>(P, flat) : ascend_kernel_of<T, true, false>(P, flat);
+  return pairs ? ascend_kernel_of<T, false, true>(P, flat) : ascend_kernel_of<T, false, false>(P, flat);
+}
+
+constexpr int kMarchSmem = 224 * 1024;
+
+// Lets every instantiation use the largest tile's shared memory.
+template <typename T>
+void march_attributes(const PoissonPlan* P) {
+  auto attr = [](auto kern) {
+    OFB_CHECK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kMarchSmem));
+  };
+  for(const bool flat : {false, true}) {
+    attr(descend_kernel<T>(P, flat));
+    for(const bool fine : {false, true})
+      for(const bool pairs : {false, true}) attr(ascend_kernel<T>(P, flat, fine, pairs));
+  }
+}
+
+// Tile and grid of a march kernel on one level: the split with the least
+// modelled time.  A block of `threads` marches chunk + 3 planes (its halo
+// planes and the pipeline's fill included); an SM takes about kPlaneLatency
+// cycles for a plane when few threads are resident (barrier, shared-memory and
+// arithmetic latency) and kThreadCycles per resident thread when many are
+// (measured: 510 threads, 1000 cycles per plane at 256^3), and the blocks run
+// in waves of what the SMs hold at once.  Small levels so get many thin
+// chunks, large ones tiles near 64 x 26 with long chunks.
+constexpr double kPlaneLatency = 500.0, kThreadCycles = 2.0;
+
+template <typename T>
+void plan_tile(const CLay& L, int rz, int streams, int sms, march::Tile& best, dim3& grid) {
+  constexpr int W = march::kW<T>, halo_rows = 2;
+  auto even = [](int v) { return (v + 1) / 2 * 2; };
+  const bool flat = L.nz == 1;
+  double best_cost = 0.0;
+  bool found = false;
+  int last_ix = 0;
+  for(int ntx = 1; ntx <= (L.nx + 7) / 8 || ntx == 1; ++ntx) {
+    march::Tile t{};
+    t.ix = ((L.nx + ntx - 1) / ntx + W - 1) / W * W;
+    if(t.ix == last_ix) continue;
+    last_ix = t.ix;
+    t.px = t.ix / W + 2;
+    if(t.px > march::kPX) continue;
+    t.tx = (L.nx + t.ix - 1) / t.ix;
+    const int max_rows = march::kMaxThreads / t.px * 2 - 2 * halo_rows;
+    if(max_rows < 2) continue;
+    int last_iy = 0;
+    const int nty0 = (L.ny + max_rows - 1) / max_rows;
+    for(int nty = nty0; nty <= std::max(nty0, (L.ny + 3) / 4) && nty < nty0 + 64; ++nty) {
+      t.iy = std::min(even((L.ny + nty - 1) / nty), max_rows);
+      if(t.iy == last_iy) continue;
+      last_iy = t.iy;
+      t.ey = t.iy + 2 * halo_rows;
+      const int threads = t.px * t.ey / 2;
+      const size_t smem = march::smem_bytes<T>(t, streams);
+      if(smem > kMarchSmem) continue;
+      const int resident = std::min<int>({march::kMaxThreads / ((threads + 31) / 32 * 32),
+                                          static_cast<int>(228 * 1024 / (smem + 2048)), 16});
+      if(resident < 1) continue;
+      const long long tiles = static_cast<long long>(t.tx) * ((L.ny + t.iy - 1) / t.iy);
+      if(tiles > kMaxBlocks) continue;
+      const int units = (L.nz + rz - 1) / rz;
+      for(int nch = 1; nch <= units && tiles * nch <= kMaxBlocks; nch < 48 ? ++nch : nch *= 2) {
+        t.chunk = (units + nch - 1) / nch * rz;
+        const long long blocks = tiles * ((L.nz + t.chunk - 1) / t.chunk);
+        const long long waves = (blocks + static_cast<long long>(sms) * resident - 1) / (static_cast<long long>(sms) * resident);
+        const long long per_sm = std::min<long long>(resident, (blocks + sms - 1) / sms);
+        const double plane = std::max(kPlaneLatency, kThreadCycles * static_cast<double>(per_sm) * threads);
+        const double cost = static_cast<double>(waves) * (flat ? 3 : t.chunk + 3) * plane;
+        if(!found || cost < best_cost) {
+          found = true;
+          best_cost = cost;
+          best = t;
+          grid = dim3(static_cast<unsigned>(tiles), static_cast<unsigned>((L.nz + t.chunk - 1) / t.chunk), 1);
+        }
+        if(flat) break;
+      }
+    }
+  }
+  if(!found) throw std::invalid_argument("grid too large for the pressure solve's tiles");
+}
+
 }  // namespace
 
 PoissonPlan* poisson_plan_create(const Grid& g, const PBC& pbc_in, int precision) {
@@ -3212,7 +3308,12 @@ PoissonPlan* poisson_plan_create(const Grid& g, const PBC& pbc_in, int precision
   P->all_periodic = true;
   for(int f = 0; f < 6; ++f)
     if(P->pbc.type[f] != kPPeriodic) P->all_periodic = false;
+  for(int l = 0; l < P->tail_first; ++l)
+    (precision == 1 ? plan_tile<float> : plan_tile<double>)(P->levels[l].L, P->levels[l].rz, 2, P->sms,
+                                                            P->levels[l].tile, P->levels[l].tgrid);
   setup_tma(P, tsz);
+  if(precision == 1) march_attributes<float>(P);
+  else march_attributes<double>(P);
   const char* no_graph = std::getenv("ORCHARD_B200_NO_GRAPH");
   P->use_graph = !(no_graph != nullptr && no_graph[0] == '1');
   return P;
@@ -3334,11 +3435,8 @@ TGrid tgrid(const PoissonPlan* P, const CLay& L, size_t elem, const void* kernel
 template <typename T, typename V>
 void v_cycle(PoissonPlan* P, int l, const V* r0, SolveScalars* sc, RedBuf rb, cudaStream_t s) {
   Level& lv = P->levels[l];
-  const int nl = static_cast<int>(P->levels.size());
-  const int zm = P->zero_mean;
   LevelScalars* ls = P->ls + l;
-  const double* sb_ptr = l == 0 ? &sc->sr : &ls->sb;
-  SolveScalars* rz_sc = l == 0 ? sc : nullptr;
+  const double* sb_ptr = l == 0 ? &sc->sr : &ls->sb;  // ls->sb stays 0 (k_descend)
   T* a = static_cast<T*>(lv.a);
   T* x = static_cast<T*>(lv.x);
   if(l == P->tail_first) {
@@ -3354,111 +3452,31 @@ void v_cycle(PoissonPlan* P, int l, const V* r0, SolveScalars* sc, RedBuf rb, cu
     OFB_LAUNCH_CHECK("k_dense_apply");
     return;
   }
-  const Launch3 ln = launch3(lv.L.nx, lv.L.ny, lv.L.nz);
   Level& cv = P->levels[l + 1];
-  const Launch3 lc = launch3(cv.L.nx, cv.L.ny, cv.L.nz);
-  LevelScalars* lsc = P->ls + (l + 1);
-  auto smooth_chain = [&](auto* bptr) {
-    using B = std::remove_cv_t<std::remove_pointer_t<decltype(bptr)>>;
-    const bool fine = l == 0;
-    const bool vec = vfits<T>(lv.L) && vec_enabled();
-    const bool vsm = vec && vec_enabled("smooth");
-    const bool vpr = vec && vec_enabled("prolong");
-    const bool vre = vec && vec_enabled("restrict");
-    const vst::RowLaunch lr = vst::row_launch(lv.L.nx, lv.L.ny, lv.L.nz, vst::Width<T>::W, 16);
-    if(lv.tma && vec_enabled("tma")) {
-      ProfScope ps(fine ? kKSmoothFirstFine : kKCoarseLevels, s);
-      const size_t sm = tround(static_cast<size_t>(1024 / lv.L.nx + 2) * lv.L.nx * sizeof(B)) * kTSlots;
-      const auto kern = P->all_periodic ? k_tsmooth_pre<T, B, 4, true> : k_tsmooth_pre<T, B, 4, false>;
-      const TGrid tg = tgrid(P, lv.L, sizeof(T), reinterpret_cast<const void*>(kern), sm, 288);
-      launch_pdl(kern, tg.grid, 288, sm, s, lv.op, lv.tm_bm, lv.tm_bh, sb_ptr, x, ls, zm, rb, P->fault);
-    } else if(vsm && vec_enabled("pre")) {
-      ProfScope ps(fine ? kKSmoothFirstFine : kKCoarseLevels, s);
-      launch_pdl(k_vsmooth_pre<T, B>, lr.grid, lr.block, 0, s, lv.op, bptr, sb_ptr, x, ls, zm, lr.kchunk, rb);
-    } else {
-      {
-        ProfScope ps(fine ? kKSmoothFirstFine : kKCoarseLevels, s);
-        launch_pdl(k_smooth_first<T, B>, ln.grid, ln.block, 0, s, lv.op, bptr, sb_ptr, a, ls, zm, ln.kchunk,
-                   rb);
-      }
-      ProfScope ps(fine ? kKSmoothFine : kKCoarseLevels, s);
-      if(vsm)
-        launch_pdl(k_vsmooth<T, B>, lr.grid, lr.block, 0, s, lv.op, bptr, sb_ptr, a, &ls->sa, x, ls, zm,
-                   nullptr, lr.kchunk, rb);
-      else
-        launch_pdl(k_smooth<T, B>, ln.grid, ln.block, 0, s, lv.op, bptr, sb_ptr, a, &ls->sa, x, ls, 1, zm,
-                   nullptr, ln.kchunk, rb);
-    }
-    if(lv.tma_prolong && vec_enabled("tma")) {
-      ProfScope ps(fine ? kKRestrictFine : kKCoarseLevels, s);
-      const int ty = 1024 / lv.L.nx;
-      const size_t sm = tslot_bytes<T, B>(lv.L.nx) * kTSlots + static_cast<size_t>(ty) * (lv.L.nx / 2) * sizeof(T);
-      const auto kern = P->all_periodic ? k_trestrict<T, B, kTSlots, true> : k_trestrict<T, B, kTSlots, false>;
-      const int per_sm = std::min(tper_sm(sizeof(T)), resident_blocks(reinterpret_cast<const void*>(kern), sm));
-      const long long g = tgrid_blocks(P, lv.L.ny / ty, lv.L.nz / 2, per_sm, 2, std::is_same_v<T, double>);
-      launch_pdl(kern, static_cast<int>(g), 256, sm, s, lv.op, cv.op, lv.tm_xm, lv.tm_xh, lv.tm_bm, sb_ptr,
-                 &ls->sx, static_cast<T*>(cv.b), lsc, zm, rb, P->fault);
-    } else {
-      ProfScope ps(fine ? kKRestrictFine : kKCoarseLevels, s);
-      if(vre && lv.rx == 2 && lv.ry == 2 && lv.rz == 2) {
-        const vst::RowLaunch lrc =
-            vst::row_launch(lv.L.nx, cv.L.ny, cv.L.nz, vst::Width<T>::W, 8);
-        launch_pdl(k_vrestrict<T, B>, lrc.grid, lrc.block, 0, s, lv.op, cv.op, bptr, sb_ptr, x, &ls->sx,
-                   static_cast<T*>(cv.b), lsc, zm, lrc.kchunk, rb);
-      } else
-        launch_restrict<T, B>(lv, cv, bptr, sb_ptr, x, &ls->sx, static_cast<T*>(cv.b), lsc, zm,
-                              lc, rb, s);
-    }
-    OFB_LAUNCH_CHECK("v_cycle descent");
-    if(l == 0) {
-      // the coarse levels are ~16 short dependent launches: time them as one
-      // chain (one event pair per V-cycle, the coarse solve at the bottom
-      // included) so that the measurement does not add an event pair's
-      // overhead to each of them
-      ProfSpan span(kKCoarseLevels, s);
-      v_cycle<T, V>(P, l + 1, r0, sc, rb, s);
-    } else {
-      v_cycle<T, V>(P, l + 1, r0, sc, rb, s);
-    }
-    if(lv.tma_prolong && vec_enabled("tma")) {
-      ProfScope ps(fine ? kKProlongFine : kKCoarseLevels, s);
-      const size_t sm = tprolong_bytes<T, B>(lv.L.nx) * 4;
-      const auto kern = P->all_periodic ? k_tprolong<T, B, 4, 4, true> : k_tprolong<T, B, 4, 4, false>;
-      const TGrid tg = tgrid(P, lv.L, sizeof(T), reinterpret_cast<const void*>(kern), sm);
-      launch_pdl(kern, tg.grid, 256, sm, s, lv.op, lv.tm_xm, lv.tm_xh, lv.tm_bm, lv.tm_em, lv.tm_eh, sb_ptr,
-                 &ls->sx, &lsc->sx, a, ls, zm, rb, P->fault);
-    } else {
-      ProfScope ps(fine ? kKProlongFine : kKCoarseLevels, s);
-      if(vpr)
-        launch_pdl(k_vprolong_smooth<T, B>, lr.grid, lr.block, 0, s, lv.op, cv.L, bptr, sb_ptr, x, &ls->sx,
-                   static_cast<const T*>(cv.x), &lsc->sx, a, ls, lv.rx == 2 ? 1 : 0, lv.ry == 2 ? 1 : 0,
-                   lv.rz == 2 ? 1 : 0, zm, lr.kchunk, rb);
-      else
-        launch_pdl(k_prolong_smooth<T, B>, ln.grid, ln.block, 0, s, lv.op, cv.L, bptr, sb_ptr, x, &ls->sx,
-                   static_cast<const T*>(cv.x), &lsc->sx, a, ls, lv.rx == 2 ? 1 : 0, lv.ry == 2 ? 1 : 0,
-                   lv.rz == 2 ? 1 : 0, zm, ln.kchunk, rb);
-    }
-    if(lv.tma && vec_enabled("tma")) {
-      ProfScope ps(fine ? kKSmoothFine : kKCoarseLevels, s);
-      const size_t sm = tslot_bytes<T, B>(lv.L.nx) * kTSlots;
-      const auto kern = P->all_periodic ? k_tsmooth<T, B, 4, true> : k_tsmooth<T, B, 4, false>;
-      const TGrid tg =
-          tgrid(P, lv.L, sizeof(T), reinterpret_cast<const void*>(kern), sm, 256, std::is_same_v<T, double>);
-      launch_pdl(kern, tg.grid, 256, sm, s, lv.op, lv.tm_am, lv.tm_ah, lv.tm_bm, sb_ptr, &ls->sa, x, ls, zm,
-                 rz_sc, rb, P->fault);
-    } else {
-      ProfScope ps(fine ? kKSmoothFine : kKCoarseLevels, s);
-      if(vsm)
-        launch_pdl(k_vsmooth<T, B>, lr.grid, lr.block, 0, s, lv.op, bptr, sb_ptr, a, &ls->sa, x, ls, zm,
-                   rz_sc, lr.kchunk, rb);
-      else
-        launch_pdl(k_smooth<T, B>, ln.grid, ln.block, 0, s, lv.op, bptr, sb_ptr, a, &ls->sa, x, ls, 1, zm,
-                   rz_sc, ln.kchunk, rb);
-    }
-    OFB_LAUNCH_CHECK("v_cycle ascent");
-  };
-  if(l == 0) smooth_chain(r0);
-  else smooth_chain(static_cast<const T*>(lv.b));
+  const T* b = l == 0 ? static_cast<const T*>(r0) : static_cast<const T*>(lv.b);
+  const size_t smem1 = march::smem_bytes<T>(lv.tile, 1), smem2 = march::smem_bytes<T>(lv.tile, 2);
+  const int threads = lv.tile.px * lv.tile.ey / 2;
+  {
+    ProfScope ps(l == 0 ? kKSmoothFirstFine : kKCoarseLevels, s);
+    launch_pdl(descend_kernel<T>(P, lv.L.nz == 1), lv.tgrid, threads, smem1, s, lv.op, cv.L, lv.tile, b, sb_ptr,
+               a, static_cast<T*>(cv.b), lv.rx, lv.ry, lv.rz);
+  }
+  if(l == 0) {
+    // the coarse levels are short dependent launches: time them as one chain
+    // (one event pair per V-cycle) so that the measurement does not add an
+    // event pair's overhead to each of them
+    ProfSpan span(kKCoarseLevels, s);
+    v_cycle<T, V>(P, l + 1, r0, sc, rb, s);
+  } else {
+    v_cycle<T, V>(P, l + 1, r0, sc, rb, s);
+  }
+  {
+    ProfScope ps(l == 0 ? kKSmoothFine : kKCoarseLevels, s);
+    launch_pdl(ascend_kernel<T>(P, lv.L.nz == 1, l == 0, lv.rx == 2 && lv.ry == 2), lv.tgrid, threads, smem2, s, lv.op, cv.L, lv.tile, b,
+               sb_ptr, static_cast<const T*>(a), static_cast<const T*>(cv.x), x, lv.rx - 1, lv.ry - 1,
+               lv.rz - 1, ls, sc, rb);
+  }
+  OFB_LAUNCH_CHECK("v_cycle");
 }
 
 // The vectors of one CG loop: FP64 for the reference's solve, FP32 for the
