@@ -82,22 +82,14 @@ def bytes_per_launch(n, precision):
         "adi_sweep": 2 * d * N,
         "divergence_rhs": 5 * d * N,
         "pcg_initial_residual": 3 * d * N,
-        "pcg_apply_ap": 2 * s * N,
-        "pcg_update_xr": 6 * s * N,
-        "pcg_update_p": 3 * s * N,
-        "vcycle_smooth_first_fine": 2 * s * N,        # read b, write x
-        "vcycle_smooth_fine": 3 * s * N,              # read a, b; write x
-        "vcycle_restrict_fine": (2 + 1 / 8) * s * N,  # read b, x; write coarse b
-        "vcycle_prolong_smooth_fine": (3 + 1 / 8) * s * N,  # read x, b, coarse x; write a
+        "pcg_apply_ap": 3 * s * N,                    # direction: read z, p; write p
+        "pcg_update_xr": 5 * s * N,                   # advance: read p, x, r; write x, r
+        "vcycle_smooth_first_fine": (2 + 1 / 8) * s * N,  # descend: read b; write x, coarse b
+        "vcycle_smooth_fine": (3 + 1 / 8) * s * N,    # ascend: read x, b, coarse x; write out
         "correct_velocity": (1 + 3 + 3) * d * N / 3 + d * N,  # per component launch
         "cell_pass": 7 * d * N,
     }
     if precision == "mixed":
-        # the FP32 inner CG fuses the p update, A p and the deferred x update
-        # into one plane-pipelined launch (read z, p_old, x; write p, A p, x)
-        # and updates r alone (read r, A p; write r)
-        out["pcg_apply_ap"] = 6 * s * N
-        out["pcg_update_xr"] = 3 * s * N
         out["defect_correction"] = 20 * N
     return out
 

@@ -13,7 +13,7 @@ namespace ofb {
 // step.
 struct SolveScalars {
   // pressure solve (linsolve/poisson_solver.cpp:678-809)
-  double sb, sx, sr, sp, sap, sz;  // pending mean shifts of b, x, r, p, Ap, z
+  double sb, sx, sr;               // pending mean shifts of b, x, r
   double rz, pap, alpha, beta;
   double sum_r;                    // sum of the stored residual
   double r0, rnorm, rel;

@@ -312,8 +312,8 @@ __device__ __forceinline__ void fetch_wait() {
 }
 
 // Words of one published plane, its guard rows included, and of one ring
-// slot; the shared memory of a kernel that publishes two fields (two planes
-// each) and streams `streams` vectors: rings, planes, diagonal table.
+// slot; the shared memory of a kernel that streams `streams` vectors and
+// publishes `fields` fields (two planes each): rings, planes, diagonal table.
 template <typename T>
 __host__ __device__ inline int plane_words(const Tile& t) {
   return (t.ey + 2) * kRow<T>;
@@ -323,9 +323,9 @@ __host__ __device__ inline int slot_words(const Tile& t) {
   return kW<T> * t.px * t.ey;
 }
 template <typename T>
-inline size_t smem_bytes(const Tile& t, int streams) {
-  return (static_cast<size_t>(kRing) * streams * slot_words<T>(t) + static_cast<size_t>(4) * plane_words<T>(t) + 64) *
-         sizeof(T);
+inline size_t smem_bytes(const Tile& t, int streams, int fields) {
+  return (static_cast<size_t>(kRing) * streams * slot_words<T>(t) +
+          static_cast<size_t>(2) * fields * plane_words<T>(t) + 64) * sizeof(T);
 }
 
 // The image plane of k, -2 <= k <= nz + 1 with nz >= 2, and whether it is a
@@ -707,6 +707,242 @@ __global__ void __launch_bounds__(kMaxThreads, 1)
       sc->rz = rz_new;
     });
   }
+}
+
+
+constexpr double kBreakdown = 1.0e-30;  // linsolve/poisson_solver.cpp:757
+
+// The buffers of the search direction: an iteration reads one and writes the
+// other (a tile's halo still needs the old values when its neighbour writes).
+template <typename T>
+struct Direction {
+  T* p[2];
+};
+
+// New search direction and its products (linsolve/poisson_solver.cpp:750-761):
+// p = (z - sz) + beta p (first iteration: z - sz) and p.Ap; A p itself is not
+// stored -- k_advance forms it again from p, which costs its seven operations
+// instead of a vector written and read back.  The means of p and A p that the
+// reference removes are zero up to rounding (z - sz has none, A annihilates
+// constants) and are left in; the residual's, which they would move, is
+// removed every iteration.  Bound: reads z and p, writes p (3 vectors); at
+// 256^3 76 us in FP64, where the separate p update and A p took 71 + 66.
+template <typename T, bool SGN, bool FLAT>
+__global__ void __launch_bounds__(kMaxThreads, 1)
+    k_direction(OpInfo o, Tile t, const T* __restrict__ z, const LevelScalars* ls0, Direction<T> d,
+                SolveScalars* sc, RedBuf rb) {
+  extern __shared__ __align__(16) unsigned char march_sm[];
+  T* ring = reinterpret_cast<T*>(march_sm);
+  const int sw = slot_words<T>(t), pw = plane_words<T>(t);
+  T* pring = ring + kRing * sw;
+  const Place<T, SGN> pl(o, t, 1);
+  const Coef<T> co(o, FLAT);
+  const int nxy = o.L.nxy;
+  const int k0 = blockIdx.y * t.chunk, k1 = min(k0 + t.chunk, o.L.nz);
+  T* me = ring + 2 * kRing * sw + (pl.row0 + 1) * kRow<T> + pl.p;
+  pdl_enter();
+  const bool first = sc->first != 0;
+  const int turn = sc->body_runs & 1;
+  const T* __restrict__ po = d.p[turn ^ 1];
+  T* __restrict__ pn = d.p[turn];
+  const T sz = SGN ? T(0) : T(ls0->sx);
+  const T beta = first ? T(0) : T(sc->beta);
+  double acc[1] = {0.0};
+  auto combine = [&](Patch<T>& q, const Patch<T>& old, bool zn) {
+#pragma unroll
+    for(int r = 0; r < 2; ++r)
+#pragma unroll
+      for(int c = 0; c < kW<T>; ++c) {
+        const T zv = q.v[r][c] - sz;
+        q.v[r][c] = first ? zv : zv + beta * old.v[r][c];
+      }
+    if constexpr(SGN) pl.settle(q, T(0), zn);
+  };
+  auto point = [&](int k, const Patch<T>& v, const Patch<T>& minus_av) {
+    pl.store(pn, k * nxy, v);
+#pragma unroll
+    for(int r = 0; r < 2; ++r)
+#pragma unroll
+      for(int c = 0; c < kW<T>; ++c)
+        if(pl.interior(r, c)) acc[0] -= double(v.v[r][c]) * double(minus_av.v[r][c]);
+  };
+  const Patch<T> none = {};
+  Patch<T> xs, ys;
+  bool zn;
+  if constexpr(FLAT) {
+    Patch<T> q = pl.load(z, 0);
+    combine(q, first ? none : pl.load(po, 0), false);
+    publish(me, q);
+    __syncthreads();
+    neighbour_sums(me, q, xs, ys);
+    point(0, q, residual<T, true>(co, none, q, xs, ys, q, q));
+  } else {
+    // step s: p(s + 1) is combined, A p(s) formed
+    Patch<T> P[4];
+    Walk f(o, k0 + 1);
+    for(int q = 1; q <= 3; ++q) {
+      if(f.k <= k1) {
+        pl.fetch(ring + (q & 3) * sw, z, f.kz * nxy);
+        pl.fetch(pring + (q & 3) * sw, po, f.kz * nxy);
+      }
+      fetch_commit();
+      f.next(o);
+    }
+    P[3] = pl.load(z, zplane(o, k0 - 1, zn) * nxy);
+    combine(P[3], pl.load(po, zplane(o, k0 - 1, zn) * nxy), zn);
+    P[0] = pl.load(z, k0 * nxy);
+    combine(P[0], pl.load(po, k0 * nxy), false);
+    ring4(k0, k1 - 1, [&](auto jc, int s) {
+      constexpr int J = jc, M = (J + 3) & 3, N = (J + 1) & 3;
+      fetch_wait<2>();
+      P[N] = pl.take(ring + N * sw);
+      const Patch<T> old = pl.take(pring + N * sw);
+      if(f.k <= k1) {  // plane s + 4
+        pl.fetch(ring + J * sw, z, f.kz * nxy);
+        pl.fetch(pring + J * sw, po, f.kz * nxy);
+      }
+      __syncwarp();
+      fetch_commit();
+      f.next(o);
+      T* pa = me + (J & 1) * pw;
+      publish(pa, P[J]);
+      combine(P[N], old, SGN && zneg(o, s + 1));
+      __syncthreads();
+      neighbour_sums(pa, P[J], xs, ys);
+      point(s, P[J], residual<T, false>(co, none, P[J], xs, ys, P[M], P[N]));
+      __syncwarp();
+    });
+  }
+  const bool mx[1] = {false};
+  reduce_finish<1>(acc, mx, rb, [=](const Sums<1>& s) {
+    sc->first = 0;
+    sc->pap = s.v[0];
+    if(fabs(s.v[0]) < kBreakdown) sc->stop = 1;
+    else sc->alpha = sc->rz / s.v[0];
+  });
+}
+
+// Solution and residual update (linsolve/poisson_solver.cpp:762-782):
+// x = (x - sx) + alpha p, r = (r - sr) - alpha A p (in FP64 arithmetic), the
+// residual's norm and the convergence test.  x keeps a zero mean up to
+// rounding (p has none).  Bound: reads p, x and r, writes x and r (5 vectors);
+// at 256^3 119 us in FP64, where the update from a stored A p took 142.
+template <typename T, bool SGN, bool FLAT>
+__global__ void __launch_bounds__(kMaxThreads, 1)
+    k_advance(OpInfo o, Tile t, Direction<T> d, T* __restrict__ x, T* __restrict__ r, SolveScalars* sc, RedBuf rb,
+              cudaGraphConditionalHandle cond) {
+  extern __shared__ __align__(16) unsigned char march_sm[];
+  T* ring = reinterpret_cast<T*>(march_sm);
+  const int sw = slot_words<T>(t), pw = plane_words<T>(t);
+  T *xring = ring + kRing * sw, *rring = xring + kRing * sw;
+  const Place<T, SGN> pl(o, t, 1);
+  const Coef<T> co(o, FLAT);
+  const int nxy = o.L.nxy;
+  const int k0 = blockIdx.y * t.chunk, k1 = min(k0 + t.chunk, o.L.nz);
+  T* me = rring + kRing * sw + (pl.row0 + 1) * kRow<T> + pl.p;
+  pdl_enter();
+  const int stop = sc->stop;
+  const T* __restrict__ p = d.p[sc->body_runs & 1];
+  const double alpha = sc->alpha, sr = sc->sr;
+  const T sx = T(sc->sx), ax = T(alpha);
+  double acc[2] = {0.0, 0.0};
+  auto point = [&](int k, const Patch<T>& pv, const Patch<T>& minus_av, const Patch<T>& xv, const Patch<T>& rv) {
+    Patch<T> xn, rn;
+#pragma unroll
+    for(int q = 0; q < 2; ++q)
+#pragma unroll
+      for(int c = 0; c < kW<T>; ++c) {
+        const double vr = (double(rv.v[q][c]) - sr) + alpha * double(minus_av.v[q][c]);
+        xn.v[q][c] = (xv.v[q][c] - sx) + ax * pv.v[q][c];
+        rn.v[q][c] = T(vr);
+        if(pl.interior(q, c)) {
+          acc[0] += vr;
+          acc[1] += vr * vr;
+        }
+      }
+    pl.store(x, k * nxy, xn);
+    pl.store(r, k * nxy, rn);
+  };
+  const Patch<T> none = {};
+  Patch<T> xs, ys;
+  bool zn;
+  if(stop) {
+  } else if constexpr(FLAT) {
+    Patch<T> q = pl.load(p, 0);
+    if constexpr(SGN) pl.settle(q, T(0), false);
+    publish(me, q);
+    const Patch<T> xv = pl.load(x, 0), rv = pl.load(r, 0);
+    __syncthreads();
+    neighbour_sums(me, q, xs, ys);
+    point(0, q, residual<T, true>(co, none, q, xs, ys, q, q), xv, rv);
+  } else {
+    // step s: plane s; p three planes ahead, x and r (own cells only) likewise
+    Patch<T> P[4];
+    int zo = k0 * nxy;
+    Walk f(o, k0 + 1);
+    for(int q = 1; q <= 3; ++q) {
+      const int zp = f.kz * nxy;
+      if(f.k <= k1) pl.fetch(ring + (q & 3) * sw, p, zp);
+      if(f.k <= k1 && pl.in != 0) {
+        pl.fetch(xring + (q - 1) * sw, x, zo);
+        pl.fetch(rring + (q - 1) * sw, r, zo);
+      }
+      fetch_commit();
+      zo = zp;
+      f.next(o);
+    }
+    P[3] = pl.load(p, zplane(o, k0 - 1, zn) * nxy);
+    if constexpr(SGN) pl.settle(P[3], T(0), zn);
+    P[0] = pl.load(p, k0 * nxy);
+    if constexpr(SGN) pl.settle(P[0], T(0), false);
+    ring4(k0, k1 - 1, [&](auto jc, int s) {
+      constexpr int J = jc, M = (J + 3) & 3, N = (J + 1) & 3;
+      fetch_wait<2>();
+      P[N] = pl.take(ring + N * sw);
+      const int zp = f.kz * nxy;
+      if(f.k <= k1) pl.fetch(ring + J * sw, p, zp);  // plane s + 4
+      if(f.k <= k1 && pl.in != 0) {                  // plane s + 3
+        pl.fetch(xring + M * sw, x, zo);
+        pl.fetch(rring + M * sw, r, zo);
+      }
+      __syncwarp();
+      fetch_commit();
+      zo = zp;
+      f.next(o);
+      T* pa = me + (J & 1) * pw;
+      publish(pa, P[J]);
+      if constexpr(SGN) pl.settle(P[N], T(0), zneg(o, s + 1));
+      __syncthreads();
+      neighbour_sums(pa, P[J], xs, ys);
+      point(s, P[J], residual<T, false>(co, none, P[J], xs, ys, P[M], P[N]), pl.take(xring + J * sw),
+            pl.take(rring + J * sw));
+      __syncwarp();
+    });
+  }
+  const bool mx[2] = {false, false};
+  reduce_finish<2>(acc, mx, rb, [=](const Sums<2>& s) {
+    sc->body_runs += 1;
+    if(sc->stop) {
+      sc->cont = 0;
+      if(cond) cudaGraphSetConditional(cond, 0);
+      return;
+    }
+    const int n = sc->n;
+    const int zm = sc->zero_mean;
+    sc->sx = 0.0;
+    const double srn = zm ? s.v[0] / n : 0.0;
+    sc->sr = srn;
+    sc->sum_r = s.v[0];
+    const double ss = fmax(s.v[1] - n * srn * srn, 0.0);
+    sc->rnorm = sqrt(ss / n);
+    sc->iterations += 1;
+    sc->rel = sc->r0 > 0.0 ? sc->rnorm / sc->r0 : 0.0;
+    if(sc->rel <= sc->tol) sc->converged = 1;
+    if(sc->hist != nullptr && sc->iterations < sc->hist_cap) sc->hist[sc->iterations] = sc->rnorm;
+    // the reference's loop: at most max_iterations iterations, stop on convergence
+    sc->cont = (sc->converged || sc->iterations >= sc->max_it) ? 0 : 1;
+    if(cond) cudaGraphSetConditional(cond, sc->cont);
+  });
 }
 
 }  // namespace march

@@ -8,20 +8,16 @@
 // coarsest grid, and the zero-mean projection on singular (periodic /
 // all-Neumann) problems after every update.
 //
-// B200 form: each vector update is one kernel that also produces the sums the
-// next step needs (deterministic two-stage reduction, common.cuh).  A mean
-// removal is never a separate pass: the kernel that produces a vector records
-// its mean as a pending shift, and every consumer subtracts the shift as it
-// loads the vector -- the same arithmetic as the reference's
-// subtract_active_mean, one kernel later.  The Jacobi diagonal is a 64-entry
-// table per level (it only depends on whether a cell touches a boundary), the
-// V-cycle's residual is restricted on the fly (never stored) and the
-// prolongation is folded into the first post-smoothing sweep.  The V-cycle
-// storage type T is double (OF_FP64) or float (OF_MIXED: FP32 storage and
-// arithmetic inside the FP64 CG loop).
+// B200 form: an iteration passes over the fine level's vectors four times
+// (march.cuh): k_descend, k_ascend, k_direction and k_advance, each several
+// steps of the algorithm pipelined over the planes of a tile, with the sums the
+// next one needs (deterministic two-stage reduction, common.cuh).  The coarse
+// levels take the same two V-cycle kernels each, down to the level that is one
+// matrix.  A mean removal is never a separate pass: the kernel that produces
+// a vector records its mean as a pending shift that consumers subtract on load.
+// The V-cycle storage type T is double (OF_FP64) or float (OF_MIXED: FP32
+// storage and arithmetic inside an FP64 defect correction).
 #include "kernels.hpp"
-#include "vstencil.cuh"
-#include "tma.cuh"
 #include "march.cuh"
 
 #include <cmath>
@@ -39,11 +35,6 @@ namespace {
 constexpr double kSmallNumber = 1.0e-30;
 constexpr double kOmega = 2.0 / 3.0;
 constexpr int kMaxCoarse = 1024;
-
-__device__ __forceinline__ double inv_diag(const OpInfo& o, int i, int j, int k) {
-  const int t = axis_class(i, o.L.nx) + 4 * axis_class(j, o.L.ny) + 16 * axis_class(k, o.L.nz);
-  return __ldg(&o.invd[t]);
-}
 
 // Neighbour coordinates along one axis, branch-free: the in-range neighbour,
 // the periodic image, or the cell itself with sign +1 (homogeneous Neumann,
@@ -131,1847 +122,6 @@ __device__ __forceinline__ void k_batched(int k0, int k1, Compute compute, Commi
   const bool valid = i < (L).nx && j < (L).ny;              \
   const int k0 = blockIdx.z * kchunk;                       \
   const int k1 = min(k0 + kchunk, (L).nz);
-
-template <typename A>
-struct Pair {
-  A v;
-  double w;
-};
-
-// ---------------------------------------------------------------------------
-// V-cycle kernels.  Level vectors are T; shifts and scalars are double.
-// ---------------------------------------------------------------------------
-
-// Pre-smoothing sweep 1 from a zero correction: a = omega (b - sb) / D.
-template <typename T, typename B>
-__global__ void __launch_bounds__(kTX* kTY)
-    k_smooth_first(OpInfo o, const B* __restrict__ b, const double* sb_ptr, T* __restrict__ a,
-                   LevelScalars* ls, int zm, int kchunk, RedBuf rb) {
-  pdl_enter();
-  STENCIL_PROLOGUE(o.L)
-  using A = T;
-  const double sb = *sb_ptr;
-  double acc[1];
-  zero(acc);
-  if(valid) {
-    const A om = A(kOmega);
-    k_batched<kBatch>(
-        k0, k1,
-        [&](int k) { return om * A(double(b[o.L.idx(i, j, k)]) - sb) * A(inv_diag(o, i, j, k)); },
-        [&](int k, A v) {
-          a[o.L.idx(i, j, k)] = T(v);
-          acc[0] += double(v);
-        });
-  }
-  const bool mx[1] = {false};
-  const int n = o.L.count();
-  reduce_finish<1>(acc, mx, rb, [=](const Sums<1>& s) { ls->sa = zm ? s.v[0] / n : 0.0; });
-}
-
-// Jacobi sweep (smooth_jacobi, linsolve/poisson_solver.cpp:569-595):
-// out = x + omega (b - sb - A x) / D with x = in - s_in; records mean(out).
-// `which` selects the LevelScalars slot for the output mean (0: sa, 1: sx).
-// On the finest level with sc != nullptr it also forms r.z for the CG.
-template <typename T, typename B>
-__global__ void __launch_bounds__(kTX* kTY)
-    k_smooth(OpInfo o, const B* __restrict__ b, const double* sb_ptr, const T* __restrict__ in,
-             const double* sin_ptr, T* __restrict__ out, LevelScalars* ls, int which, int zm,
-             SolveScalars* sc, int kchunk, RedBuf rb) {
-  pdl_enter();
-  STENCIL_PROLOGUE(o.L)
-  using A = T;
-  const double sb = *sb_ptr;
-  const A sin = A(*sin_ptr);
-  double acc[2];
-  zero(acc);
-  if(valid) {
-    const ColNb nb = col_nb(o, i, j);
-    const A om = A(kOmega);
-    auto val = [&](int ii, int jj, int kk) { return A(in[o.L.idx(ii, jj, kk)]) - sin; };
-    k_batched<kBatch>(
-        k0, k1,
-        [&](int k) {
-          A c;
-          const A ax = apply_op<A>(o, nb, i, j, k, val, c);
-          const double bq = double(b[o.L.idx(i, j, k)]) - sb;
-          return Pair<A>{c + om * (A(bq) - ax) * A(inv_diag(o, i, j, k)), bq};
-        },
-        [&](int k, Pair<A> r) {
-          out[o.L.idx(i, j, k)] = T(r.v);
-          acc[0] += double(r.v);
-          acc[1] += r.w * double(r.v);
-        });
-  }
-  const bool mx[2] = {false, false};
-  const int n = o.L.count();
-  reduce_finish<2>(acc, mx, rb, [=](const Sums<2>& s) {
-    const double mean = zm ? s.v[0] / n : 0.0;
-    if(which == 0) ls->sa = mean;
-    else {
-      ls->sx = mean;
-      ls->sum_x = s.v[0];
-    }
-    if(sc != nullptr) {
-      // r.z with z = out - mean (linsolve/poisson_solver.cpp:749, :791)
-      const double rz_new = s.v[1] - mean * (sc->sum_r - sc->n * sc->sr);
-      if(sc->first) {
-        sc->rz = rz_new;
-      } else {
-        sc->beta = rz_new / sc->rz;
-        sc->rz = rz_new;
-      }
-    }
-  });
-}
-
-// Residual + restriction (v_cycle :611-624 and restrict_full_weighting
-// :397-424): coarse b = mean of the children's (b - sb - A x); x = in - s_in.
-// RX, RY, RZ are the refinement ratios (1 or 2); children summed in the
-// reference's dz, dy, dx order.
-template <typename T, typename B, int RX, int RY, int RZ>
-__global__ void __launch_bounds__(kTX* kTY)
-    k_restrict_residual(OpInfo o, OpInfo oc, const B* __restrict__ b, const double* sb_ptr,
-                        const T* __restrict__ in, const double* sin_ptr, T* __restrict__ bc,
-                        LevelScalars* lsc, int zm, int kchunk, RedBuf rb) {
-  pdl_enter();
-  STENCIL_PROLOGUE(oc.L)
-  using A = T;
-  const double sb = *sb_ptr;
-  const A sin = A(*sin_ptr);
-  const A inv_children = A(1.0 / double(RX * RY * RZ));
-  double acc[1];
-  zero(acc);
-  if(valid) {
-    ColNb nb[RY][RX];
-#pragma unroll
-    for(int dy = 0; dy < RY; ++dy)
-#pragma unroll
-      for(int dx = 0; dx < RX; ++dx) nb[dy][dx] = col_nb(o, i * RX + dx, j * RY + dy);
-    auto val = [&](int ii, int jj, int kk) { return A(in[o.L.idx(ii, jj, kk)]) - sin; };
-    k_batched<2>(
-        k0, k1,
-        [&](int kc) {
-          A sum = A(0);
-#pragma unroll
-          for(int dz = 0; dz < RZ; ++dz)
-#pragma unroll
-            for(int dy = 0; dy < RY; ++dy)
-#pragma unroll
-              for(int dx = 0; dx < RX; ++dx) {
-                const int fi = i * RX + dx, fj = j * RY + dy, fk = kc * RZ + dz;
-                A c;
-                const A ax = apply_op<A>(o, nb[dy][dx], fi, fj, fk, val, c);
-                sum += A(double(b[o.L.idx(fi, fj, fk)]) - sb) - ax;
-              }
-          return inv_children * sum;
-        },
-        [&](int kc, A v) {
-          bc[oc.L.idx(i, j, kc)] = T(v);
-          acc[0] += double(v);
-        });
-  }
-  const bool mx[1] = {false};
-  const int n = oc.L.count();
-  reduce_finish<1>(acc, mx, rb, [=](const Sums<1>& s) { lsc->sb = zm ? s.v[0] / n : 0.0; });
-}
-
-// Prolongation + first post-smoothing sweep (prolongate_and_add :426-451,
-// then smooth_jacobi): x3 = (in - s_in) + (e_parent - s_e); out = x3 +
-// omega (b - sb - A x3) / D.  SX, SY, SZ are log2 of the refinement ratios.
-template <typename T, typename B>
-__global__ void __launch_bounds__(kTX* kTY)
-    k_prolong_smooth(OpInfo o, CLay Lc, const B* __restrict__ b, const double* sb_ptr,
-                     const T* __restrict__ in, const double* sin_ptr, const T* __restrict__ ec,
-                     const double* sec_ptr, T* __restrict__ out, LevelScalars* ls, int sx, int sy,
-                     int sz, int zm, int kchunk, RedBuf rb) {
-  pdl_enter();
-  STENCIL_PROLOGUE(o.L)
-  using A = T;
-  const double sb = *sb_ptr;
-  const A sin = A(*sin_ptr);
-  const A sec = A(*sec_ptr);
-  double acc[1];
-  zero(acc);
-  if(valid) {
-    const ColNb nb = col_nb(o, i, j);
-    const A om = A(kOmega);
-    auto val = [&](int ii, int jj, int kk) {
-      return (A(in[o.L.idx(ii, jj, kk)]) - sin) + (A(ec[Lc.idx(ii >> sx, jj >> sy, kk >> sz)]) - sec);
-    };
-    k_batched<kBatch>(
-        k0, k1,
-        [&](int k) {
-          A c;
-          const A ax = apply_op<A>(o, nb, i, j, k, val, c);
-          const A bq = A(double(b[o.L.idx(i, j, k)]) - sb);
-          return c + om * (bq - ax) * A(inv_diag(o, i, j, k));
-        },
-        [&](int k, A v) {
-          out[o.L.idx(i, j, k)] = T(v);
-          acc[0] += double(v);
-        });
-  }
-  const bool mx[1] = {false};
-  const int n = o.L.count();
-  reduce_finish<1>(acc, mx, rb, [=](const Sums<1>& s) { ls->sa = zm ? s.v[0] / n : 0.0; });
-}
-
-// ---------------------------------------------------------------------------
-// Row-vector kernels (vstencil.cuh) for levels whose rows split into 16-byte
-// vectors; the column kernels above serve the rest.
-// ---------------------------------------------------------------------------
-
-template <typename T>
-inline bool vfits(const CLay& L) {
-  return vst::row_fits(L.nx, vst::Width<T>::W);
-}
-
-// Vector kernels can be switched off for comparisons: ORCHARD_B200_NO_VEC=1
-// (all) or a comma list of smooth, pre, prolong, restrict, ap.  Read at each use so
-// that a process can compare both forms.
-bool vec_enabled(const char* which = "") {
-  const char* e = std::getenv("ORCHARD_B200_NO_VEC");
-  if(e == nullptr || e[0] == '\0' || e[0] == '0') return true;
-  if(e[0] == '1') return false;
-  return std::strstr(e, which) == nullptr || which[0] == '\0';
-}
-
-#define ROW_PROLOGUE(T)                                                          \
-  constexpr int W = vst::Width<T>::W;                                             \
-  const vst::RowGeom g = vst::row_geom<W>(o.L, o.periodic, o.dir_lo, o.dir_hi);   \
-  const int k0 = blockIdx.z * kchunk;                                             \
-  const int k1 = min(k0 + kchunk, o.L.nz);
-
-// Jacobi sweep (smooth_jacobi); same contract as k_smooth with which = 1.
-template <typename T, typename B>
-__global__ void __launch_bounds__(256)
-    k_vsmooth(OpInfo o, const B* __restrict__ b, const double* sb_ptr, const T* __restrict__ in,
-              const double* sin_ptr, T* __restrict__ out, LevelScalars* ls, int zm,
-              SolveScalars* sc, int kchunk, RedBuf rb) {
-  pdl_enter();
-  using A = T;
-  ROW_PROLOGUE(T)
-  using R = vst::Row<A, W>;
-  using RB = vst::Row<double, W>;
-  const double sb = *sb_ptr;
-  const A sin = A(*sin_ptr);
-  const A om = A(kOmega);
-  double acc[2] = {0.0, 0.0};
-  vst::march<A, W, RB>(
-      o, g, k0, k1,
-      [&](int i0, int jj, int kk) {
-        R r = vst::ld<A, W>(in + o.L.idx(i0, jj, kk));
-#pragma unroll
-        for(int t = 0; t < W; ++t) r.v[t] -= sin;
-        return r;
-      },
-      [&](int ii, int jj, int kk) { return A(in[o.L.idx(ii, jj, kk)]) - sin; },
-      [&](int i0, int jj, int kk) { return vst::ld<double, W>(b + o.L.idx(i0, jj, kk)); },
-      [&](int k, const R& c, const R& ax, const RB& bb) {
-        R v;
-        double bq[W];
-#pragma unroll
-        for(int t = 0; t < W; ++t) {
-          bq[t] = bb.v[t] - sb;
-          v.v[t] = c.v[t] + om * (A(bq[t]) - ax.v[t]) * A(inv_diag(o, g.i0 + t, g.j, k));
-        }
-        if(g.act) {
-          vst::st<T, W>(out + o.L.idx(g.i0, g.j, k), v);
-#pragma unroll
-          for(int t = 0; t < W; ++t) {
-            acc[0] += double(v.v[t]);
-            acc[1] += bq[t] * double(v.v[t]);
-          }
-        }
-      });
-  const bool mx[2] = {false, false};
-  const int n = o.L.count();
-  reduce_finish<2>(acc, mx, rb, [=](const Sums<2>& s) {
-    const double mean = zm ? s.v[0] / n : 0.0;
-    ls->sx = mean;
-    ls->sum_x = s.v[0];
-    if(sc != nullptr) {
-      // r.z with z = out - mean (linsolve/poisson_solver.cpp:749, :791)
-      const double rz_new = s.v[1] - mean * (sc->sum_r - sc->n * sc->sr);
-      if(sc->first) {
-        sc->rz = rz_new;
-      } else {
-        sc->beta = rz_new / sc->rz;
-        sc->rz = rz_new;
-      }
-    }
-  });
-}
-
-// Both pre-smoothing sweeps from a zero correction in one pass over b: the
-// first sweep is pointwise, a = omega (b - sb) / D, so the second one,
-// out = a + omega (b - sb - A a) / D, reads b alone (a is formed on load for
-// every neighbour).  The reference removes mean(a) between the sweeps; A
-// annihilates constants on the problems where it does that (periodic /
-// all-Neumann), so the shift only moves out by a constant, which the mean
-// recorded here (ls->sx) removes as before.
-template <typename T, typename B>
-__global__ void __launch_bounds__(256)
-    k_vsmooth_pre(OpInfo o, const B* __restrict__ b, const double* sb_ptr, T* __restrict__ out,
-                  LevelScalars* ls, int zm, int kchunk, RedBuf rb) {
-  pdl_enter();
-  using A = T;
-  ROW_PROLOGUE(T)
-  using R = vst::Row<A, W>;
-  using RB = vst::Row<double, W>;
-  const double sb = *sb_ptr;
-  const A om = A(kOmega);
-  auto a_at = [&](int ii, int jj, int kk, double bv) {
-    return om * A(bv - sb) * A(inv_diag(o, ii, jj, kk));
-  };
-  double acc[1] = {0.0};
-  vst::march<A, W, RB>(
-      o, g, k0, k1,
-      [&](int i0, int jj, int kk) {
-        const RB bb = vst::ld<double, W>(b + o.L.idx(i0, jj, kk));
-        R r;
-#pragma unroll
-        for(int t = 0; t < W; ++t) r.v[t] = a_at(i0 + t, jj, kk, bb.v[t]);
-        return r;
-      },
-      [&](int ii, int jj, int kk) { return a_at(ii, jj, kk, double(b[o.L.idx(ii, jj, kk)])); },
-      [&](int i0, int jj, int kk) { return vst::ld<double, W>(b + o.L.idx(i0, jj, kk)); },
-      [&](int k, const R& c, const R& ax, const RB& bb) {
-        R v;
-#pragma unroll
-        for(int t = 0; t < W; ++t)
-          v.v[t] = c.v[t] + om * (A(bb.v[t] - sb) - ax.v[t]) * A(inv_diag(o, g.i0 + t, g.j, k));
-        if(g.act) {
-          vst::st<T, W>(out + o.L.idx(g.i0, g.j, k), v);
-#pragma unroll
-          for(int t = 0; t < W; ++t) acc[0] += double(v.v[t]);
-        }
-      });
-  const bool mx[1] = {false};
-  const int n = o.L.count();
-  reduce_finish<1>(acc, mx, rb, [=](const Sums<1>& s) {
-    ls->sx = zm ? s.v[0] / n : 0.0;
-    ls->sum_x = s.v[0];
-  });
-}
-
-// Prolongation + first post-smoothing sweep; same contract as k_prolong_smooth.
-template <typename T, typename B>
-__global__ void __launch_bounds__(256)
-    k_vprolong_smooth(OpInfo o, CLay Lc, const B* __restrict__ b, const double* sb_ptr,
-                      const T* __restrict__ in, const double* sin_ptr, const T* __restrict__ ec,
-                      const double* sec_ptr, T* __restrict__ out, LevelScalars* ls, int sx, int sy,
-                      int sz, int zm, int kchunk, RedBuf rb) {
-  pdl_enter();
-  using A = T;
-  ROW_PROLOGUE(T)
-  using R = vst::Row<A, W>;
-  using RB = vst::Row<double, W>;
-  const double sb = *sb_ptr;
-  const A sin = A(*sin_ptr);
-  const A sec = A(*sec_ptr);
-  const A om = A(kOmega);
-  double acc[1] = {0.0};
-  vst::march<A, W, RB>(
-      o, g, k0, k1,
-      [&](int i0, int jj, int kk) {
-        R r = vst::ld<A, W>(in + o.L.idx(i0, jj, kk));
-        const int pj = jj >> sy, pk = kk >> sz;
-#pragma unroll
-        for(int t = 0; t < W; ++t) r.v[t] = (r.v[t] - sin) + (A(ec[Lc.idx((i0 + t) >> sx, pj, pk)]) - sec);
-        return r;
-      },
-      [&](int ii, int jj, int kk) {
-        return (A(in[o.L.idx(ii, jj, kk)]) - sin) + (A(ec[Lc.idx(ii >> sx, jj >> sy, kk >> sz)]) - sec);
-      },
-      [&](int i0, int jj, int kk) { return vst::ld<double, W>(b + o.L.idx(i0, jj, kk)); },
-      [&](int k, const R& c, const R& ax, const RB& bb) {
-        R v;
-#pragma unroll
-        for(int t = 0; t < W; ++t)
-          v.v[t] = c.v[t] + om * (A(bb.v[t] - sb) - ax.v[t]) * A(inv_diag(o, g.i0 + t, g.j, k));
-        if(g.act) {
-          vst::st<T, W>(out + o.L.idx(g.i0, g.j, k), v);
-#pragma unroll
-          for(int t = 0; t < W; ++t) acc[0] += double(v.v[t]);
-        }
-      });
-  const bool mx[1] = {false};
-  const int n = o.L.count();
-  reduce_finish<1>(acc, mx, rb, [=](const Sums<1>& s) { ls->sa = zm ? s.v[0] / n : 0.0; });
-}
-
-// A p; same contract as k_apply_ap.  V is the vector type (arithmetic FP64).
-template <typename V>
-__global__ void __launch_bounds__(256)
-    k_vapply_ap(OpInfo o, const V* __restrict__ p, V* __restrict__ ap, SolveScalars* sc,
-                int kchunk, RedBuf rb) {
-  pdl_enter();
-  ROW_PROLOGUE(V)
-  using R = vst::Row<double, W>;
-  const double sp = sc->sp;
-  double acc[3] = {0.0, 0.0, 0.0};
-  vst::march<double, W, int>(
-      o, g, k0, k1,
-      [&](int i0, int jj, int kk) {
-        R r = vst::ld<double, W>(p + o.L.idx(i0, jj, kk));
-#pragma unroll
-        for(int t = 0; t < W; ++t) r.v[t] -= sp;
-        return r;
-      },
-      [&](int ii, int jj, int kk) { return double(p[o.L.idx(ii, jj, kk)]) - sp; },
-      [&](int, int, int) { return 0; },
-      [&](int k, const R& c, const R& ax, int) {
-        if(g.act) {
-          vst::st<V, W>(ap + o.L.idx(g.i0, g.j, k), ax);
-#pragma unroll
-          for(int t = 0; t < W; ++t) {
-            acc[0] += ax.v[t];
-            acc[1] += c.v[t] * ax.v[t];
-            acc[2] += c.v[t];
-          }
-        }
-      });
-  const bool mx[3] = {false, false, false};
-  reduce_finish<3>(acc, mx, rb, [=](const Sums<3>& s) {
-    const double sap = sc->zero_mean ? s.v[0] / sc->n : 0.0;
-    sc->sap = sap;
-    const double pap = s.v[1] - sap * s.v[2];
-    sc->pap = pap;
-    if(fabs(pap) < kSmallNumber) {
-      sc->stop = 1;
-    } else {
-      sc->alpha = sc->rz / pap;
-    }
-  });
-}
-
-// Residual + 2x2x2 restriction on row vectors: a thread owns W fine cells of
-// the two fine rows of a coarse row (W/2 coarse cells) and marches coarse
-// planes (two fine planes each).
-template <typename T, typename B>
-__global__ void __launch_bounds__(256)
-    k_vrestrict(OpInfo o, OpInfo oc, const B* __restrict__ b, const double* sb_ptr,
-                const T* __restrict__ in, const double* sin_ptr, T* __restrict__ bc,
-                LevelScalars* lsc, int zm, int kchunk, RedBuf rb) {
-  pdl_enter();
-  using A = T;
-  constexpr int W = vst::Width<T>::W;
-  using R = vst::Row<A, W>;
-  const CLay& L = o.L;
-  const int lane = threadIdx.x;
-  int i0 = (blockIdx.x * 32 + lane) * W;
-  const int jc = blockIdx.y * 8 + threadIdx.y;
-  const bool act = i0 < L.nx && jc < oc.L.ny;
-  if(i0 >= L.nx) i0 = L.nx - W;
-  const int jcc = jc < oc.L.ny ? jc : oc.L.ny - 1;
-  const int kc0 = blockIdx.z * kchunk;
-  const int kc1 = min(kc0 + kchunk, oc.L.nz);
-  const double sb = *sb_ptr;
-  const A sin = A(*sin_ptr);
-  const A ix = A(o.inv2[0]), iy = A(o.inv2[1]), iz = A(o.inv2[2]);
-  const int jr[2] = {2 * jcc, 2 * jcc + 1};
-  int jdn, jup;
-  double sdn, sup;
-  nb_lo(jr[0], L.ny, o.periodic[1], o.dir_lo[1], jdn, sdn);
-  nb_hi(jr[1], L.ny, o.periodic[1], o.dir_hi[1], jup, sup);
-  const bool need_l = lane == 0 || i0 == 0;
-  const bool need_r = lane == 31 || i0 + W >= L.nx;
-  int xl, xr;
-  double sxl, sxr;
-  nb_lo(i0, L.nx, o.periodic[0], o.dir_lo[0], xl, sxl);
-  nb_hi(i0 + W - 1, L.nx, o.periodic[0], o.dir_hi[0], xr, sxr);
-  auto rowv = [&](int jj, int kk) {
-    R r = vst::ld<A, W>(in + L.idx(i0, jj, kk));
-#pragma unroll
-    for(int t = 0; t < W; ++t) r.v[t] -= sin;
-    return r;
-  };
-  auto zrowv = [&](int jj, int kk) {
-    double sg;
-    const int kz = vst::zrow(kk, L.nz, o.periodic[2], o.dir_lo[2], o.dir_hi[2], sg);
-    R r = rowv(jj, kz);
-#pragma unroll
-    for(int t = 0; t < W; ++t) r.v[t] *= A(sg);
-    return r;
-  };
-  double acc[1] = {0.0};
-  for(int kc = kc0; kc < kc1; ++kc) {
-    const int kf = 2 * kc;
-    // rows j0, j1 at planes kf-1 .. kf+2, neighbour rows at kf, kf+1
-    R q[2][4];
-#pragma unroll
-    for(int r = 0; r < 2; ++r)
-#pragma unroll
-      for(int z = 0; z < 4; ++z) q[r][z] = zrowv(jr[r], kf - 1 + z);
-    R dn[2], up[2];
-    A hl[2][2], hr[2][2];
-    vst::Row<double, W> bb[2][2];
-#pragma unroll
-    for(int z = 0; z < 2; ++z) {
-      dn[z] = rowv(jdn, kf + z);
-      up[z] = rowv(jup, kf + z);
-#pragma unroll
-      for(int t = 0; t < W; ++t) {
-        dn[z].v[t] *= A(sdn);
-        up[z].v[t] *= A(sup);
-      }
-#pragma unroll
-      for(int r = 0; r < 2; ++r) {
-        hl[r][z] = need_l ? A(sxl) * (A(in[L.idx(xl, jr[r], kf + z)]) - sin) : A(0);
-        hr[r][z] = need_r ? A(sxr) * (A(in[L.idx(xr, jr[r], kf + z)]) - sin) : A(0);
-        bb[r][z] = vst::ld<double, W>(b + L.idx(i0, jr[r], kf + z));
-      }
-    }
-    A csum[W / 2];
-#pragma unroll
-    for(int c = 0; c < W / 2; ++c) csum[c] = A(0);
-#pragma unroll
-    for(int z = 0; z < 2; ++z)
-#pragma unroll
-      for(int r = 0; r < 2; ++r) {
-        const R& cen = q[r][z + 1];
-        const A from_l = __shfl_up_sync(0xffffffffu, cen.v[W - 1], 1);
-        const A from_r = __shfl_down_sync(0xffffffffu, cen.v[0], 1);
-        const A left = need_l ? hl[r][z] : from_l;
-        const A right = need_r ? hr[r][z] : from_r;
-        const R& d = r == 0 ? dn[z] : q[0][z + 1];
-        const R& u = r == 0 ? q[1][z + 1] : up[z];
-        const R ax = vst::row_ax<A, W>(cen, left, right, d, u, q[r][z], q[r][z + 2], ix, iy, iz);
-#pragma unroll
-        for(int t = 0; t < W; ++t) csum[t / 2] += A(bb[r][z].v[t] - sb) - ax.v[t];
-      }
-    if(act) {
-#pragma unroll
-      for(int c = 0; c < W / 2; ++c) {
-        const A v = A(0.125) * csum[c];
-        bc[oc.L.idx(i0 / 2 + c, jc, kc)] = T(v);
-        acc[0] += double(v);
-      }
-    }
-  }
-  const bool mx[1] = {false};
-  const int n = oc.L.count();
-  reduce_finish<1>(acc, mx, rb, [=](const Sums<1>& s) { lsc->sb = zm ? s.v[0] / n : 0.0; });
-}
-
-// ---------------------------------------------------------------------------
-// Plane-pipelined stencil kernels.  A block owns a tile of whole rows (all nx
-// cells, TY = 1024 / nx rows) and a chunk of k planes.  One thread stages each
-// plane of the operand -- the tile rows plus the two neighbour rows, fetched at
-// their boundary images (periodic wrap or the mirrored row) -- and of the
-// rhs into a ring of kTSlots shared-memory slots with TMA, kTSlots - 2 planes
-// ahead of the compute; an mbarrier per slot carries the arrival.  Each
-// thread owns four consecutive cells of one row: their z-neighbours come from
-// a register queue, the in-plane neighbours from the staged plane.  Boundary
-// signs (Dirichlet mirrors) and mean shifts are applied on read.  Used where
-// nx is 64, 128 or 256 and TY divides ny.
-// ---------------------------------------------------------------------------
-constexpr int kTSlots = 5;
-
-__host__ __device__ inline size_t tround(size_t b) { return (b + 127) / 128 * 128; }
-
-template <typename T, typename B>
-__host__ __device__ inline size_t tslot_bytes(int nx) {
-  const int ty = 1024 / nx;
-  return tround(static_cast<size_t>(ty + 2) * nx * sizeof(T)) + tround(static_cast<size_t>(ty) * nx * sizeof(B));
-}
-
-template <typename T, typename B>
-__host__ __device__ inline size_t tprolong_bytes(int nx) {
-  const int ty = 1024 / nx;
-  return tround(static_cast<size_t>(ty + 2) * nx * sizeof(T)) + tround(static_cast<size_t>(ty) * nx * sizeof(B)) +
-         tround(static_cast<size_t>(ty / 2 + 2) * (nx / 2) * sizeof(T));
-}
-
-// Four consecutive values from shared (or global) memory.  SWAP (FP64 only):
-// lanes 32 bytes apart read their two 16-byte halves in an order that
-// alternates with (lane ^ lane / 4), so that each quarter-warp phase of a
-// 128-bit shared-memory load touches eight distinct 16-byte bank groups
-// instead of four (no 2-way bank conflict); the same values either way, at
-// the cost of a few registers for the lane-dependent select.
-template <typename A, typename S, bool SWAP = false>
-__device__ __forceinline__ void tload4(const S* p, A (&v)[4]) {
-  if constexpr(std::is_same_v<S, double>) {
-    double2 a, b;
-    if constexpr(SWAP) {
-      const int lane = threadIdx.x & 31;
-      const int h = (lane ^ (lane >> 2)) & 1;
-      const double2* q = reinterpret_cast<const double2*>(p);
-      const double2 f = q[h];
-      const double2 g = q[h ^ 1];
-      a = h ? g : f;
-      b = h ? f : g;
-    } else {
-      a = *reinterpret_cast<const double2*>(p);
-      b = *reinterpret_cast<const double2*>(p + 2);
-    }
-    v[0] = A(a.x);
-    v[1] = A(a.y);
-    v[2] = A(b.x);
-    v[3] = A(b.y);
-  } else {
-    const float4 a = *reinterpret_cast<const float4*>(p);
-    v[0] = A(a.x);
-    v[1] = A(a.y);
-    v[2] = A(a.z);
-    v[3] = A(a.w);
-  }
-}
-
-template <typename S, typename A>
-__device__ __forceinline__ void tstore4(S* p, const A (&v)[4]) {
-  if constexpr(std::is_same_v<S, double>) {
-    *reinterpret_cast<double2*>(p) = make_double2(double(v[0]), double(v[1]));
-    *reinterpret_cast<double2*>(p + 2) = make_double2(double(v[2]), double(v[3]));
-  } else {
-    *reinterpret_cast<float4*>(p) = make_float4(float(v[0]), float(v[1]), float(v[2]), float(v[3]));
-  }
-}
-
-// Persistent schedule of the plane pipeline: the tile-planes (tile, k) of a
-// level, k fastest, are split into gridDim.x contiguous ranges of equal length
-// (within one); a block walks its range as segments (one per tile it touches)
-// and streams each segment's planes k_begin - 1 .. k_end through one ring, so
-// the pipeline is filled once per block and no block waits for a tail wave.
-constexpr int kTMaxSeg = 8;
-
-struct TSeg {
-  int tile, kb, ke, lbase;  // planes [kb, ke) of `tile`; first load index
-};
-
-__device__ __forceinline__ int tsegments(int tiles, int nz, TSeg (&seg)[kTMaxSeg], int& nload) {
-  if(gridDim.x % tiles == 0) {
-    // z-aligned schedule (the host selects it by launching a multiple of the
-    // tile count, tgrid_blocks): block b owns tile b % tiles and z chunk
-    // b / tiles, so the blocks
-    // of neighbouring tiles stream the same planes at the same time and a
-    // tile's halo rows -- its neighbours' edge rows -- come from L2, not DRAM
-    const int nzc = gridDim.x / tiles;
-    const int tile = blockIdx.x % tiles, zc = blockIdx.x / tiles;
-    const int kb = static_cast<int>(static_cast<long long>(nz) * zc / nzc);
-    const int ke = static_cast<int>(static_cast<long long>(nz) * (zc + 1) / nzc);
-    seg[0] = TSeg{tile, kb, ke, 0};
-    nload = ke > kb ? ke - kb + 2 : 0;
-    return ke > kb ? 1 : 0;
-  }
-  const long long total = static_cast<long long>(tiles) * nz;
-  const long long f0 = total * blockIdx.x / gridDim.x;
-  const long long f1 = total * (blockIdx.x + 1) / gridDim.x;
-  int ns = 0;
-  nload = 0;
-  for(long long f = f0; f < f1 && ns < kTMaxSeg;) {
-    const int tile = static_cast<int>(f / nz);
-    const int kb = static_cast<int>(f % nz);
-    const int ke = static_cast<int>(min(static_cast<long long>(nz), kb + (f1 - f)));
-    seg[ns] = TSeg{tile, kb, ke, nload};
-    nload += ke - kb + 2;
-    f += ke - kb;
-    ++ns;
-  }
-  return ns;
-}
-
-// Jacobi sweep (smooth_jacobi, linsolve/poisson_solver.cpp:569-595) on the
-// plane pipeline: out = x + omega (b - sb - A x) / D with x = in - s_in;
-// records mean(out) (ls->sx) and, on the finest level, r.z (sc).  Same
-// contract as k_vsmooth.  CPT cells per thread (4 or 2), 1024 / CPT threads.
-template <typename T, typename B, int CPT, bool PER>
-__global__ void __launch_bounds__(1024 / CPT)
-    k_tsmooth(OpInfo o, const __grid_constant__ CUtensorMap um, const __grid_constant__ CUtensorMap uh,
-              const __grid_constant__ CUtensorMap bm, const double* sb_ptr, const double* sin_ptr,
-              T* __restrict__ out, LevelScalars* ls, int zm, SolveScalars* sc, RedBuf rb, int* fault) {
-  pdl_enter();
-  using A = T;
-  constexpr int D = kTSlots;
-  extern __shared__ __align__(128) unsigned char tsm[];
-  __shared__ uint64_t bars[D];
-  __shared__ double invd_s[64];
-  const int NX = o.L.nx, NY = o.L.ny, NZ = o.L.nz;
-  const int TY = 1024 / NX;
-  const int tpr = NX / CPT;
-  const int r = threadIdx.x / tpr;
-  const int i0 = (threadIdx.x % tpr) * CPT;
-  const size_t ubytes = tround(static_cast<size_t>(TY + 2) * NX * sizeof(T));
-  const size_t sbytes = tslot_bytes<T, B>(NX);
-  const uint32_t tx_bytes = static_cast<uint32_t>((TY + 2) * NX * sizeof(T) + TY * NX * sizeof(B));
-  auto uslot = [&](int s) { return reinterpret_cast<T*>(tsm + s * sbytes); };
-  auto bslot = [&](int s) { return reinterpret_cast<B*>(tsm + s * sbytes + ubytes); };
-  TSeg seg[kTMaxSeg];
-  int nload = 0;
-  const int nseg = tsegments(NY / TY, NZ, seg, nload);
-  // producer (thread 0): load l -> its segment's tile and plane image
-  auto issue = [&](int l) {
-    int q = 0;
-    while(q + 1 < nseg && seg[q + 1].lbase <= l) ++q;
-    const int j0 = seg[q].tile * TY;
-    int jm, jp;
-    double sg;
-    nb_lo(j0, NY, o.periodic[1], o.dir_lo[1], jm, sg);
-    nb_hi(j0 + TY - 1, NY, o.periodic[1], o.dir_hi[1], jp, sg);
-    const int kz = vst::zrow(seg[q].kb - 1 + (l - seg[q].lbase), NZ, o.periodic[2], o.dir_lo[2],
-                             o.dir_hi[2], sg);
-    const int sl = l % D;
-    tma::mbar_arrive_expect_tx(&bars[sl], tx_bytes);
-    tma::load_3d(uslot(sl) + NX, &um, &bars[sl], 0, j0, kz);
-    tma::load_3d(uslot(sl), &uh, &bars[sl], 0, jm, kz);
-    tma::load_3d(uslot(sl) + (TY + 1) * NX, &uh, &bars[sl], 0, jp, kz);
-    tma::load_3d(bslot(sl), &bm, &bars[sl], 0, j0, kz);
-  };
-  if(threadIdx.x == 0) {
-    for(int sl = 0; sl < D; ++sl) tma::mbar_init(&bars[sl], 1);
-    tma::fence_barrier_init();
-  }
-  if(threadIdx.x < 64) invd_s[threadIdx.x] = o.invd[threadIdx.x];
-  __syncthreads();
-  int next = 0;  // next load to issue (meaningful on thread 0)
-  if(threadIdx.x == 0)
-    while(next < nload && next < D) issue(next++);
-  const double sb = *sb_ptr;
-  const A sin = A(*sin_ptr);
-  const A om = A(kOmega);
-  const A ix = A(o.inv2[0]), iy = A(o.inv2[1]), iz = A(o.inv2[2]);
-  auto ldrow = [&](const T* p, A (&v)[CPT]) {
-    if constexpr(CPT == 4) {
-      tload4<A>(p, v);
-    } else if constexpr(std::is_same_v<T, double>) {
-      const double2 a = *reinterpret_cast<const double2*>(p);
-      v[0] = A(a.x);
-      v[1] = A(a.y);
-    } else {
-      const float2 a = *reinterpret_cast<const float2*>(p);
-      v[0] = A(a.x);
-      v[1] = A(a.y);
-    }
-  };
-  double acc[2] = {0.0, 0.0};
-  int xl, xr;
-  double sxl, sxr;
-  nb_lo(i0, NX, o.periodic[0], o.dir_lo[0], xl, sxl);
-  nb_hi(i0 + CPT - 1, NX, o.periodic[0], o.dir_hi[0], xr, sxr);
-  for(int q = 0; q < nseg; ++q) {
-    const TSeg sg = seg[q];
-    const int j0 = sg.tile * TY;
-    const int j = j0 + r;
-    int jm, jp;
-    double sylo, syhi;
-    nb_lo(j0, NY, o.periodic[1], o.dir_lo[1], jm, sylo);
-    nb_hi(j0 + TY - 1, NY, o.periodic[1], o.dir_hi[1], jp, syhi);
-    int cls[CPT];
-#pragma unroll
-    for(int t = 0; t < CPT; ++t) cls[t] = axis_class(i0 + t, NX) + 4 * axis_class(j, NY);
-    auto own = [&](int l, A (&v)[CPT]) {
-      tma::mbar_wait(&bars[l % D], (l / D) & 1, fault, 1);
-      double zs;
-      vst::zrow(sg.kb - 1 + (l - sg.lbase), NZ, o.periodic[2], o.dir_lo[2], o.dir_hi[2], zs);
-      ldrow(uslot(l % D) + (r + 1) * NX + i0, v);
-      if constexpr(!PER) {
-#pragma unroll
-        for(int t = 0; t < CPT; ++t) v[t] = A(zs) * (v[t] - sin);
-      }
-    };
-    // one output plane k from its staged slot and the z-queue (below, cen, above)
-    auto plane = [&](int k, int c, const A (&below)[CPT], const A (&cen)[CPT], const A (&above)[CPT]) {
-      const T* pk = uslot(c % D);
-      const B* bk = bslot(c % D);
-      A dn[CPT], up[CPT];
-      ldrow(pk + r * NX + i0, dn);
-      ldrow(pk + (r + 2) * NX + i0, up);
-      A left = pk[(r + 1) * NX + xl], right = pk[(r + 1) * NX + xr];
-      if constexpr(!PER) {
-        // boundary signs and the mean shift (on a fully periodic grid the
-        // operator annihilates the shift, so raw values are used there)
-        const A sd = r == 0 ? A(sylo) : A(1), su = r == TY - 1 ? A(syhi) : A(1);
-#pragma unroll
-        for(int t = 0; t < CPT; ++t) {
-          dn[t] = sd * (dn[t] - sin);
-          up[t] = su * (up[t] - sin);
-        }
-        left = A(sxl) * (left - sin);
-        right = A(sxr) * (right - sin);
-      }
-      double bq[CPT];
-      if constexpr(CPT == 4) {
-        tload4<double>(bk + r * NX + i0, bq);
-      } else {
-#pragma unroll
-        for(int t = 0; t < CPT; ++t) bq[t] = double(bk[r * NX + i0 + t]);
-      }
-      const int cz = 16 * axis_class(k, NZ);
-      A v[CPT];
-#pragma unroll
-      for(int t = 0; t < CPT; ++t) {
-        const double bd = bq[t] - sb;
-        const A l = t > 0 ? cen[t - 1] : left;
-        const A rr = t < CPT - 1 ? cen[t + 1] : right;
-        const A two_c = A(2) * cen[t];
-        const A ax = -(rr - two_c + l) * ix - (up[t] - two_c + dn[t]) * iy - (above[t] - two_c + below[t]) * iz;
-        if constexpr(PER)
-          v[t] = (cen[t] - sin) + om * (A(bd) - ax) * A(invd_s[0]);
-        else
-          v[t] = cen[t] + om * (A(bd) - ax) * A(invd_s[cls[t] + cz]);
-        acc[0] += double(v[t]);
-        acc[1] += bd * double(v[t]);
-      }
-      if constexpr(CPT == 4) {
-        tstore4<T>(out + o.L.idx(i0, j, k), v);
-      } else if constexpr(std::is_same_v<T, double>) {
-        *reinterpret_cast<double2*>(out + o.L.idx(i0, j, k)) = make_double2(v[0], v[1]);
-      } else {
-        *reinterpret_cast<float2*>(out + o.L.idx(i0, j, k)) = make_float2(v[0], v[1]);
-      }
-    };
-    A q0[CPT], q1[CPT], q2[CPT], q3[CPT];
-    own(sg.lbase, q0);
-    own(sg.lbase + 1, q1);
-    __syncthreads();
-    // two planes per step (one when a single plane is left)
-    for(int k = sg.kb; k < sg.ke;) {
-      const int c = sg.lbase + 1 + (k - sg.kb);  // load of plane k
-      const bool two = k + 1 < sg.ke;
-      if(threadIdx.x == 0) {
-        tma::fence_proxy_async();
-        while(next < nload && next <= c - 1 + D) issue(next++);
-      }
-      own(c + 1, q2);
-      if(two) own(c + 2, q3);
-      plane(k, c, q0, q1, q2);
-      if(two) plane(k + 1, c + 1, q1, q2, q3);
-#pragma unroll
-      for(int t = 0; t < CPT; ++t) {
-        q0[t] = two ? q2[t] : q1[t];
-        q1[t] = two ? q3[t] : q2[t];
-      }
-      k += two ? 2 : 1;
-      __syncthreads();
-    }
-  }
-  const bool mx[2] = {false, false};
-  const int n = o.L.count();
-  reduce_finish<2>(acc, mx, rb, [=](const Sums<2>& st) {
-    const double mean = zm ? st.v[0] / n : 0.0;
-    ls->sx = mean;
-    ls->sum_x = st.v[0];
-    if(sc != nullptr) {
-      const double rz_new = st.v[1] - mean * (sc->sum_r - sc->n * sc->sr);
-      if(sc->first) {
-        sc->rz = rz_new;
-      } else {
-        sc->beta = rz_new / sc->rz;
-        sc->rz = rz_new;
-      }
-    }
-  });
-}
-
-// Both pre-smoothing sweeps from a zero correction on the plane pipeline
-// (same contract as k_vsmooth_pre): the staged operand is b itself, and the
-// first sweep's a = omega (b - sb) / D is formed on read for every stencil
-// point, with the diagonal of the point's boundary image.  Warp-specialised:
-// 1024 / CPT consumer threads and one producer warp that issues the TMA loads;
-// each consumer warp releases a slot through an mbarrier when it has read it,
-// so there is no block barrier per plane (at 256^3: 65.5 -> 60.7 us FP64,
-// 45 -> 43 us FP32 per launch).
-template <typename T, typename B, int CPT, bool PER>
-__global__ void __launch_bounds__(1024 / CPT + 32)
-    k_tsmooth_pre(OpInfo o, const __grid_constant__ CUtensorMap bm, const __grid_constant__ CUtensorMap bh,
-                  const double* sb_ptr, T* __restrict__ out, LevelScalars* ls, int zm, RedBuf rb,
-                  int* fault) {
-  pdl_enter();
-  using A = T;
-  constexpr int D = kTSlots;
-  extern __shared__ __align__(128) unsigned char tsm[];
-  __shared__ uint64_t bars[D], empt[D];  // slot loaded / slot released
-  __shared__ A invd_s[64];
-  using L = std::conditional_t<std::is_same_v<T, float>, float, double>;  // loaded rhs values
-  const int NX = o.L.nx, NY = o.L.ny, NZ = o.L.nz;
-  const int TY = 1024 / NX;
-  const int tpr = NX / CPT;
-  const int r = threadIdx.x / tpr;
-  const int i0 = (threadIdx.x % tpr) * CPT;
-  const size_t sbytes = tround(static_cast<size_t>(TY + 2) * NX * sizeof(B));
-  const uint32_t tx_bytes = static_cast<uint32_t>((TY + 2) * NX * sizeof(B));
-  auto slot = [&](int s) { return reinterpret_cast<B*>(tsm + s * sbytes); };
-  TSeg seg[kTMaxSeg];
-  int nload = 0;
-  const int nseg = tsegments(NY / TY, NZ, seg, nload);
-  auto issue = [&](int l) {
-    int q = 0;
-    while(q + 1 < nseg && seg[q + 1].lbase <= l) ++q;
-    const int j0 = seg[q].tile * TY;
-    int jm, jp;
-    double sg;
-    nb_lo(j0, NY, o.periodic[1], o.dir_lo[1], jm, sg);
-    nb_hi(j0 + TY - 1, NY, o.periodic[1], o.dir_hi[1], jp, sg);
-    const int kz = vst::zrow(seg[q].kb - 1 + (l - seg[q].lbase), NZ, o.periodic[2], o.dir_lo[2],
-                             o.dir_hi[2], sg);
-    const int sl = l % D;
-    tma::mbar_arrive_expect_tx(&bars[sl], tx_bytes);
-    tma::load_3d(slot(sl) + NX, &bm, &bars[sl], 0, j0, kz);
-    tma::load_3d(slot(sl), &bh, &bars[sl], 0, jm, kz);
-    tma::load_3d(slot(sl) + (TY + 1) * NX, &bh, &bars[sl], 0, jp, kz);
-  };
-  constexpr int NC = 1024 / CPT;  // consumer threads; the warp after them is the producer
-  if(threadIdx.x == 0) {
-    for(int sl = 0; sl < D; ++sl) {
-      tma::mbar_init(&bars[sl], 1);
-      tma::mbar_init(&empt[sl], NC / 32);
-    }
-    tma::fence_barrier_init();
-  }
-  if(threadIdx.x < 64) invd_s[threadIdx.x] = A(o.invd[threadIdx.x]);
-  __syncthreads();
-  const double sb = *sb_ptr;
-  const A om = A(kOmega);
-  const A ix = A(o.inv2[0]), iy = A(o.inv2[1]), iz = A(o.inv2[2]);
-  auto ldrow = [&](const B* p, L (&v)[CPT]) {
-    if constexpr(CPT == 4) {
-      tload4<L, B, std::is_same_v<B, double>>(p, v);
-    } else {
-#pragma unroll
-      for(int t = 0; t < CPT; ++t) v[t] = L(p[t]);
-    }
-  };
-  double acc[1] = {0.0};
-  int xl, xr;
-  double sxl, sxr;
-  nb_lo(i0, NX, o.periodic[0], o.dir_lo[0], xl, sxl);
-  nb_hi(i0 + CPT - 1, NX, o.periodic[0], o.dir_hi[0], xr, sxr);
-  // a consumer warp releases slot l once its lanes have read it
-  auto release = [&](int l) {
-    __syncwarp();
-    if((threadIdx.x & 31) == 0) tma::mbar_arrive(&empt[l % D]);
-  };
-  if(threadIdx.x >= NC) {
-    // producer: load l goes into slot l % D once every consumer warp has
-    // released load l - D there (bounded waits, as for the loads)
-    if(threadIdx.x == NC) {
-      for(int l = 0; l < nload; ++l) {
-        if(l >= D) tma::mbar_wait(&empt[l % D], ((l / D) - 1) & 1, fault, 1);
-        issue(l);
-      }
-    }
-  } else
-  for(int q = 0; q < nseg; ++q) {
-    const TSeg sg = seg[q];
-    const int j0 = sg.tile * TY;
-    const int j = j0 + r;
-    int jm, jp;
-    double sylo, syhi;
-    nb_lo(j0, NY, o.periodic[1], o.dir_lo[1], jm, sylo);
-    nb_hi(j0 + TY - 1, NY, o.periodic[1], o.dir_hi[1], jp, syhi);
-    // boundary classes (x + 4 y) of the own cells and of their in-plane neighbours' images
-    const int jd = r == 0 ? jm : j - 1, ju = r == TY - 1 ? jp : j + 1;
-    const A sd = r == 0 ? A(sylo) : A(1), su = r == TY - 1 ? A(syhi) : A(1);
-    int cown[CPT], cdn[CPT], cup[CPT];
-#pragma unroll
-    for(int t = 0; t < CPT; ++t) {
-      const int cx = axis_class(i0 + t, NX);
-      cown[t] = cx + 4 * axis_class(j, NY);
-      cdn[t] = cx + 4 * axis_class(jd, NY);
-      cup[t] = cx + 4 * axis_class(ju, NY);
-    }
-    const int cl = axis_class(xl, NX) + 4 * axis_class(j, NY);
-    const int cr = axis_class(xr, NX) + 4 * axis_class(j, NY);
-    // a of the own cells at load l (its plane's image and sign)
-    auto own = [&](int l, A (&v)[CPT]) {
-      tma::mbar_wait(&bars[l % D], (l / D) & 1, fault, 1);
-      double zs;
-      const int kz = vst::zrow(sg.kb - 1 + (l - sg.lbase), NZ, o.periodic[2], o.dir_lo[2], o.dir_hi[2], zs);
-      const int cz = 16 * axis_class(kz, NZ);
-      L b[CPT];
-      ldrow(slot(l % D) + (r + 1) * NX + i0, b);
-      if constexpr(PER) {
-        // raw b: the operator annihilates the constant omega sb / D
-#pragma unroll
-        for(int t = 0; t < CPT; ++t) v[t] = A(b[t]);
-      } else {
-#pragma unroll
-        for(int t = 0; t < CPT; ++t) v[t] = A(zs) * om * A(b[t] - L(sb)) * A(invd_s[cown[t] + cz]);
-      }
-    };
-    A below[CPT], cen[CPT], above[CPT];
-    own(sg.lbase, below);
-    release(sg.lbase);
-    own(sg.lbase + 1, cen);
-    for(int k = sg.kb; k < sg.ke; ++k) {
-      const int c = sg.lbase + 1 + (k - sg.kb);
-      own(c + 1, above);
-      const B* pk = slot(c % D);
-      const int cz = 16 * axis_class(k, NZ);
-      L bd[CPT], bu[CPT], bc[CPT];
-      ldrow(pk + r * NX + i0, bd);
-      ldrow(pk + (r + 2) * NX + i0, bu);
-      ldrow(pk + (r + 1) * NX + i0, bc);
-      A dn[CPT], up[CPT], left, right;
-      if constexpr(PER) {
-#pragma unroll
-        for(int t = 0; t < CPT; ++t) {
-          dn[t] = A(bd[t]);
-          up[t] = A(bu[t]);
-        }
-        left = A(pk[(r + 1) * NX + xl]);
-        right = A(pk[(r + 1) * NX + xr]);
-      } else {
-#pragma unroll
-        for(int t = 0; t < CPT; ++t) {
-          dn[t] = sd * om * A(bd[t] - L(sb)) * A(invd_s[cdn[t] + cz]);
-          up[t] = su * om * A(bu[t] - L(sb)) * A(invd_s[cup[t] + cz]);
-        }
-        left = A(sxl) * om * A(L(pk[(r + 1) * NX + xl]) - L(sb)) * A(invd_s[cl + cz]);
-        right = A(sxr) * om * A(L(pk[(r + 1) * NX + xr]) - L(sb)) * A(invd_s[cr + cz]);
-      }
-      A v[CPT];
-      A ps0 = A(0);  // FP32: per-plane partial sum
-      const A w0 = om * A(invd_s[0]);
-#pragma unroll
-      for(int t = 0; t < CPT; ++t) {
-        const A l = t > 0 ? cen[t - 1] : left;
-        const A rr = t < CPT - 1 ? cen[t + 1] : right;
-        const A two_c = A(2) * cen[t];
-        const A ax = -(rr - two_c + l) * ix - (up[t] - two_c + dn[t]) * iy - (above[t] - two_c + below[t]) * iz;
-        if constexpr(PER) {
-          // a = w (b - sb) on every point, so A a = w A b
-          const A bcs = A(bc[t] - L(sb));
-          v[t] = w0 * bcs + w0 * (bcs - w0 * ax);
-        } else {
-          v[t] = cen[t] + om * (A(bc[t] - L(sb)) - ax) * A(invd_s[cown[t] + cz]);
-        }
-        if constexpr(std::is_same_v<T, float>) ps0 += v[t];
-        else acc[0] += double(v[t]);
-      }
-      if constexpr(std::is_same_v<T, float>) acc[0] += double(ps0);
-      if constexpr(CPT == 4) {
-        tstore4<T>(out + o.L.idx(i0, j, k), v);
-      } else if constexpr(std::is_same_v<T, double>) {
-        *reinterpret_cast<double2*>(out + o.L.idx(i0, j, k)) = make_double2(v[0], v[1]);
-      } else {
-        *reinterpret_cast<float2*>(out + o.L.idx(i0, j, k)) = make_float2(v[0], v[1]);
-      }
-#pragma unroll
-      for(int t = 0; t < CPT; ++t) {
-        below[t] = cen[t];
-        cen[t] = above[t];
-      }
-      release(c);
-    }
-    release(sg.lbase + 1 + (sg.ke - sg.kb));
-  }
-  const bool mx[1] = {false};
-  const int n = o.L.count();
-  reduce_finish<1>(acc, mx, rb, [=](const Sums<1>& st) {
-    ls->sx = zm ? st.v[0] / n : 0.0;
-    ls->sum_x = st.v[0];
-  });
-}
-
-// Prolongation + first post-smoothing sweep on the plane pipeline (same
-// contract as k_vprolong_smooth, 2x2x2 coarsening): the staged operand is the
-// level's correction x and the coarse correction ec (parent rows and the
-// parents of the halo rows), combined on read as (x - sx) + (ec - sec).
-template <typename T, typename B, int CPT, int D, bool PER>
-__global__ void __launch_bounds__(1024 / CPT)
-    k_tprolong(OpInfo o, const __grid_constant__ CUtensorMap xm, const __grid_constant__ CUtensorMap xh,
-               const __grid_constant__ CUtensorMap bm, const __grid_constant__ CUtensorMap em,
-               const __grid_constant__ CUtensorMap eh, const double* sb_ptr, const double* sin_ptr,
-               const double* sec_ptr, T* __restrict__ out, LevelScalars* ls, int zm, RedBuf rb,
-               int* fault) {
-  pdl_enter();
-  using A = T;
-  extern __shared__ __align__(128) unsigned char tsm[];
-  __shared__ uint64_t bars[D];
-  __shared__ A invd_s[64];
-  using L = std::conditional_t<std::is_same_v<T, float>, float, double>;  // loaded rhs values
-  const int NX = o.L.nx, NY = o.L.ny, NZ = o.L.nz;
-  const int NXc = NX / 2, NZc = NZ / 2;
-  const int TY = 1024 / NX;
-  const int TYc = TY / 2;
-  const int tpr = NX / CPT;
-  const int r = threadIdx.x / tpr;
-  const int i0 = (threadIdx.x % tpr) * CPT;
-  const size_t xbytes = tround(static_cast<size_t>(TY + 2) * NX * sizeof(T));
-  const size_t bbytes = tround(static_cast<size_t>(TY) * NX * sizeof(B));
-  const size_t ebytes = tround(static_cast<size_t>(TYc + 2) * NXc * sizeof(T));
-  const size_t sbytes = xbytes + bbytes + ebytes;
-  const uint32_t tx_bytes = static_cast<uint32_t>((TY + 2) * NX * sizeof(T) + TY * NX * sizeof(B) +
-                                                  (TYc + 2) * NXc * sizeof(T));
-  auto xslot = [&](int s) { return reinterpret_cast<T*>(tsm + s * sbytes); };
-  auto bslot = [&](int s) { return reinterpret_cast<B*>(tsm + s * sbytes + xbytes); };
-  auto eslot = [&](int s) { return reinterpret_cast<T*>(tsm + s * sbytes + xbytes + bbytes); };
-  TSeg seg[kTMaxSeg];
-  int nload = 0;
-  const int nseg = tsegments(NY / TY, NZ, seg, nload);
-  auto issue = [&](int l) {
-    int q = 0;
-    while(q + 1 < nseg && seg[q + 1].lbase <= l) ++q;
-    const int j0 = seg[q].tile * TY;
-    int jm, jp;
-    double sg;
-    nb_lo(j0, NY, o.periodic[1], o.dir_lo[1], jm, sg);
-    nb_hi(j0 + TY - 1, NY, o.periodic[1], o.dir_hi[1], jp, sg);
-    const int kz = vst::zrow(seg[q].kb - 1 + (l - seg[q].lbase), NZ, o.periodic[2], o.dir_lo[2],
-                             o.dir_hi[2], sg);
-    const int sl = l % D;
-    tma::mbar_arrive_expect_tx(&bars[sl], tx_bytes);
-    tma::load_3d(xslot(sl) + NX, &xm, &bars[sl], 0, j0, kz);
-    tma::load_3d(xslot(sl), &xh, &bars[sl], 0, jm, kz);
-    tma::load_3d(xslot(sl) + (TY + 1) * NX, &xh, &bars[sl], 0, jp, kz);
-    tma::load_3d(bslot(sl), &bm, &bars[sl], 0, j0, kz);
-    tma::load_3d(eslot(sl) + NXc, &em, &bars[sl], 0, j0 >> 1, kz >> 1);
-    tma::load_3d(eslot(sl), &eh, &bars[sl], 0, jm >> 1, kz >> 1);
-    tma::load_3d(eslot(sl) + (TYc + 1) * NXc, &eh, &bars[sl], 0, jp >> 1, kz >> 1);
-  };
-  (void)NZc;
-  if(threadIdx.x == 0) {
-    for(int sl = 0; sl < D; ++sl) tma::mbar_init(&bars[sl], 1);
-    tma::fence_barrier_init();
-  }
-  if(threadIdx.x < 64) invd_s[threadIdx.x] = A(o.invd[threadIdx.x]);
-  __syncthreads();
-  int next = 0;
-  if(threadIdx.x == 0)
-    while(next < nload && next < D) issue(next++);
-  const double sb = *sb_ptr;
-  const A sin = A(*sin_ptr);
-  const A sec = A(*sec_ptr);
-  const A om = A(kOmega);
-  const A ix = A(o.inv2[0]), iy = A(o.inv2[1]), iz = A(o.inv2[2]);
-  // fine slot row (0 .. TY+1) -> coarse slot row of its parent
-  auto crow = [&](int fr) { return fr == 0 ? 0 : (fr == TY + 1 ? TYc + 1 : ((fr - 1) >> 1) + 1); };
-  // combined operand of the CPT cells at fine slot row fr (shifted, unsigned)
-  // (on a fully periodic grid the shifts are left out: the operator
-  // annihilates constants, and only the centre value needs them)
-  const A shx = PER ? A(0) : sin, she = PER ? A(0) : sec;
-  auto operand = [&](const T* xs, const T* es, int fr, A (&v)[CPT]) {
-    A xv[CPT];
-    tload4<A>(xs + fr * NX + i0, xv);
-    const T* erow = es + crow(fr) * NXc + (i0 >> 1);
-    const A e0 = A(erow[0]) - she, e1 = A(erow[1]) - she;
-    v[0] = (xv[0] - shx) + e0;
-    v[1] = (xv[1] - shx) + e0;
-    v[2] = (xv[2] - shx) + e1;
-    v[3] = (xv[3] - shx) + e1;
-  };
-  double acc[1] = {0.0};
-  int xl, xr;
-  double sxl, sxr;
-  nb_lo(i0, NX, o.periodic[0], o.dir_lo[0], xl, sxl);
-  nb_hi(i0 + CPT - 1, NX, o.periodic[0], o.dir_hi[0], xr, sxr);
-  for(int q = 0; q < nseg; ++q) {
-    const TSeg sg = seg[q];
-    const int j0 = sg.tile * TY;
-    const int j = j0 + r;
-    int jm, jp;
-    double sylo, syhi;
-    nb_lo(j0, NY, o.periodic[1], o.dir_lo[1], jm, sylo);
-    nb_hi(j0 + TY - 1, NY, o.periodic[1], o.dir_hi[1], jp, syhi);
-    int cls[CPT];
-#pragma unroll
-    for(int t = 0; t < CPT; ++t) cls[t] = axis_class(i0 + t, NX) + 4 * axis_class(j, NY);
-    auto own = [&](int l, A (&v)[CPT]) {
-      tma::mbar_wait(&bars[l % D], (l / D) & 1, fault, 1);
-      double zs;
-      vst::zrow(sg.kb - 1 + (l - sg.lbase), NZ, o.periodic[2], o.dir_lo[2], o.dir_hi[2], zs);
-      operand(xslot(l % D), eslot(l % D), r + 1, v);
-      if constexpr(!PER) {
-#pragma unroll
-        for(int t = 0; t < CPT; ++t) v[t] *= A(zs);
-      }
-    };
-    A below[CPT], cen[CPT], above[CPT];
-    own(sg.lbase, below);
-    own(sg.lbase + 1, cen);
-    __syncthreads();
-    for(int k = sg.kb; k < sg.ke; ++k) {
-      const int c = sg.lbase + 1 + (k - sg.kb);
-      if(threadIdx.x == 0) {
-        tma::fence_proxy_async();
-        while(next < nload && next <= c - 1 + D) issue(next++);
-      }
-      own(c + 1, above);
-      const T* xs = xslot(c % D);
-      const T* es = eslot(c % D);
-      const B* bk = bslot(c % D);
-      A dn[CPT], up[CPT];
-      operand(xs, es, r, dn);
-      operand(xs, es, r + 2, up);
-      if constexpr(!PER) {
-        const A sd = r == 0 ? A(sylo) : A(1), su = r == TY - 1 ? A(syhi) : A(1);
-#pragma unroll
-        for(int t = 0; t < CPT; ++t) {
-          dn[t] *= sd;
-          up[t] *= su;
-        }
-      }
-      const T* erow = es + crow(r + 1) * NXc;
-      A left = (A(xs[(r + 1) * NX + xl]) - shx) + (A(erow[xl >> 1]) - she);
-      A right = (A(xs[(r + 1) * NX + xr]) - shx) + (A(erow[xr >> 1]) - she);
-      if constexpr(!PER) {
-        left *= A(sxl);
-        right *= A(sxr);
-      }
-      L bq[CPT];
-      tload4<L>(bk + r * NX + i0, bq);
-      const int cz = 16 * axis_class(k, NZ);
-      A v[CPT];
-      A ps0 = A(0);  // FP32: per-plane partial sum
-#pragma unroll
-      for(int t = 0; t < CPT; ++t) {
-        const A l = t > 0 ? cen[t - 1] : left;
-        const A rr = t < CPT - 1 ? cen[t + 1] : right;
-        const A two_c = A(2) * cen[t];
-        const A ax = -(rr - two_c + l) * ix - (up[t] - two_c + dn[t]) * iy - (above[t] - two_c + below[t]) * iz;
-        if constexpr(PER)
-          v[t] = (cen[t] - sin - sec) + om * (A(bq[t] - L(sb)) - ax) * A(invd_s[0]);
-        else
-          v[t] = cen[t] + om * (A(bq[t] - L(sb)) - ax) * A(invd_s[cls[t] + cz]);
-        if constexpr(std::is_same_v<T, float>) ps0 += v[t];
-        else acc[0] += double(v[t]);
-      }
-      if constexpr(std::is_same_v<T, float>) acc[0] += double(ps0);
-      tstore4<T>(out + o.L.idx(i0, j, k), v);
-#pragma unroll
-      for(int t = 0; t < CPT; ++t) {
-        below[t] = cen[t];
-        cen[t] = above[t];
-      }
-      __syncthreads();
-    }
-  }
-  const bool mx[1] = {false};
-  const int n = o.L.count();
-  reduce_finish<1>(acc, mx, rb, [=](const Sums<1>& st) { ls->sa = zm ? st.v[0] / n : 0.0; });
-}
-
-// A p on the plane pipeline (same contract as k_vapply_ap).
-template <typename V, int CPT, bool PER>
-__global__ void __launch_bounds__(1024 / CPT)
-    k_tap(OpInfo o, const __grid_constant__ CUtensorMap pm, const __grid_constant__ CUtensorMap ph,
-          V* __restrict__ ap, SolveScalars* sc, RedBuf rb, int* fault) {
-  pdl_enter();
-  constexpr int D = kTSlots;
-  extern __shared__ __align__(128) unsigned char tsm[];
-  __shared__ uint64_t bars[D];
-  const int NX = o.L.nx, NY = o.L.ny, NZ = o.L.nz;
-  const int TY = 1024 / NX;
-  const int tpr = NX / CPT;
-  const int r = threadIdx.x / tpr;
-  const int i0 = (threadIdx.x % tpr) * CPT;
-  const size_t sbytes = tround(static_cast<size_t>(TY + 2) * NX * sizeof(V));
-  const uint32_t tx_bytes = static_cast<uint32_t>((TY + 2) * NX * sizeof(V));
-  auto slot = [&](int s) { return reinterpret_cast<V*>(tsm + s * sbytes); };
-  TSeg seg[kTMaxSeg];
-  int nload = 0;
-  const int nseg = tsegments(NY / TY, NZ, seg, nload);
-  auto issue = [&](int l) {
-    int q = 0;
-    while(q + 1 < nseg && seg[q + 1].lbase <= l) ++q;
-    const int j0 = seg[q].tile * TY;
-    int jm, jp;
-    double sg;
-    nb_lo(j0, NY, o.periodic[1], o.dir_lo[1], jm, sg);
-    nb_hi(j0 + TY - 1, NY, o.periodic[1], o.dir_hi[1], jp, sg);
-    const int kz = vst::zrow(seg[q].kb - 1 + (l - seg[q].lbase), NZ, o.periodic[2], o.dir_lo[2],
-                             o.dir_hi[2], sg);
-    const int sl = l % D;
-    tma::mbar_arrive_expect_tx(&bars[sl], tx_bytes);
-    tma::load_3d(slot(sl) + NX, &pm, &bars[sl], 0, j0, kz);
-    tma::load_3d(slot(sl), &ph, &bars[sl], 0, jm, kz);
-    tma::load_3d(slot(sl) + (TY + 1) * NX, &ph, &bars[sl], 0, jp, kz);
-  };
-  if(threadIdx.x == 0) {
-    for(int sl = 0; sl < D; ++sl) tma::mbar_init(&bars[sl], 1);
-    tma::fence_barrier_init();
-  }
-  __syncthreads();
-  int next = 0;
-  if(threadIdx.x == 0)
-    while(next < nload && next < D) issue(next++);
-  const double sp = sc->sp;
-  const double ix = o.inv2[0], iy = o.inv2[1], iz = o.inv2[2];
-  double acc[3] = {0.0, 0.0, 0.0};
-  int xl, xr;
-  double sxl, sxr;
-  nb_lo(i0, NX, o.periodic[0], o.dir_lo[0], xl, sxl);
-  nb_hi(i0 + CPT - 1, NX, o.periodic[0], o.dir_hi[0], xr, sxr);
-  for(int q = 0; q < nseg; ++q) {
-    const TSeg sg = seg[q];
-    const int j0 = sg.tile * TY;
-    const int j = j0 + r;
-    int jm, jp;
-    double sylo, syhi;
-    nb_lo(j0, NY, o.periodic[1], o.dir_lo[1], jm, sylo);
-    nb_hi(j0 + TY - 1, NY, o.periodic[1], o.dir_hi[1], jp, syhi);
-    auto own = [&](int l, double (&v)[CPT]) {
-      tma::mbar_wait(&bars[l % D], (l / D) & 1, fault, 1);
-      double zs;
-      vst::zrow(sg.kb - 1 + (l - sg.lbase), NZ, o.periodic[2], o.dir_lo[2], o.dir_hi[2], zs);
-      tload4<double>(slot(l % D) + (r + 1) * NX + i0, v);
-      if constexpr(!PER) {
-#pragma unroll
-        for(int t = 0; t < CPT; ++t) v[t] = zs * (v[t] - sp);
-      }
-    };
-    double below[CPT], cen[CPT], above[CPT];
-    own(sg.lbase, below);
-    own(sg.lbase + 1, cen);
-    __syncthreads();
-    for(int k = sg.kb; k < sg.ke; ++k) {
-      const int c = sg.lbase + 1 + (k - sg.kb);
-      if(threadIdx.x == 0) {
-        tma::fence_proxy_async();
-        while(next < nload && next <= c - 1 + D) issue(next++);
-      }
-      own(c + 1, above);
-      const V* pk = slot(c % D);
-      double dn[CPT], up[CPT];
-      tload4<double>(pk + r * NX + i0, dn);
-      tload4<double>(pk + (r + 2) * NX + i0, up);
-      double left = double(pk[(r + 1) * NX + xl]), right = double(pk[(r + 1) * NX + xr]);
-      if constexpr(!PER) {
-        const double sd = r == 0 ? sylo : 1.0, su = r == TY - 1 ? syhi : 1.0;
-#pragma unroll
-        for(int t = 0; t < CPT; ++t) {
-          dn[t] = sd * (dn[t] - sp);
-          up[t] = su * (up[t] - sp);
-        }
-        left = sxl * (left - sp);
-        right = sxr * (right - sp);
-      }
-      double v[CPT];
-#pragma unroll
-      for(int t = 0; t < CPT; ++t) {
-        const double l = t > 0 ? cen[t - 1] : left;
-        const double rr = t < CPT - 1 ? cen[t + 1] : right;
-        const double two_c = 2.0 * cen[t];
-        v[t] = -(rr - two_c + l) * ix - (up[t] - two_c + dn[t]) * iy - (above[t] - two_c + below[t]) * iz;
-        const double cs = PER ? cen[t] - sp : cen[t];
-        acc[0] += v[t];
-        acc[1] += cs * v[t];
-        acc[2] += cs;
-      }
-      tstore4<V>(ap + o.L.idx(i0, j, k), v);
-#pragma unroll
-      for(int t = 0; t < CPT; ++t) {
-        below[t] = cen[t];
-        cen[t] = above[t];
-      }
-      __syncthreads();
-    }
-  }
-  const bool mx[3] = {false, false, false};
-  reduce_finish<3>(acc, mx, rb, [=](const Sums<3>& st) {
-    const double sap = sc->zero_mean ? st.v[0] / sc->n : 0.0;
-    sc->sap = sap;
-    const double pap = st.v[1] - sap * st.v[2];
-    sc->pap = pap;
-    if(fabs(pap) < kSmallNumber) {
-      sc->stop = 1;
-    } else {
-      sc->alpha = sc->rz / pap;
-    }
-  });
-}
-
-// Fused CG step on the plane pipeline: p = (z - sz) + beta (p_old - sp_old)
-// (p = z - sz on the first body), A p, and the previous iteration's deferred
-// solution update x = (x - sx) + alpha_old (p_old - sp_old)
-// (linsolve/poisson_solver.cpp:762-766, one body later).  The staged operand
-// is z + beta p_old: the operator annihilates the mean shifts wherever they
-// are nonzero (periodic / all-Neumann problems).  Records sp, sap, pap and
-// alpha as k_update_p and k_apply_ap do, and mean(x).
-// Ring depth of k_tpap: its registers allow two blocks per SM, so FP32
-// planes (half the bytes) get twice the slots to keep as many bytes in flight.
-template <typename V>
-constexpr int tpap_slots() {
-  return 4;
-}
-
-template <typename T, typename V, bool PER>
-__global__ void __launch_bounds__(256)
-    k_tpap(OpInfo o, const __grid_constant__ CUtensorMap zm_, const __grid_constant__ CUtensorMap zh,
-           const __grid_constant__ CUtensorMap pm0, const __grid_constant__ CUtensorMap ph0,
-           const __grid_constant__ CUtensorMap pm1, const __grid_constant__ CUtensorMap ph1,
-           const LevelScalars* ls0, V* p0, V* p1, V* __restrict__ ap, V* __restrict__ x,
-           SolveScalars* sc, RedBuf rb, int* fault) {
-  pdl_enter();
-  using A = V;  // arithmetic of the vector type: FP64, or FP32 on the mixed path's inner solve
-  constexpr int CPT = 4;
-  constexpr int D = tpap_slots<V>();
-  extern __shared__ __align__(128) unsigned char tsm[];
-  __shared__ uint64_t bars[D];
-  const int NX = o.L.nx, NY = o.L.ny, NZ = o.L.nz;
-  const int TY = 1024 / NX;
-  const int tpr = NX / CPT;
-  const int r = threadIdx.x / tpr;
-  const int i0 = (threadIdx.x % tpr) * CPT;
-  const size_t zbytes = tround(static_cast<size_t>(TY + 2) * NX * sizeof(T));
-  const size_t sbytes = zbytes + tround(static_cast<size_t>(TY + 2) * NX * sizeof(V));
-  const uint32_t tx_bytes = static_cast<uint32_t>((TY + 2) * NX * (sizeof(T) + sizeof(V)));
-  auto zslot = [&](int s) { return reinterpret_cast<T*>(tsm + s * sbytes); };
-  auto pslot = [&](int s) { return reinterpret_cast<V*>(tsm + s * sbytes + zbytes); };
-  // p ping-pongs between two buffers: body b reads p_old from buffer
-  // (b + 1) & 1 and writes p to buffer b & 1 (other blocks still read p_old)
-  const int par = sc->body_runs & 1;
-  const CUtensorMap* pm = par ? &pm0 : &pm1;
-  const CUtensorMap* ph = par ? &ph0 : &ph1;
-  V* p_out = par ? p1 : p0;
-  TSeg seg[kTMaxSeg];
-  int nload = 0;
-  const int nseg = tsegments(NY / TY, NZ, seg, nload);
-  auto issue = [&](int l) {
-    int q = 0;
-    while(q + 1 < nseg && seg[q + 1].lbase <= l) ++q;
-    const int j0 = seg[q].tile * TY;
-    int jm, jp;
-    double sg;
-    nb_lo(j0, NY, o.periodic[1], o.dir_lo[1], jm, sg);
-    nb_hi(j0 + TY - 1, NY, o.periodic[1], o.dir_hi[1], jp, sg);
-    const int kz = vst::zrow(seg[q].kb - 1 + (l - seg[q].lbase), NZ, o.periodic[2], o.dir_lo[2],
-                             o.dir_hi[2], sg);
-    const int sl = l % D;
-    tma::mbar_arrive_expect_tx(&bars[sl], tx_bytes);
-    tma::load_3d(zslot(sl) + NX, &zm_, &bars[sl], 0, j0, kz);
-    tma::load_3d(zslot(sl), &zh, &bars[sl], 0, jm, kz);
-    tma::load_3d(zslot(sl) + (TY + 1) * NX, &zh, &bars[sl], 0, jp, kz);
-    tma::load_3d(pslot(sl) + NX, pm, &bars[sl], 0, j0, kz);
-    tma::load_3d(pslot(sl), ph, &bars[sl], 0, jm, kz);
-    tma::load_3d(pslot(sl) + (TY + 1) * NX, ph, &bars[sl], 0, jp, kz);
-  };
-  if(threadIdx.x == 0) {
-    for(int sl = 0; sl < D; ++sl) tma::mbar_init(&bars[sl], 1);
-    tma::fence_barrier_init();
-  }
-  __syncthreads();
-  int next = 0;
-  if(threadIdx.x == 0)
-    while(next < nload && next < D) issue(next++);
-  const int first = sc->first;
-  const A beta = A(first ? 0.0 : sc->beta);
-  const A sz = A(ls0->sx), spo = A(sc->sp);
-  const A alpha_old = A(sc->alpha), sx = A(sc->sx);
-  const A ix = A(o.inv2[0]), iy = A(o.inv2[1]), iz = A(o.inv2[2]);
-  // raw operand z + beta p_old of the 4 cells at slot row fr
-  auto operand = [&](int sl, int fr, A (&v)[CPT]) {
-    A zv[CPT], pv[CPT];
-    tload4<A>(zslot(sl) + fr * NX + i0, zv);
-    tload4<A>(pslot(sl) + fr * NX + i0, pv);
-#pragma unroll
-    for(int t = 0; t < CPT; ++t) v[t] = zv[t] + beta * pv[t];
-  };
-  auto point = [&](int sl, int fr, int ii) {
-    return A(zslot(sl)[fr * NX + ii]) + beta * A(pslot(sl)[fr * NX + ii]);
-  };
-  double acc[4] = {0.0, 0.0, 0.0, 0.0};
-  int xl, xr;
-  double sxl, sxr;
-  nb_lo(i0, NX, o.periodic[0], o.dir_lo[0], xl, sxl);
-  nb_hi(i0 + CPT - 1, NX, o.periodic[0], o.dir_hi[0], xr, sxr);
-  for(int q = 0; q < nseg; ++q) {
-    const TSeg sg = seg[q];
-    const int j0 = sg.tile * TY;
-    const int j = j0 + r;
-    int jm, jp;
-    double sylo, syhi;
-    nb_lo(j0, NY, o.periodic[1], o.dir_lo[1], jm, sylo);
-    nb_hi(j0 + TY - 1, NY, o.periodic[1], o.dir_hi[1], jp, syhi);
-    auto own = [&](int l, A (&v)[CPT]) {
-      tma::mbar_wait(&bars[l % D], (l / D) & 1, fault, 1);
-      operand(l % D, r + 1, v);
-      if constexpr(!PER) {
-        double zs;
-        vst::zrow(sg.kb - 1 + (l - sg.lbase), NZ, o.periodic[2], o.dir_lo[2], o.dir_hi[2], zs);
-#pragma unroll
-        for(int t = 0; t < CPT; ++t) v[t] *= A(zs);
-      }
-    };
-    A below[CPT], cen[CPT], above[CPT];
-    own(sg.lbase, below);
-    own(sg.lbase + 1, cen);
-    // x of the own cells one plane ahead (plain loads, prefetched a step early)
-    A xn[CPT] = {A(0), A(0), A(0), A(0)};
-    if(!first) tload4<A>(x + o.L.idx(i0, j, sg.kb), xn);
-    __syncthreads();
-    for(int k = sg.kb; k < sg.ke; ++k) {
-      const int c = sg.lbase + 1 + (k - sg.kb);
-      if(threadIdx.x == 0) {
-        tma::fence_proxy_async();
-        while(next < nload && next <= c - 1 + D) issue(next++);
-      }
-      own(c + 1, above);
-      const int sl = c % D;
-      A dn[CPT], up[CPT];
-      operand(sl, r, dn);
-      operand(sl, r + 2, up);
-      A left = point(sl, r + 1, xl), right = point(sl, r + 1, xr);
-      if constexpr(!PER) {
-        const A sd = A(r == 0 ? sylo : 1.0), su = A(r == TY - 1 ? syhi : 1.0);
-#pragma unroll
-        for(int t = 0; t < CPT; ++t) {
-          dn[t] *= sd;
-          up[t] *= su;
-        }
-        left *= A(sxl);
-        right *= A(sxr);
-      }
-      // own cells: exact p (with shifts), the deferred x update
-      A zc[CPT], pc[CPT];
-      tload4<A>(zslot(sl) + (r + 1) * NX + i0, zc);
-      tload4<A>(pslot(sl) + (r + 1) * NX + i0, pc);
-      A pn[CPT], apv[CPT];
-#pragma unroll
-      for(int t = 0; t < CPT; ++t) {
-        const A l = t > 0 ? cen[t - 1] : left;
-        const A rr = t < CPT - 1 ? cen[t + 1] : right;
-        const A two_c = A(2) * cen[t];
-        apv[t] = -(rr - two_c + l) * ix - (up[t] - two_c + dn[t]) * iy - (above[t] - two_c + below[t]) * iz;
-        pn[t] = first ? zc[t] - sz : (zc[t] - sz) + beta * (pc[t] - spo);
-      }
-      const size_t gq = o.L.idx(i0, j, k);
-      tstore4<V>(p_out + gq, pn);
-      tstore4<V>(ap + gq, apv);
-      if(!first) {
-        A xv[CPT];
-#pragma unroll
-        for(int t = 0; t < CPT; ++t) xv[t] = xn[t];
-        if(k + 1 < sg.ke) tload4<A>(x + o.L.idx(i0, j, k + 1), xn);
-#pragma unroll
-        for(int t = 0; t < CPT; ++t) {
-          xv[t] = (xv[t] - sx) + alpha_old * (pc[t] - spo);
-          acc[3] += double(xv[t]);
-        }
-        tstore4<V>(x + gq, xv);
-      }
-#pragma unroll
-      for(int t = 0; t < CPT; ++t) {
-        acc[0] += double(pn[t]);
-        acc[1] += double(apv[t]);
-        acc[2] += double(pn[t]) * double(apv[t]);
-        below[t] = cen[t];
-        cen[t] = above[t];
-      }
-      __syncthreads();
-    }
-  }
-  const bool mx[4] = {false, false, false, false};
-  reduce_finish<4>(acc, mx, rb, [=](const Sums<4>& st) {
-    const int n = sc->n;
-    const int zmn = sc->zero_mean;
-    const double sp = zmn ? st.v[0] / n : 0.0;
-    const double sap = zmn ? st.v[1] / n : 0.0;
-    sc->sp = sp;
-    sc->sap = sap;
-    if(!first) sc->sx = zmn ? st.v[3] / n : 0.0;
-    sc->first = 0;
-    const double pap = st.v[2] - sp * st.v[1] - sap * st.v[0] + n * sp * sap;
-    sc->pap = pap;
-    if(fabs(pap) < kSmallNumber) {
-      sc->stop = 1;
-    } else {
-      sc->alpha = sc->rz / pap;
-    }
-  });
-}
-
-// r = (r - sr) - alpha (Ap - sap), its norm and the convergence test: the
-// residual half of k_update_xr for the fused CG step (x is updated one body
-// later by k_tpap, and after the loop by k_x_final).  The compact vector is
-// one contiguous array, so it is swept flat, 16 bytes per load (float4 /
-// double2) with kFlatUnroll loads of each operand in flight per thread.
-constexpr int kFlatUnroll = 4;
-constexpr int kFlatThreads = 256;
-
-template <typename V>
-struct Vec16;
-template <>
-struct Vec16<float> {
-  using T = float4;
-  static constexpr int W = 4;
-};
-template <>
-struct Vec16<double> {
-  using T = double2;
-  static constexpr int W = 2;
-};
-
-template <typename V>
-__global__ void __launch_bounds__(kFlatThreads)
-    k_update_r_flat(int n, V* __restrict__ r, const V* __restrict__ ap, SolveScalars* sc, RedBuf rb,
-                    cudaGraphConditionalHandle cond) {
-  pdl_enter();
-  using VT = typename Vec16<V>::T;
-  constexpr int W = Vec16<V>::W;
-  const int stop = sc->stop;
-  const double alpha = sc->alpha, sr = sc->sr, sap = sc->sap;
-  double acc[2];
-  zero(acc);
-  if(!stop) {
-    const int nv = n / W;
-    const int stride = gridDim.x * blockDim.x;
-    VT* rv = reinterpret_cast<VT*>(r);
-    const VT* av = reinterpret_cast<const VT*>(ap);
-    for(int base = blockIdx.x * blockDim.x + threadIdx.x; base < nv; base += kFlatUnroll * stride) {
-      VT rr[kFlatUnroll], aa[kFlatUnroll];
-#pragma unroll
-      for(int u = 0; u < kFlatUnroll; ++u) {
-        const int q = base + u * stride;
-        if(q < nv) {
-          rr[u] = rv[q];
-          aa[u] = av[q];
-        }
-      }
-#pragma unroll
-      for(int u = 0; u < kFlatUnroll; ++u) {
-        const int q = base + u * stride;
-        if(q < nv) {
-          V* rs = reinterpret_cast<V*>(&rr[u]);
-          const V* as = reinterpret_cast<const V*>(&aa[u]);
-#pragma unroll
-          for(int w = 0; w < W; ++w) {
-            const double v = (double(rs[w]) - sr) - alpha * (double(as[w]) - sap);
-            rs[w] = V(v);
-            acc[0] += v;
-            acc[1] += v * v;
-          }
-          rv[q] = rr[u];
-        }
-      }
-    }
-    // the n % W elements past the last full vector
-    for(int q = nv * W + blockIdx.x * blockDim.x + threadIdx.x; q < n; q += stride) {
-      const double v = (double(r[q]) - sr) - alpha * (double(ap[q]) - sap);
-      r[q] = V(v);
-      acc[0] += v;
-      acc[1] += v * v;
-    }
-  }
-  const bool mx[2] = {false, false};
-  reduce_finish<2>(acc, mx, rb, [=](const Sums<2>& s) {
-    sc->body_runs += 1;
-    if(sc->stop) {
-      sc->cont = 0;
-      if(cond) cudaGraphSetConditional(cond, 0);
-      return;
-    }
-    const int nn = sc->n;
-    const int zm = sc->zero_mean;
-    const double srn = zm ? s.v[0] / nn : 0.0;
-    sc->sr = srn;
-    sc->sum_r = s.v[0];
-    const double ss = fmax(s.v[1] - nn * srn * srn, 0.0);
-    sc->rnorm = sqrt(ss / nn);
-    sc->iterations += 1;
-    sc->rel = sc->r0 > 0.0 ? sc->rnorm / sc->r0 : 0.0;
-    if(sc->rel <= sc->tol) sc->converged = 1;
-    if(sc->hist != nullptr && sc->iterations < sc->hist_cap) sc->hist[sc->iterations] = sc->rnorm;
-    sc->cont = (sc->converged || sc->iterations >= sc->max_it) ? 0 : 1;
-    if(cond) cudaGraphSetConditional(cond, sc->cont);
-  });
-}
-
-// After a fused-step loop: the last deferred update x = (x - sx) + alpha (p - sp)
-// unless the loop stopped on a vanishing p.Ap (then the reference skips it).
-template <typename V>
-__global__ void __launch_bounds__(kTX* kTY)
-    k_x_final(CLay L, V* __restrict__ x, const V* p0, const V* p1, SolveScalars* sc, int kchunk, RedBuf rb) {
-  STENCIL_PROLOGUE(L)
-  const int skip = sc->stop || sc->body_runs == 0;
-  const V* __restrict__ p = ((sc->body_runs - 1) & 1) ? p1 : p0;
-  const double alpha = sc->alpha, sx = sc->sx, sp = sc->sp;
-  double acc[1];
-  zero(acc);
-  if(valid && !skip) {
-    for(int k = k0; k < k1; ++k) {
-      const int q = L.idx(i, j, k);
-      const double v = (double(x[q]) - sx) + alpha * (double(p[q]) - sp);
-      x[q] = V(v);
-      acc[0] += v;
-    }
-  }
-  const bool mx[1] = {false};
-  reduce_finish<1>(acc, mx, rb, [=](const Sums<1>& s) {
-    if(!skip) sc->sx = sc->zero_mean ? s.v[0] / sc->n : 0.0;
-  });
-}
-
-// Residual + 2x2x2 restriction on the plane pipeline (same contract as
-// k_vrestrict): each step forms the residual (b - sb) - A (x - sx) on the two
-// fine planes of one coarse plane; a thread sums its cells pairwise in x and
-// over the two planes, and the row pairs are combined through shared memory.
-// The schedule runs over coarse planes, so each segment streams fine planes
-// 2 kc_begin - 1 .. 2 kc_end.
-template <typename T, typename B, int D, bool PER>
-__global__ void __launch_bounds__(256)
-    k_trestrict(OpInfo o, OpInfo oc, const __grid_constant__ CUtensorMap xm,
-                const __grid_constant__ CUtensorMap xh, const __grid_constant__ CUtensorMap bm,
-                const double* sb_ptr, const double* sin_ptr, T* __restrict__ bc, LevelScalars* lsc,
-                int zm, RedBuf rb, int* fault) {
-  pdl_enter();
-  using A = T;
-  constexpr int CPT = 4;
-  extern __shared__ __align__(128) unsigned char tsm[];
-  __shared__ uint64_t bars[D];
-  const int NX = o.L.nx, NY = o.L.ny, NZ = o.L.nz;
-  const int TY = 1024 / NX;
-  const int tpr = NX / CPT;
-  const int r = threadIdx.x / tpr;
-  const int i0 = (threadIdx.x % tpr) * CPT;
-  const size_t ubytes = tround(static_cast<size_t>(TY + 2) * NX * sizeof(T));
-  const size_t sbytes = tslot_bytes<T, B>(NX);
-  const uint32_t tx_bytes = static_cast<uint32_t>((TY + 2) * NX * sizeof(T) + TY * NX * sizeof(B));
-  auto uslot = [&](int s) { return reinterpret_cast<T*>(tsm + s * sbytes); };
-  auto bslot = [&](int s) { return reinterpret_cast<B*>(tsm + s * sbytes + ubytes); };
-  A* part = reinterpret_cast<A*>(tsm + D * sbytes);  // [TY][NX / 2] row partials
-  // segments over coarse planes; loads count fine planes
-  TSeg seg[kTMaxSeg];
-  int nseg = 0, nload = 0;
-  if(gridDim.x % (NY / TY) == 0) {
-    // z-aligned schedule over coarse planes (as in tsegments)
-    const int tiles = NY / TY, nzc = NZ / 2, nch = gridDim.x / tiles;
-    const int tile = blockIdx.x % tiles, zc = blockIdx.x / tiles;
-    const int kb = static_cast<int>(static_cast<long long>(nzc) * zc / nch);
-    const int ke = static_cast<int>(static_cast<long long>(nzc) * (zc + 1) / nch);
-    if(ke > kb) {
-      seg[nseg++] = TSeg{tile, kb, ke, 0};
-      nload = 2 * (ke - kb) + 2;
-    }
-  } else {
-    const int nzc = NZ / 2;
-    const long long total = static_cast<long long>(NY / TY) * nzc;
-    const long long f0 = total * blockIdx.x / gridDim.x;
-    const long long f1 = total * (blockIdx.x + 1) / gridDim.x;
-    for(long long f = f0; f < f1 && nseg < kTMaxSeg;) {
-      const int tile = static_cast<int>(f / nzc);
-      const int kb = static_cast<int>(f % nzc);
-      const int ke = static_cast<int>(min(static_cast<long long>(nzc), kb + (f1 - f)));
-      seg[nseg++] = TSeg{tile, kb, ke, nload};
-      nload += 2 * (ke - kb) + 2;
-      f += ke - kb;
-    }
-  }
-  auto fine_plane = [&](const TSeg& sg, int l) { return 2 * sg.kb - 1 + (l - sg.lbase); };
-  auto issue = [&](int l) {
-    int q = 0;
-    while(q + 1 < nseg && seg[q + 1].lbase <= l) ++q;
-    const int j0 = seg[q].tile * TY;
-    int jm, jp;
-    double sg;
-    nb_lo(j0, NY, o.periodic[1], o.dir_lo[1], jm, sg);
-    nb_hi(j0 + TY - 1, NY, o.periodic[1], o.dir_hi[1], jp, sg);
-    const int kz = vst::zrow(fine_plane(seg[q], l), NZ, o.periodic[2], o.dir_lo[2], o.dir_hi[2], sg);
-    const int sl = l % D;
-    tma::mbar_arrive_expect_tx(&bars[sl], tx_bytes);
-    tma::load_3d(uslot(sl) + NX, &xm, &bars[sl], 0, j0, kz);
-    tma::load_3d(uslot(sl), &xh, &bars[sl], 0, jm, kz);
-    tma::load_3d(uslot(sl) + (TY + 1) * NX, &xh, &bars[sl], 0, jp, kz);
-    tma::load_3d(bslot(sl), &bm, &bars[sl], 0, j0, kz);
-  };
-  if(threadIdx.x == 0) {
-    for(int sl = 0; sl < D; ++sl) tma::mbar_init(&bars[sl], 1);
-    tma::fence_barrier_init();
-  }
-  __syncthreads();
-  int next = 0;
-  if(threadIdx.x == 0)
-    while(next < nload && next < D) issue(next++);
-  const double sb = *sb_ptr;
-  const A sin = A(*sin_ptr);
-  const A ix = A(o.inv2[0]), iy = A(o.inv2[1]), iz = A(o.inv2[2]);
-  double acc[1] = {0.0};
-  int xl, xr;
-  double sxl, sxr;
-  nb_lo(i0, NX, o.periodic[0], o.dir_lo[0], xl, sxl);
-  nb_hi(i0 + CPT - 1, NX, o.periodic[0], o.dir_hi[0], xr, sxr);
-  for(int q = 0; q < nseg; ++q) {
-    const TSeg sg = seg[q];
-    const int j0 = sg.tile * TY;
-    const int j = j0 + r;
-    int jm, jp;
-    double sylo, syhi;
-    nb_lo(j0, NY, o.periodic[1], o.dir_lo[1], jm, sylo);
-    nb_hi(j0 + TY - 1, NY, o.periodic[1], o.dir_hi[1], jp, syhi);
-    auto own = [&](int l, A (&v)[CPT]) {
-      tma::mbar_wait(&bars[l % D], (l / D) & 1, fault, 1);
-      double zs;
-      vst::zrow(fine_plane(sg, l), NZ, o.periodic[2], o.dir_lo[2], o.dir_hi[2], zs);
-      tload4<A>(uslot(l % D) + (r + 1) * NX + i0, v);
-      if constexpr(!PER) {
-#pragma unroll
-        for(int t = 0; t < CPT; ++t) v[t] = A(zs) * (v[t] - sin);
-      }
-    };
-    // residual of the CPT cells at the plane staged in load c
-    auto residual = [&](int c, const A (&below)[CPT], const A (&cen)[CPT], const A (&above)[CPT],
-                        A (&res)[CPT]) {
-      const T* pk = uslot(c % D);
-      const B* bk = bslot(c % D);
-      A dn[CPT], up[CPT];
-      tload4<A>(pk + r * NX + i0, dn);
-      tload4<A>(pk + (r + 2) * NX + i0, up);
-      A left = pk[(r + 1) * NX + xl], right = pk[(r + 1) * NX + xr];
-      if constexpr(!PER) {
-        const A sd = r == 0 ? A(sylo) : A(1), su = r == TY - 1 ? A(syhi) : A(1);
-#pragma unroll
-        for(int t = 0; t < CPT; ++t) {
-          dn[t] = sd * (dn[t] - sin);
-          up[t] = su * (up[t] - sin);
-        }
-        left = A(sxl) * (left - sin);
-        right = A(sxr) * (right - sin);
-      }
-      double bq[CPT];
-      tload4<double>(bk + r * NX + i0, bq);
-#pragma unroll
-      for(int t = 0; t < CPT; ++t) {
-        const A l = t > 0 ? cen[t - 1] : left;
-        const A rr = t < CPT - 1 ? cen[t + 1] : right;
-        const A two_c = A(2) * cen[t];
-        const A ax = -(rr - two_c + l) * ix - (up[t] - two_c + dn[t]) * iy - (above[t] - two_c + below[t]) * iz;
-        res[t] = A(bq[t] - sb) - ax;
-      }
-    };
-    A q0[CPT], q1[CPT], q2[CPT], q3[CPT];
-    own(sg.lbase, q0);
-    own(sg.lbase + 1, q1);
-    __syncthreads();
-    for(int kc = sg.kb; kc < sg.ke; ++kc) {
-      const int c = sg.lbase + 1 + 2 * (kc - sg.kb);  // load of fine plane 2 kc
-      if(threadIdx.x == 0) {
-        tma::fence_proxy_async();
-        while(next < nload && next <= c - 1 + D) issue(next++);
-      }
-      own(c + 1, q2);
-      own(c + 2, q3);
-      A r0[CPT], r1[CPT];
-      residual(c, q0, q1, q2, r0);
-      residual(c + 1, q1, q2, q3, r1);
-      part[r * (NX / 2) + (i0 >> 1)] = (r0[0] + r0[1]) + (r1[0] + r1[1]);
-      part[r * (NX / 2) + (i0 >> 1) + 1] = (r0[2] + r0[3]) + (r1[2] + r1[3]);
-#pragma unroll
-      for(int t = 0; t < CPT; ++t) {
-        q0[t] = q2[t];
-        q1[t] = q3[t];
-      }
-      __syncthreads();
-      if((r & 1) == 0) {
-        const int m = i0 >> 1;
-        const A c0 = A(0.125) * (part[r * (NX / 2) + m] + part[(r + 1) * (NX / 2) + m]);
-        const A c1 = A(0.125) * (part[r * (NX / 2) + m + 1] + part[(r + 1) * (NX / 2) + m + 1]);
-        T* dst = bc + oc.L.idx(m, j >> 1, kc);
-        if constexpr(std::is_same_v<T, double>) {
-          *reinterpret_cast<double2*>(dst) = make_double2(c0, c1);
-        } else {
-          *reinterpret_cast<float2*>(dst) = make_float2(c0, c1);
-        }
-        acc[0] += double(c0) + double(c1);
-      }
-      __syncthreads();
-    }
-  }
-  const bool mx[1] = {false};
-  const int n = oc.L.count();
-  reduce_finish<1>(acc, mx, rb, [=](const Sums<1>& st) { lsc->sb = zm ? st.v[0] / n : 0.0; });
-}
 
 // ---------------------------------------------------------------------------
 // The small end of the hierarchy as one matrix.  From the first level of at
@@ -2434,135 +584,6 @@ __global__ void __launch_bounds__(kTX* kTY)
   });
 }
 
-// p = (z - sz) + beta (p - sp); first iteration p = z - sz.
-template <typename T, typename V>
-__global__ void __launch_bounds__(kTX* kTY)
-    k_update_p(CLay L, const T* __restrict__ z, const LevelScalars* ls0, V* __restrict__ p,
-               SolveScalars* sc, int kchunk, RedBuf rb) {
-  pdl_enter();
-  STENCIL_PROLOGUE(L)
-  const int first = sc->first;
-  const double sz = ls0->sx;
-  const double beta = first ? 0.0 : sc->beta;
-  const double sp = sc->sp;
-  double acc[1];
-  zero(acc);
-  if(valid) {
-    k_batched<kBatch>(
-        k0, k1,
-        [&](int k) {
-          const int q = L.idx(i, j, k);
-          return first ? double(z[q]) - sz : (double(z[q]) - sz) + beta * (double(p[q]) - sp);
-        },
-        [&](int k, double v) {
-          p[L.idx(i, j, k)] = V(v);
-          acc[0] += v;
-        });
-  }
-  const bool mx[1] = {false};
-  reduce_finish<1>(acc, mx, rb, [=](const Sums<1>& s) {
-    sc->sp = sc->zero_mean ? s.v[0] / sc->n : 0.0;
-    sc->first = 0;
-  });
-}
-
-// Ap = A (p - sp); mean shift of Ap; p.Ap; alpha (linsolve/poisson_solver.cpp:751-761).
-template <typename V>
-__global__ void __launch_bounds__(kTX* kTY)
-    k_apply_ap(OpInfo o, const V* __restrict__ p, V* __restrict__ ap, SolveScalars* sc,
-               int kchunk, RedBuf rb) {
-  pdl_enter();
-  STENCIL_PROLOGUE(o.L)
-  const double sp = sc->sp;
-  double acc[3];
-  zero(acc);
-  if(valid) {
-    const ColNb nb = col_nb(o, i, j);
-    auto val = [&](int ii, int jj, int kk) { return double(p[o.L.idx(ii, jj, kk)]) - sp; };
-    k_batched<kBatch>(
-        k0, k1,
-        [&](int k) {
-          double c;
-          const double v = apply_op<double>(o, nb, i, j, k, val, c);
-          return Pair<double>{v, c};
-        },
-        [&](int k, Pair<double> r) {
-          ap[o.L.idx(i, j, k)] = V(r.v);
-          acc[0] += r.v;
-          acc[1] += r.w * r.v;
-          acc[2] += r.w;
-        });
-  }
-  const bool mx[3] = {false, false, false};
-  reduce_finish<3>(acc, mx, rb, [=](const Sums<3>& s) {
-    const double sap = sc->zero_mean ? s.v[0] / sc->n : 0.0;
-    sc->sap = sap;
-    const double pap = s.v[1] - sap * s.v[2];
-    sc->pap = pap;
-    if(fabs(pap) < kSmallNumber) {
-      sc->stop = 1;
-    } else {
-      sc->alpha = sc->rz / pap;
-    }
-  });
-}
-
-// x = (x - sx) + alpha (p - sp); r = (r - sr) - alpha (Ap - sap); norms and
-// the convergence test (linsolve/poisson_solver.cpp:762-782).
-template <typename V>
-__global__ void __launch_bounds__(kTX* kTY)
-    k_update_xr(CLay L, V* __restrict__ x, V* __restrict__ r,
-                const V* __restrict__ p, const V* __restrict__ ap, SolveScalars* sc,
-                int kchunk, RedBuf rb, cudaGraphConditionalHandle cond) {
-  pdl_enter();
-  STENCIL_PROLOGUE(L)
-  const int stop = sc->stop;
-  const double alpha = sc->alpha, sx = sc->sx, sr = sc->sr, sp = sc->sp, sap = sc->sap;
-  double acc[3];
-  zero(acc);
-  if(valid && !stop) {
-    k_batched<kBatch>(
-        k0, k1,
-        [&](int k) {
-          const int q = L.idx(i, j, k);
-          return Pair<double>{(double(x[q]) - sx) + alpha * (double(p[q]) - sp),
-                              (double(r[q]) - sr) - alpha * (double(ap[q]) - sap)};
-        },
-        [&](int k, Pair<double> v) {
-          const int q = L.idx(i, j, k);
-          x[q] = V(v.v);
-          r[q] = V(v.w);
-          acc[0] += v.v;
-          acc[1] += v.w;
-          acc[2] += v.w * v.w;
-        });
-  }
-  const bool mx[3] = {false, false, false};
-  reduce_finish<3>(acc, mx, rb, [=](const Sums<3>& s) {
-    sc->body_runs += 1;
-    if(sc->stop) {
-      sc->cont = 0;
-      if(cond) cudaGraphSetConditional(cond, 0);
-      return;
-    }
-    const int n = sc->n;
-    const int zm = sc->zero_mean;
-    sc->sx = zm ? s.v[0] / n : 0.0;
-    const double srn = zm ? s.v[1] / n : 0.0;
-    sc->sr = srn;
-    sc->sum_r = s.v[1];
-    const double ss = fmax(s.v[2] - n * srn * srn, 0.0);
-    sc->rnorm = sqrt(ss / n);
-    sc->iterations += 1;
-    sc->rel = sc->r0 > 0.0 ? sc->rnorm / sc->r0 : 0.0;
-    if(sc->rel <= sc->tol) sc->converged = 1;
-    if(sc->hist != nullptr && sc->iterations < sc->hist_cap) sc->hist[sc->iterations] = sc->rnorm;
-    // the reference's loop: at most max_iterations iterations, stop on convergence
-    sc->cont = (sc->converged || sc->iterations >= sc->max_it) ? 0 : 1;
-    if(cond) cudaGraphSetConditional(cond, sc->cont);
-  });
-}
-
 // Mixed path: the FP64 residual scaled to unit RMS into the FP32 inner rhs,
 // the inner correction cleared, and the inner loop's scalars initialised the
 // way k_initial_residual does it for a zero initial guess.
@@ -2601,7 +622,6 @@ __global__ void __launch_bounds__(kTX* kTY)
     si->first = 1;
     si->body_runs = 0;
     si->sx = 0.0;
-    si->sp = 0.0;
     si->hist = nullptr;
     si->hist_cap = 0;
     si->cont = r0 > 0.0 ? 1 : 0;
@@ -2707,11 +727,6 @@ struct Level {
   int rx = 1, ry = 1, rz = 1;  // refinement ratio to the next coarser level
   march::Tile tile{};          // of k_descend and k_ascend
   dim3 tgrid;
-  // plane-pipeline (TMA) maps: a (main rows, one halo row) and the rhs
-  bool tma = false;
-  CUtensorMap tm_am, tm_ah, tm_bm, tm_bh;
-  bool tma_prolong = false;  // 2x2x2 coarsening: correction x and the coarse result
-  CUtensorMap tm_xm, tm_xh, tm_em, tm_eh;
 };
 
 struct PoissonPlan {
@@ -2735,11 +750,10 @@ struct PoissonPlan {
   // mixed path: inner (FP32) CG vectors and scalars
   float *r32 = nullptr, *e32 = nullptr, *p32 = nullptr, *ap32 = nullptr;
   SolveScalars* sc_in = nullptr;
-  int* fault = nullptr;  // device: a bounded wait in a plane-pipelined kernel gave up
   int sms = 148;         // streaming multiprocessors of the plan's device
-  bool tma_ap = false;   // plane-pipelined A p on the finest level
   bool all_periodic = false;  // every face periodic: constant diagonal, no boundary signs
-  CUtensorMap tm_pm, tm_ph, tm_pm2, tm_ph2;
+  march::Tile cg_tile{};      // of k_direction and k_advance
+  dim3 cg_grid;
   double* p2 = nullptr;     // second p buffer of the fused CG step
   float* p32b = nullptr;
   // levels tail_first.. run as one matrix-vector product (k_dense_apply)
@@ -2972,91 +986,6 @@ void setup_dense(PoissonPlan* P, const int* swaps, const double* factors) {
   throw std::invalid_argument("the coarsest multigrid level does not fit the dense solve");
 }
 
-// Tensor maps of the plane-pipelined kernels for every level above the
-// single-block tail whose rows fit one TMA box (nx of 64, 128 or 256) and
-// whose row tiles divide ny.  ORCHARD_B200_NO_TMA=1 keeps the row kernels.
-bool tma_fits(const CLay& L) {
-  if(L.nx != 64 && L.nx != 128 && L.nx != 256) return false;
-  const int ty = 1024 / L.nx;
-  return L.ny % ty == 0 && L.nz >= 1;
-}
-
-void setup_tma(PoissonPlan* P, size_t tsz) {
-  const char* e = std::getenv("ORCHARD_B200_NO_TMA");
-  if(e != nullptr && e[0] == '1') return;
-  const int nl = static_cast<int>(P->levels.size());
-  const int last = P->tail_first >= 0 ? P->tail_first : nl - 1;
-  for(int l = 0; l < last; ++l) {
-    Level& lv = P->levels[l];
-    if(!tma_fits(lv.L)) continue;
-    const int ty = 1024 / lv.L.nx;
-    const int es = static_cast<int>(tsz);
-    lv.tm_am = tma::make_map_3d(lv.a, es, lv.L.nx, lv.L.ny, lv.L.nz, lv.L.nx, ty);
-    lv.tm_ah = tma::make_map_3d(lv.a, es, lv.L.nx, lv.L.ny, lv.L.nz, lv.L.nx, 1);
-    // the finest level's rhs is the CG residual: FP64, or FP32 on the mixed path
-    const void* bp = l > 0 ? lv.b : (P->precision == 1 ? static_cast<const void*>(P->r32) : P->r);
-    const int bes = l > 0 ? es : (P->precision == 1 ? 4 : 8);
-    lv.tm_bm = tma::make_map_3d(bp, bes, lv.L.nx, lv.L.ny, lv.L.nz, lv.L.nx, ty);
-    lv.tm_bh = tma::make_map_3d(bp, bes, lv.L.nx, lv.L.ny, lv.L.nz, lv.L.nx, 1);
-    lv.tma = true;
-    if(lv.rx == 2 && lv.ry == 2 && lv.rz == 2 && l + 1 < nl) {
-      const Level& cv = P->levels[l + 1];
-      lv.tm_xm = tma::make_map_3d(lv.x, es, lv.L.nx, lv.L.ny, lv.L.nz, lv.L.nx, ty);
-      lv.tm_xh = tma::make_map_3d(lv.x, es, lv.L.nx, lv.L.ny, lv.L.nz, lv.L.nx, 1);
-      lv.tm_em = tma::make_map_3d(cv.x, es, cv.L.nx, cv.L.ny, cv.L.nz, cv.L.nx, ty / 2);
-      lv.tm_eh = tma::make_map_3d(cv.x, es, cv.L.nx, cv.L.ny, cv.L.nz, cv.L.nx, 1);
-      lv.tma_prolong = true;
-    }
-    if(l == 0) {
-      const void* pp = P->precision == 1 ? static_cast<const void*>(P->p32) : P->p;
-      const void* pp2 = P->precision == 1 ? static_cast<const void*>(P->p32b) : P->p2;
-      const int pes = P->precision == 1 ? 4 : 8;
-      P->tm_pm = tma::make_map_3d(pp, pes, lv.L.nx, lv.L.ny, lv.L.nz, lv.L.nx, ty);
-      P->tm_ph = tma::make_map_3d(pp, pes, lv.L.nx, lv.L.ny, lv.L.nz, lv.L.nx, 1);
-      P->tm_pm2 = tma::make_map_3d(pp2, pes, lv.L.nx, lv.L.ny, lv.L.nz, lv.L.nx, ty);
-      P->tm_ph2 = tma::make_map_3d(pp2, pes, lv.L.nx, lv.L.ny, lv.L.nz, lv.L.nx, 1);
-      P->tma_ap = true;
-    }
-  }
-  auto attr = [](const void* fn, size_t bytes) {
-    OFB_CHECK(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(bytes)));
-  };
-  attr(reinterpret_cast<const void*>(k_tprolong<double, double, 4, 4, false>), tprolong_bytes<double, double>(256) * 4);
-  attr(reinterpret_cast<const void*>(k_tprolong<double, double, 4, 4, true>), tprolong_bytes<double, double>(256) * 4);
-  attr(reinterpret_cast<const void*>(k_tprolong<float, float, 4, 4, false>), tprolong_bytes<float, float>(256) * 4);
-  attr(reinterpret_cast<const void*>(k_tprolong<float, float, 4, 4, true>), tprolong_bytes<float, float>(256) * 4);
-  attr(reinterpret_cast<const void*>(k_tpap<double, double, false>), tround(6 * 256 * 8) * 2 * 4);
-  attr(reinterpret_cast<const void*>(k_tpap<double, double, true>), tround(6 * 256 * 8) * 2 * 4);
-  attr(reinterpret_cast<const void*>(k_tpap<float, float, false>), tround(6 * 256 * 4) * 2 * tpap_slots<float>());
-  attr(reinterpret_cast<const void*>(k_tpap<float, float, true>), tround(6 * 256 * 4) * 2 * tpap_slots<float>());
-  attr(reinterpret_cast<const void*>(k_tap<double, 4, false>), tround(static_cast<size_t>(6) * 256 * 8) * kTSlots);
-  attr(reinterpret_cast<const void*>(k_tap<double, 4, true>), tround(static_cast<size_t>(6) * 256 * 8) * kTSlots);
-  attr(reinterpret_cast<const void*>(k_tap<float, 4, false>), tround(static_cast<size_t>(6) * 256 * 4) * kTSlots);
-  attr(reinterpret_cast<const void*>(k_tap<float, 4, true>), tround(static_cast<size_t>(6) * 256 * 4) * kTSlots);
-  attr(reinterpret_cast<const void*>(k_trestrict<double, double, kTSlots, false>),
-       tslot_bytes<double, double>(256) * kTSlots + 4 * 128 * 8);
-  attr(reinterpret_cast<const void*>(k_trestrict<double, double, kTSlots, true>),
-       tslot_bytes<double, double>(256) * kTSlots + 4 * 128 * 8);
-  attr(reinterpret_cast<const void*>(k_trestrict<float, float, kTSlots, false>),
-       tslot_bytes<float, float>(256) * kTSlots + 4 * 128 * 4);
-  attr(reinterpret_cast<const void*>(k_trestrict<float, float, kTSlots, true>),
-       tslot_bytes<float, float>(256) * kTSlots + 4 * 128 * 4);
-  // the largest slot is that of nx = 256 (TY = 4): (TY + 2 + TY) rows of 256
-  for(const void* fn : {reinterpret_cast<const void*>(k_tsmooth<double, double, 4, false>),
-                         reinterpret_cast<const void*>(k_tsmooth<double, double, 4, true>)})
-    attr(fn, tslot_bytes<double, double>(256) * kTSlots);
-  for(const void* fn : {reinterpret_cast<const void*>(k_tsmooth<float, float, 4, false>),
-                         reinterpret_cast<const void*>(k_tsmooth<float, float, 4, true>)})
-    attr(fn, tslot_bytes<float, float>(256) * kTSlots);
-  for(const void* fn : {reinterpret_cast<const void*>(k_tsmooth_pre<double, double, 4, false>),
-                         reinterpret_cast<const void*>(k_tsmooth_pre<double, double, 4, true>)})
-    attr(fn, tslot_bytes<double, double>(256) * kTSlots);
-  for(const void* fn : {reinterpret_cast<const void*>(k_tsmooth_pre<float, float, 4, false>),
-                         reinterpret_cast<const void*>(k_tsmooth_pre<float, float, 4, true>)})
-    attr(fn, tslot_bytes<float, float>(256) * kTSlots);
-
-}
-
 // The instantiation for the plan's boundary conditions: sign images where a
 // face is Dirichlet, one diagonal value where every face is periodic.
 template <typename T>
@@ -3083,6 +1012,20 @@ auto ascend_kernel(const PoissonPlan* P, bool flat, bool fine, bool pairs) {
   return pairs ? ascend_kernel_of<T, false, true>(P, flat) : ascend_kernel_of<T, false, false>(P, flat);
 }
 
+template <typename T>
+auto direction_kernel(const PoissonPlan* P, bool flat) {
+  using namespace march;
+  if(!P->zero_mean) return flat ? k_direction<T, true, true> : k_direction<T, true, false>;
+  return flat ? k_direction<T, false, true> : k_direction<T, false, false>;
+}
+
+template <typename T>
+auto advance_kernel(const PoissonPlan* P, bool flat) {
+  using namespace march;
+  if(!P->zero_mean) return flat ? k_advance<T, true, true> : k_advance<T, true, false>;
+  return flat ? k_advance<T, false, true> : k_advance<T, false, false>;
+}
+
 constexpr int kMarchSmem = 224 * 1024;
 
 // Lets every instantiation use the largest tile's shared memory.
@@ -3093,6 +1036,8 @@ void march_attributes(const PoissonPlan* P) {
   };
   for(const bool flat : {false, true}) {
     attr(descend_kernel<T>(P, flat));
+    attr(direction_kernel<T>(P, flat));
+    attr(advance_kernel<T>(P, flat));
     for(const bool fine : {false, true})
       for(const bool pairs : {false, true}) attr(ascend_kernel<T>(P, flat, fine, pairs));
   }
@@ -3109,8 +1054,9 @@ void march_attributes(const PoissonPlan* P) {
 constexpr double kPlaneLatency = 500.0, kThreadCycles = 2.0;
 
 template <typename T>
-void plan_tile(const CLay& L, int rz, int streams, int sms, march::Tile& best, dim3& grid) {
-  constexpr int W = march::kW<T>, halo_rows = 2;
+void plan_tile(const CLay& L, int halo_rows, int rz, int streams, int fields, int sms, march::Tile& best,
+               dim3& grid) {
+  constexpr int W = march::kW<T>;
   auto even = [](int v) { return (v + 1) / 2 * 2; };
   const bool flat = L.nz == 1;
   double best_cost = 0.0;
@@ -3134,7 +1080,7 @@ void plan_tile(const CLay& L, int rz, int streams, int sms, march::Tile& best, d
       last_iy = t.iy;
       t.ey = t.iy + 2 * halo_rows;
       const int threads = t.px * t.ey / 2;
-      const size_t smem = march::smem_bytes<T>(t, streams);
+      const size_t smem = march::smem_bytes<T>(t, streams, fields);
       if(smem > kMarchSmem) continue;
       const int resident = std::min<int>({march::kMaxThreads / ((threads + 31) / 32 * 32),
                                           static_cast<int>(228 * 1024 / (smem + 2048)), 16});
@@ -3303,15 +1249,13 @@ PoissonPlan* poisson_plan_create(const Grid& g, const PBC& pbc_in, int precision
     OFB_CHECK(cudaGetDevice(&dev));
     OFB_CHECK(cudaDeviceGetAttribute(&P->sms, cudaDevAttrMultiProcessorCount, dev));
   }
-  OFB_CHECK(cudaMalloc(&P->fault, sizeof(int)));
-  OFB_CHECK(cudaMemset(P->fault, 0, sizeof(int)));
   P->all_periodic = true;
   for(int f = 0; f < 6; ++f)
     if(P->pbc.type[f] != kPPeriodic) P->all_periodic = false;
   for(int l = 0; l < P->tail_first; ++l)
-    (precision == 1 ? plan_tile<float> : plan_tile<double>)(P->levels[l].L, P->levels[l].rz, 2, P->sms,
+    (precision == 1 ? plan_tile<float> : plan_tile<double>)(P->levels[l].L, 2, P->levels[l].rz, 2, 2, P->sms,
                                                             P->levels[l].tile, P->levels[l].tgrid);
-  setup_tma(P, tsz);
+  (precision == 1 ? plan_tile<float> : plan_tile<double>)(P->levels[0].L, 1, 1, 3, 1, P->sms, P->cg_tile, P->cg_grid);
   if(precision == 1) march_attributes<float>(P);
   else march_attributes<double>(P);
   const char* no_graph = std::getenv("ORCHARD_B200_NO_GRAPH");
@@ -3343,7 +1287,6 @@ void poisson_plan_destroy(PoissonPlan* P) {
   cudaFree(P->p2);
   cudaFree(P->p32b);
   cudaFree(P->sc_in);
-  cudaFree(P->fault);
   cudaFree(P->dense);
   delete P;
 }
@@ -3355,80 +1298,6 @@ double* poisson_b(PoissonPlan* P) { return P->b; }
 double* poisson_x(PoissonPlan* P) { return P->x; }
 
 namespace {
-
-template <typename T, typename B, int RX, int RY, int RZ>
-void launch_restrict_r(const Level& lv, const Level& cv, const B* b, const double* sb_ptr,
-                       const T* x, const double* sx_ptr, T* bc, LevelScalars* lsc, int zm,
-                       const Launch3& lc, RedBuf rb, cudaStream_t s) {
-  launch_pdl(k_restrict_residual<T, B, RX, RY, RZ>, lc.grid, lc.block, 0, s, lv.op, cv.op, b, sb_ptr, x,
-             sx_ptr, bc, lsc, zm, lc.kchunk, rb);
-}
-
-template <typename T, typename B>
-void launch_restrict(const Level& lv, const Level& cv, const B* b, const double* sb_ptr, const T* x,
-                     const double* sx_ptr, T* bc, LevelScalars* lsc, int zm, const Launch3& lc,
-                     RedBuf rb, cudaStream_t s) {
-  const int code = (lv.rx == 2 ? 4 : 0) + (lv.ry == 2 ? 2 : 0) + (lv.rz == 2 ? 1 : 0);
-  switch(code) {
-    case 7: launch_restrict_r<T, B, 2, 2, 2>(lv, cv, b, sb_ptr, x, sx_ptr, bc, lsc, zm, lc, rb, s); break;
-    case 6: launch_restrict_r<T, B, 2, 2, 1>(lv, cv, b, sb_ptr, x, sx_ptr, bc, lsc, zm, lc, rb, s); break;
-    case 5: launch_restrict_r<T, B, 2, 1, 2>(lv, cv, b, sb_ptr, x, sx_ptr, bc, lsc, zm, lc, rb, s); break;
-    case 4: launch_restrict_r<T, B, 2, 1, 1>(lv, cv, b, sb_ptr, x, sx_ptr, bc, lsc, zm, lc, rb, s); break;
-    case 3: launch_restrict_r<T, B, 1, 2, 2>(lv, cv, b, sb_ptr, x, sx_ptr, bc, lsc, zm, lc, rb, s); break;
-    case 2: launch_restrict_r<T, B, 1, 2, 1>(lv, cv, b, sb_ptr, x, sx_ptr, bc, lsc, zm, lc, rb, s); break;
-    case 1: launch_restrict_r<T, B, 1, 1, 2>(lv, cv, b, sb_ptr, x, sx_ptr, bc, lsc, zm, lc, rb, s); break;
-    default: launch_restrict_r<T, B, 1, 1, 1>(lv, cv, b, sb_ptr, x, sx_ptr, bc, lsc, zm, lc, rb, s); break;
-  }
-}
-
-// Grid of a persistent plane-pipelined launch on a level: at most two blocks
-// per SM, each with a range of at least four tile-planes that fits kTMaxSeg
-// segments.
-struct TGrid {
-  int grid, ty;
-};
-
-// Blocks per SM of the plane-pipeline kernels: four, or as many as fit (the
-// rings of the FP64 kernels on a 256-wide level hold ~100 KB, so two of
-// those; the lighter A p ring and the FP32 kernels, whose planes carry half
-// the bytes, fit three or four and keep more bytes in flight per SM).
-int tper_sm(size_t) { return 4; }
-
-// Blocks of one plane-pipeline launch: tper_sm blocks per SM, no more than
-// fit on an SM at once (the persistent schedule gives every block an equal
-// share), at least 4 tile-planes per block.
-int resident_blocks(const void* kernel, size_t smem, int threads = 256) {
-  int n = 0;
-  OFB_CHECK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, kernel, threads, smem));
-  return std::max(1, n);
-}
-
-// Grid of a plane-pipeline launch over `tiles` row tiles and `nzu` planes (or
-// coarse planes): a multiple of the tile count (the z-aligned schedule of
-// tsegments) where the kernel gains from it (`aligned_always`: its halo rows
-// come from L2) or where that keeps at least 95 % of the blocks that fit,
-// else the contiguous ranges.  Measured at 256^3: the aligned schedule takes
-// the FP64 k_tsmooth from 88 to 80 us and k_trestrict from 72 to 68 us
-// although their 2 blocks per SM round down from 296 to 256; k_tprolong (both
-// precisions), the FP32 k_tsmooth and k_tap (3 blocks per SM, 444 -> 384) lose
-// more to the rounding down than they gain.
-long long tgrid_blocks(const PoissonPlan* P, int tiles, int nzu, int per_sm, int min_units,
-                       bool aligned_always) {
-  const long long items = static_cast<long long>(tiles) * nzu;
-  long long g = std::min<long long>(static_cast<long long>(per_sm) * P->sms, std::max(1LL, items / min_units));
-  const long long aligned = tiles * std::min<long long>(nzu, g / tiles);
-  if(aligned > 0 && (aligned_always || aligned * 20 >= g * 19)) return aligned;
-  while((items / g + 1) / nzu + 2 > kTMaxSeg) ++g;
-  if(g % tiles == 0) ++g;  // a multiple of the tile count would select the aligned schedule
-  return g;
-}
-
-TGrid tgrid(const PoissonPlan* P, const CLay& L, size_t elem, const void* kernel, size_t smem,
-            int threads = 256, bool aligned_always = false) {
-  const int ty = 1024 / L.nx;
-  const int per_sm = std::min(tper_sm(elem), resident_blocks(kernel, smem, threads));
-  return TGrid{static_cast<int>(tgrid_blocks(P, L.ny / ty, L.nz, per_sm, 4, aligned_always)), ty};
-}
 
 // v_cycle (linsolve/poisson_solver.cpp:597-633) from level l; the finest
 // level's rhs is the CG residual r0 (type V, shift sc->sr).
@@ -3454,7 +1323,7 @@ void v_cycle(PoissonPlan* P, int l, const V* r0, SolveScalars* sc, RedBuf rb, cu
   }
   Level& cv = P->levels[l + 1];
   const T* b = l == 0 ? static_cast<const T*>(r0) : static_cast<const T*>(lv.b);
-  const size_t smem1 = march::smem_bytes<T>(lv.tile, 1), smem2 = march::smem_bytes<T>(lv.tile, 2);
+  const size_t smem1 = march::smem_bytes<T>(lv.tile, 1, 2), smem2 = march::smem_bytes<T>(lv.tile, 2, 2);
   const int threads = lv.tile.px * lv.tile.ey / 2;
   {
     ProfScope ps(l == 0 ? kKSmoothFirstFine : kKCoarseLevels, s);
@@ -3499,29 +1368,7 @@ void enqueue_pre(PoissonPlan* P, const CGVec<V>& v, SolveScalars* sc, RedBuf rb,
   OFB_LAUNCH_CHECK("k_initial_residual");
 }
 
-// The fused CG step needs the plane-pipeline maps of the finest level's
-// correction (z) and of p.  It is used for the FP32 inner solves of the mixed
-// path, where it is measurably faster; in FP64 the separate kernels are as
-// fast.  ORCHARD_B200_NO_VEC containing "fuse" keeps the separate kernels.
-bool fused_cg(const PoissonPlan* P) {
-  const char* f64 = std::getenv("ORCHARD_B200_FUSE64");
-  const bool fp64_fused = f64 != nullptr && f64[0] == '1';
-  return (P->precision == 1 || fp64_fused) && P->tma_ap && P->levels[0].tma_prolong &&
-         vec_enabled("tma") && vec_enabled("fuse");
-}
-
-// The last deferred x update of a fused-step loop.
-template <typename V>
-void enqueue_x_final(PoissonPlan* P, const CGVec<V>& v, SolveScalars* sc, RedBuf rb, cudaStream_t s) {
-  if(!fused_cg(P)) return;
-  const Level& l0 = P->levels[0];
-  const Launch3 ln = launch3(l0.L.nx, l0.L.ny, l0.L.nz);
-  ProfScope ps(kKUpdateXr, s);
-  k_x_final<V><<<ln.grid, ln.block, 0, s>>>(l0.L, v.x, v.p, v.p2, sc, ln.kchunk, rb);
-  OFB_LAUNCH_CHECK("k_x_final");
-}
-
-// One body of the rotated PCG loop: z = M r, p = z + beta p, A p, x/r update
+// One body of the rotated PCG loop: z = M r, p = z + beta p and p.Ap, x/r update
 // and the convergence test -- the reference's iteration (:750-806) with the
 // preconditioner moved to the top; the body count is the reference's
 // iteration count, and the first body forms p = z as the reference does
@@ -3530,52 +1377,20 @@ template <typename T, typename V>
 void enqueue_body(PoissonPlan* P, const CGVec<V>& v, SolveScalars* sc, RedBuf rb, cudaStream_t s,
                   cudaGraphConditionalHandle cond) {
   const Level& l0 = P->levels[0];
-  const Launch3 ln = launch3(l0.L.nx, l0.L.ny, l0.L.nz);
   v_cycle<T, V>(P, 0, v.r, sc, rb, s);
-  if(fused_cg(P)) {
-    // fused p update + A p + deferred x update, then the residual update
-    {
-      ProfScope ps(kKApplyAp, s);
-      const int ty = 1024 / l0.L.nx;
-      const size_t sm = (tround(static_cast<size_t>(ty + 2) * l0.L.nx * sizeof(T)) +
-                         tround(static_cast<size_t>(ty + 2) * l0.L.nx * sizeof(V))) * tpap_slots<V>();
-      const auto kern = P->all_periodic ? k_tpap<T, V, true> : k_tpap<T, V, false>;
-      const TGrid tg = tgrid(P, l0.L, sizeof(V), reinterpret_cast<const void*>(kern), sm);
-      launch_pdl(kern, tg.grid, 256, sm, s, l0.op, l0.tm_xm, l0.tm_xh, P->tm_pm, P->tm_ph, P->tm_pm2,
-                 P->tm_ph2, P->ls, v.p, v.p2, v.ap, v.x, sc, rb, P->fault);
-    }
-    {
-      ProfScope ps(kKUpdateXr, s);
-      const int n = l0.L.count();
-      const int blocks = static_cast<int>(std::min<long long>(
-          kTargetBlocks, std::max(1LL, (static_cast<long long>(n) + kFlatThreads - 1) / kFlatThreads)));
-      launch_pdl(k_update_r_flat<V>, blocks, kFlatThreads, 0, s, n, v.r, v.ap, sc, rb, cond);
-    }
-    OFB_LAUNCH_CHECK("fused pcg body");
-    return;
-  }
-  {
-    ProfScope ps(kKUpdateP, s);
-    launch_pdl(k_update_p<T, V>, ln.grid, ln.block, 0, s, l0.L, static_cast<const T*>(l0.x), P->ls, v.p, sc,
-               ln.kchunk, rb);
-  }
+  const march::Tile& t = P->cg_tile;
+  const int threads = t.px * t.ey / 2;
+  const bool flat = l0.L.nz == 1;
+  const march::Direction<V> d{{v.p, v.p2}};
   {
     ProfScope ps(kKApplyAp, s);
-    if(P->tma_ap && vec_enabled("tma")) {
-      const size_t sm = tround(static_cast<size_t>(1024 / l0.L.nx + 2) * l0.L.nx * sizeof(V)) * kTSlots;
-      const auto kern = P->all_periodic ? k_tap<V, 4, true> : k_tap<V, 4, false>;
-      const TGrid tg = tgrid(P, l0.L, sizeof(V), reinterpret_cast<const void*>(kern), sm);
-      launch_pdl(kern, tg.grid, 256, sm, s, l0.op, P->tm_pm, P->tm_ph, v.ap, sc, rb, P->fault);
-    } else if(vfits<V>(l0.L) && vec_enabled() && vec_enabled("ap")) {
-      const vst::RowLaunch lr = vst::row_launch(l0.L.nx, l0.L.ny, l0.L.nz, vst::Width<V>::W, 16);
-      launch_pdl(k_vapply_ap<V>, lr.grid, lr.block, 0, s, l0.op, v.p, v.ap, sc, lr.kchunk, rb);
-    }
-    else
-      launch_pdl(k_apply_ap<V>, ln.grid, ln.block, 0, s, l0.op, v.p, v.ap, sc, ln.kchunk, rb);
+    launch_pdl(direction_kernel<V>(P, flat), P->cg_grid, threads, march::smem_bytes<V>(t, 2, 1), s, l0.op, t,
+               static_cast<const V*>(l0.x), P->ls, d, sc, rb);
   }
   {
     ProfScope ps(kKUpdateXr, s);
-    launch_pdl(k_update_xr<V>, ln.grid, ln.block, 0, s, l0.L, v.x, v.r, v.p, v.ap, sc, ln.kchunk, rb, cond);
+    launch_pdl(advance_kernel<V>(P, flat), P->cg_grid, threads, march::smem_bytes<V>(t, 3, 1), s, l0.op, t, d,
+               v.x, v.r, sc, rb, cond);
   }
   OFB_LAUNCH_CHECK("pcg body");
 }
@@ -3650,7 +1465,6 @@ SolveScalars init_scalars(PoissonPlan* P, int max_iterations, double tolerance, 
     init.sx = 0.0;
     init.removed_rhs_mean = 0.0;
   }
-  init.sp = 0.0;
   return init;
 }
 
@@ -3669,7 +1483,6 @@ void solve_impl(PoissonPlan* P, int max_iterations, double tolerance, SolveScala
           [&](cudaGraphConditionalHandle c) { enqueue_body<T, double>(P, v, sc, rb, s, c); },
           &P->graph);
     OFB_CHECK(cudaGraphLaunch(P->exec, s));
-    enqueue_x_final<double>(P, v, sc, rb, s);
     OFB_CHECK(cudaMemcpyAsync(host, sc, sizeof(SolveScalars), cudaMemcpyDeviceToHost, s));
     OFB_CHECK(cudaStreamSynchronize(s));
     prof_add_counts(P->pre_counts, 1);
@@ -3685,7 +1498,6 @@ void solve_impl(PoissonPlan* P, int max_iterations, double tolerance, SolveScala
       OFB_CHECK(cudaStreamSynchronize(s));
       prof_collect();
     }
-    enqueue_x_final<double>(P, v, sc, rb, s);
     OFB_CHECK(cudaMemcpyAsync(host, sc, sizeof(SolveScalars), cudaMemcpyDeviceToHost, s));
     OFB_CHECK(cudaStreamSynchronize(s));
     prof_collect();
@@ -3741,7 +1553,6 @@ void solve_dc(PoissonPlan* P, int max_iterations, double tolerance, SolveScalars
   };
   auto body = [&](cudaGraphConditionalHandle c) { enqueue_body<T, float>(P, v, si, rb, s, c); };
   auto post = [&]() {
-    enqueue_x_final<float>(P, v, si, rb, s);
     ProfScope ps(kKDefectCorrection, s, 2);
     k_dc_update_x<<<ln.grid, ln.block, 0, s>>>(l0.L, P->x, P->e32, sc, si, ln.kchunk, rb);
     k_dc_residual<<<ln.grid, ln.block, 0, s>>>(l0.op, P->b, P->x, P->r, sc, si, ln.kchunk, rb);
@@ -3788,25 +1599,15 @@ void solve_dc(PoissonPlan* P, int max_iterations, double tolerance, SolveScalars
 void poisson_solve(PoissonPlan* P, int max_iterations, double tolerance, SolveScalars* sc_dev,
                    SolveScalars* sc_host, RedBuf rb, cudaStream_t s, double* history,
                    int history_cap) {
-  // the fault word describes this solve only: a wait that gave up in an
-  // earlier solve does not fail the next one
-  OFB_CHECK(cudaMemsetAsync(P->fault, 0, sizeof(int), s));
   if(P->precision == 1)
     solve_dc<float>(P, max_iterations, tolerance, sc_dev, sc_host, rb, s, history, history_cap);
   else
     solve_impl<double>(P, max_iterations, tolerance, sc_dev, sc_host, rb, s, history, history_cap);
-  int fault = 0;
-  OFB_CHECK(cudaMemcpyAsync(&fault, P->fault, sizeof(int), cudaMemcpyDeviceToHost, s));
-  OFB_CHECK(cudaStreamSynchronize(s));
-  if(fault != 0)
-    throw TimeoutError("a bounded wait for a TMA plane load gave up in the pressure solve (code " +
-                       std::to_string(fault) + ")");
 }
 
 double poisson_time_coarse_chain(PoissonPlan* P, RedBuf rb, cudaStream_t s, int reps, int* launches) {
   *launches = 0;
   if(P->levels.size() < 2 || reps < 1) return 0.0;
-  OFB_CHECK(cudaMemsetAsync(P->fault, 0, sizeof(int), s));
   long long counts[kKernelCount] = {};
   cudaGraph_t g = nullptr;
   cudaGraphExec_t ge = nullptr;
@@ -3835,12 +1636,6 @@ double poisson_time_coarse_chain(PoissonPlan* P, RedBuf rb, cudaStream_t s, int 
   cudaEventDestroy(e1);
   cudaGraphExecDestroy(ge);
   cudaGraphDestroy(g);
-  int fault = 0;
-  OFB_CHECK(cudaMemcpyAsync(&fault, P->fault, sizeof(int), cudaMemcpyDeviceToHost, s));
-  OFB_CHECK(cudaStreamSynchronize(s));
-  if(fault != 0)
-    throw TimeoutError("a bounded wait for a TMA plane load gave up in the coarse-level chain (code " +
-                       std::to_string(fault) + ")");
   return 1000.0 * ms / reps;
 }
 

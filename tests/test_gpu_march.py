@@ -1,0 +1,87 @@
+"""Pressure solves whose shapes sit at the edges of the marching kernels' tiles.
+
+The V-cycle levels above 1024 cells and the CG updates run on tiles of row
+patches (2 cells in FP64, 4 in FP32) that march k, with image cells outside
+the domain; levels of at most 1024 cells are one matrix.  The shapes below
+take rows that split into no whole patch, axes shorter than the halo, axes
+that do not coarsen, one plane, one more cell than a tile and a finest level
+that is itself the matrix, under every kind of boundary image.
+
+The residual history of the first iterations is the reference's algorithm
+iteration by iteration (a wrong image, weight or restriction changes it in the
+first digits): it must agree to 1e-9 relative, far above the rounding of a few
+V-cycles (about 1e-15 each) and far below any such error.  The solutions each
+satisfy |b - A x| <= 1e-12 |b|, so they agree to 2e-12 times the condition
+number of A (on the zero-mean subspace for singular problems).
+"""
+import numpy as np
+import pytest
+
+import pyoracle as po
+from conftest import to_gpu_grid, to_gpu_pbc
+
+pytestmark = pytest.mark.gpu
+
+PER = [po.P_PERIODIC] * 6
+NEU = [po.P_NEUMANN] * 6
+MIX = [po.P_DIRICHLET, po.P_NEUMANN, po.P_PERIODIC, po.P_PERIODIC, po.P_NEUMANN, po.P_DIRICHLET]
+DIR = [po.P_DIRICHLET] * 6
+
+SHAPES = [
+    (66, 28, 6),    # one more patch than a tile's 64 cells
+    (130, 5, 3),    # odd rows, three planes
+    (37, 20, 6),    # odd nx: no whole patches, x not coarsened
+    (2, 36, 30),    # rows shorter than the halo
+    (15, 18, 14),   # odd nx in a tile of one row of patches
+    (20, 150, 2),   # two planes, many row tiles
+    (70, 72, 1),    # one plane
+    (257, 6, 1),    # one plane, odd nx above four tiles
+    (32, 32, 2),    # level 1 is the matrix
+    (16, 8, 8),     # the finest level is the matrix
+]
+
+
+def _condition(shape, h, types):
+    """Largest over smallest non-zero eigenvalue of the separable operator."""
+    lo, hi = [], []
+    for a, n in enumerate(shape):
+        m = np.zeros((n, n))
+        for i in range(n):
+            m[i, i] += 2.0
+            for j, t in ((i - 1, types[2 * a]), (i + 1, types[2 * a + 1])):
+                if 0 <= j < n:
+                    m[i, j] -= 1.0
+                elif t == po.P_PERIODIC:
+                    m[i, j % n] -= 1.0
+                else:
+                    m[i, i] += 1.0 if t == po.P_DIRICHLET else -1.0
+        e = np.sort(np.linalg.eigvalsh(m)) / h[a] ** 2
+        lo.append(e)
+        hi.append(e[-1])
+    s = (lo[0][:, None, None] + lo[1][None, :, None] + lo[2][None, None, :]).ravel()
+    return sum(hi) / np.min(s[s > 1e-9 * sum(hi)])
+
+
+@pytest.mark.parametrize("precision", ["fp64", "mixed"])
+@pytest.mark.parametrize("types", [PER, NEU, MIX, DIR], ids=["periodic", "neumann", "mixed", "dirichlet"])
+@pytest.mark.parametrize("shape", SHAPES, ids=lambda s: "x".join(map(str, s)))
+def test_pressure_solve_at_tile_edges(oracle, shape, types, precision):
+    import solver_b200 as sb
+    h = (0.1, 0.12, 0.09)
+    g = po.Grid(*shape, *h)
+    rng = np.random.default_rng(sum(shape))
+    rhs = rng.standard_normal(po.shape(g, "p"))
+    pbc = po.pbc_from(types)
+    ref = np.zeros(po.shape(g, "p"))
+    dref, href = oracle.poisson_solve(g, pbc, 400, 1e-12, rhs, ref)
+    assert dref.converged
+    ctx = sb.Context(to_gpu_grid(g), [sb.PERIODIC] * 6,
+                     precision=sb.OF_MIXED if precision == "mixed" else sb.OF_FP64)
+    got, d = ctx.solve_pressure_poisson(rhs, to_gpu_pbc(pbc), 2000, 1e-12)
+    ctx.close()
+    assert d["converged"] and d["relative_residual"] <= 1e-12
+    if precision == "fp64":
+        n = min(6, len(href), len(d["residual_history"]))
+        np.testing.assert_allclose(d["residual_history"][:n], href[:n], rtol=1e-9, atol=1e-12 * href[0])
+    a, b = po.active(got), po.active(ref)
+    assert np.linalg.norm(a - b) <= 2e-12 * _condition(shape, h, types) * np.linalg.norm(b)
