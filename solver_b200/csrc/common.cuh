@@ -141,6 +141,21 @@ inline Launch3 launch3(int nx, int ny, int nz) {
   return l;
 }
 
+// One launch over the three face components: blockIdx.x % 3 is the component,
+// the other indices cover the largest extents.  Sizes are limited as if each
+// component were launched by itself; at most three times kMaxBlocks blocks.
+inline Launch3 launch3_components(const Grid& g) {
+  Launch3 l = launch3(g.nx + 1, g.ny, g.nz);
+  for(const Launch3& o : {launch3(g.nx, g.ny + 1, g.nz), launch3(g.nx, g.ny, g.nz + 1)}) {
+    l.grid.x = l.grid.x > o.grid.x ? l.grid.x : o.grid.x;
+    l.grid.y = l.grid.y > o.grid.y ? l.grid.y : o.grid.y;
+    l.kchunk = l.kchunk > o.kchunk ? l.kchunk : o.kchunk;
+  }
+  l.grid.x *= 3;
+  l.grid.z = (g.nz + 1 + l.kchunk - 1) / l.kchunk;
+  return l;
+}
+
 inline int blocks_of(const Launch3& l) { return l.grid.x * l.grid.y * l.grid.z; }
 
 // ---------------------------------------------------------------------------

@@ -10,6 +10,21 @@ namespace {
 
 constexpr double kSmallDenominator = 1.0e-14;  // solver/momentum_terms.cpp:14
 
+// n / d for 1e-14 <= |d| < 2^1022: the hardware's reciprocal approximation
+// (relative error 2^-23), one step of Halley's cubic iteration (2^-69) and
+// Markstein's residual correction of the quotient (Markstein, IBM J. Res. Dev.
+// 34, 1990), so the result is within one ulp.  The limiter's one division per
+// face in the general form was most of the advection's FP64 issue.
+__device__ __forceinline__ double quotient(double n, double d) {
+  double r;
+  asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(d));
+  double e = fma(-d, r, 1.0);
+  e = fma(e, e, e);
+  r = fma(r, e, r);
+  const double q = n * r;
+  return fma(fma(-d, q, n), r, q);
+}
+
 // Branch-free form of one reconstruct_face call: every candidate value is
 // loaded before the velocity sign is known and the reference's three cases
 // (first-order upwind for |u_f| < 1e-14 or near the storage bounds, van Leer
@@ -23,10 +38,11 @@ __device__ __forceinline__ double tvd_face(double vel, double left, double right
   // 0.5 phi(r) delta with r = num / delta (0 when |delta| < 1e-14) and
   // phi = (r + |r|) / (1 + |r|): zero unless r > 0, and then equal to
   // num delta / (delta + num) -- one division instead of two; the value
-  // differs from the two-division form by rounding only, the branches not
-  // at all (the sign of r is the product of exact signs).
-  const bool positive = fabs(delta) >= kSmallDenominator && num != 0.0 && ((num > 0.0) == (delta > 0.0));
-  const double half_phi_delta = positive ? num * delta / (delta + num) : 0.0;
+  // differs from the two-division form by rounding only (r > 0 is read off
+  // the product num delta, whose underflow stands for a value below 1e-290).
+  const double nd = num * delta;
+  const bool positive = fabs(delta) >= kSmallDenominator && nd > 0.0;
+  const double half_phi_delta = positive ? quotient(nd, delta + num) : 0.0;
   const double muscl = up ? left + half_phi_delta : right - half_phi_delta;
   const bool first_order = fabs(vel) < kSmallDenominator || (up ? !far_left_ok : !far_right_ok);
   return first_order ? (up ? left : right) : muscl;
@@ -77,14 +93,23 @@ __device__ __forceinline__ double advection_bf(const Grid& g, const double* __re
   return flux_div;
 }
 
-// Advection term of component C at every active point, written to adv[C]
-// (the first half of assemble_predictor_rhs, solver/taylor_green.cpp:238).
+// The three components of one launch: consecutive blocks take the same tile
+// of u, v and w, which read the same velocity cells (from L2), and a step of a
+// small grid is one launch instead of three.  Extents are the largest
+// component's; a block clips to its own.
+struct Tile3 {
+  int comp, bx;
+};
+__device__ __forceinline__ Tile3 component_tile() {
+  return Tile3{static_cast<int>(blockIdx.x % 3), static_cast<int>(blockIdx.x / 3)};
+}
+
 template <int C>
-__global__ void __launch_bounds__(kTX* kTY)
-    k_advect_bf(Grid g, const double* __restrict__ u, const double* __restrict__ v,
-                const double* __restrict__ w, double* __restrict__ out, int kchunk) {
+__device__ __forceinline__ void advect_tile(const Grid& g, const double* __restrict__ u,
+                                            const double* __restrict__ v, const double* __restrict__ w,
+                                            double* __restrict__ out, int bx, int kchunk) {
   const Lay L = make_lay(g, kFaceX + C);
-  const int i = blockIdx.x * kTX + threadIdx.x + 1;
+  const int i = bx * kTX + threadIdx.x + 1;
   const int j = blockIdx.y * kTY + threadIdx.y + 1;
   if(i > L.nx || j > L.ny) return;
   const int k0 = blockIdx.z * kchunk + 1;
@@ -93,86 +118,99 @@ __global__ void __launch_bounds__(kTX* kTY)
   for(int k = k0; k < k1; ++k) out[L.idx(i, j, k)] = advection_bf<C>(g, u, v, w, i, j, k, inv_h);
 }
 
+// Advection term of every component at its active points (the first half of
+// assemble_predictor_rhs, solver/taylor_green.cpp:238).  Bound by its FP64
+// arithmetic (six limited faces per point).
+__global__ void __launch_bounds__(kTX* kTY)
+    k_advect_bf(Grid g, const double* __restrict__ u, const double* __restrict__ v,
+                const double* __restrict__ w, double* __restrict__ au, double* __restrict__ av,
+                double* __restrict__ aw, int kchunk) {
+  const Tile3 t = component_tile();
+  if(t.comp == 0) advect_tile<0>(g, u, v, w, au, t.bx, kchunk);
+  else if(t.comp == 1) advect_tile<1>(g, u, v, w, av, t.bx, kchunk);
+  else advect_tile<2>(g, u, v, w, aw, t.bx, kchunk);
+}
+
+// What one plane contributes to the predictor at a point: the value and its
+// second differences in x, in y and in both.
+struct PlaneTerms {
+  double c, xx, yy, xy;
+};
+
+__device__ __forceinline__ PlaneTerms plane_terms(const double* __restrict__ f, int q, int sx, double ix,
+                                                  double iy) {
+  double m[3][3];
+#pragma unroll
+  for(int b = 0; b < 3; ++b)
+#pragma unroll
+    for(int e = 0; e < 3; ++e) m[b][e] = f[q + (e - 1) + (b - 1) * sx];
+  double d[3];
+#pragma unroll
+  for(int b = 0; b < 3; ++b) d[b] = (m[b][2] - 2.0 * m[b][1] + m[b][0]) * ix;
+  return PlaneTerms{m[1][1], d[1], (m[2][1] - 2.0 * m[1][1] + m[0][1]) * iy, (d[2] - 2.0 * d[1] + d[0]) * iy};
+}
+
 // The rest of assemble_predictor_rhs (solver/taylor_green.cpp:239-255):
 // diffusion, total-pressure gradient, factorisation correction and the AB2
-// combination with the advection term computed by k_advect_bf.  The 27-point
-// correction is evaluated column by column (second z-differences first), so
-// only 18 neighbourhood values are live at once.
+// combination with the advection term computed by k_advect_bf.  A thread
+// marches k with the terms of three planes in registers: the 27-point
+// correction is the z second difference of the planes' xx, yy and xy, so a
+// point loads the nine cells of one new plane instead of 27.
 template <int C>
-__global__ void __launch_bounds__(kTX* kTY) k_predictor_rest(PredictorArgs a, int kchunk) {
+__device__ __forceinline__ void predictor_tile(const PredictorArgs& a, int bx, int kchunk) {
   const Grid& g = a.g;
   const Lay L = make_lay(g, kFaceX + C);
   const Lay P = make_lay(g, kCell);
-  const int i = blockIdx.x * kTX + threadIdx.x + 1;
+  const int i = bx * kTX + threadIdx.x + 1;
   const int j = blockIdx.y * kTY + threadIdx.y + 1;
   if(i > L.nx || j > L.ny) return;
   const int k0 = blockIdx.z * kchunk + 1;
   const int k1 = min(k0 + kchunk, L.nz + 1);
+  if(k0 >= k1) return;
   const double ih = 1.0 / g.h(C);
   const double ix = 1.0 / (g.dx * g.dx), iy = 1.0 / (g.dy * g.dy), iz = 1.0 / (g.dz * g.dz);
-  const double dy2 = g.dy * g.dy;
-  const bool three_d = g.nz != 1;
+  const bool three_d = a.variant != 1 && g.nz != 1;
   const double s_gp = -a.dt;
-  const double s_dif = 0.5 * a.dt;
+  const double s_dif = 0.5 * a.dt * a.nu;
   const double s_adv = a.has_prev ? -1.5 * a.dt : -a.dt;
   const double s_prev = 0.5 * a.dt;
   const double s_corr = a.alpha * a.alpha;
   const double* __restrict__ f = a.cur[C];
+  const double* __restrict__ p = a.p;
   const int pstC = P.stride(C);
-  for(int k = k0; k < k1; ++k) {
-    const int q = L.idx(i, j, k);
-    // in-plane values m[dy][dx] and second z-differences z2[dy][dx]
-    double m[3][3], z2[3][3];
-    double fzm = 0.0, fzp = 0.0;
-#pragma unroll
-    for(int b = 0; b < 3; ++b)
-#pragma unroll
-      for(int e = 0; e < 3; ++e) {
-        const int qq = q + (e - 1) + (b - 1) * L.sx;
-        const double lo = f[qq - L.sxy], mid = f[qq], hi = f[qq + L.sxy];
-        m[b][e] = mid;
-        z2[b][e] = (hi - 2.0 * mid + lo) * iz;
-        if(b == 1 && e == 1) {
-          fzm = lo;
-          fzp = hi;
-        }
-      }
-    const double c2 = 2.0 * m[1][1];
-    const double lap = (m[1][2] - c2 + m[1][0]) * ix + (m[2][1] - c2 + m[0][1]) * iy +
-                       (fzp - c2 + fzm) * iz;
-    const double dif = lap * a.nu;
+  int q = L.idx(i, j, k0);
+  PlaneTerms lo = plane_terms(f, q - L.sxy, L.sx, ix, iy), mid = plane_terms(f, q, L.sx, ix, iy);
+#pragma unroll 2
+  for(int k = k0; k < k1; ++k, q += L.sxy) {
+    const PlaneTerms hi = plane_terms(f, q + L.sxy, L.sx, ix, iy);
     const int pq = P.idx(i, j, k);
-    const double gp = (a.p[pq] - a.p[pq - pstC]) * ih;
-    double corr;
-    if(a.variant == 1) {
-      double dyy[3];
-#pragma unroll
-      for(int e = 0; e < 3; ++e) dyy[e] = (m[2][e] - 2.0 * m[1][e] + m[0][e]) / dy2;
-      corr = (dyy[2] - 2.0 * dyy[1] + dyy[0]) * ix;
-    } else {
-      double d2y[3];
-#pragma unroll
-      for(int e = 0; e < 3; ++e) d2y[e] = (m[2][e] - 2.0 * m[1][e] + m[0][e]) * iy;
-      corr = (d2y[2] - 2.0 * d2y[1] + d2y[0]) * ix;
-      if(three_d) {
-        const double mxz = (z2[1][2] - 2.0 * z2[1][1] + z2[1][0]) * ix;
-        double myz[3];
-#pragma unroll
-        for(int e = 0; e < 3; ++e) myz[e] = (z2[2][e] - 2.0 * z2[1][e] + z2[0][e]) * iy;
-        const double triple = (myz[2] - 2.0 * myz[1] + myz[0]) * ix;
-        corr += mxz;
-        corr += myz[1];
-        corr -= a.alpha * triple;
-      }
+    const double gp = (p[pq] - p[pq - pstC]) * ih;
+    const double adv = a.adv[C][q];
+    const double prev = a.has_prev ? a.prev[C][q] : 0.0;
+    const double lap = mid.xx + mid.yy + (hi.c - 2.0 * mid.c + lo.c) * iz;
+    double corr = mid.xy;
+    if(three_d) {
+      corr += (hi.xx - 2.0 * mid.xx + lo.xx) * iz;
+      corr += (hi.yy - 2.0 * mid.yy + lo.yy) * iz;
+      corr -= a.alpha * ((hi.xy - 2.0 * mid.xy + lo.xy) * iz);
     }
-    double r = m[1][1];
+    double r = mid.c;
     r += s_gp * gp;
-    r += s_dif * dif;
-    r += s_adv * a.adv[C][q];
-    if(a.has_prev) r += s_prev * a.prev[C][q];
+    r += s_dif * lap;
+    r += s_adv * adv;
+    if(a.has_prev) r += s_prev * prev;
     r += s_corr * corr;
     a.rhs[C][q] = r;
+    lo = mid;
+    mid = hi;
   }
+}
+
+__global__ void __launch_bounds__(kTX* kTY) k_predictor_rest(PredictorArgs a, int kchunk) {
+  const Tile3 t = component_tile();
+  if(t.comp == 0) predictor_tile<0>(a, t.bx, kchunk);
+  else if(t.comp == 1) predictor_tile<1>(a, t.bx, kchunk);
+  else predictor_tile<2>(a, t.bx, kchunk);
 }
 
 // initialize_exact_state (solver/taylor_green.cpp:335-395), active entries.
@@ -205,42 +243,28 @@ __global__ void k_tg_init(Grid g, int mode, int loc, double* f) {
 }  // namespace
 
 void launch_predictor_rhs(const PredictorArgs& a, cudaStream_t s) {
-  const Lay Lu = make_lay(a.g, kFaceX), Lv = make_lay(a.g, kFaceY), Lw = make_lay(a.g, kFaceZ);
-  const Launch3 l0 = launch3(Lu.nx, Lu.ny, Lu.nz);
-  const Launch3 l1 = launch3(Lv.nx, Lv.ny, Lv.nz);
-  const Launch3 l2 = launch3(Lw.nx, Lw.ny, Lw.nz);
+  const Launch3 l = launch3_components(a.g);
   {
-    ProfScope ps(kKAdvection, s, 3);
-    k_advect_bf<0><<<l0.grid, l0.block, 0, s>>>(a.g, a.cur[0], a.cur[1], a.cur[2], a.adv[0], l0.kchunk);
-    k_advect_bf<1><<<l1.grid, l1.block, 0, s>>>(a.g, a.cur[0], a.cur[1], a.cur[2], a.adv[1], l1.kchunk);
-    k_advect_bf<2><<<l2.grid, l2.block, 0, s>>>(a.g, a.cur[0], a.cur[1], a.cur[2], a.adv[2], l2.kchunk);
+    ProfScope ps(kKAdvection, s);
+    k_advect_bf<<<l.grid, l.block, 0, s>>>(a.g, a.cur[0], a.cur[1], a.cur[2], a.adv[0], a.adv[1], a.adv[2],
+                                           l.kchunk);
     OFB_LAUNCH_CHECK("k_advect_bf");
   }
   launch_predictor_rest(a, s);
 }
 
 void launch_predictor_rest(const PredictorArgs& a, cudaStream_t s) {
-  const Lay Lu = make_lay(a.g, kFaceX), Lv = make_lay(a.g, kFaceY), Lw = make_lay(a.g, kFaceZ);
-  const Launch3 l0 = launch3(Lu.nx, Lu.ny, Lu.nz);
-  const Launch3 l1 = launch3(Lv.nx, Lv.ny, Lv.nz);
-  const Launch3 l2 = launch3(Lw.nx, Lw.ny, Lw.nz);
-  ProfScope ps(kKPredictor, s, 3);
-  k_predictor_rest<0><<<l0.grid, l0.block, 0, s>>>(a, l0.kchunk);
-  k_predictor_rest<1><<<l1.grid, l1.block, 0, s>>>(a, l1.kchunk);
-  k_predictor_rest<2><<<l2.grid, l2.block, 0, s>>>(a, l2.kchunk);
+  const Launch3 l = launch3_components(a.g);
+  ProfScope ps(kKPredictor, s);
+  k_predictor_rest<<<l.grid, l.block, 0, s>>>(a, l.kchunk);
   OFB_LAUNCH_CHECK("k_predictor_rest");
 }
 
 void launch_advection(const Grid& g, const double* u, const double* v, const double* w,
                       double* au, double* av, double* aw, cudaStream_t s) {
-  const Lay Lu = make_lay(g, kFaceX), Lv = make_lay(g, kFaceY), Lw = make_lay(g, kFaceZ);
-  ProfScope ps(kKOther, s, 3);
-  Launch3 l0 = launch3(Lu.nx, Lu.ny, Lu.nz);
-  k_advect_bf<0><<<l0.grid, l0.block, 0, s>>>(g, u, v, w, au, l0.kchunk);
-  Launch3 l1 = launch3(Lv.nx, Lv.ny, Lv.nz);
-  k_advect_bf<1><<<l1.grid, l1.block, 0, s>>>(g, u, v, w, av, l1.kchunk);
-  Launch3 l2 = launch3(Lw.nx, Lw.ny, Lw.nz);
-  k_advect_bf<2><<<l2.grid, l2.block, 0, s>>>(g, u, v, w, aw, l2.kchunk);
+  const Launch3 l = launch3_components(g);
+  ProfScope ps(kKOther, s);
+  k_advect_bf<<<l.grid, l.block, 0, s>>>(g, u, v, w, au, av, aw, l.kchunk);
   OFB_LAUNCH_CHECK("k_advection");
 }
 
