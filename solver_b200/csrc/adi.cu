@@ -4,12 +4,13 @@
 // Dirichlet/ghost-relation end rows on walls, cyclic with Sherman-Morrison on
 // periodic axes -- so the Thomas factors (modified upper diagonal and inverse
 // pivots) and the Sherman-Morrison correction vector are computed once on the
-// host in FP64 and shared.  On the device one thread solves one line: forward
-// elimination, back substitution and the Sherman-Morrison update, in place in
-// the output field.  Threads of a warp own adjacent lines, so y and z sweeps
-// read and write unit-stride rows.
+// host in FP64 and shared.  Lines whose coupling decays within a few dozen cells
+// (every projection step here: alpha / h^2 is well below one) are solved in
+// independent chunks (k_adi_lines, k_adi_rows); the others by one warp per line
+// (k_adi_scan) or one thread per line (k_adi_tile).
 #include "kernels.hpp"
 
+#include <algorithm>
 #include <cmath>
 #include <vector>
 
@@ -33,6 +34,13 @@ struct AdiAxis {
   // 32 on periodic axes; wall lines are padded to a multiple of 32):
   // per-lane segment factors, spikes and the interface operator, all laid
   // out [element][lane] so that a warp reads them with one coalesced load
+  // chunked solver (see k_adi_lines), used when the decay length fits
+  bool decay = false;
+  int reach = 0;            // K: cells after which the coupling is below rounding
+  double lambda = 0.0, scale = 0.0;
+  int node_lo = 0, node_hi = 0;            // the wall is a node (else half a cell off the first unknown)
+  double sign_lo = 0.0, sign_hi = 0.0;     // image of unknown x: add + sign x
+  double add_lo = 0.0, add_hi = 0.0;       // (at a node: add / 2 is the wall's value)
   bool partition = false;
   int seg = 0;              // K = ceil(n / 32)
   size_t poff = 0;          // offset: cu[K][32], ip[K][32], v[K][32], w[K][32], gl[64][32], gr[64][32]
@@ -45,6 +53,11 @@ struct AdiPlan {
 };
 
 namespace {
+
+// When a line takes the chunked solver: its cost grows with (chunk + 2 reach),
+// so up to a reach of 64 cells (coupling alpha / h^2 up to about 2.5); shorter
+// lines than 8 unknowns go to k_adi_tile; a row must fit a block's threads.
+constexpr int kDecayMaxReach = 64, kDecayMinLine = 8, kRowMaxLine = 4096;
 
 double tangential_coef(int type) {
   return (type == kNoSlip || type == kPrescribed) ? -1.0 : (type == kSymmetry || type == kFixedPressure) ? 1.0 : 0.0;
@@ -175,6 +188,24 @@ AdiPlan* adi_plan_create(const Grid& g, const VBC& bc, double alpha) {
           cu[q] = q + 1 < n ? up[q] / pivot : 0.0;
           ip[q] = 1.0 / pivot;
         }
+      }
+      // The infinite line's inverse is (lambda / beta) / (1 - lambda^2) times
+      // lambda^|distance|; reach is where its tail drops below 2^-56.
+      if(beta > 0.0) {
+        const double root = (1.0 + 2.0 * beta) + std::sqrt(1.0 + 4.0 * beta);
+        A.lambda = 2.0 * beta / root;
+        A.scale = 2.0 / root;
+        A.reach = static_cast<int>(std::ceil((std::log(1.0 - A.lambda) - 56.0 * std::log(2.0)) / std::log(A.lambda)));
+        A.decay = n >= kDecayMinLine && A.reach <= kDecayMaxReach && (a != 0 || n <= kRowMaxLine);
+        auto wall = [&](int type, int face, int& node, double& sign, double& add) {
+          node = c == a && is_dirichlet_velocity(type);
+          const double v = bc.vel[face][c];
+          const bool fixed = node || type == kNoSlip || type == kPrescribed;
+          sign = fixed ? -1.0 : 1.0;
+          add = !fixed || (node && type == kSymmetry) ? 0.0 : 2.0 * v;
+        };
+        wall(bc.type[2 * a], 2 * a, A.node_lo, A.sign_lo, A.add_lo);
+        wall(bc.type[2 * a + 1], 2 * a + 1, A.node_hi, A.sign_hi, A.add_hi);
       }
       A.off = host.size();
       host.insert(host.end(), cu.begin(), cu.end());
@@ -565,12 +596,239 @@ void launch_scan(const SweepArgs& a, const ScanArgs& sa, int axis, int a1, int a
   }
 }
 
+// ---------------------------------------------------------------------------
+// Chunked line solver.  Away from the ends the Thomas factors of
+// (1 + 2 beta) x_q - beta (x_{q-1} + x_{q+1}) = r_q are constants: with lambda
+// the smaller root of beta l^2 - (1 + 2 beta) l + beta = 0,
+//   m_q = r_q + lambda m_{q-1},  y_q = m_q + lambda y_{q+1},  x = (lambda / beta) y,
+// and the influence of r fades as lambda^distance.  A chunk started K cells
+// before its first unknown and ended K cells after its last, with lambda^K
+// below the rounding, so gives the line's solution without the rest of the
+// line.  The ends are images: periodic wrap, or the reflection a wall row
+// stands for (its ghost relation x_{-1} = add + sign x_0, or x_{-1} = the wall's
+// value at a node and x_{-1-q} = add - x_{-1+q} beyond it), which r obeys too.
+// Replaces the per-line scans (k_adi_scan 116-127 us per sweep at 256^3 against
+// 42 us of traffic; k_adi_tile 61-98 us at 144 x 80 x 112).
+// ---------------------------------------------------------------------------
+struct LineArgs {
+  Lay L;
+  int n, begin, dup_index, periodic, copy_duplicate, reach;
+  double lambda, scale;
+  int node_lo, node_hi;
+  double sign_lo, sign_hi, add_lo, add_hi;
+  const double* in;
+  double* out;
+};
+
+struct Lines3 {
+  LineArgs c[3];  // the components of this launch
+};
+
+// r at unknown index q of a line (st apart from base), images included.
+__device__ __forceinline__ double line_at(const LineArgs& a, const double* base, int st, int q) {
+  if(q >= 0 && q < a.n) return base[q * st];
+  double add = 0.0, sign = 1.0;
+  while(q < 0 || q >= a.n) {
+    if(a.periodic) {
+      q += q < 0 ? a.n : -a.n;
+    } else if(q < 0) {
+      if(a.node_lo && q == -1) return add + sign * 0.5 * a.add_lo;
+      add += sign * a.add_lo;
+      sign *= a.sign_lo;
+      q = a.node_lo ? -2 - q : -1 - q;
+    } else {
+      if(a.node_hi && q == a.n) return add + sign * 0.5 * a.add_hi;
+      add += sign * a.add_hi;
+      sign *= a.sign_hi;
+      q = a.node_hi ? 2 * a.n - q : 2 * a.n - 1 - q;
+    }
+  }
+  return add + sign * base[q * st];
+}
+
+// Unknowns [q0, q0 + S) of a line into y (y[t] valid for q0 + t < n).
+template <int S>
+__device__ __forceinline__ void solve_chunk(const LineArgs& a, const double* base, int st, int q0, double (&y)[S]) {
+  const double l = a.lambda;
+  const int K = a.reach;
+  double m = 0.0;
+  if(q0 - K >= 0 && q0 + S + K <= a.n) {  // no images
+    const double* r = base + (q0 - K) * st;
+#pragma unroll 4
+    for(int t = 0; t < K; ++t, r += st) m = *r + l * m;
+#pragma unroll
+    for(int t = 0; t < S; ++t, r += st) {
+      m = *r + l * m;
+      y[t] = m;
+    }
+    double z = 0.0, w = l;
+#pragma unroll 4
+    for(int t = 0; t < K; ++t, r += st) {
+      m = *r + l * m;
+      z += w * m;
+      w *= l;
+    }
+    y[S - 1] += z;
+  } else {
+    for(int t = -K; t < 0; ++t) m = line_at(a, base, st, q0 + t) + l * m;
+#pragma unroll
+    for(int t = 0; t < S; ++t) {
+      m = line_at(a, base, st, q0 + t) + l * m;
+      y[t] = m;
+    }
+    double z = 0.0, w = l;
+    for(int t = S; t < S + K; ++t) {
+      m = line_at(a, base, st, q0 + t) + l * m;
+      z += w * m;
+      w *= l;
+    }
+    y[S - 1] += z;
+  }
+#pragma unroll
+  for(int t = S - 2; t >= 0; --t) y[t] += l * y[t + 1];
+#pragma unroll
+  for(int t = 0; t < S; ++t) y[t] *= a.scale;
+}
+
+// y and z sweeps: a thread solves kLineChunk unknowns of a line, a warp's
+// lines are adjacent in x (coalesced rows).  The chunk's redundant reads
+// (2 K of chunk + 2 K) come from L2: 32 unknowns per thread took 245 us per axis
+// for the three components at 256^3 (reach 7), 16 take 210 (more loads in flight).
+constexpr int kLineChunk = 16, kLineThreads = 128;
+
+__global__ void __launch_bounds__(kLineThreads) k_adi_lines(Lines3 s, int axis) {
+  const LineArgs& a = s.c[blockIdx.y];
+  const Lay& L = a.L;
+  const int iblocks = (L.nx + kLineThreads - 1) / kLineThreads;
+  const int chunks = (a.n + kLineChunk - 1) / kLineChunk;
+  const int other = axis == 1 ? 2 : 1;
+  int b = blockIdx.x;
+  const int i = (b % iblocks) * kLineThreads + threadIdx.x;
+  b /= iblocks;
+  const int q0 = (b % chunks) * kLineChunk, o = b / chunks;
+  if(i >= L.nx || o >= L.n(other)) return;
+  const int st = L.stride(axis);
+  const int at = L.idx(i + 1, axis == 1 ? 0 : o + 1, axis == 1 ? o + 1 : 0);
+  double y[kLineChunk];
+  solve_chunk<kLineChunk>(a, a.in + at + a.begin * st, st, q0, y);
+  double* out = a.out + at + (a.begin + q0) * st;
+#pragma unroll
+  for(int t = 0; t < kLineChunk; ++t)
+    if(q0 + t < a.n) out[t * st] = y[t];
+  if(a.copy_duplicate && q0 == 0) a.out[at + a.dup_index * st] = y[0];
+}
+
+// x sweeps: a block stages whole rows in shared memory (odd row stride: lanes
+// on adjacent rows touch different banks), a thread solves kRowChunk unknowns
+// of one row, and the rows are stored back from shared memory (coalesced both
+// ways).
+constexpr int kRowChunk = 16;
+
+__global__ void __launch_bounds__(1024, 1) k_adi_rows(Lines3 s, int rows) {
+  extern __shared__ double line_sm[];
+  const LineArgs& a = s.c[blockIdx.y];
+  const Lay& L = a.L;
+  const int total = L.ny * L.nz;
+  const int first = blockIdx.x * rows;
+  if(first >= total) return;
+  const int stride = a.n | 1;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, warps = (blockDim.x + 31) >> 5;
+  for(int l = warp; l < rows && first + l < total; l += warps) {
+    const int at = L.idx(a.begin, (first + l) % L.ny + 1, (first + l) / L.ny + 1);
+    for(int q = lane; q < a.n; q += 32) line_sm[l * stride + q] = a.in[at + q];
+  }
+  __syncthreads();
+  const int l = threadIdx.x % rows, q0 = threadIdx.x / rows * kRowChunk;
+  const bool work = q0 < a.n && first + l < total;
+  double y[kRowChunk];
+  if(work) solve_chunk<kRowChunk>(a, line_sm + l * stride, 1, q0, y);
+  __syncthreads();
+  if(work) {
+#pragma unroll
+    for(int t = 0; t < kRowChunk; ++t)
+      if(q0 + t < a.n) line_sm[l * stride + q0 + t] = y[t];
+  }
+  __syncthreads();
+  for(int w = warp; w < rows && first + w < total; w += warps) {
+    const int at = L.idx(a.begin, (first + w) % L.ny + 1, (first + w) / L.ny + 1);
+    for(int q = lane; q < a.n; q += 32) a.out[at + q] = line_sm[w * stride + q];
+    if(a.copy_duplicate && lane == 0) a.out[at - a.begin + a.dup_index] = line_sm[w * stride];
+  }
+}
+
+void launch_decay(const AdiPlan* p, const int* comps, int count, int axis, const double* const* in,
+                  double* const* out, cudaStream_t s) {
+  Lines3 q{};
+  long long blocks = 0;
+  int longest = 0, most_rows = 0;
+  for(int t = 0; t < count; ++t) {
+    const AdiAxis& A = p->ax[comps[t]][axis];
+    LineArgs& a = q.c[t];
+    a.L = make_lay(p->g, kFaceX + comps[t]);
+    a.n = A.n;
+    a.begin = A.begin;
+    a.dup_index = A.dup_index;
+    a.periodic = A.periodic ? 1 : 0;
+    a.copy_duplicate = A.copy_duplicate ? 1 : 0;
+    a.reach = A.reach;
+    a.lambda = A.lambda;
+    a.scale = A.scale;
+    a.node_lo = A.node_lo;
+    a.node_hi = A.node_hi;
+    a.sign_lo = A.sign_lo;
+    a.sign_hi = A.sign_hi;
+    a.add_lo = A.add_lo;
+    a.add_hi = A.add_hi;
+    a.in = in[comps[t]];
+    a.out = out[comps[t]];
+    longest = std::max(longest, A.n);
+    most_rows = std::max(most_rows, a.L.ny * a.L.nz);
+    if(axis != 0) {
+      const long long b = static_cast<long long>((a.L.nx + kLineThreads - 1) / kLineThreads) *
+                          ((A.n + kLineChunk - 1) / kLineChunk) * a.L.n(axis == 1 ? 2 : 1);
+      blocks = std::max(blocks, b);
+    }
+  }
+  ProfScope ps(kKAdi, s);
+  if(axis != 0) {
+    k_adi_lines<<<dim3(static_cast<unsigned>(blocks), count), kLineThreads, 0, s>>>(q, axis);
+    OFB_LAUNCH_CHECK("k_adi_lines");
+    return;
+  }
+  // 16 rows per block (4 when that leaves fewer than two blocks per SM, or a
+  // row so long that 16 pass the block's threads or 100 KB)
+  const int chunks = (longest + kRowChunk - 1) / kRowChunk;
+  const size_t row = static_cast<size_t>(longest | 1) * sizeof(double);
+  int rows = 16;
+  if(most_rows < 2 * 148 * 16 || rows * chunks > 1024 || rows * row > 100 * 1024) rows = 4;
+  OFB_CHECK(cudaFuncSetAttribute(k_adi_rows, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                 static_cast<int>(rows * row)));
+  k_adi_rows<<<dim3((most_rows + rows - 1) / rows, count), (rows * chunks + 31) / 32 * 32, rows * row, s>>>(q, rows);
+  OFB_LAUNCH_CHECK("k_adi_rows");
+}
+
 }  // namespace
+
+void launch_adi_sweeps(const AdiPlan* p, int axis, const double* const* in, double* const* out, cudaStream_t s) {
+  int together[3], count = 0;
+  for(int c = 0; c < 3; ++c) {
+    if(!p->ax[c][axis].active) continue;
+    if(p->ax[c][axis].decay) together[count++] = c;
+    else launch_adi_sweep(p, c, axis, in[c], out[c], s);
+  }
+  if(count > 0) launch_decay(p, together, count, axis, in, out, s);
+}
 
 void launch_adi_sweep(const AdiPlan* p, int comp, int axis, const double* in, double* out,
                       cudaStream_t s) {
   const AdiAxis& A = p->ax[comp][axis];
   if(!A.active) return;
+  if(A.decay) {
+    const double* ins[3] = {in, in, in};
+    double* outs[3] = {out, out, out};
+    launch_decay(p, &comp, 1, axis, ins, outs, s);
+    return;
+  }
   SweepArgs a;
   a.L = make_lay(p->g, kFaceX + comp);
   a.axis = axis;

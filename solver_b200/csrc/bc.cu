@@ -26,11 +26,11 @@ __device__ __forceinline__ int base_index(const Lay& L, int axis, int a1, int p1
 
 // apply_velocity_component_boundaries for one axis (solver/projection.cpp:451-462):
 // apply_periodic_pair (:207-300) or apply_face_field_boundary (:384-449).
-__global__ void k_velocity_bc_axis(Grid g, VBC bc, int axis, int comp0, double* f0, double* f1,
-                                   double* f2) {
-  const int comp = comp0 + blockIdx.z;
+// axis < 0: each component's own axis.
+__global__ void k_velocity_bc_axis(Grid g, VBC bc, int axis_, double* f0, double* f1, double* f2) {
+  const int comp = blockIdx.z;
+  const int axis = axis_ < 0 ? comp : axis_;
   double* f = comp == 0 ? f0 : comp == 1 ? f1 : f2;
-  if(f == nullptr) return;
   const Lay L = make_lay(g, kFaceX + comp);
   int a1, a2;
   other_axes(axis, a1, a2);
@@ -140,18 +140,15 @@ __global__ void k_total_pressure_bc(Grid g, VBC bc, double nu, const double* u, 
 
 }  // namespace
 
-void launch_component_bc(const Grid& g, const VBC& bc, int comp, double* f, cudaStream_t s) {
-  for(int axis = 0; axis < 3; ++axis) {
-    const int d1 = (axis == 0 ? g.ny : g.nx) + 1;
-    const int d2 = (axis == 2 ? g.ny : g.nz) + 1;
-    dim3 block(32, 8, 1);
-    dim3 grid((d1 + 31) / 32, (d2 + 7) / 8, 1);
-    double* fs[3] = {nullptr, nullptr, nullptr};
-    fs[comp] = f;
-    ProfScope ps(kKVelocityBc, s);
-    k_velocity_bc_axis<<<grid, block, 0, s>>>(g, bc, axis, comp, fs[0], fs[1], fs[2]);
-    OFB_LAUNCH_CHECK("k_velocity_bc_axis");
-  }
+void launch_normal_faces(const Grid& g, const VBC& bc, double* u, double* v, double* w, cudaStream_t s) {
+  // the faces normal to x span (ny, nz), to y (nx, nz), to z (nx, ny)
+  const int d1 = g.nx > g.ny ? g.nx : g.ny;
+  const int d2 = g.ny > g.nz ? g.ny : g.nz;
+  dim3 block(32, 8, 1);
+  dim3 grid((d1 + 31) / 32, (d2 + 7) / 8, 3);
+  ProfScope ps(kKVelocityBc, s);
+  k_velocity_bc_axis<<<grid, block, 0, s>>>(g, bc, -1, u, v, w);
+  OFB_LAUNCH_CHECK("k_velocity_bc_axis");
 }
 
 void launch_velocity_bc(const Grid& g, const VBC& bc, double* u, double* v, double* w,
@@ -165,7 +162,7 @@ void launch_velocity_bc(const Grid& g, const VBC& bc, double* u, double* v, doub
     dim3 block(32, 8, 1);
     dim3 grid((d1 + 31) / 32, (d2 + 7) / 8, 3);
     ProfScope ps(kKVelocityBc, s);
-    k_velocity_bc_axis<<<grid, block, 0, s>>>(g, bc, axis, 0, u, v, w);
+    k_velocity_bc_axis<<<grid, block, 0, s>>>(g, bc, axis, u, v, w);
     OFB_LAUNCH_CHECK("k_velocity_bc_axis");
   }
 }

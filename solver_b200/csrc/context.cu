@@ -314,36 +314,43 @@ ofb::SolveScalars run_poisson(of_ctx* ctx, int max_iterations, double tolerance,
 }
 
 // solve_predictor_adi on the context's rhs buffers; returns pointers to the
-// three predicted components (rhs[] or adi_b[]).  With sweep_out, sweep
-// (component, axis) writes into sweep_out[component][axis] instead of the
-// ping-pong buffers, so every sweep's output survives the call (the adjoint
-// needs them for the viscosity derivative).
+// three predicted components (rhs[] or adi_b[]).  The reference applies each
+// component's boundary conditions before the sweeps and after each one; of
+// what they write, a later sweep or the projection reads only the active
+// faces of the component's own axis.  Those are set before the first sweep and
+// after the last -- between sweeps only where a fixed-pressure face copies its
+// neighbour: a wall face stays out of the sweep along its axis and sweeps
+// across it solve separate lines, and a duplicated periodic face keeps its
+// image's value through every sweep.  The ghosts are left to the callers that
+// return them.  With sweep_out, sweep (component, axis) writes into
+// sweep_out[component][axis] instead of the ping-pong buffers, so every sweep's
+// output survives the call (the adjoint needs them for the viscosity
+// derivative).
 void predictor_adi(of_ctx* ctx, double alpha, double* out[3], int* line_solves,
                    double* const (*sweep_out)[3] = nullptr) {
   ofb::AdiPlan* plan = alpha != 0.0 ? ctx->adi_for(alpha) : nullptr;
   int lines = 0;
+  double* b[3];
+  bool copies = false;
+  for(int f = 0; f < 6; ++f) copies = copies || ctx->bc.type[f] == ofb::kFixedPressure;
   for(int c = 0; c < 3; ++c) {
-    double* a = ctx->rhs[c];
-    double* b = ctx->adi_b[c];
-    ofb::launch_component_bc(ctx->g, ctx->bc, c, a, ctx->stream);
-    if(alpha == 0.0) {
-      out[c] = a;
-      continue;
+    out[c] = ctx->rhs[c];
+    b[c] = ctx->adi_b[c];
+  }
+  ofb::launch_normal_faces(ctx->g, ctx->bc, out[0], out[1], out[2], ctx->stream);
+  for(int axis = 0; plan != nullptr && axis < 3; ++axis) {
+    const double* from[3] = {out[0], out[1], out[2]};
+    double* to[3];
+    for(int c = 0; c < 3; ++c) to[c] = sweep_out != nullptr ? sweep_out[c][axis] : b[c];
+    ofb::launch_adi_sweeps(plan, axis, from, to, ctx->stream);
+    for(int c = 0; c < 3; ++c) {
+      if(!ofb::adi_axis_active(plan, c, axis)) continue;
+      lines += ofb::adi_line_count(plan, c, axis);
+      b[c] = out[c];
+      out[c] = to[c];
     }
-    for(int axis = 0; axis < 3; ++axis) {
-      if(ofb::adi_axis_active(plan, c, axis)) {
-        if(sweep_out != nullptr) {
-          ofb::launch_adi_sweep(plan, c, axis, a, sweep_out[c][axis], ctx->stream);
-          a = sweep_out[c][axis];
-        } else {
-          ofb::launch_adi_sweep(plan, c, axis, a, b, ctx->stream);
-          std::swap(a, b);
-        }
-        lines += ofb::adi_line_count(plan, c, axis);
-      }
-      ofb::launch_component_bc(ctx->g, ctx->bc, c, a, ctx->stream);
-    }
-    out[c] = a;
+    if(copies || axis == 2)
+      ofb::launch_normal_faces(ctx->g, ctx->bc, out[0], out[1], out[2], ctx->stream);
   }
   if(line_solves) *line_solves = lines;
 }
@@ -942,6 +949,7 @@ of_status of_solve_predictor_adi(of_ctx* ctx, double alpha, const double* rhs_u,
     }
     double* res[3];
     predictor_adi(ctx, alpha, res, line_solves);
+    ofb::launch_velocity_bc(ctx->g, ctx->bc, res[0], res[1], res[2], ctx->stream);
     for(int c = 0; c < 3; ++c) ctx->download(outp[c], res[c], 1 + c);
     ctx->sync();
   });

@@ -52,8 +52,9 @@ struct LevelScalars {
 // face fields in place.
 void launch_velocity_bc(const Grid& g, const VBC& bc, double* u, double* v, double* w,
                         cudaStream_t s);
-// Same on a single component (solve_component_adi's per-component calls).
-void launch_component_bc(const Grid& g, const VBC& bc, int comp, double* f, cudaStream_t s);
+// Of the same, only the part that writes active entries: each component along
+// its own axis (duplicated periodic faces, wall faces).
+void launch_normal_faces(const Grid& g, const VBC& bc, double* u, double* v, double* w, cudaStream_t s);
 // apply_total_pressure_boundary_conditions (solver/projection.cpp:986-1026) with
 // the wall-normal source nu * Laplacian(velocity) evaluated at the wall faces.
 void launch_total_pressure_bc(const Grid& g, const VBC& bc, double nu, const double* u,
@@ -88,6 +89,10 @@ void adi_plan_destroy(AdiPlan* p);
 // active lines of `in`, writes the solved lines of `out`.
 void launch_adi_sweep(const AdiPlan* p, int comp, int axis, const double* in, double* out,
                       cudaStream_t s);
+// The sweeps of one axis for the three components (in[c] -> out[c]; a component
+// whose axis is inactive is left alone), in one launch where they allow it.
+void launch_adi_sweeps(const AdiPlan* p, int axis, const double* const* in, double* const* out,
+                       cudaStream_t s);
 int adi_line_count(const AdiPlan* p, int comp, int axis);
 bool adi_axis_active(const AdiPlan* p, int comp, int axis);
 
