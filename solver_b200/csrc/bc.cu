@@ -99,7 +99,8 @@ __device__ __forceinline__ double diffusion_at(const Lay& L, const Grid& g, doub
 // Dirichlet ghosts (:302-337).  blockIdx.z selects the axis; axes are
 // independent because every source is an active cell.
 __global__ void k_total_pressure_bc(Grid g, VBC bc, double nu, const double* u, const double* v,
-                                    const double* w, double* p) {
+                                    const double* w, double* p, const SolveScalars* guard) {
+  if(guard != nullptr && !guard->converged) return;
   const int axis = blockIdx.z;
   const Lay P = make_lay(g, kCell);
   int a1, a2;
@@ -168,14 +169,15 @@ void launch_velocity_bc(const Grid& g, const VBC& bc, double* u, double* v, doub
 }
 
 void launch_total_pressure_bc(const Grid& g, const VBC& bc, double nu, const double* u,
-                              const double* v, const double* w, double* p, cudaStream_t s) {
+                              const double* v, const double* w, double* p, const SolveScalars* guard,
+                              cudaStream_t s) {
   const int d1 = g.nx > g.ny ? g.nx : g.ny;
   const int d2 = g.ny > g.nz ? g.ny : g.nz;
   const int dm = d1 > d2 ? d1 : d2;
   dim3 block(32, 8, 1);
   dim3 grid((dm + 31) / 32, (dm + 7) / 8, 3);
   ProfScope ps(kKTotalPressureBc, s);
-  k_total_pressure_bc<<<grid, block, 0, s>>>(g, bc, nu, u, v, w, p);
+  k_total_pressure_bc<<<grid, block, 0, s>>>(g, bc, nu, u, v, w, p, guard);
   OFB_LAUNCH_CHECK("k_total_pressure_bc");
 }
 

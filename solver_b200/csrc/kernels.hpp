@@ -57,8 +57,10 @@ void launch_velocity_bc(const Grid& g, const VBC& bc, double* u, double* v, doub
 void launch_normal_faces(const Grid& g, const VBC& bc, double* u, double* v, double* w, cudaStream_t s);
 // apply_total_pressure_boundary_conditions (solver/projection.cpp:986-1026) with
 // the wall-normal source nu * Laplacian(velocity) evaluated at the wall faces.
+// With a guard, nothing is written unless guard->converged.
 void launch_total_pressure_bc(const Grid& g, const VBC& bc, double nu, const double* u,
-                              const double* v, const double* w, double* p, cudaStream_t s);
+                              const double* v, const double* w, double* p, const SolveScalars* guard,
+                              cudaStream_t s);
 
 // ---- momentum (momentum.cu) ----
 struct PredictorArgs {
@@ -109,28 +111,25 @@ void launch_rhs_to_system(const Grid& g, const PBC& pbc, const double* rhs_padde
 // Compact initial guess from the padded pressure; sum -> sx.
 void launch_pressure_to_compact(const Grid& g, const double* p_padded, double* x,
                                 SolveScalars* sc, int zm, RedBuf rb, cudaStream_t s);
-// correct_velocity (solver/projection.cpp:1066-1095) active faces, and the
-// max |corrected - previous| reduction when prev != nullptr.
-void launch_correct_velocity(const Grid& g, const PBC& pbc, const double* x,
-                             const SolveScalars* sc, const double* pu, const double* pv,
-                             const double* pw, double scale, double* cu, double* cv, double* cw,
-                             const double* prev_u, const double* prev_v, const double* prev_w,
-                             SolveScalars* sc_out, RedBuf rb, cudaStream_t s);
-// Post-correction cell pass: divergence after, pressure mean, optional write of
-// the padded pressure correction, optional total-pressure update and CFL.
-struct CellPassArgs {
+// correct_velocity (solver/projection.cpp:1066-1095) on the active faces and
+// every cell quantity of the step's end, in one pass.
+struct FinishArgs {
   Grid g;
-  const double* u;
-  const double* v;
-  const double* w;
+  PBC pbc;
   const double* x;           // compact pressure correction (shift sc->sx)
+  const double* pred[3];
+  double scale;              // -dt / density
+  double* out[3];
+  const double* prev[3];     // for max |corrected - previous|, may be null
+  int open[6];               // fixed-pressure faces (velocity copied from inside)
   double* phi_padded;        // out (active), may be null
   double* p_total;           // in/out, may be null
   const double* rhs_padded;  // pressure rhs for the total-pressure update
   double p_rhs_scale;        // -0.5 nu dt
   double dt;                 // for the CFL diagnostic (0: skip)
+  int guard;                 // leave p_total alone unless sc->converged
 };
-void launch_cell_pass(const CellPassArgs& a, SolveScalars* sc, RedBuf rb, cudaStream_t s);
+void launch_finish(const FinishArgs& a, SolveScalars* sc, RedBuf rb, cudaStream_t s);
 
 // ---- Poisson (poisson.cu) ----
 struct PoissonPlan;  // hierarchy, coarse factorisation, work vectors
@@ -141,12 +140,19 @@ int poisson_coarse_unknowns(const PoissonPlan* p);
 size_t poisson_device_bytes(const PoissonPlan* p);
 double* poisson_b(PoissonPlan* p);  // compact system rhs
 double* poisson_x(PoissonPlan* p);  // compact solution
-// Runs the MG-PCG loop on b (with shift sc->sb) and x (shift sc->sx).  Returns
-// after the device scalars hold the final diagnostics.  `history` (host) gets
-// the residual norms when non-null.
+// Runs the MG-PCG loop on b (with shift sc->sb) and x (shift sc->sx; with
+// zero_guess x is set to zero here).  Returns after the device scalars hold the
+// final diagnostics and sc_host their copy.  `history` (host) gets the residual
+// norms when non-null.
 void poisson_solve(PoissonPlan* p, int max_iterations, double tolerance, SolveScalars* sc_dev,
                    SolveScalars* sc_host, RedBuf rb, cudaStream_t s, double* history,
-                   int history_cap);
+                   int history_cap, bool zero_guess);
+// The same, but where the whole loop runs on the device it is only enqueued:
+// returns true, and the caller copies the scalars to the host after its own
+// work on the stream and hands them to poisson_account.  Else as poisson_solve.
+bool poisson_solve_enqueue(PoissonPlan* p, int max_iterations, double tolerance, SolveScalars* sc_dev,
+                           SolveScalars* sc_host, RedBuf rb, cudaStream_t s, bool zero_guess);
+void poisson_account(PoissonPlan* p, const SolveScalars& sc_host);
 // Device time (us) of the V-cycle's coarse-level chain -- levels 1 .. coarsest,
 // as each CG iteration runs it -- replayed `reps` times from a CUDA graph of
 // that chain alone on the level-1 rhs of the last solve (nothing it writes is

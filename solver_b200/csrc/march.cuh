@@ -945,5 +945,154 @@ __global__ void __launch_bounds__(kMaxThreads, 1)
   });
 }
 
+
+// What a solve starts with; see start_solve.
+struct SolveStart {
+  double tol;
+  int max_it, n, zero_mean;
+  double* hist;
+  int hist_cap;
+};
+
+// The scalars of a new solve from its residual's sum and sum of squares
+// (linsolve/poisson_solver.cpp:717-739).
+__device__ __forceinline__ void start_solve(SolveScalars* sc, const SolveStart& a, double sum, double squares) {
+  if(!a.zero_mean) {
+    sc->sb = 0.0;
+    sc->sx = 0.0;
+    sc->removed_rhs_mean = 0.0;
+  }
+  const double sr = a.zero_mean ? sum / a.n : 0.0;
+  const double r0 = sqrt(fmax(squares - a.n * sr * sr, 0.0) / a.n);
+  sc->zero_mean = a.zero_mean;
+  sc->n = a.n;
+  sc->tol = a.tol;
+  sc->max_it = a.max_it;
+  sc->hist = a.hist;
+  sc->hist_cap = a.hist_cap;
+  sc->outer = 0;
+  sc->sr = sr;
+  sc->sum_r = sum;
+  sc->r0 = r0;
+  sc->rnorm = r0;
+  sc->iterations = 0;
+  sc->stop = 0;
+  sc->converged = r0 <= a.tol ? 1 : 0;
+  sc->rel = sc->converged || r0 <= 0.0 ? 0.0 : 1.0;
+  sc->first = 1;
+  sc->body_runs = 0;
+  sc->cont = sc->converged ? 0 : 1;
+  if(a.hist != nullptr && a.hist_cap > 0) a.hist[0] = r0;
+}
+
+// The residual r = (b - sb) - A (x - sx) in FP64.  START: of the initial guess,
+// beginning a solve; else of the mixed path's corrected solution: its norm, the
+// convergence test and the outer loop's control (si: the inner solve's scalars).
+// Bound: reads x and b, writes r (3 vectors); the column kernel it replaces took
+// 125 us at 256^3.
+template <bool SGN, bool FLAT, bool START>
+__global__ void __launch_bounds__(kMaxThreads, 1)
+    k_residual(OpInfo o, Tile t, const double* __restrict__ x, const double* __restrict__ b,
+               double* __restrict__ res, SolveScalars* sc, const SolveScalars* si, SolveStart start, RedBuf rb) {
+  using T = double;
+  extern __shared__ __align__(16) unsigned char march_sm[];
+  T* ring = reinterpret_cast<T*>(march_sm);
+  const int sw = slot_words<T>(t), pw = plane_words<T>(t);
+  T* bring = ring + kRing * sw;
+  const Place<T, SGN> pl(o, t, 1);
+  const Coef<T> co(o, FLAT);
+  const int nxy = o.L.nxy;
+  const int k0 = blockIdx.y * t.chunk, k1 = min(k0 + t.chunk, o.L.nz);
+  T* me = bring + kRing * sw + (pl.row0 + 1) * kRow<T> + pl.p;
+  pdl_enter();
+  const T sb = SGN ? 0.0 : sc->sb, sx = SGN ? 0.0 : sc->sx;
+  double acc[2] = {0.0, 0.0};
+  auto point = [&](int k, const Patch<T>& v) {
+    pl.store(res, k * nxy, v);
+#pragma unroll
+    for(int r = 0; r < 2; ++r)
+#pragma unroll
+      for(int c = 0; c < kW<T>; ++c)
+        if(pl.interior(r, c)) {
+          acc[0] += v.v[r][c];
+          acc[1] += v.v[r][c] * v.v[r][c];
+        }
+  };
+  auto centred = [&](Patch<T> q) {
+#pragma unroll
+    for(int r = 0; r < 2; ++r)
+#pragma unroll
+      for(int c = 0; c < kW<T>; ++c) q.v[r][c] -= sb;
+    return q;
+  };
+  Patch<T> xs, ys;
+  bool zn;
+  if constexpr(FLAT) {
+    Patch<T> q = pl.load(x, 0);
+    pl.settle(q, sx, false);
+    publish(me, q);
+    const Patch<T> bq = centred(pl.load(b, 0));
+    __syncthreads();
+    neighbour_sums(me, q, xs, ys);
+    point(0, residual<T, true>(co, bq, q, xs, ys, q, q));
+  } else {
+    Patch<T> X[4];
+    int zo = k0 * nxy;
+    Walk f(o, k0 + 1);
+    for(int q = 1; q <= 3; ++q) {
+      const int zx = f.kz * nxy;
+      if(f.k <= k1) pl.fetch(ring + (q & 3) * sw, x, zx);
+      if(f.k <= k1 && pl.in != 0) pl.fetch(bring + (q - 1) * sw, b, zo);
+      fetch_commit();
+      zo = zx;
+      f.next(o);
+    }
+    X[3] = pl.load(x, zplane(o, k0 - 1, zn) * nxy);
+    pl.settle(X[3], sx, zn);
+    X[0] = pl.load(x, k0 * nxy);
+    pl.settle(X[0], sx, false);
+    ring4(k0, k1 - 1, [&](auto jc, int s) {
+      constexpr int J = jc, M = (J + 3) & 3, N = (J + 1) & 3;
+      fetch_wait<2>();
+      X[N] = pl.take(ring + N * sw);
+      const int zx = f.kz * nxy;
+      if(f.k <= k1) pl.fetch(ring + J * sw, x, zx);                  // plane s + 4
+      if(f.k <= k1 && pl.in != 0) pl.fetch(bring + M * sw, b, zo);   // plane s + 3
+      __syncwarp();
+      fetch_commit();
+      zo = zx;
+      f.next(o);
+      T* pa = me + (J & 1) * pw;
+      publish(pa, X[J]);
+      pl.settle(X[N], sx, SGN && zneg(o, s + 1));
+      __syncthreads();
+      neighbour_sums(pa, X[J], xs, ys);
+      point(s, residual<T, false>(co, centred(pl.take(bring + J * sw)), X[J], xs, ys, X[M], X[N]));
+      __syncwarp();
+    });
+  }
+  const bool mx[2] = {false, false};
+  reduce_finish<2>(acc, mx, rb, [=](const Sums<2>& s) {
+    if constexpr(START) {
+      start_solve(sc, start, s.v[0], s.v[1]);
+    } else {
+      const int n = sc->n;
+      const double sr = sc->zero_mean ? s.v[0] / n : 0.0;
+      sc->sr = sr;
+      sc->sum_r = s.v[0];
+      const double rn = sqrt(fmax(s.v[1] - n * sr * sr, 0.0) / n);
+      sc->rnorm = rn;
+      sc->iterations += si->iterations;
+      sc->body_runs += si->body_runs;
+      sc->outer += 1;
+      sc->rel = sc->r0 > 0.0 ? rn / sc->r0 : 0.0;
+      if(sc->rel <= sc->tol) sc->converged = 1;
+      if(sc->hist != nullptr && sc->outer < sc->hist_cap) sc->hist[sc->outer] = rn;
+      const bool stalled = si->iterations == 0;
+      sc->cont = (sc->converged || sc->iterations >= sc->max_it || sc->outer >= 100 || stalled) ? 0 : 1;
+    }
+  });
+}
+
 }  // namespace march
 }  // namespace ofb

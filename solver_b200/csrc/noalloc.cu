@@ -52,12 +52,14 @@ __global__ void __launch_bounds__(kTX* kTY)
   const double idx = 1.0 / g.dx, idy = 1.0 / g.dy, idz = 1.0 / g.dz;
   double acc[2] = {0.0, 0.0};
   if(valid) {
+    double w0 = w[W.idx(i + 1, j + 1, k0 + 1)];  // the cell's lower z face
+#pragma unroll 2
     for(int k = k0; k < k1; ++k) {
-      const int uq = U.idx(i + 1, j + 1, k + 1), vq = V.idx(i + 1, j + 1, k + 1),
-                wq = W.idx(i + 1, j + 1, k + 1);
+      const int uq = U.idx(i + 1, j + 1, k + 1), vq = V.idx(i + 1, j + 1, k + 1);
+      const double w1 = w[W.idx(i + 1, j + 1, k + 2)];
       // compute_divergence (operators/discrete_operators.cpp:98-113)
-      const double div = (u[uq + 1] - u[uq]) * idx + (v[vq + V.sx] - v[vq]) * idy +
-                         (w[wq + W.sxy] - w[wq]) * idz;
+      const double div = (u[uq + 1] - u[uq]) * idx + (v[vq + V.sx] - v[vq]) * idy + (w1 - w0) * idz;
+      w0 = w1;
       const double r = div * scale;
       rhs[P.idx(i + 1, j + 1, k + 1)] = r;
       acc[0] += div * div;
@@ -102,7 +104,7 @@ long long noalloc_max_plane_blocks() { return kMaxBlocks; }
 void launch_pressure_rhs_noalloc(const Grid& g, const double* u, const double* v, const double* w,
                                  double scale, double* rhs, double* scratch, double* norms_host,
                                  cudaStream_t s) {
-  const Launch3 l = launch3(g.nx, g.ny, g.nz);
+  const Launch3 l = launch3(g.nx, g.ny, g.nz, kReducingBlocks);
   unsigned int* ticket = reinterpret_cast<unsigned int*>(scratch + kNaTicket);
   // the ticket must start at zero; it resets itself, but a launch that never
   // completed would leave it set

@@ -36,84 +36,10 @@ constexpr double kSmallNumber = 1.0e-30;
 constexpr double kOmega = 2.0 / 3.0;
 constexpr int kMaxCoarse = 1024;
 
-// Neighbour coordinates along one axis, branch-free: the in-range neighbour,
-// the periodic image, or the cell itself with sign +1 (homogeneous Neumann,
-// ghost = centre) or -1 (homogeneous Dirichlet, ghost = -centre)
-// (neighbor_value, linsolve/poisson_solver.cpp:195-242).  Every load is then
-// unconditional and in bounds, so a thread can keep many loads in flight.
-__device__ __forceinline__ void nb_lo(int c, int n, int per, int dir, int& cc, double& sg) {
-  const bool in = c > 0;
-  cc = in ? c - 1 : (per ? n - 1 : c);
-  sg = (in || per || !dir) ? 1.0 : -1.0;
-}
-
-__device__ __forceinline__ void nb_hi(int c, int n, int per, int dir, int& cc, double& sg) {
-  const bool in = c < n - 1;
-  cc = in ? c + 1 : (per ? 0 : c);
-  sg = (in || per || !dir) ? 1.0 : -1.0;
-}
-
-// In-plane neighbours of one (i, j) column; fixed while the thread marches in k.
-struct ColNb {
-  int xl, xr, yd, yu;
-  double sxl, sxr, syd, syu;
-};
-
-__device__ __forceinline__ ColNb col_nb(const OpInfo& o, int i, int j) {
-  ColNb c;
-  nb_lo(i, o.L.nx, o.periodic[0], o.dir_lo[0], c.xl, c.sxl);
-  nb_hi(i, o.L.nx, o.periodic[0], o.dir_hi[0], c.xr, c.sxr);
-  nb_lo(j, o.L.ny, o.periodic[1], o.dir_lo[1], c.yd, c.syd);
-  nb_hi(j, o.L.ny, o.periodic[1], o.dir_hi[1], c.yu, c.syu);
-  return c;
-}
-
-// apply_poisson_operator at (i, j, k) (linsolve/poisson_solver.cpp:244-269):
-// -(r - 2c + l)/dx^2 - (u - 2c + d)/dy^2 - (f - 2c + b)/dz^2 with the boundary
-// rules above.  val(i, j, k) returns the operand at an in-range cell.
-template <typename A, typename F>
-__device__ __forceinline__ A apply_op(const OpInfo& o, const ColNb& nb, int i, int j, int k, F val,
-                                      A& center) {
-  int kb, kf;
-  double sb, sf;
-  nb_lo(k, o.L.nz, o.periodic[2], o.dir_lo[2], kb, sb);
-  nb_hi(k, o.L.nz, o.periodic[2], o.dir_hi[2], kf, sf);
-  const A c = val(i, j, k);
-  const A l = A(nb.sxl) * val(nb.xl, j, k);
-  const A r = A(nb.sxr) * val(nb.xr, j, k);
-  const A d = A(nb.syd) * val(i, nb.yd, k);
-  const A u = A(nb.syu) * val(i, nb.yu, k);
-  const A b = A(sb) * val(i, j, kb);
-  const A f = A(sf) * val(i, j, kf);
-  center = c;
-  const A two_c = A(2) * c;
-  return -(r - two_c + l) * A(o.inv2[0]) - (u - two_c + d) * A(o.inv2[1]) -
-         (f - two_c + b) * A(o.inv2[2]);
-}
-
 template <int K>
 __device__ __forceinline__ void zero(double (&v)[K]) {
 #pragma unroll
   for(int q = 0; q < K; ++q) v[q] = 0.0;
-}
-
-// Marches k in [k0, k1) in batches of KB planes: compute(k) holds only loads
-// and arithmetic, commit(k, r) the stores and reductions, so the loads of a
-// whole batch are independent and issued together.
-constexpr int kBatch = 4;
-
-template <int KB, typename Compute, typename Commit>
-__device__ __forceinline__ void k_batched(int k0, int k1, Compute compute, Commit commit) {
-  using R = decltype(compute(0));
-  int k = k0;
-  for(; k + KB <= k1; k += KB) {
-    R r[KB];
-#pragma unroll
-    for(int t = 0; t < KB; ++t) r[t] = compute(k + t);
-#pragma unroll
-    for(int t = 0; t < KB; ++t) commit(k + t, r[t]);
-  }
-  for(; k < k1; ++k) commit(k, compute(k));
 }
 
 #define STENCIL_PROLOGUE(L)                                 \
@@ -535,53 +461,40 @@ __global__ void __launch_bounds__(kDenseThreads)
 // CG kernels (FP64 vectors).
 // ---------------------------------------------------------------------------
 
-// r = (b - sb) - A (x - sx); initial residual (linsolve/poisson_solver.cpp:717-739).
-template <typename V>
-__global__ void __launch_bounds__(kTX* kTY)
-    k_initial_residual(OpInfo o, const V* __restrict__ b, const V* __restrict__ x,
-                       V* __restrict__ r, SolveScalars* sc, int kchunk, RedBuf rb,
-                       cudaGraphConditionalHandle cond) {
-  STENCIL_PROLOGUE(o.L)
-  const double sb = sc->sb, sx = sc->sx;
-  double acc[2];
-  zero(acc);
-  if(valid) {
-    const ColNb nb = col_nb(o, i, j);
-    auto val = [&](int ii, int jj, int kk) { return double(x[o.L.idx(ii, jj, kk)]) - sx; };
-    k_batched<kBatch>(
-        k0, k1,
-        [&](int k) {
-          double c;
-          const double ax = apply_op<double>(o, nb, i, j, k, val, c);
-          return (double(b[o.L.idx(i, j, k)]) - sb) - ax;
-        },
-        [&](int k, double v) {
-          r[o.L.idx(i, j, k)] = V(v);
-          acc[0] += v;
-          acc[1] += v * v;
-        });
+// A solve from a zero guess: r = b - sb, x = 0 and the solve's scalars, in one
+// flat pass (1 vector read, 2 written; clearing x and the general residual
+// took 21 + 125 us at 256^3).
+constexpr int kFlatThreads = 256, kFlatUnroll = 4;
+
+__global__ void __launch_bounds__(kFlatThreads)
+    k_start_from_zero(int n, const double* __restrict__ b, double* __restrict__ x, double* __restrict__ r,
+                      SolveScalars* sc, march::SolveStart start, RedBuf rb) {
+  const double sb = start.zero_mean ? sc->sb : 0.0;
+  const int stride = gridDim.x * blockDim.x;
+  double acc[2] = {0.0, 0.0};
+  for(int q = blockIdx.x * blockDim.x + threadIdx.x; q < n; q += kFlatUnroll * stride) {
+    double v[kFlatUnroll];
+#pragma unroll
+    for(int u = 0; u < kFlatUnroll; ++u) v[u] = q + u * stride < n ? b[q + u * stride] - sb : 0.0;
+#pragma unroll
+    for(int u = 0; u < kFlatUnroll; ++u)
+      if(q + u * stride < n) {
+        r[q + u * stride] = v[u];
+        x[q + u * stride] = 0.0;
+        acc[0] += v[u];
+        acc[1] += v[u] * v[u];
+      }
   }
   const bool mx[2] = {false, false};
   reduce_finish<2>(acc, mx, rb, [=](const Sums<2>& s) {
-    const int n = sc->n;
-    const double sr = sc->zero_mean ? s.v[0] / n : 0.0;
-    sc->sr = sr;
-    sc->sum_r = s.v[0];
-    const double ss = fmax(s.v[1] - n * sr * sr, 0.0);
-    const double r0 = sqrt(ss / n);
-    sc->r0 = r0;
-    sc->rnorm = r0;
-    sc->rel = r0 > 0.0 ? 1.0 : 0.0;
-    sc->iterations = 0;
-    sc->stop = 0;
-    sc->converged = r0 <= sc->tol ? 1 : 0;
-    if(sc->converged) sc->rel = 0.0;
-    sc->first = 1;
-    sc->body_runs = 0;
-    sc->cont = sc->converged ? 0 : 1;
-    if(sc->hist != nullptr && sc->hist_cap > 0) sc->hist[0] = r0;
-    if(cond) cudaGraphSetConditional(cond, sc->cont);
+    sc->sx = 0.0;
+    march::start_solve(sc, start, s.v[0], s.v[1]);
   });
+}
+
+// First node of the loop graph: run the body at all?
+__global__ void k_loop_gate(const SolveScalars* sc, cudaGraphConditionalHandle cond) {
+  cudaGraphSetConditional(cond, sc->cont);
 }
 
 // Mixed path: the FP64 residual scaled to unit RMS into the FP32 inner rhs,
@@ -589,8 +502,8 @@ __global__ void __launch_bounds__(kTX* kTY)
 // way k_initial_residual does it for a zero initial guess.
 __global__ void __launch_bounds__(kTX* kTY)
     k_dc_to_inner(CLay L, const double* __restrict__ r, const SolveScalars* sc,
-                  float* __restrict__ r32, float* __restrict__ e32, SolveScalars* si, int kchunk,
-                  RedBuf rb, cudaGraphConditionalHandle cond) {
+                  float* __restrict__ r32, float* __restrict__ e32, SolveScalars* si, double inner_tol,
+                  int inner_max_it, int kchunk, RedBuf rb, cudaGraphConditionalHandle cond) {
   STENCIL_PROLOGUE(L)
   const double sr = sc->sr;
   const double inv = sc->rnorm > 0.0 ? 1.0 / sc->rnorm : 1.0;
@@ -608,7 +521,11 @@ __global__ void __launch_bounds__(kTX* kTY)
   }
   const bool mx[2] = {false, false};
   reduce_finish<2>(acc, mx, rb, [=](const Sums<2>& s) {
-    const int n = si->n;
+    const int n = sc->n;
+    si->n = n;
+    si->zero_mean = sc->zero_mean;
+    si->tol = inner_tol;
+    si->max_it = inner_max_it;
     const double srn = si->zero_mean ? s.v[0] / n : 0.0;
     si->sr = srn;
     si->sum_r = s.v[0];
@@ -653,52 +570,6 @@ __global__ void __launch_bounds__(kTX* kTY)
   });
 }
 
-// Mixed path: the FP64 residual r = (b - sb) - A (x - sx) after a correction,
-// its norm, the convergence test against the reference's relative tolerance
-// and the loop control (the total of inner iterations is the iteration count).
-__global__ void __launch_bounds__(kTX* kTY)
-    k_dc_residual(OpInfo o, const double* __restrict__ b, const double* __restrict__ x,
-                  double* __restrict__ r, SolveScalars* sc, const SolveScalars* si, int kchunk,
-                  RedBuf rb) {
-  STENCIL_PROLOGUE(o.L)
-  const double sb = sc->sb, sx = sc->sx;
-  double acc[2];
-  zero(acc);
-  if(valid) {
-    const ColNb nb = col_nb(o, i, j);
-    auto val = [&](int ii, int jj, int kk) { return x[o.L.idx(ii, jj, kk)] - sx; };
-    k_batched<kBatch>(
-        k0, k1,
-        [&](int k) {
-          double c;
-          const double ax = apply_op<double>(o, nb, i, j, k, val, c);
-          return (b[o.L.idx(i, j, k)] - sb) - ax;
-        },
-        [&](int k, double v) {
-          r[o.L.idx(i, j, k)] = v;
-          acc[0] += v;
-          acc[1] += v * v;
-        });
-  }
-  const bool mx[2] = {false, false};
-  reduce_finish<2>(acc, mx, rb, [=](const Sums<2>& s) {
-    const int n = sc->n;
-    const double srn = sc->zero_mean ? s.v[0] / n : 0.0;
-    sc->sr = srn;
-    sc->sum_r = s.v[0];
-    const double rn = sqrt(fmax(s.v[1] - n * srn * srn, 0.0) / n);
-    sc->rnorm = rn;
-    sc->iterations += si->iterations;
-    sc->body_runs += si->body_runs;
-    sc->outer += 1;
-    sc->rel = sc->r0 > 0.0 ? rn / sc->r0 : 0.0;
-    if(sc->rel <= sc->tol) sc->converged = 1;
-    if(sc->hist != nullptr && sc->outer < sc->hist_cap) sc->hist[sc->outer] = rn;
-    const bool stalled = si->iterations == 0;
-    sc->cont = (sc->converged || sc->iterations >= sc->max_it || sc->outer >= 100 || stalled) ? 0 : 1;
-  });
-}
-
 __global__ void k_compact_to_pressure(Grid g, const double* __restrict__ x, const SolveScalars* sc,
                                       double* __restrict__ p) {
   const Lay P = make_lay(g, kCell);
@@ -737,7 +608,7 @@ struct PoissonPlan {
   std::vector<Level> levels;
   int coarse_n = 0;
   LevelScalars* ls = nullptr;  // device, one per level
-  double *b = nullptr, *x = nullptr, *r = nullptr, *p = nullptr, *ap = nullptr;
+  double *b = nullptr, *x = nullptr, *r = nullptr, *p = nullptr;
   double* hist = nullptr;
   int hist_cap = 0;
   size_t bytes = 0;
@@ -748,13 +619,13 @@ struct PoissonPlan {
   long long pre_counts[kKernelCount] = {};
   long long body_counts[kKernelCount] = {};
   // mixed path: inner (FP32) CG vectors and scalars
-  float *r32 = nullptr, *e32 = nullptr, *p32 = nullptr, *ap32 = nullptr;
+  float *r32 = nullptr, *e32 = nullptr, *p32 = nullptr;
   SolveScalars* sc_in = nullptr;
   int sms = 148;         // streaming multiprocessors of the plan's device
   bool all_periodic = false;  // every face periodic: constant diagonal, no boundary signs
-  march::Tile cg_tile{};      // of k_direction and k_advance
-  dim3 cg_grid;
-  double* p2 = nullptr;     // second p buffer of the fused CG step
+  march::Tile cg_tile{}, res_tile{};  // of k_direction and k_advance; of k_residual
+  dim3 cg_grid, res_grid;
+  double* p2 = nullptr;     // second p buffer
   float* p32b = nullptr;
   // levels tail_first.. run as one matrix-vector product (k_dense_apply)
   int tail_first = -1;
@@ -1026,6 +897,13 @@ auto advance_kernel(const PoissonPlan* P, bool flat) {
   return flat ? k_advance<T, false, true> : k_advance<T, false, false>;
 }
 
+template <bool START>
+auto residual_kernel(const PoissonPlan* P, bool flat) {
+  using namespace march;
+  if(!P->zero_mean) return flat ? k_residual<true, true, START> : k_residual<true, false, START>;
+  return flat ? k_residual<false, true, START> : k_residual<false, false, START>;
+}
+
 constexpr int kMarchSmem = 224 * 1024;
 
 // Lets every instantiation use the largest tile's shared memory.
@@ -1038,6 +916,8 @@ void march_attributes(const PoissonPlan* P) {
     attr(descend_kernel<T>(P, flat));
     attr(direction_kernel<T>(P, flat));
     attr(advance_kernel<T>(P, flat));
+    attr(residual_kernel<true>(P, flat));
+    attr(residual_kernel<false>(P, flat));
     for(const bool fine : {false, true})
       for(const bool pairs : {false, true}) attr(ascend_kernel<T>(P, flat, fine, pairs));
   }
@@ -1230,19 +1110,18 @@ PoissonPlan* poisson_plan_create(const Grid& g, const PBC& pbc_in, int precision
   OFB_CHECK(cudaMalloc(&P->x, nf * sizeof(double)));
   OFB_CHECK(cudaMalloc(&P->r, nf * sizeof(double)));
   OFB_CHECK(cudaMalloc(&P->p, nf * sizeof(double)));
-  OFB_CHECK(cudaMalloc(&P->ap, nf * sizeof(double)));
   OFB_CHECK(cudaMemset(P->p, 0, nf * sizeof(double)));
   OFB_CHECK(cudaMalloc(&P->p2, nf * sizeof(double)));
   OFB_CHECK(cudaMemset(P->p2, 0, nf * sizeof(double)));
-  P->bytes += 6 * nf * sizeof(double);
+  P->bytes += 5 * nf * sizeof(double);
   if(precision == 1) {
-    for(float** v : {&P->r32, &P->e32, &P->p32, &P->ap32, &P->p32b}) {
+    for(float** v : {&P->r32, &P->e32, &P->p32, &P->p32b}) {
       OFB_CHECK(cudaMalloc(v, nf * sizeof(float)));
       OFB_CHECK(cudaMemset(*v, 0, nf * sizeof(float)));
     }
     OFB_CHECK(cudaMalloc(&P->sc_in, sizeof(SolveScalars)));
     OFB_CHECK(cudaMemset(P->sc_in, 0, sizeof(SolveScalars)));
-    P->bytes += 5 * nf * sizeof(float);
+    P->bytes += 4 * nf * sizeof(float);
   }
   {
     int dev = 0;
@@ -1256,6 +1135,7 @@ PoissonPlan* poisson_plan_create(const Grid& g, const PBC& pbc_in, int precision
     (precision == 1 ? plan_tile<float> : plan_tile<double>)(P->levels[l].L, 2, P->levels[l].rz, 2, 2, P->sms,
                                                             P->levels[l].tile, P->levels[l].tgrid);
   (precision == 1 ? plan_tile<float> : plan_tile<double>)(P->levels[0].L, 1, 1, 3, 1, P->sms, P->cg_tile, P->cg_grid);
+  plan_tile<double>(P->levels[0].L, 1, 1, 2, 1, P->sms, P->res_tile, P->res_grid);
   if(precision == 1) march_attributes<float>(P);
   else march_attributes<double>(P);
   const char* no_graph = std::getenv("ORCHARD_B200_NO_GRAPH");
@@ -1279,11 +1159,9 @@ void poisson_plan_destroy(PoissonPlan* P) {
   cudaFree(P->x);
   cudaFree(P->r);
   cudaFree(P->p);
-  cudaFree(P->ap);
   cudaFree(P->r32);
   cudaFree(P->e32);
   cudaFree(P->p32);
-  cudaFree(P->ap32);
   cudaFree(P->p2);
   cudaFree(P->p32b);
   cudaFree(P->sc_in);
@@ -1352,20 +1230,27 @@ void v_cycle(PoissonPlan* P, int l, const V* r0, SolveScalars* sc, RedBuf rb, cu
 // inner solves of the mixed path's defect correction.
 template <typename V>
 struct CGVec {
-  V *b, *x, *r, *p, *ap, *p2;  // p2: the fused step's second p buffer
+  V *x, *r, *p, *p2;  // p and p2 alternate (march::Direction)
 };
 
-CGVec<double> cg64(PoissonPlan* P) { return CGVec<double>{P->b, P->x, P->r, P->p, P->ap, P->p2}; }
+CGVec<double> cg64(PoissonPlan* P) { return CGVec<double>{P->x, P->r, P->p, P->p2}; }
 
 // Initial residual and convergence test (linsolve/poisson_solver.cpp:717-739).
-template <typename V>
-void enqueue_pre(PoissonPlan* P, const CGVec<V>& v, SolveScalars* sc, RedBuf rb, cudaStream_t s,
-                 cudaGraphConditionalHandle cond) {
+void enqueue_start(PoissonPlan* P, const march::SolveStart& start, SolveScalars* sc, RedBuf rb, cudaStream_t s,
+                   bool zero_guess) {
   const Level& l0 = P->levels[0];
-  const Launch3 ln = launch3(l0.L.nx, l0.L.ny, l0.L.nz);
   ProfScope ps(kKInitResidual, s);
-  k_initial_residual<V><<<ln.grid, ln.block, 0, s>>>(l0.op, v.b, v.x, v.r, sc, ln.kchunk, rb, cond);
-  OFB_LAUNCH_CHECK("k_initial_residual");
+  if(zero_guess) {
+    const int n = l0.L.count();
+    const int blocks = std::min(kTargetBlocks, (n + kFlatThreads - 1) / kFlatThreads);
+    k_start_from_zero<<<blocks, kFlatThreads, 0, s>>>(n, P->b, P->x, P->r, sc, start, rb);
+    OFB_LAUNCH_CHECK("k_start_from_zero");
+    return;
+  }
+  const march::Tile& t = P->res_tile;
+  launch_pdl(residual_kernel<true>(P, l0.L.nz == 1), P->res_grid, t.px * t.ey / 2, march::smem_bytes<double>(t, 2, 1),
+             s, l0.op, t, P->x, P->b, P->r, sc, static_cast<const SolveScalars*>(nullptr), start, rb);
+  OFB_LAUNCH_CHECK("k_residual");
 }
 
 // One body of the rotated PCG loop: z = M r, p = z + beta p and p.Ap, x/r update
@@ -1446,61 +1331,47 @@ void ensure_history(PoissonPlan* P, int max_iterations) {
   }
 }
 
-// Host-side initialisation of the solve scalars (b and x shifts were set by
-// the kernels that filled them).
-SolveScalars init_scalars(PoissonPlan* P, int max_iterations, double tolerance, SolveScalars* sc,
-                          SolveScalars* host, cudaStream_t s) {
-  OFB_CHECK(cudaMemcpyAsync(host, sc, sizeof(SolveScalars), cudaMemcpyDeviceToHost, s));
-  OFB_CHECK(cudaStreamSynchronize(s));
-  SolveScalars init = *host;
-  init.zero_mean = P->zero_mean;
-  init.n = P->levels[0].L.count();
-  init.tol = tolerance;
-  init.max_it = max_iterations;
-  init.hist = P->hist;
-  init.hist_cap = P->hist_cap;
-  init.outer = 0;
-  if(!P->zero_mean) {
-    init.sb = 0.0;
-    init.sx = 0.0;
-    init.removed_rhs_mean = 0.0;
+march::SolveStart solve_start(PoissonPlan* P, int max_iterations, double tolerance) {
+  ensure_history(P, max_iterations);
+  return march::SolveStart{tolerance, max_iterations, P->levels[0].L.count(), P->zero_mean, P->hist, P->hist_cap};
+}
+
+bool loop_on_device(const PoissonPlan* P) { return P->use_graph && !prof_enabled(); }
+
+// Enqueues an FP64 solve as one graph launch after its start.
+template <typename T>
+void enqueue_solve(PoissonPlan* P, int max_iterations, double tolerance, SolveScalars* sc, RedBuf rb,
+                   cudaStream_t s, bool zero_guess) {
+  enqueue_start(P, solve_start(P, max_iterations, tolerance), sc, rb, s, zero_guess);
+  if(P->exec == nullptr) {
+    const CGVec<double> v = cg64(P);
+    P->exec = build_loop_graph(
+        P, s,
+        [&](cudaGraphConditionalHandle c) {
+          k_loop_gate<<<1, 1, 0, s>>>(sc, c);
+          OFB_LAUNCH_CHECK("k_loop_gate");
+        },
+        [&](cudaGraphConditionalHandle c) { enqueue_body<T, double>(P, v, sc, rb, s, c); }, &P->graph);
   }
-  return init;
+  OFB_CHECK(cudaGraphLaunch(P->exec, s));
 }
 
 template <typename T>
 void solve_impl(PoissonPlan* P, int max_iterations, double tolerance, SolveScalars* sc,
-                SolveScalars* host, RedBuf rb, cudaStream_t s, double* history, int history_cap) {
-  ensure_history(P, max_iterations);
-  *host = init_scalars(P, max_iterations, tolerance, sc, host, s);
-  OFB_CHECK(cudaMemcpyAsync(sc, host, sizeof(SolveScalars), cudaMemcpyHostToDevice, s));
-  const CGVec<double> v = cg64(P);
-  const bool use_graph = P->use_graph && !prof_enabled();
-  if(use_graph) {
-    if(P->exec == nullptr)
-      P->exec = build_loop_graph(
-          P, s, [&](cudaGraphConditionalHandle c) { enqueue_pre<double>(P, v, sc, rb, s, c); },
-          [&](cudaGraphConditionalHandle c) { enqueue_body<T, double>(P, v, sc, rb, s, c); },
-          &P->graph);
-    OFB_CHECK(cudaGraphLaunch(P->exec, s));
+                SolveScalars* host, RedBuf rb, cudaStream_t s, double* history, int history_cap, bool zero_guess) {
+  auto read = [&] {
     OFB_CHECK(cudaMemcpyAsync(host, sc, sizeof(SolveScalars), cudaMemcpyDeviceToHost, s));
     OFB_CHECK(cudaStreamSynchronize(s));
-    prof_add_counts(P->pre_counts, 1);
-    prof_add_counts(P->body_counts, host->body_runs);
+    prof_collect();
+  };
+  if(loop_on_device(P)) {
+    enqueue_solve<T>(P, max_iterations, tolerance, sc, rb, s, zero_guess);
+    read();
+    poisson_account(P, *host);
   } else {
-    enqueue_pre<double>(P, v, sc, rb, s, 0);
-    OFB_CHECK(cudaMemcpyAsync(host, sc, sizeof(SolveScalars), cudaMemcpyDeviceToHost, s));
-    OFB_CHECK(cudaStreamSynchronize(s));
-    prof_collect();
-    while(host->cont) {
-      enqueue_body<T, double>(P, v, sc, rb, s, 0);
-      OFB_CHECK(cudaMemcpyAsync(host, sc, sizeof(SolveScalars), cudaMemcpyDeviceToHost, s));
-      OFB_CHECK(cudaStreamSynchronize(s));
-      prof_collect();
-    }
-    OFB_CHECK(cudaMemcpyAsync(host, sc, sizeof(SolveScalars), cudaMemcpyDeviceToHost, s));
-    OFB_CHECK(cudaStreamSynchronize(s));
-    prof_collect();
+    const CGVec<double> v = cg64(P);
+    enqueue_start(P, solve_start(P, max_iterations, tolerance), sc, rb, s, zero_guess);
+    for(read(); host->cont; read()) enqueue_body<T, double>(P, v, sc, rb, s, 0);
   }
   if(history != nullptr && history_cap > 0) {
     const int n = std::min(history_cap, std::min(host->iterations + 1, P->hist_cap));
@@ -1522,43 +1393,32 @@ constexpr int kInnerMaxIt = 60;
 
 template <typename T>
 void solve_dc(PoissonPlan* P, int max_iterations, double tolerance, SolveScalars* sc,
-              SolveScalars* host, RedBuf rb, cudaStream_t s, double* history, int history_cap) {
-  ensure_history(P, max_iterations);
-  SolveScalars init = init_scalars(P, max_iterations, tolerance, sc, host, s);
-  *host = init;
-  OFB_CHECK(cudaMemcpyAsync(sc, host, sizeof(SolveScalars), cudaMemcpyHostToDevice, s));
-  SolveScalars in{};
-  in.zero_mean = P->zero_mean;
-  in.n = init.n;
-  in.tol = kInnerTol;
-  in.max_it = kInnerMaxIt;
-  OFB_CHECK(cudaMemcpyAsync(P->sc_in, &in, sizeof(SolveScalars), cudaMemcpyHostToDevice, s));
+              SolveScalars* host, RedBuf rb, cudaStream_t s, double* history, int history_cap, bool zero_guess) {
   const Level& l0 = P->levels[0];
-  const Launch3 ln = launch3(l0.L.nx, l0.L.ny, l0.L.nz);
-  // outer residual of the initial guess
-  {
-    ProfScope ps(kKInitResidual, s);
-    k_initial_residual<double><<<ln.grid, ln.block, 0, s>>>(l0.op, P->b, P->x, P->r, sc, ln.kchunk,
-                                                            rb, 0);
-    OFB_LAUNCH_CHECK("k_initial_residual");
-  }
+  const Launch3 ln = launch3(l0.L.nx, l0.L.ny, l0.L.nz, kReducingBlocks);
+  const march::SolveStart start = solve_start(P, max_iterations, tolerance);
+  enqueue_start(P, start, sc, rb, s, zero_guess);
   OFB_CHECK(cudaMemcpyAsync(host, sc, sizeof(SolveScalars), cudaMemcpyDeviceToHost, s));
   OFB_CHECK(cudaStreamSynchronize(s));
-  const CGVec<float> v{nullptr, P->e32, P->r32, P->p32, P->ap32, P->p32b};
+  const CGVec<float> v{P->e32, P->r32, P->p32, P->p32b};
   SolveScalars* si = P->sc_in;
   auto pre = [&](cudaGraphConditionalHandle c) {
     ProfScope ps(kKDefectCorrection, s);
-    k_dc_to_inner<<<ln.grid, ln.block, 0, s>>>(l0.L, P->r, sc, P->r32, P->e32, si, ln.kchunk, rb, c);
+    k_dc_to_inner<<<ln.grid, ln.block, 0, s>>>(l0.L, P->r, sc, P->r32, P->e32, si, kInnerTol,
+                                               kInnerMaxIt, ln.kchunk, rb, c);
     OFB_LAUNCH_CHECK("k_dc_to_inner");
   };
   auto body = [&](cudaGraphConditionalHandle c) { enqueue_body<T, float>(P, v, si, rb, s, c); };
   auto post = [&]() {
     ProfScope ps(kKDefectCorrection, s, 2);
     k_dc_update_x<<<ln.grid, ln.block, 0, s>>>(l0.L, P->x, P->e32, sc, si, ln.kchunk, rb);
-    k_dc_residual<<<ln.grid, ln.block, 0, s>>>(l0.op, P->b, P->x, P->r, sc, si, ln.kchunk, rb);
+    const march::Tile& t = P->res_tile;
+    launch_pdl(residual_kernel<false>(P, l0.L.nz == 1), P->res_grid, t.px * t.ey / 2,
+               march::smem_bytes<double>(t, 2, 1), s, l0.op, t, P->x, P->b, P->r, sc,
+               static_cast<const SolveScalars*>(si), start, rb);
     OFB_LAUNCH_CHECK("defect correction update");
   };
-  const bool use_graph = P->use_graph && !prof_enabled();
+  const bool use_graph = loop_on_device(P);
   long long inner_runs = 0;
   while(host->cont) {
     if(use_graph) {
@@ -1596,13 +1456,28 @@ void solve_dc(PoissonPlan* P, int max_iterations, double tolerance, SolveScalars
 
 }  // namespace
 
+void poisson_account(PoissonPlan* P, const SolveScalars& host) {
+  prof_add_counts(P->pre_counts, 1);
+  prof_add_counts(P->body_counts, host.body_runs);
+}
+
 void poisson_solve(PoissonPlan* P, int max_iterations, double tolerance, SolveScalars* sc_dev,
                    SolveScalars* sc_host, RedBuf rb, cudaStream_t s, double* history,
-                   int history_cap) {
+                   int history_cap, bool zero_guess) {
   if(P->precision == 1)
-    solve_dc<float>(P, max_iterations, tolerance, sc_dev, sc_host, rb, s, history, history_cap);
+    solve_dc<float>(P, max_iterations, tolerance, sc_dev, sc_host, rb, s, history, history_cap, zero_guess);
   else
-    solve_impl<double>(P, max_iterations, tolerance, sc_dev, sc_host, rb, s, history, history_cap);
+    solve_impl<double>(P, max_iterations, tolerance, sc_dev, sc_host, rb, s, history, history_cap, zero_guess);
+}
+
+bool poisson_solve_enqueue(PoissonPlan* P, int max_iterations, double tolerance, SolveScalars* sc_dev,
+                           SolveScalars* sc_host, RedBuf rb, cudaStream_t s, bool zero_guess) {
+  if(P->precision == 1 || !loop_on_device(P)) {
+    poisson_solve(P, max_iterations, tolerance, sc_dev, sc_host, rb, s, nullptr, 0, zero_guess);
+    return false;
+  }
+  enqueue_solve<double>(P, max_iterations, tolerance, sc_dev, rb, s, zero_guess);
+  return true;
 }
 
 double poisson_time_coarse_chain(PoissonPlan* P, RedBuf rb, cudaStream_t s, int reps, int* launches) {
