@@ -3,6 +3,7 @@
 // each entry point validates its arguments with the reference's messages,
 // enqueues the kernels and returns after the diagnostics are on the host.
 #include "../../include/orchard_b200.h"
+#include "hostcopy.hpp"
 #include "kernels.hpp"
 
 #include <algorithm>
@@ -156,6 +157,11 @@ struct of_ctx {
   size_t bytes = 0;
   AdjWork* adj = nullptr;
 
+  cudaEvent_t slot_done[ofb::kStagingSlots] = {};  // staged transfers
+
+  of_ctx() { ofb::staging_retain(); }
+  of_ctx(const of_ctx&) = delete;
+  of_ctx& operator=(const of_ctx&) = delete;
   ~of_ctx() {
     cudaSetDevice(device);
     if(stream) cudaStreamSynchronize(stream);
@@ -183,7 +189,10 @@ struct of_ctx {
       cudaStreamDestroy(side);
     }
     if(adv_ready) cudaEventDestroy(adv_ready);
+    for(cudaEvent_t e : slot_done)
+      if(e) cudaEventDestroy(e);
     if(stream) cudaStreamDestroy(stream);
+    ofb::staging_release();
   }
 
   double* alloc(size_t n) {
@@ -196,11 +205,142 @@ struct of_ctx {
 
   size_t size(int loc) const { return lay[loc].size(); }
 
+  // A whole field between the caller's array and the device.  active_only (to
+  // the host): the array's ghost entries are left as they are.
+  struct Transfer {
+    double* dev;
+    double* host;
+    int loc;
+    bool active_only;
+  };
+
+  // Uploads / downloads fields in order on the stream.  Pageable arrays of
+  // kStagedBytes and more go through the pinned staging slots (hostcopy.hpp),
+  // chunk by chunk; the rest by plain copies.  Staged downloads have arrived
+  // on return, plain ones with the next sync().
+  static constexpr size_t kStagedBytes = size_t(128) << 10;
+
+  void upload(const std::vector<Transfer>& list) { transfer(list, true); }
+  void download(const std::vector<Transfer>& list) { transfer(list, false); }
   void upload(double* dst, const double* src, int loc) {
-    OFB_CHECK(cudaMemcpyAsync(dst, src, size(loc) * sizeof(double), cudaMemcpyHostToDevice, stream));
+    upload({Transfer{dst, const_cast<double*>(src), loc, false}});
   }
   void download(double* dst, const double* src, int loc) {
-    OFB_CHECK(cudaMemcpyAsync(dst, src, size(loc) * sizeof(double), cudaMemcpyDeviceToHost, stream));
+    download({Transfer{const_cast<double*>(src), dst, loc, false}});
+  }
+
+  static bool pageable(const void* p) {
+    cudaPointerAttributes a{};
+    if(cudaPointerGetAttributes(&a, p) != cudaSuccess) {
+      cudaGetLastError();
+      return true;
+    }
+    return a.type == cudaMemoryTypeUnregistered;
+  }
+
+  void transfer(const std::vector<Transfer>& list, bool up) {
+    struct Chunk {
+      const Transfer* t;
+      size_t first, count;  // doubles
+    };
+    std::vector<Chunk> staged;
+    std::vector<const Transfer*> plain;
+    for(const Transfer& t : list) {
+      if(size(t.loc) * sizeof(double) < kStagedBytes || !pageable(t.host)) {
+        plain.push_back(&t);
+        continue;
+      }
+      const size_t n = size(t.loc), step = ofb::kStagingBytes / sizeof(double);
+      for(size_t f = 0; f < n; f += step) staged.push_back(Chunk{&t, f, std::min(step, n - f)});
+    }
+    if(!staged.empty()) {
+      ofb::StagingLease lease;
+      if(lease) {
+        for(cudaEvent_t& e : slot_done)
+          if(e == nullptr) OFB_CHECK(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
+        constexpr int S = ofb::kStagingSlots;
+        const int n = static_cast<int>(staged.size());
+        auto slot = [&](int i) { return reinterpret_cast<double*>(lease.slot(i % S)); };
+        auto done = [&](int i) { OFB_CHECK(cudaEventSynchronize(slot_done[i % S])); };
+        auto send = [&](int i) {  // the bus's part of chunk i
+          const Chunk& c = staged[i];
+          double* dev = c.t->dev + c.first;
+          if(up)
+            OFB_CHECK(cudaMemcpyAsync(dev, slot(i), c.count * sizeof(double), cudaMemcpyHostToDevice, stream));
+          else
+            OFB_CHECK(cudaMemcpyAsync(slot(i), dev, c.count * sizeof(double), cudaMemcpyDeviceToHost, stream));
+          OFB_CHECK(cudaEventRecord(slot_done[i % S], stream));
+        };
+        auto copy = [&](int i) {  // the host's part of chunk i
+          const Chunk& c = staged[i];
+          const size_t part = size_t(16) << 10;  // doubles
+          const int parts = static_cast<int>((c.count + part - 1) / part);
+          lease.parallel(parts, [&](int p) {
+            const size_t f = p * part, m = std::min(part, c.count - f);
+            if(up) std::memcpy(slot(i) + f, c.t->host + c.first + f, m * sizeof(double));
+            else if(!c.t->active_only) std::memcpy(c.t->host + c.first + f, slot(i) + f, m * sizeof(double));
+            else copy_active(lay[c.t->loc], c.t->host, slot(i) + f, c.first + f, m);
+          });
+        };
+        if(up) {
+          for(int i = 0; i < n; ++i) {
+            if(i >= S) done(i);
+            copy(i);
+            send(i);
+          }
+        } else {
+          for(int i = 0; i < std::min(n, S); ++i) send(i);
+          // fresh result arrays: their pages are mapped while the device works,
+          // a worker to a chunk (whole huge pages)
+          if(n > 2 * S)
+            lease.parallel(n, [&](int i) {
+              ofb::populate(staged[i].t->host + staged[i].first, staged[i].count * sizeof(double));
+            });
+          for(int i = 0; i < n; ++i) {
+            done(i);
+            copy(i);
+            if(i + S < n) send(i + S);
+          }
+        }
+        // the slots go to the next lease idle
+        for(int i = std::max(0, n - S); i < n; ++i) done(i);
+      } else {
+        for(const Transfer& t : list)
+          if(std::find(plain.begin(), plain.end(), &t) == plain.end()) plain.push_back(&t);
+      }
+    }
+    for(const Transfer* t : plain) {
+      const size_t bytes = size(t->loc) * sizeof(double);
+      if(up) {
+        OFB_CHECK(cudaMemcpyAsync(t->dev, t->host, bytes, cudaMemcpyHostToDevice, stream));
+      } else if(!t->active_only) {
+        OFB_CHECK(cudaMemcpyAsync(t->host, t->dev, bytes, cudaMemcpyDeviceToHost, stream));
+      } else if(pageable(t->host)) {
+        std::vector<double> whole(size(t->loc));
+        OFB_CHECK(cudaMemcpyAsync(whole.data(), t->dev, bytes, cudaMemcpyDeviceToHost, stream));
+        sync();
+        copy_active(lay[t->loc], t->host, whole.data(), 0, whole.size());
+      } else {
+        const Lay& L = lay[t->loc];
+        cudaMemcpy3DParms c = {};
+        c.srcPtr = make_cudaPitchedPtr(t->dev, L.sx * sizeof(double), L.sx, L.sy);
+        c.dstPtr = make_cudaPitchedPtr(t->host, L.sx * sizeof(double), L.sx, L.sy);
+        c.srcPos = c.dstPos = make_cudaPos(sizeof(double), 1, 1);
+        c.extent = make_cudaExtent(L.nx * sizeof(double), L.ny, L.nz);
+        c.kind = cudaMemcpyDeviceToHost;
+        OFB_CHECK(cudaMemcpy3DAsync(&c, stream));
+      }
+    }
+  }
+
+  // Entries [first, first + count) of a field's storage from src, active ones only.
+  static void copy_active(const Lay& L, double* field, const double* src, size_t first, size_t count) {
+    for(size_t row = first / L.sx; row * L.sx < first + count; ++row) {
+      const int j = static_cast<int>(row % L.sy), k = static_cast<int>(row / L.sy);
+      if(j < 1 || j > L.ny || k < 1 || k > L.nz) continue;
+      const size_t lo = std::max(first, row * L.sx + 1), hi = std::min(first + count, row * L.sx + 1 + L.nx);
+      if(lo < hi) std::memcpy(field + lo, src + (lo - first), (hi - lo) * sizeof(double));
+    }
   }
   void d2d(double* dst, const double* src, int loc) {
     OFB_CHECK(cudaMemcpyAsync(dst, src, size(loc) * sizeof(double), cudaMemcpyDeviceToDevice, stream));
@@ -937,13 +1077,16 @@ of_status of_compute_advection_term(of_ctx* ctx, const double* u, const double* 
     require_ptr(aw, "advection z");
     const double* in[3] = {u, v, w};
     double* out[3] = {au, av, aw};
+    using T = of_ctx::Transfer;
+    std::vector<T> up, down;
     for(int c = 0; c < 3; ++c) {
-      ctx->upload(ctx->corrected[c], in[c], 1 + c);
-      ctx->upload(ctx->adv_cur[c], out[c], 1 + c);
+      up.push_back(T{ctx->corrected[c], const_cast<double*>(in[c]), 1 + c, false});
+      down.push_back(T{ctx->adv_cur[c], out[c], 1 + c, true});
     }
+    ctx->upload(up);
     ofb::launch_advection(ctx->g, ctx->corrected[0], ctx->corrected[1], ctx->corrected[2],
                           ctx->adv_cur[0], ctx->adv_cur[1], ctx->adv_cur[2], ctx->stream);
-    for(int c = 0; c < 3; ++c) ctx->download(out[c], ctx->adv_cur[c], 1 + c);
+    ctx->download(down);
     ctx->sync();
     ctx->state_clean = false;
   });
@@ -960,13 +1103,17 @@ of_status of_solve_predictor_adi(of_ctx* ctx, double alpha, const double* rhs_u,
     for(int c = 0; c < 3; ++c) {
       require_ptr(in[c], "predictor rhs");
       require_ptr(outp[c], "predicted velocity");
-      ctx->upload(ctx->rhs[c], in[c], 1 + c);
-      ctx->d2d(ctx->adi_b[c], ctx->rhs[c], 1 + c);  // edge ghosts follow the input
     }
+    using T = of_ctx::Transfer;
+    std::vector<T> up, down;
+    for(int c = 0; c < 3; ++c) up.push_back(T{ctx->rhs[c], const_cast<double*>(in[c]), 1 + c, false});
+    ctx->upload(up);
+    for(int c = 0; c < 3; ++c) ctx->d2d(ctx->adi_b[c], ctx->rhs[c], 1 + c);  // edge ghosts follow the input
     double* res[3];
     predictor_adi(ctx, alpha, res, line_solves);
     ofb::launch_velocity_bc(ctx->g, ctx->bc, res[0], res[1], res[2], ctx->stream);
-    for(int c = 0; c < 3; ++c) ctx->download(outp[c], res[c], 1 + c);
+    for(int c = 0; c < 3; ++c) down.push_back(T{res[c], outp[c], 1 + c, false});
+    ctx->download(down);
     ctx->sync();
   });
 }
@@ -987,8 +1134,8 @@ of_status of_solve_pressure_poisson(of_ctx* ctx, const of_pbc* pbc_in, int max_i
     int zm = 1;
     for(int f = 0; f < 6; ++f)
       if(p.type[f] == ofb::kPDirichlet) zm = 0;
-    ctx->upload(ctx->prhs, rhs, 0);
-    ctx->upload(ctx->phi, pressure, 0);
+    ctx->upload({of_ctx::Transfer{ctx->prhs, const_cast<double*>(rhs), 0, false},
+                 of_ctx::Transfer{ctx->phi, pressure, 0, false}});
     ofb::launch_rhs_to_system(ctx->g, p, ctx->prhs, ofb::poisson_b(plan), ctx->sc, ctx->rb, ctx->stream);
     ofb::launch_pressure_to_compact(ctx->g, ctx->phi, ofb::poisson_x(plan), ctx->sc, zm, ctx->rb,
                                     ctx->stream);
@@ -1025,10 +1172,12 @@ of_status of_project_velocity(of_ctx* ctx, double dt, double density, int max_it
     int zm = 1;
     for(int f = 0; f < 6; ++f)
       if(ctx->pbc.type[f] == ofb::kPDirichlet) zm = 0;
-    for(int c = 0; c < 3; ++c) ctx->upload(ctx->rhs[c], in[c], 1 + c);
+    using T = of_ctx::Transfer;
+    std::vector<T> up, down;
+    for(int c = 0; c < 3; ++c) up.push_back(T{ctx->rhs[c], const_cast<double*>(in[c]), 1 + c, false});
+    up.push_back(T{ctx->phi, pressure_correction, 0, false});
+    ctx->upload(up);
     ofb::launch_velocity_bc(ctx->g, ctx->bc, ctx->rhs[0], ctx->rhs[1], ctx->rhs[2], ctx->stream);
-    ctx->upload(ctx->phi, pressure_correction, 0);
-    if(pressure_rhs) ctx->upload(ctx->prhs, pressure_rhs, 0);
     ofb::launch_divergence_rhs(ctx->g, ctx->pbc, ctx->rhs[0], ctx->rhs[1], ctx->rhs[2],
                                density / dt, ctx->prhs, ofb::poisson_b(plan), ctx->sc, ctx->rb,
                                ctx->stream);
@@ -1044,9 +1193,10 @@ of_status of_project_velocity(of_ctx* ctx, double dt, double density, int max_it
                             ctx->corrected[2], ctx->stream);
     OFB_CHECK(cudaMemcpyAsync(ctx->sc_host, ctx->sc, sizeof(ofb::SolveScalars),
                               cudaMemcpyDeviceToHost, ctx->stream));
-    for(int c = 0; c < 3; ++c) ctx->download(outp[c], ctx->corrected[c], 1 + c);
-    ctx->download(pressure_correction, ctx->phi, 0);
-    if(pressure_rhs) ctx->download(pressure_rhs, ctx->prhs, 0);
+    for(int c = 0; c < 3; ++c) down.push_back(T{ctx->corrected[c], outp[c], 1 + c, false});
+    down.push_back(T{ctx->phi, pressure_correction, 0, true});
+    if(pressure_rhs) down.push_back(T{ctx->prhs, pressure_rhs, 0, true});
+    ctx->download(down);
     ctx->sync();
     s = *ctx->sc_host;
     if(diag) {

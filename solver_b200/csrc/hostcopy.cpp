@@ -1,0 +1,163 @@
+#include "hostcopy.hpp"
+
+#include <cuda_runtime.h>
+#include <sys/mman.h>
+#include <unistd.h>
+
+#include <algorithm>
+#include <atomic>
+#include <chrono>
+#include <condition_variable>
+#include <cstdint>
+#include <memory>
+#include <mutex>
+#include <thread>
+#include <vector>
+
+namespace ofb {
+
+namespace {
+
+// Workers wait for the next job actively for a short while (the chunks of one
+// transfer follow each other within it), then asleep.
+constexpr auto kSpin = std::chrono::microseconds(200);
+
+class Workers {
+ public:
+  explicit Workers(int n) {
+    for(int i = 0; i < n; ++i) {
+      try {
+        threads_.emplace_back([this] { loop(); });
+      } catch(...) {
+        break;  // the calling thread does the work alone
+      }
+    }
+  }
+  ~Workers() {
+    {
+      std::lock_guard<std::mutex> lock(mutex_);
+      quit_ = true;
+    }
+    wake_.notify_all();
+    for(std::thread& t : threads_) t.join();
+  }
+
+  void run(int parts, const std::function<void(int)>& fn) {
+    auto job = std::make_shared<Job>();
+    job->fn = &fn;
+    job->parts = parts;
+    {
+      std::lock_guard<std::mutex> lock(mutex_);
+      job_ = job;
+      epoch_.fetch_add(1, std::memory_order_release);
+    }
+    if(asleep_.load(std::memory_order_acquire) > 0) wake_.notify_all();
+    job->work();
+    while(job->done.load(std::memory_order_acquire) < parts) std::this_thread::yield();
+  }
+
+ private:
+  // Parts are taken from a counter, so a worker that comes late finds none and
+  // never touches fn after run() has returned.
+  struct Job {
+    const std::function<void(int)>* fn;
+    int parts;
+    std::atomic<int> next{0}, done{0};
+    void work() {
+      for(int i; (i = next.fetch_add(1)) < parts;) {
+        (*fn)(i);
+        done.fetch_add(1, std::memory_order_release);
+      }
+    }
+  };
+
+  void loop() {
+    unsigned seen = 0;
+    for(;;) {
+      const auto until = std::chrono::steady_clock::now() + kSpin;
+      while(epoch_.load(std::memory_order_acquire) == seen && std::chrono::steady_clock::now() < until)
+        std::this_thread::yield();
+      std::shared_ptr<Job> job;
+      {
+        std::unique_lock<std::mutex> lock(mutex_);
+        asleep_.fetch_add(1);
+        wake_.wait(lock, [&] { return quit_ || epoch_.load() != seen; });
+        asleep_.fetch_sub(1);
+        if(quit_) return;
+        seen = epoch_.load();
+        job = job_;
+      }
+      job->work();
+    }
+  }
+
+  std::vector<std::thread> threads_;
+  std::mutex mutex_;
+  std::condition_variable wake_;
+  std::shared_ptr<Job> job_;
+  std::atomic<unsigned> epoch_{0};
+  std::atomic<int> asleep_{0};
+  bool quit_ = false;
+};
+
+std::mutex g_mutex;  // guards the three below
+int g_contexts = 0;
+bool g_leased = false;
+char* g_slots = nullptr;
+std::unique_ptr<Workers> g_workers;
+
+}  // namespace
+
+void populate(void* p, size_t bytes) {
+#ifndef MADV_POPULATE_WRITE
+#define MADV_POPULATE_WRITE 23  // Linux 5.14; older kernels refuse it
+#endif
+  static const uintptr_t page = static_cast<uintptr_t>(sysconf(_SC_PAGESIZE));
+  const uintptr_t lo = reinterpret_cast<uintptr_t>(p) / page * page;
+  const uintptr_t hi = (reinterpret_cast<uintptr_t>(p) + bytes + page - 1) / page * page;
+  madvise(reinterpret_cast<void*>(lo), hi - lo, MADV_POPULATE_WRITE);
+}
+
+void staging_retain() {
+  std::lock_guard<std::mutex> lock(g_mutex);
+  ++g_contexts;
+}
+
+void staging_release() {
+  std::unique_ptr<Workers> workers;
+  std::lock_guard<std::mutex> lock(g_mutex);
+  if(--g_contexts > 0 || g_leased) return;
+  workers = std::move(g_workers);
+  if(g_slots != nullptr) cudaFreeHost(g_slots);
+  g_slots = nullptr;
+}
+
+StagingLease::StagingLease() {
+  std::lock_guard<std::mutex> lock(g_mutex);
+  if(g_leased) return;
+  if(g_slots == nullptr) {
+    void* p = nullptr;
+    if(cudaHostAlloc(&p, kStagingSlots * kStagingBytes, cudaHostAllocPortable) != cudaSuccess) {
+      cudaGetLastError();
+      return;
+    }
+    g_slots = static_cast<char*>(p);
+  }
+  if(g_workers == nullptr) {
+    const int cores = static_cast<int>(std::thread::hardware_concurrency());
+    g_workers = std::make_unique<Workers>(std::min(7, std::max(0, cores - 1)));
+  }
+  g_leased = held_ = true;
+}
+
+StagingLease::~StagingLease() {
+  if(!held_) return;
+  std::lock_guard<std::mutex> lock(g_mutex);
+  g_leased = false;
+}
+
+char* StagingLease::slot(int i) const { return g_slots + i * kStagingBytes; }
+
+void StagingLease::parallel(int parts, const std::function<void(int)>& fn) const { g_workers->run(parts, fn); }
+
+}  // namespace ofb

@@ -1,0 +1,75 @@
+"""Seam calls on pageable arrays large enough for the staged transfers.
+
+Staged (pageable), plain (pinned) and contended (two threads at once, one of
+which finds the staging slots taken) transfers move the same bytes: results
+must be bitwise equal, and entries the reference leaves alone -- the ghosts of
+the advection term and of the pressure fields -- must come back as passed in.
+The sizes give fields below and above one slot (2 MiB) and storage rows that
+straddle its chunks.
+"""
+import threading
+
+import numpy as np
+import pytest
+
+import solver_b200 as sb
+
+pytestmark = pytest.mark.gpu
+
+SIZES = [(28, 30, 24), (64, 62, 60), (96, 56, 144)]
+
+
+def _pinned(a):
+    import torch
+    t = torch.empty(a.shape, dtype=torch.float64, pin_memory=True)
+    t.numpy()[...] = a
+    return t.numpy()
+
+
+def _calls(ctx, g, vel, wrap):
+    rng = np.random.default_rng(7)
+    adv = [wrap(rng.standard_normal(g.shape(c))) for c in "uvw"]
+    before = [a.copy() for a in adv]
+    ctx.compute_advection_term(*[wrap(v) for v in vel], out=adv)
+    for a, b in zip(adv, before):
+        ghost = np.ones(a.shape, bool)
+        ghost[1:-1, 1:-1, 1:-1] = False
+        assert np.array_equal(a[ghost], b[ghost])
+        assert not np.array_equal(a[~ghost], b[~ghost])
+    pred, lines = ctx.solve_predictor_adi([wrap(v) for v in vel], 0.002)
+    phi, rhs = wrap(np.full(g.shape("p"), 0.25)), wrap(np.full(g.shape("p"), 0.5))
+    out, _, _, _ = ctx.project_velocity([wrap(v) for v in vel], 0.01, 1.0, 60, 1e-6, pressure_correction=phi,
+                                        pressure_rhs=rhs)
+    for a, v in ((phi, 0.25), (rhs, 0.5)):
+        ghost = np.ones(a.shape, bool)
+        ghost[1:-1, 1:-1, 1:-1] = False
+        assert np.all(a[ghost] == v)
+    return [np.array(x) for x in adv + pred + out + [phi, rhs]]
+
+
+@pytest.mark.parametrize("size", SIZES, ids=lambda s: "x".join(map(str, s)))
+def test_staged_transfers_equal_plain_ones(size):
+    g = sb.Grid(*size, 0.1, 0.1, 0.1)
+    bc = [sb.PERIODIC, sb.PERIODIC, sb.NO_SLIP_WALL, sb.NO_SLIP_WALL, sb.PERIODIC, sb.PERIODIC]
+    rng = np.random.default_rng(1)
+    vel = [rng.standard_normal(g.shape(c)) for c in "uvw"]
+    with sb.Context(g, bc) as ctx:
+        plain = _calls(ctx, g, vel, _pinned)
+        staged = _calls(ctx, g, vel, np.array)
+    for a, b in zip(plain, staged):
+        assert np.array_equal(a, b)
+
+    got = {}
+
+    def work(k):
+        with sb.Context(g, bc) as c:
+            got[k] = _calls(c, g, vel, np.array)
+
+    threads = [threading.Thread(target=work, args=(k,)) for k in range(2)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    for k in range(2):
+        for a, b in zip(plain, got[k]):
+            assert np.array_equal(a, b)
