@@ -293,15 +293,22 @@ inline void check_cuda(cudaError_t e, const char* what) {
 // a CUDA graph the dependency becomes a programmatic edge.  Every kernel
 // launched this way calls pdl_enter() before it touches global memory: it
 // waits until the grids it depends on have completed and their writes are
-// visible (a no-op under a plain launch).  No kernel triggers its dependents
-// early (griddepcontrol.launch_dependents): at 256^3 that made the graph-run
-// step 5 % slower, the resident waiting blocks of the next kernel getting in
-// the way of the running one, while the implicit trigger at block exit gains
-// 0.3 % in the graph and 16 % on the coarse levels of a host-driven loop.
+// visible (a no-op under a plain launch).  Kernels on few blocks also let their
+// dependents launch at once (pdl_early): the next kernel's blocks then set up
+// on idle SMs and wait there (2D 512^2 step 866 -> 814 us,
+// 128^3 3483 -> 3320).  On grids that fill the GPU the waiting blocks get in the
+// way of the running ones (5 % of a 256^3 step), so those trigger at exit.  A
+// waiting grid holds no block back: it launches only when every block of the
+// one before it is resident.
 // ORCHARD_B200_NO_PDL=1 makes every launch plain.
 // ---------------------------------------------------------------------------
 
 __device__ __forceinline__ void pdl_enter() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+
+constexpr unsigned kEarlyBlocks = 400;
+__device__ __forceinline__ void pdl_early() {
+  if(gridDim.x * gridDim.y <= kEarlyBlocks) asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
 
 inline bool pdl_enabled() {
   static const bool on = [] {

@@ -314,6 +314,8 @@ __device__ __forceinline__ void fetch_wait() {
 // Words of one published plane, its guard rows included, and of one ring
 // slot; the shared memory of a kernel that streams `streams` vectors and
 // publishes `fields` fields (two planes each): rings, planes, diagonal table.
+// A grid one cell deep streams nothing and needs one plane per field.
+// `parents`: room for the coarse correction's ring (k_ascend).
 template <typename T>
 __host__ __device__ inline int plane_words(const Tile& t) {
   return (t.ey + 2) * kRow<T>;
@@ -323,9 +325,11 @@ __host__ __device__ inline int slot_words(const Tile& t) {
   return kW<T> * t.px * t.ey;
 }
 template <typename T>
-inline size_t smem_bytes(const Tile& t, int streams, int fields) {
+inline size_t smem_bytes(const Tile& t, int streams, int fields, bool flat, bool parents = false) {
+  if(flat) return (static_cast<size_t>(fields) * plane_words<T>(t) + 64) * sizeof(T);
   return (static_cast<size_t>(kRing) * streams * slot_words<T>(t) +
-          static_cast<size_t>(2) * fields * plane_words<T>(t) + 64) * sizeof(T);
+          static_cast<size_t>(2) * fields * plane_words<T>(t) + 64) * sizeof(T) +
+         (parents ? static_cast<size_t>(kRing) * (t.px * t.ey / 2) * 8 : 0);
 }
 
 // The image plane of k, -2 <= k <= nz + 1 with nz >= 2, and whether it is a
@@ -446,8 +450,8 @@ __global__ void __launch_bounds__(kMaxThreads, 1)
   extern __shared__ __align__(16) unsigned char march_sm[];
   T* ring = reinterpret_cast<T*>(march_sm);
   const int sw = slot_words<T>(t), pw = plane_words<T>(t);
-  T* planes = ring + kRing * 1 * sw;
-  T* tab = planes + 4 * pw;
+  T* planes = FLAT ? ring : ring + kRing * sw;
+  T* tab = planes + (FLAT ? 2 : 4) * pw;
   if constexpr(!CD) {
     for(int q = threadIdx.x; q < 64; q += blockDim.x) tab[q] = T(2.0 / 3.0 * o.invd[q]);
     __syncthreads();
@@ -459,6 +463,7 @@ __global__ void __launch_bounds__(kMaxThreads, 1)
   const int nxy = o.L.nxy;
   const int k0 = blockIdx.y * t.chunk, k1 = min(k0 + t.chunk, o.L.nz);
   T* me = planes + (pl.row0 + 1) * kRow<T> + pl.p;  // field 0 of the even planes
+  pdl_early();
   pdl_enter();
   const T sb = SGN ? T(0) : T(*sb_ptr);
   bool zn;
@@ -569,8 +574,8 @@ __global__ void __launch_bounds__(kMaxThreads, 1)
   extern __shared__ __align__(16) unsigned char march_sm[];
   T* ring = reinterpret_cast<T*>(march_sm);
   const int sw = slot_words<T>(t), pw = plane_words<T>(t);
-  T* planes = ring + kRing * 2 * sw;
-  T* tab = planes + 4 * pw;
+  T* planes = FLAT ? ring : ring + kRing * 2 * sw;
+  T* tab = planes + (FLAT ? 2 : 4) * pw;
   if constexpr(!CD) {
     for(int q = threadIdx.x; q < 64; q += blockDim.x) tab[q] = T(2.0 / 3.0 * o.invd[q]);
     __syncthreads();
@@ -581,16 +586,22 @@ __global__ void __launch_bounds__(kMaxThreads, 1)
   const int nxy = o.L.nxy;
   const int k0 = blockIdx.y * t.chunk, k1 = min(k0 + t.chunk, o.L.nz);
   T* me = planes + (pl.row0 + 1) * kRow<T> + pl.p;
+  pdl_early();
   pdl_enter();
   const T sb = SGN ? T(0) : T(*sb_ptr);
   bool zn;
-  // the coarse correction of the patch: W / 2 parents where both x and y
-  // coarsen (PAIRS), else one per cell; loaded two planes ahead, always from
-  // valid cells (under a condition the merge would wait for the load)
+  // the coarse correction of the patch: W / 2 parents (8 bytes) where both x
+  // and y coarsen (PAIRS), streamed through a ring like x and b -- loaded into
+  // registers two planes ahead they cost 18 us at 256^3 in FP64 and 18 of 84 in
+  // FP32; else one per cell, loaded two planes ahead, always from valid cells
+  // (under a condition the merge would wait for the load)
   constexpr int NR = PAIRS ? 1 : 2, NE = PAIRS ? kW<T> / 2 : kW<T>;
   struct Parents {
     T v[NR][NE];
   };
+  T* ering = tab + 64;
+  const int ew = PAIRS ? NE * blockDim.x : 0;
+  const int e0 = lc.nx * (pl.yj[0] >> 1);
   auto lde = [&](int kz) {
     Parents q;
     const T* ep = e + lc.nxy * (kz >> sz);
@@ -598,8 +609,23 @@ __global__ void __launch_bounds__(kMaxThreads, 1)
     for(int r = 0; r < NR; ++r)
 #pragma unroll
       for(int c = 0; c < NE; ++c)
-        q.v[r][c] = PAIRS ? ep[lc.nx * (pl.yj[0] >> 1) + (pl.xi[2 * c] >> 1)]
-                          : ep[lc.nx * (pl.yj[r] >> sy) + (pl.xi[c] >> sx)];
+        q.v[r][c] = PAIRS ? ep[e0 + (pl.xi[2 * c] >> 1)] : ep[lc.nx * (pl.yj[r] >> sy) + (pl.xi[c] >> sx)];
+    return q;
+  };
+  auto fetch_e = [&](int slot, int kz) {
+    const T* ep = e + (lc.nxy * (kz >> sz) + e0);
+    const unsigned d = static_cast<unsigned>(__cvta_generic_to_shared(ering + slot * ew + NE * threadIdx.x));
+    if(NE == 1 || pl.vec) {
+      asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(d), "l"(ep + (pl.xi[0] >> 1)) : "memory");
+    } else {
+      asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(d), "l"(ep + (pl.xi[0] >> 1)) : "memory");
+      asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(d + 4), "l"(ep + (pl.xi[NE] >> 1)) : "memory");
+    }
+  };
+  auto take_e = [&](int slot) {
+    Parents q;
+#pragma unroll
+    for(int c = 0; c < NE; ++c) q.v[0][c] = ering[slot * ew + NE * threadIdx.x + c];
     return q;
   };
   // y = x + P e with the signs of Dirichlet images
@@ -650,9 +676,13 @@ __global__ void __launch_bounds__(kMaxThreads, 1)
       const int zx = f.kz * nxy;
       if(f.k <= k1 + 1) pl.fetch(ring + (q & 3) * sw, x, zx);
       if(f.k <= k1 + 1) pl.fetch(bring + (q - 1) * sw, b, zb);
+      if constexpr(PAIRS) {
+        if(f.k <= k1 + 1) fetch_e(q, f.kz);
+      } else {
+        if(q == 1) E[1] = lde(f.kz);
+        if(q == 2) E[2] = lde(f.kz);
+      }
       fetch_commit();
-      if(q == 1) E[1] = lde(f.kz);
-      if(q == 2) E[2] = lde(f.kz);
       zb = zx;
       f.next(o);
     }
@@ -669,12 +699,16 @@ __global__ void __launch_bounds__(kMaxThreads, 1)
       Y[N] = pl.take(ring + N * sw);
       B[J] = pl.take(bring + J * sw);
       const int zx = f.kz * nxy;
+      if constexpr(PAIRS) E[N] = take_e(N);
       if(f.k <= k1 + 1) pl.fetch(ring + J * sw, x, zx);       // plane s + 4
+      if constexpr(PAIRS) {
+        if(f.k <= k1 + 1) fetch_e(J, f.kz);
+      }
       if(f.k <= k1 + 2) pl.fetch(bring + M * sw, b, zb);      // plane s + 3
       __syncwarp();
       fetch_commit();
       join(Y[N], E[N], s + 1);
-      E[M] = lde(ke);
+      if constexpr(!PAIRS) E[M] = lde(ke);
       zb = zx;
       ke = max(0, min(f.kz, o.L.nz - 1));
       f.next(o);
@@ -739,7 +773,8 @@ __global__ void __launch_bounds__(kMaxThreads, 1)
   const Coef<T> co(o, FLAT);
   const int nxy = o.L.nxy;
   const int k0 = blockIdx.y * t.chunk, k1 = min(k0 + t.chunk, o.L.nz);
-  T* me = ring + 2 * kRing * sw + (pl.row0 + 1) * kRow<T> + pl.p;
+  T* me = (FLAT ? ring : ring + 2 * kRing * sw) + (pl.row0 + 1) * kRow<T> + pl.p;
+  pdl_early();
   pdl_enter();
   const bool first = sc->first != 0;
   const int turn = sc->body_runs & 1;
@@ -839,7 +874,8 @@ __global__ void __launch_bounds__(kMaxThreads, 1)
   const Coef<T> co(o, FLAT);
   const int nxy = o.L.nxy;
   const int k0 = blockIdx.y * t.chunk, k1 = min(k0 + t.chunk, o.L.nz);
-  T* me = rring + kRing * sw + (pl.row0 + 1) * kRow<T> + pl.p;
+  T* me = (FLAT ? ring : rring + kRing * sw) + (pl.row0 + 1) * kRow<T> + pl.p;
+  pdl_early();
   pdl_enter();
   const int stop = sc->stop;
   const T* __restrict__ p = d.p[sc->body_runs & 1];
@@ -1003,7 +1039,8 @@ __global__ void __launch_bounds__(kMaxThreads, 1)
   const Coef<T> co(o, FLAT);
   const int nxy = o.L.nxy;
   const int k0 = blockIdx.y * t.chunk, k1 = min(k0 + t.chunk, o.L.nz);
-  T* me = bring + kRing * sw + (pl.row0 + 1) * kRow<T> + pl.p;
+  T* me = (FLAT ? ring : bring + kRing * sw) + (pl.row0 + 1) * kRow<T> + pl.p;
+  pdl_early();
   pdl_enter();
   const T sb = SGN ? 0.0 : sc->sb, sx = SGN ? 0.0 : sc->sx;
   double acc[2] = {0.0, 0.0};

@@ -414,6 +414,7 @@ template <typename T, typename B>
 __global__ void __launch_bounds__(kDenseThreads)
     k_dense_apply(int n, const T* __restrict__ G, const B* __restrict__ b, T* __restrict__ x,
                   LevelScalars* ls, SolveScalars* sc, RedBuf rb) {
+  pdl_early();
   pdl_enter();
   constexpr int kGroups = kDenseThreads / kDenseRows;
   __shared__ double part[kGroups][kDenseRows + 1];
@@ -932,6 +933,8 @@ void march_attributes(const PoissonPlan* P) {
 // in waves of what the SMs hold at once.  Small levels so get many thin
 // chunks, large ones tiles near 64 x 26 with long chunks.
 constexpr double kPlaneLatency = 500.0, kThreadCycles = 2.0;
+// Resident threads of the kernels on grids one cell deep (56-80 registers).
+constexpr int kFlatResident = 768;
 
 template <typename T>
 void plan_tile(const CLay& L, int halo_rows, int rz, int streams, int fields, int sms, march::Tile& best,
@@ -960,9 +963,9 @@ void plan_tile(const CLay& L, int halo_rows, int rz, int streams, int fields, in
       last_iy = t.iy;
       t.ey = t.iy + 2 * halo_rows;
       const int threads = t.px * t.ey / 2;
-      const size_t smem = march::smem_bytes<T>(t, streams, fields);
+      const size_t smem = march::smem_bytes<T>(t, streams, fields, flat, fields == 2);
       if(smem > kMarchSmem) continue;
-      const int resident = std::min<int>({march::kMaxThreads / ((threads + 31) / 32 * 32),
+      const int resident = std::min<int>({(flat ? kFlatResident : march::kMaxThreads) / ((threads + 31) / 32 * 32),
                                           static_cast<int>(228 * 1024 / (smem + 2048)), 16});
       if(resident < 1) continue;
       const long long tiles = static_cast<long long>(t.tx) * ((L.ny + t.iy - 1) / t.iy);
@@ -1201,7 +1204,8 @@ void v_cycle(PoissonPlan* P, int l, const V* r0, SolveScalars* sc, RedBuf rb, cu
   }
   Level& cv = P->levels[l + 1];
   const T* b = l == 0 ? static_cast<const T*>(r0) : static_cast<const T*>(lv.b);
-  const size_t smem1 = march::smem_bytes<T>(lv.tile, 1, 2), smem2 = march::smem_bytes<T>(lv.tile, 2, 2);
+  const size_t smem1 = march::smem_bytes<T>(lv.tile, 1, 2, lv.L.nz == 1),
+               smem2 = march::smem_bytes<T>(lv.tile, 2, 2, lv.L.nz == 1, true);
   const int threads = lv.tile.px * lv.tile.ey / 2;
   {
     ProfScope ps(l == 0 ? kKSmoothFirstFine : kKCoarseLevels, s);
@@ -1248,7 +1252,7 @@ void enqueue_start(PoissonPlan* P, const march::SolveStart& start, SolveScalars*
     return;
   }
   const march::Tile& t = P->res_tile;
-  launch_pdl(residual_kernel<true>(P, l0.L.nz == 1), P->res_grid, t.px * t.ey / 2, march::smem_bytes<double>(t, 2, 1),
+  launch_pdl(residual_kernel<true>(P, l0.L.nz == 1), P->res_grid, t.px * t.ey / 2, march::smem_bytes<double>(t, 2, 1, l0.L.nz == 1),
              s, l0.op, t, P->x, P->b, P->r, sc, static_cast<const SolveScalars*>(nullptr), start, rb);
   OFB_LAUNCH_CHECK("k_residual");
 }
@@ -1269,12 +1273,12 @@ void enqueue_body(PoissonPlan* P, const CGVec<V>& v, SolveScalars* sc, RedBuf rb
   const march::Direction<V> d{{v.p, v.p2}};
   {
     ProfScope ps(kKApplyAp, s);
-    launch_pdl(direction_kernel<V>(P, flat), P->cg_grid, threads, march::smem_bytes<V>(t, 2, 1), s, l0.op, t,
+    launch_pdl(direction_kernel<V>(P, flat), P->cg_grid, threads, march::smem_bytes<V>(t, 2, 1, flat), s, l0.op, t,
                static_cast<const V*>(l0.x), P->ls, d, sc, rb);
   }
   {
     ProfScope ps(kKUpdateXr, s);
-    launch_pdl(advance_kernel<V>(P, flat), P->cg_grid, threads, march::smem_bytes<V>(t, 3, 1), s, l0.op, t, d,
+    launch_pdl(advance_kernel<V>(P, flat), P->cg_grid, threads, march::smem_bytes<V>(t, 3, 1, flat), s, l0.op, t, d,
                v.x, v.r, sc, rb, cond);
   }
   OFB_LAUNCH_CHECK("pcg body");
@@ -1414,7 +1418,7 @@ void solve_dc(PoissonPlan* P, int max_iterations, double tolerance, SolveScalars
     k_dc_update_x<<<ln.grid, ln.block, 0, s>>>(l0.L, P->x, P->e32, sc, si, ln.kchunk, rb);
     const march::Tile& t = P->res_tile;
     launch_pdl(residual_kernel<false>(P, l0.L.nz == 1), P->res_grid, t.px * t.ey / 2,
-               march::smem_bytes<double>(t, 2, 1), s, l0.op, t, P->x, P->b, P->r, sc,
+               march::smem_bytes<double>(t, 2, 1, l0.L.nz == 1), s, l0.op, t, P->x, P->b, P->r, sc,
                static_cast<const SolveScalars*>(si), start, rb);
     OFB_LAUNCH_CHECK("defect correction update");
   };
