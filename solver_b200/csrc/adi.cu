@@ -275,6 +275,7 @@ AdiPlan* adi_plan_create(const Grid& g, const VBC& bc, double alpha) {
   if(!host.empty()) {
     OFB_CHECK(cudaMalloc(&p->coef, host.size() * sizeof(double)));
     OFB_CHECK(cudaMemcpy(p->coef, host.data(), host.size() * sizeof(double), cudaMemcpyHostToDevice));
+    OFB_CHECK(cudaStreamSynchronize(nullptr));  // the context's stream does not wait for the default one
   }
   return p;
 }

@@ -1143,6 +1143,10 @@ PoissonPlan* poisson_plan_create(const Grid& g, const PBC& pbc_in, int precision
   else march_attributes<double>(P);
   const char* no_graph = std::getenv("ORCHARD_B200_NO_GRAPH");
   P->use_graph = !(no_graph != nullptr && no_graph[0] == '1');
+  // what was set up above went through the default stream, with which the
+  // context's stream does not synchronise: behind another thread's plan it
+  // would still be on its way when the first solve runs
+  OFB_CHECK(cudaStreamSynchronize(nullptr));
   return P;
 }
 
