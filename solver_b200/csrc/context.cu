@@ -477,18 +477,20 @@ ofb::FinishArgs finish_args(of_ctx* ctx, const double* const* pred, double scale
 // after the last -- between sweeps only where a fixed-pressure face copies its
 // neighbour: a wall face stays out of the sweep along its axis and sweeps
 // across it solve separate lines, and a duplicated periodic face keeps its
-// image's value through every sweep.  The ghosts are left to the callers that
-// return them.  With sweep_out, sweep (component, axis) writes into
-// sweep_out[component][axis] instead of the ping-pong buffers, so every sweep's
-// output survives the call (the adjoint needs them for the viscosity
-// derivative).
-void predictor_adi(of_ctx* ctx, double alpha, double* out[3], int* line_solves,
+// image's value through every sweep.  With `ghosts` (the entry point that
+// returns the fields) the faces are set after every sweep and the last set is
+// the full one: the ghosts beside a wall face are filled from what the last
+// sweep made of it, before it is reset.  With sweep_out, sweep (component,
+// axis) writes into sweep_out[component][axis] instead of the ping-pong
+// buffers, so every sweep's output survives the call (the adjoint needs them
+// for the viscosity derivative).
+void predictor_adi(of_ctx* ctx, double alpha, double* out[3], int* line_solves, bool ghosts,
                    double* const (*sweep_out)[3] = nullptr) {
   ofb::AdiPlan* plan = alpha != 0.0 ? ctx->adi_for(alpha) : nullptr;
   int lines = 0;
   double* b[3];
-  bool copies = false;
-  for(int f = 0; f < 6; ++f) copies = copies || ctx->bc.type[f] == ofb::kFixedPressure;
+  bool between = ghosts;
+  for(int f = 0; f < 6; ++f) between = between || ctx->bc.type[f] == ofb::kFixedPressure;
   for(int c = 0; c < 3; ++c) {
     out[c] = ctx->rhs[c];
     b[c] = ctx->adi_b[c];
@@ -505,9 +507,10 @@ void predictor_adi(of_ctx* ctx, double alpha, double* out[3], int* line_solves,
       b[c] = out[c];
       out[c] = to[c];
     }
-    if(copies || axis == 2)
+    if(axis == 2 ? !ghosts : between)
       ofb::launch_normal_faces(ctx->g, ctx->bc, out[0], out[1], out[2], ctx->stream);
   }
+  if(ghosts) ofb::launch_velocity_bc(ctx->g, ctx->bc, out[0], out[1], out[2], ctx->stream);
   if(line_solves) *line_solves = lines;
 }
 
@@ -621,7 +624,7 @@ ofb::SolveScalars forward_step(of_ctx* ctx, const of_step_params* prm, const std
   }
   // solve_predictor_adi
   double* pred[3];
-  predictor_adi(ctx, alpha, pred, nullptr, hk != nullptr ? hk->sweep_out : nullptr);
+  predictor_adi(ctx, alpha, pred, nullptr, false, hk != nullptr ? hk->sweep_out : nullptr);
   // project_velocity with a zero initial pressure correction
   ofb::launch_divergence_rhs(g, ctx->pbc, pred[0], pred[1], pred[2], prm->density / dt, ctx->prhs,
                              ofb::poisson_b(plan), ctx->sc, ctx->rb, s);
@@ -1110,8 +1113,7 @@ of_status of_solve_predictor_adi(of_ctx* ctx, double alpha, const double* rhs_u,
     ctx->upload(up);
     for(int c = 0; c < 3; ++c) ctx->d2d(ctx->adi_b[c], ctx->rhs[c], 1 + c);  // edge ghosts follow the input
     double* res[3];
-    predictor_adi(ctx, alpha, res, line_solves);
-    ofb::launch_velocity_bc(ctx->g, ctx->bc, res[0], res[1], res[2], ctx->stream);
+    predictor_adi(ctx, alpha, res, line_solves, true);
     for(int c = 0; c < 3; ++c) down.push_back(T{res[c], outp[c], 1 + c, false});
     ctx->download(down);
     ctx->sync();

@@ -85,3 +85,34 @@ def test_pressure_solve_at_tile_edges(oracle, shape, types, precision):
         np.testing.assert_allclose(d["residual_history"][:n], href[:n], rtol=1e-9, atol=1e-12 * href[0])
     a, b = po.active(got), po.active(ref)
     assert np.linalg.norm(a - b) <= 2e-12 * _condition(shape, h, types) * np.linalg.norm(b)
+
+
+@pytest.mark.parametrize("alpha", [1e-6, 0.02, 0.3])
+@pytest.mark.parametrize("types", ["periodic", "walls", "open"])
+@pytest.mark.parametrize("shape", [(8, 9, 15), (16, 17, 33), (31, 32, 8), (100, 12, 40)],
+                         ids=lambda s: "x".join(map(str, s)))
+def test_adi_chunks_at_line_ends(oracle, shape, types, alpha):
+    """Chunks of 16 unknowns whose reach (4 to 60 cells here) passes one or both
+    ends of the line, several times over on the short ones: periodic images,
+    wall reflections (with a moving lid and a wall-normal velocity) and
+    fixed-pressure faces.  The images are exact up to the truncation at 2^-56
+    and rounding: 1e-13 of the field's largest value."""
+    import solver_b200 as sb
+    from conftest import to_gpu_bc
+    g = po.Grid(*shape, 0.5, 0.6, 0.55)
+    sets = {"periodic": [po.PERIODIC] * 6,
+            "walls": [po.NO_SLIP_WALL, po.PRESCRIBED_VELOCITY, po.SYMMETRY, po.PRESCRIBED_VELOCITY,
+                      po.NO_SLIP_WALL, po.SYMMETRY],
+            "open": [po.PRESCRIBED_VELOCITY, po.FIXED_PRESSURE, po.NO_SLIP_WALL, po.NO_SLIP_WALL,
+                     po.PERIODIC, po.PERIODIC]}
+    velocities = {"periodic": [None] * 6, "walls": [None, (0.4, 0.2, -0.3), None, (0.7, -0.5, 0.1), None, None],
+                  "open": [(1.0, 0.3, -0.2), None, None, None, None, None]}
+    bc = po.bc_from(sets[types], velocities[types])
+    rng = np.random.default_rng(sum(shape))
+    rhs = [rng.standard_normal(po.shape(g, c)) for c in "uvw"]
+    with sb.Context(to_gpu_grid(g), to_gpu_bc(bc)) as ctx:
+        got, lines = ctx.solve_predictor_adi(rhs, alpha)
+    exp, lines_ref = oracle.predictor_adi(g, bc, alpha, *rhs)
+    assert lines == lines_ref
+    for a, b in zip(got, exp):
+        assert np.max(np.abs(a - b)) <= 1e-13 * np.max(np.abs(b))
