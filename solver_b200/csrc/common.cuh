@@ -156,6 +156,9 @@ inline Launch3 launch3_components(const Grid& g) {
     l.kchunk = l.kchunk > o.kchunk ? l.kchunk : o.kchunk;
   }
   l.grid.x *= 3;
+  // each chunk starts with extra planes: longer ones where 16 blocks per SM remain
+  const long long cols = static_cast<long long>(l.grid.x) * l.grid.y;
+  while(l.kchunk < 16 && cols * ((g.nz + 2 * l.kchunk) / (2 * l.kchunk)) >= 16 * 148) l.kchunk *= 2;
   l.grid.z = (g.nz + 1 + l.kchunk - 1) / l.kchunk;
   return l;
 }

@@ -87,6 +87,25 @@ def test_pressure_solve_at_tile_edges(oracle, shape, types, precision):
     assert np.linalg.norm(a - b) <= 2e-12 * _condition(shape, h, types) * np.linalg.norm(b)
 
 
+@pytest.mark.parametrize("amplitude", [1e-9, 1.0, 1e9])
+@pytest.mark.parametrize("shape", [(30, 8, 5), (31, 9, 16), (32, 7, 17), (63, 17, 2), (5, 3, 1)],
+                         ids=lambda s: "x".join(map(str, s)))
+def test_advection_at_tile_edges(oracle, shape, amplitude):
+    """Tiles of 31 points along x (the 32nd lane evaluates the last face), rows
+    of 8, chunks of planes with a carried face; amplitudes that take the
+    limiter's quotient over many binades and its small-denominator branch.  Each
+    flux is within a few rounding errors (the quotient within one ulp), so the
+    term is within 1e-13 of its largest flux difference."""
+    import solver_b200 as sb
+    g = po.Grid(*shape, 0.3, 0.25, 0.4)
+    rng = np.random.default_rng(sum(shape))
+    vel = [amplitude * rng.standard_normal(po.shape(g, c)) for c in "uvw"]
+    with sb.Context(to_gpu_grid(g), [sb.PERIODIC] * 6) as ctx:
+        got = ctx.compute_advection_term(*vel)
+    for a, b in zip(got, oracle.advection(g, *vel)):
+        assert np.max(np.abs(po.active(a) - po.active(b))) <= 1e-13 * max(1e-300, np.max(np.abs(b)))
+
+
 @pytest.mark.parametrize("alpha", [1e-6, 0.02, 0.3])
 @pytest.mark.parametrize("types", ["periodic", "walls", "open"])
 @pytest.mark.parametrize("shape", [(8, 9, 15), (16, 17, 33), (31, 32, 8), (100, 12, 40)],
