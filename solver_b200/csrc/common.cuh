@@ -191,9 +191,15 @@ __device__ __forceinline__ double warp_sum(double v) {
   return v;
 }
 
-__device__ __forceinline__ double warp_max(double v) {
+// Over the first `lanes` lanes of a warp, on lane 0.  A block's last warp may be
+// partial (the marching tiles have any number of threads), and a shuffle from a
+// lane without a thread has no defined value.
+__device__ __forceinline__ double warp_reduce(double v, bool is_max, int lane, int lanes) {
 #pragma unroll
-  for(int o = 16; o > 0; o >>= 1) v = fmax(v, __shfl_down_sync(0xffffffffu, v, o));
+  for(int o = 16; o > 0; o >>= 1) {
+    const double w = __shfl_down_sync(0xffffffffu, v, o);
+    if(lane + o < lanes) v = is_max ? fmax(v, w) : v + w;
+  }
   return v;
 }
 
@@ -207,18 +213,16 @@ __device__ __forceinline__ void block_reduce(double (&v)[K], const bool (&is_max
   const int lane = tid & 31;
   const int warp = tid >> 5;
   const int nwarps = (nthreads + 31) >> 5;
+  const int lanes = min(32, nthreads - 32 * warp);
 #pragma unroll
   for(int k = 0; k < K; ++k) {
-    double x = is_max[k] ? warp_max(v[k]) : warp_sum(v[k]);
+    const double x = warp_reduce(v[k], is_max[k], lane, lanes);
     if(lane == 0) sh[k][warp] = x;
   }
   __syncthreads();
   if(warp == 0) {
 #pragma unroll
-    for(int k = 0; k < K; ++k) {
-      double x = lane < nwarps ? sh[k][lane] : (is_max[k] ? -INFINITY : 0.0);
-      v[k] = is_max[k] ? warp_max(x) : warp_sum(x);
-    }
+    for(int k = 0; k < K; ++k) v[k] = warp_reduce(sh[k][lane], is_max[k], lane, nwarps);
   }
   __syncthreads();
 }
@@ -272,11 +276,6 @@ __device__ __forceinline__ void reduce_finish(double (&v)[K], const bool (&is_ma
 // ---------------------------------------------------------------------------
 
 struct CudaError : std::runtime_error {
-  using std::runtime_error::runtime_error;
-};
-
-// A bounded device-side wait gave up (reported as OF_TIMEOUT).
-struct TimeoutError : std::runtime_error {
   using std::runtime_error::runtime_error;
 };
 
