@@ -39,7 +39,7 @@ typedef enum {
   OF_NOT_CONVERGED = 3,    /* require_converged_pressure_projection (solver/projection.cpp:1133) */
   OF_NONFINITE = 4,        /* "... solve produced a non-finite state" (solver/taylor_green.cpp:614) */
   OF_CUDA_ERROR = 5,
-  OF_TIMEOUT = 6           /* a device-side wait gave up (never expected) */
+  OF_TIMEOUT = 6           /* kept for callers: no kernel waits on the device any more */
 } of_status;
 
 /* Grid (core/grid.hpp:57-87); ghost_layers is always 1. */
