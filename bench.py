@@ -77,17 +77,18 @@ def bytes_per_launch(n, precision):
     d = 8
     s = 4 if precision == "mixed" else 8  # inner solve vectors
     out = {
-        "predictor_rhs": 5 * d * N,  # per component: read f, p, prev, adv; write rhs
-        "advection": 4 * d * N,      # per component: read u, v, w; write adv
-        "adi_sweep": 2 * d * N,
+        # the three components share a launch
+        "predictor_rhs": 13 * d * N,  # read f, prev, adv (3 each) and p; write rhs (3)
+        "advection": 6 * d * N,       # read u, v, w; write adv (3)
+        "adi_sweep": 6 * d * N,       # one axis: read and write 3
         "divergence_rhs": 5 * d * N,
         "pcg_initial_residual": 3 * d * N,
         "pcg_apply_ap": 3 * s * N,                    # direction: read z, p; write p
         "pcg_update_xr": 5 * s * N,                   # advance: read p, x, r; write x, r
         "vcycle_smooth_first_fine": (2 + 1 / 8) * s * N,  # descend: read b; write x, coarse b
         "vcycle_smooth_fine": (3 + 1 / 8) * s * N,    # ascend: read x, b, coarse x; write out
-        "correct_velocity": (1 + 3 + 3) * d * N / 3 + d * N,  # per component launch
-        "cell_pass": 7 * d * N,
+        # end of the step: read u* (3), u (3), phi, rhs and p; write u (3) and p
+        "correct_velocity": 13 * d * N,
     }
     if precision == "mixed":
         out["defect_correction"] = 20 * N
@@ -453,7 +454,7 @@ def run_b200_arm(args, world, rank, local):
                 "frac": step_bytes / (elapsed_ms / args.steps / 1000.0) / 1e9 / peak}
     kernels = {k: {"launches_per_step": v[0] / replay_steps, "ms_per_step": round(v[2] / replay_steps, 4)}
                for k, v in prof.items() if v[0]}
-    # The coarse levels are ~13 kernels of a few microseconds per V-cycle: in
+    # The coarse levels are 9 kernels of a few microseconds per V-cycle: in
     # the host-driven replay their time is set by the host's launch rate, so
     # they are timed as the product runs them, a CUDA graph of the chain
     # replayed on the device (of_profile_coarse_chain).
