@@ -442,7 +442,9 @@ __device__ __forceinline__ void ring4(int s0, int s1, Step step) {
 // has zero mean), so no sum is formed here.
 //
 // Bound: one read of b, one write of x and of bc (2.125 vectors); in FP64 at
-// 256^3 the arithmetic and the shared-memory traffic are each near the DRAM time.
+// 256^3 the arithmetic and the shared-memory traffic are each near the DRAM time:
+// 81 us (FP32 54), where the pre-sweeps and the residual with its restriction
+// took 53 + 65 in two passes.
 template <typename T, bool SGN, bool CD, bool FLAT>
 __global__ void __launch_bounds__(kMaxThreads, 1)
     k_descend(OpInfo o, CLay oc, Tile t, const T* __restrict__ b, const double* sb_ptr, T* __restrict__ x,
@@ -565,7 +567,8 @@ __global__ void __launch_bounds__(kMaxThreads, 1)
 // level (FINE) it also forms mean(out) and r.z for the CG; on the others no
 // mean is needed (see k_descend).  sx, sy, sz: log2 of the coarsening ratios.
 //
-// Bound: reads x, b and e, writes out (3.125 vectors).
+// Bound: reads x, b and e, writes out (3.125 vectors); 97 us at 256^3 in FP64 (66
+// in FP32), where the prolongation with one sweep and the second sweep took 89 + 78.
 template <typename T, bool SGN, bool CD, bool FLAT, bool FINE, bool PAIRS>
 __global__ void __launch_bounds__(kMaxThreads, 1)
     k_ascend(OpInfo o, CLay lc, Tile t, const T* __restrict__ b, const double* sb_ptr, const T* __restrict__ x,
@@ -760,7 +763,7 @@ struct Direction {
 // reference removes are zero up to rounding (z - sz has none, A annihilates
 // constants) and are left in; the residual's, which they would move, is
 // removed every iteration.  Bound: reads z and p, writes p (3 vectors); at
-// 256^3 76 us in FP64, where the separate p update and A p took 71 + 66.
+// 256^3 72 us in FP64, where the separate p update and A p took 71 + 66.
 template <typename T, bool SGN, bool FLAT>
 __global__ void __launch_bounds__(kMaxThreads, 1)
     k_direction(OpInfo o, Tile t, const T* __restrict__ z, const LevelScalars* ls0, Direction<T> d,
@@ -861,7 +864,7 @@ __global__ void __launch_bounds__(kMaxThreads, 1)
 // x = (x - sx) + alpha p, r = (r - sr) - alpha A p (in FP64 arithmetic), the
 // residual's norm and the convergence test.  x keeps a zero mean up to
 // rounding (p has none).  Bound: reads p, x and r, writes x and r (5 vectors);
-// at 256^3 119 us in FP64, where the update from a stored A p took 142.
+// at 256^3 120 us in FP64, where the update from a stored A p took 142.
 template <typename T, bool SGN, bool FLAT>
 __global__ void __launch_bounds__(kMaxThreads, 1)
     k_advance(OpInfo o, Tile t, Direction<T> d, T* __restrict__ x, T* __restrict__ r, SolveScalars* sc, RedBuf rb,
