@@ -157,7 +157,8 @@ void poisson_account(PoissonPlan* p, const SolveScalars& sc_host);
 // as each CG iteration runs it -- replayed `reps` times from a CUDA graph of
 // that chain alone on the level-1 rhs of the last solve (nothing it writes is
 // read before the next solve's V-cycles overwrite it); *launches = kernels per
-// chain.
+// chain.  Both are zero where the finest level is the dense one: no level is
+// launched below it.
 double poisson_time_coarse_chain(PoissonPlan* p, RedBuf rb, cudaStream_t s, int reps, int* launches);
 // Writes x - sx into the active entries of a padded pressure field.
 void launch_compact_to_pressure(const Grid& g, const double* x, const SolveScalars* sc,

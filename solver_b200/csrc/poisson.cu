@@ -1288,6 +1288,42 @@ void enqueue_body(PoissonPlan* P, const CGVec<V>& v, SolveScalars* sc, RedBuf rb
   OFB_LAUNCH_CHECK("pcg body");
 }
 
+// A stream's capture with the launches counted into `counts`; an exception on
+// the way ends both, so the stream and the profiler stay usable.
+class Capture {
+ public:
+  Capture(cudaStream_t s, long long* counts, cudaGraph_t into) : s_(s) {
+    if(into != nullptr)
+      OFB_CHECK(cudaStreamBeginCaptureToGraph(s, into, nullptr, nullptr, 0, cudaStreamCaptureModeThreadLocal));
+    else
+      OFB_CHECK(cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal));
+    open_ = true;
+    owns_ = into == nullptr;
+    prof_capture_begin(counts);
+  }
+  Capture(const Capture&) = delete;
+  Capture& operator=(const Capture&) = delete;
+  cudaGraph_t end() {
+    cudaGraph_t g = nullptr;
+    open_ = false;
+    prof_capture_end();
+    OFB_CHECK(cudaStreamEndCapture(s_, &g));
+    return g;
+  }
+  ~Capture() {
+    if(!open_) return;
+    cudaGraph_t g = nullptr;
+    prof_capture_end();
+    cudaStreamEndCapture(s_, &g);
+    if(owns_ && g != nullptr) cudaGraphDestroy(g);
+    cudaGetLastError();
+  }
+
+ private:
+  cudaStream_t s_;
+  bool open_ = false, owns_ = false;
+};
+
 // A loop as one graph: pre -> WHILE(cont) { body }.  pre and body are
 // enqueue callbacks taking the conditional handle; the loop is bounded by the
 // iteration limit the body enforces (it clears the condition), so the graph
@@ -1295,21 +1331,28 @@ void enqueue_body(PoissonPlan* P, const CGVec<V>& v, SolveScalars* sc, RedBuf rb
 template <typename Pre, typename Body>
 cudaGraphExec_t build_loop_graph(PoissonPlan* P, cudaStream_t s, Pre pre, Body body,
                                  cudaGraph_t* graph_out) {
-  cudaGraph_t g = nullptr;
-  OFB_CHECK(cudaGraphCreate(&g, 0));
+  struct Graph {
+    cudaGraph_t g = nullptr;
+    ~Graph() {
+      if(g != nullptr) cudaGraphDestroy(g);
+    }
+  } graph;
+  OFB_CHECK(cudaGraphCreate(&graph.g, 0));
+  const cudaGraph_t g = graph.g;
   cudaGraphConditionalHandle cond = 0;
   OFB_CHECK(cudaGraphConditionalHandleCreate(&cond, g, 0, cudaGraphCondAssignDefault));
   for(int i = 0; i < kKernelCount; ++i) P->pre_counts[i] = P->body_counts[i] = 0;
-  prof_capture_begin(P->pre_counts);
-  OFB_CHECK(cudaStreamBeginCaptureToGraph(s, g, nullptr, nullptr, 0, cudaStreamCaptureModeThreadLocal));
-  pre(cond);
-  cudaStreamCaptureStatus status;
-  const cudaGraphNode_t* deps = nullptr;
-  size_t ndeps = 0;
-  OFB_CHECK(cudaStreamGetCaptureInfo(s, &status, nullptr, nullptr, &deps, &ndeps));
-  std::vector<cudaGraphNode_t> leaf(deps, deps + ndeps);
-  OFB_CHECK(cudaStreamEndCapture(s, &g));
-  prof_capture_end();
+  std::vector<cudaGraphNode_t> leaf;
+  {
+    Capture c(s, P->pre_counts, g);
+    pre(cond);
+    cudaStreamCaptureStatus status;
+    const cudaGraphNode_t* deps = nullptr;
+    size_t ndeps = 0;
+    OFB_CHECK(cudaStreamGetCaptureInfo(s, &status, nullptr, nullptr, &deps, &ndeps));
+    leaf.assign(deps, deps + ndeps);
+    c.end();
+  }
   cudaGraphNodeParams cp = {};
   cp.type = cudaGraphNodeTypeConditional;
   cp.conditional.handle = cond;
@@ -1317,16 +1360,15 @@ cudaGraphExec_t build_loop_graph(PoissonPlan* P, cudaStream_t s, Pre pre, Body b
   cp.conditional.size = 1;
   cudaGraphNode_t wnode;
   OFB_CHECK(cudaGraphAddNode(&wnode, g, leaf.data(), leaf.size(), &cp));
-  cudaGraph_t bodyg = cp.conditional.phGraph_out[0];
-  prof_capture_begin(P->body_counts);
-  OFB_CHECK(cudaStreamBeginCaptureToGraph(s, bodyg, nullptr, nullptr, 0,
-                                          cudaStreamCaptureModeThreadLocal));
-  body(cond);
-  OFB_CHECK(cudaStreamEndCapture(s, &bodyg));
-  prof_capture_end();
+  {
+    Capture c(s, P->body_counts, cp.conditional.phGraph_out[0]);
+    body(cond);
+    c.end();
+  }
   cudaGraphExec_t exec = nullptr;
   OFB_CHECK(cudaGraphInstantiate(&exec, g, 0));
   *graph_out = g;
+  graph.g = nullptr;
   return exec;
 }
 
@@ -1490,19 +1532,20 @@ bool poisson_solve_enqueue(PoissonPlan* P, int max_iterations, double tolerance,
 
 double poisson_time_coarse_chain(PoissonPlan* P, RedBuf rb, cudaStream_t s, int reps, int* launches) {
   *launches = 0;
-  if(P->levels.size() < 2 || reps < 1) return 0.0;
+  // a finest level that is the dense one has no chain below it
+  if(P->tail_first < 1 || reps < 1) return 0.0;
   long long counts[kKernelCount] = {};
   cudaGraph_t g = nullptr;
   cudaGraphExec_t ge = nullptr;
-  prof_capture_begin(counts);
-  OFB_CHECK(cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal));
-  // levels >= 1 read only their own level data and LevelScalars
-  if(P->precision == 1)
-    v_cycle<float, float>(P, 1, nullptr, nullptr, rb, s);
-  else
-    v_cycle<double, double>(P, 1, nullptr, nullptr, rb, s);
-  OFB_CHECK(cudaStreamEndCapture(s, &g));
-  prof_capture_end();
+  {
+    Capture c(s, counts, nullptr);
+    // levels >= 1 read only their own level data and LevelScalars
+    if(P->precision == 1)
+      v_cycle<float, float>(P, 1, nullptr, nullptr, rb, s);
+    else
+      v_cycle<double, double>(P, 1, nullptr, nullptr, rb, s);
+    g = c.end();
+  }
   for(int i = 0; i < kKernelCount; ++i) *launches += static_cast<int>(counts[i]);
   OFB_CHECK(cudaGraphInstantiate(&ge, g, 0));
   cudaEvent_t e0 = nullptr, e1 = nullptr;

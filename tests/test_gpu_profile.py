@@ -41,3 +41,29 @@ def test_coarse_chain_replays_leave_the_run_bitwise_unchanged(precision):
     assert m["pressure_iterations"] == m_ref["pressure_iterations"]
     for f in FIELDS:
         assert np.array_equal(np.asarray(out[f]), np.asarray(ref[f])), f
+
+
+@pytest.mark.parametrize("precision", [sb.OF_FP64, sb.OF_MIXED])
+@pytest.mark.parametrize("shape", [(4, 4, 4), (8, 8, 8), (16, 8, 8), (32, 32, 1), (3, 3, 3)],
+                         ids=lambda s: "x".join(map(str, s)))
+def test_no_chain_below_a_dense_finest_level(shape, precision):
+    """Grids of at most 1024 cells: the whole V-cycle is one matrix, nothing is
+    launched below it.  The call says so, and neither the context nor the
+    launch counters are left in a capture."""
+    h = 2 * np.pi / max(shape)
+    dt = 0.1 * h
+    prm = sb.step_params(0.01, dt, 400, 1e-8)  # (4^3 breaks down at 1e-10: p.Ap < 1e-30)
+    states, counts = [], []
+    for profile in (False, True):
+        with sb.Context(sb.Grid(*shape, h, h, h), [sb.PERIODIC] * 6, precision=precision) as ctx:
+            ctx.tg_init(0.01, dt, 1)
+            ctx.run_steps(prm, 1)
+            if profile:
+                assert sb.profile_coarse_chain(ctx, 3) == (0.0, 0)
+            sb.profile_reset()
+            ctx.run_steps(prm, 2)
+            counts.append({k: v[0] for k, v in sb.profile_read().items()})
+            states.append(ctx.download_state())
+    assert counts[0] == counts[1] and sum(counts[0].values()) > 0
+    for f in FIELDS:
+        assert np.array_equal(np.asarray(states[0][f]), np.asarray(states[1][f])), f
