@@ -202,7 +202,7 @@ AdiPlan* adi_plan_create(const Grid& g, const VBC& bc, double alpha) {
           const double v = bc.vel[face][c];
           const bool fixed = node || type == kNoSlip || type == kPrescribed;
           sign = fixed ? -1.0 : 1.0;
-          add = !fixed || (node && type == kSymmetry) ? 0.0 : 2.0 * v;
+          add = fixed ? 2.0 * v : 0.0;
         };
         wall(bc.type[2 * a], 2 * a, A.node_lo, A.sign_lo, A.add_lo);
         wall(bc.type[2 * a + 1], 2 * a + 1, A.node_hi, A.sign_hi, A.add_hi);

