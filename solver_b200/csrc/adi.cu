@@ -195,8 +195,10 @@ AdiPlan* adi_plan_create(const Grid& g, const VBC& bc, double alpha) {
         const double root = (1.0 + 2.0 * beta) + std::sqrt(1.0 + 4.0 * beta);
         A.lambda = 2.0 * beta / root;
         A.scale = 2.0 / root;
-        A.reach = static_cast<int>(std::ceil((std::log(1.0 - A.lambda) - 56.0 * std::log(2.0)) / std::log(A.lambda)));
-        A.decay = n >= kDecayMinLine && A.reach <= kDecayMaxReach && (a != 0 || n <= kRowMaxLine);
+        // (as a double: past beta = 1e15 it exceeds every int, and lambda = 1 has none)
+        const double reach = std::ceil((std::log(1.0 - A.lambda) - 56.0 * std::log(2.0)) / std::log(A.lambda));
+        A.decay = n >= kDecayMinLine && reach >= 0.0 && reach <= kDecayMaxReach && (a != 0 || n <= kRowMaxLine);
+        A.reach = A.decay ? static_cast<int>(reach) : 0;
         auto wall = [&](int type, int face, int& node, double& sign, double& add) {
           node = c == a && is_dirichlet_velocity(type);
           const double v = bc.vel[face][c];

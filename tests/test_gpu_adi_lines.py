@@ -41,3 +41,21 @@ def test_symmetry_wall_with_normal_velocity(oracle, shape, alpha):
     bc = po.bc_from([po.SYMMETRY, po.SYMMETRY, po.NO_SLIP_WALL, po.SYMMETRY, po.SYMMETRY, po.NO_SLIP_WALL],
                     [(0.7, 0.1, 0.2), (-0.3, 0.0, 0.0), None, (0.2, 0.4, 0.1), (0.0, 0.0, 0.9), None])
     _compare(oracle, g, bc, alpha, _rhs(g, 3))
+
+
+@pytest.mark.parametrize("alpha", [3e2, 1e14, 1e15, 1e16, 1e17, 1e19, 1e33])
+def test_couplings_without_a_decay_length(oracle, alpha):
+    """Couplings whose decay length is thousands of cells, exceeds every int or
+    does not exist (lambda rounds to 1) take the eliminations.  Fixed walls: the
+    matrix tends to the second difference, of condition 4 (n / pi)^2 = 650 for
+    the longest line (40), so the fields agree to 650 x 8 roundings: 1e-12."""
+    g = po.Grid(40, 12, 33, 0.5, 0.6, 0.55)
+    bc = po.bc_from([po.NO_SLIP_WALL, po.PRESCRIBED_VELOCITY] * 3,
+                    [None, (0.4, 0.2, -0.3), None, (0.7, -0.5, 0.1), None, (0.3, 0.2, 0.6)])
+    rhs = _rhs(g, 4)
+    with sb.Context(to_gpu_grid(g), to_gpu_bc(bc)) as ctx:
+        got, lines = ctx.solve_predictor_adi(rhs, alpha)
+    exp, lines_ref = oracle.predictor_adi(g, bc, alpha, *rhs)
+    assert lines == lines_ref
+    for a, b in zip(got, exp):
+        assert np.max(np.abs(a - b)) <= 1e-12 * np.max(np.abs(b))
