@@ -63,6 +63,8 @@ double tangential_coef(int type) {
   return (type == kNoSlip || type == kPrescribed) ? -1.0 : (type == kSymmetry || type == kFixedPressure) ? 1.0 : 0.0;
 }
 
+void adi_attributes();
+
 }  // namespace
 
 AdiPlan* adi_plan_create(const Grid& g, const VBC& bc, double alpha) {
@@ -274,6 +276,7 @@ AdiPlan* adi_plan_create(const Grid& g, const VBC& bc, double alpha) {
       }
     }
   }
+  adi_attributes();
   if(!host.empty()) {
     OFB_CHECK(cudaMalloc(&p->coef, host.size() * sizeof(double)));
     OFB_CHECK(cudaMemcpy(p->coef, host.data(), host.size() * sizeof(double), cudaMemcpyHostToDevice));
@@ -588,13 +591,9 @@ void launch_scan(const SweepArgs& a, const ScanArgs& sa, int axis, int a1, int a
   if(axis == 0) {
     const long long nl = static_cast<long long>(a.L.n(a1)) * a.L.n(a2);
     const dim3 grid(static_cast<unsigned>((nl + LB - 1) / LB), 1, 1);
-    OFB_CHECK(cudaFuncSetAttribute(k_adi_scan<true, LB>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                   static_cast<int>(smem)));
     k_adi_scan<true, LB><<<grid, block, smem, s>>>(a, sa, in, out);
   } else {
     const dim3 grid((a.L.n(a1) + LB - 1) / LB, a.L.n(a2), 1);
-    OFB_CHECK(cudaFuncSetAttribute(k_adi_scan<false, LB>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                   static_cast<int>(smem)));
     k_adi_scan<false, LB><<<grid, block, smem, s>>>(a, sa, in, out);
   }
 }
@@ -804,10 +803,25 @@ void launch_decay(const AdiPlan* p, const int* comps, int count, int axis, const
   const size_t row = static_cast<size_t>(longest | 1) * sizeof(double);
   int rows = 16;
   if(most_rows < 2 * 148 * 16 || rows * chunks > 1024 || rows * row > 100 * 1024) rows = 4;
-  OFB_CHECK(cudaFuncSetAttribute(k_adi_rows, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 static_cast<int>(rows * row)));
   k_adi_rows<<<dim3((most_rows + rows - 1) / rows, count), (rows * chunks + 31) / 32 * 32, rows * row, s>>>(q, rows);
   OFB_LAUNCH_CHECK("k_adi_rows");
+}
+
+// Lets every line solver use the shared memory of its longest line.  The
+// attribute belongs to the kernel, not to a plan: set to one launch's size it
+// would be another thread's launch that fails.
+void adi_attributes() {
+  constexpr int kMost = 227 * 1024;  // per block, all of it dynamic in these kernels
+  auto attr = [](auto kern) {
+    OFB_CHECK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kMost));
+  };
+  attr(k_adi_scan<true, 4>);
+  attr(k_adi_scan<false, 4>);
+  attr(k_adi_scan<true, 16>);
+  attr(k_adi_scan<false, 16>);
+  attr(k_adi_tile<true>);
+  attr(k_adi_tile<false>);
+  attr(k_adi_rows);
 }
 
 }  // namespace
@@ -880,13 +894,9 @@ void launch_adi_sweep(const AdiPlan* p, int comp, int axis, const double* in, do
   if(axis == 0) {
     const long long nl = static_cast<long long>(a.L.n(a1)) * a.L.n(a2);
     dim3 grid(static_cast<unsigned>((nl + lines - 1) / lines), 1, 1);
-    OFB_CHECK(cudaFuncSetAttribute(k_adi_tile<true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                   static_cast<int>(smem)));
     k_adi_tile<true><<<grid, 32, smem, s>>>(a, in, out, lines);
   } else {
     dim3 grid((a.L.n(a1) + lines - 1) / lines, a.L.n(a2), 1);
-    OFB_CHECK(cudaFuncSetAttribute(k_adi_tile<false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                   static_cast<int>(smem)));
     k_adi_tile<false><<<grid, 32, smem, s>>>(a, in, out, lines);
   }
   OFB_LAUNCH_CHECK("k_adi_tile");

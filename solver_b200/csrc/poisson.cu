@@ -842,7 +842,8 @@ void setup_dense(PoissonPlan* P, const int* swaps, const double* factors) {
     t.zm = P->zero_mean;
     const int n = P->levels[first].L.count();
     auto columns = [&](auto* G, auto kern) {
-      OFB_CHECK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(bytes)));
+      // the limit itself, whatever this plan needs: the attribute is the kernel's
+      OFB_CHECK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(kSmemLimit)));
       kern<<<n, kTailThreads, bytes>>>(t, G);
       OFB_LAUNCH_CHECK("k_dense_columns");
     };

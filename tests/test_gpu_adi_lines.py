@@ -59,3 +59,32 @@ def test_couplings_without_a_decay_length(oracle, alpha):
     assert lines == lines_ref
     for a, b in zip(got, exp):
         assert np.max(np.abs(a - b)) <= 1e-12 * np.max(np.abs(b))
+
+
+@pytest.mark.parametrize("alpha", [0.001, 1.0])
+def test_threads_with_lines_of_different_lengths(alpha):
+    """Six contexts in six threads, half of them with lines that need far more
+    shared memory than the others', solving and building plans at the same time: a
+    launch must not depend on the sizes of another thread's."""
+    failed = []
+
+    def work(shape):
+        try:
+            g = sb.Grid(*shape, 0.1, 0.1, 0.1)
+            rhs = [np.ones(g.shape(c)) for c in "uvw"]
+            for _ in range(4):
+                with sb.Context(g, [sb.PERIODIC] * 6) as ctx:
+                    ctx.project_velocity(rhs, 0.01, 1.0, 5, 1e-6)
+                    for _ in range(400):
+                        out, _ = ctx.solve_predictor_adi(rhs, alpha)
+                    for o in out:  # a constant is unchanged
+                        assert np.max(np.abs(o[1:-1, 1:-1, 1:-1] - 1.0)) <= 1e-12
+        except Exception as e:
+            failed.append((shape, e))
+
+    threads = [threading.Thread(target=work, args=(s,)) for s in ((1000, 2, 1), (16, 2, 1)) * 3]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert not failed
