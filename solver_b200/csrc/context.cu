@@ -477,7 +477,8 @@ ofb::FinishArgs finish_args(of_ctx* ctx, const double* const* pred, double scale
 // image's value through every sweep.  With `ghosts` (the entry point that
 // returns the fields) the faces are set after every sweep and the last set is
 // the full one: the ghosts beside a wall face are filled from what the last
-// sweep made of it, before it is reset.  With sweep_out, sweep (component,
+// sweep made of it, before it is reset.  Without sweeps (alpha = 0) that one
+// is the only one.  With sweep_out, sweep (component,
 // axis) writes into sweep_out[component][axis] instead of the ping-pong
 // buffers, so every sweep's output survives the call (the adjoint needs them
 // for the viscosity derivative).
@@ -492,7 +493,8 @@ void predictor_adi(of_ctx* ctx, double alpha, double* out[3], int* line_solves, 
     out[c] = ctx->rhs[c];
     b[c] = ctx->adi_b[c];
   }
-  ofb::launch_normal_faces(ctx->g, ctx->bc, out[0], out[1], out[2], ctx->stream);
+  if(plan != nullptr || !ghosts)
+    ofb::launch_normal_faces(ctx->g, ctx->bc, out[0], out[1], out[2], ctx->stream);
   for(int axis = 0; plan != nullptr && axis < 3; ++axis) {
     const double* from[3] = {out[0], out[1], out[2]};
     double* to[3];

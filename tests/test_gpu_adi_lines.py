@@ -88,3 +88,25 @@ def test_threads_with_lines_of_different_lengths(alpha):
     for t in threads:
         t.join()
     assert not failed
+
+
+@pytest.mark.parametrize("shape", [(9, 12, 10), (16, 8, 1), (1, 9, 7)], ids=lambda s: "x".join(map(str, s)))
+@pytest.mark.parametrize("types", ["walls", "open", "periodic"])
+def test_no_diffusion_fills_the_boundaries_once(oracle, shape, types):
+    """alpha = 0: no sweep, and the ghosts are filled from the faces as they were
+    passed in, which only then are set (bitwise: nothing is computed but
+    2 value - neighbour)."""
+    g = po.Grid(*shape, 0.5, 0.6, 0.55)
+    sets = {"walls": [po.NO_SLIP_WALL, po.PRESCRIBED_VELOCITY, po.SYMMETRY, po.PRESCRIBED_VELOCITY,
+                      po.NO_SLIP_WALL, po.SYMMETRY],
+            "open": [po.PRESCRIBED_VELOCITY, po.FIXED_PRESSURE, po.NO_SLIP_WALL, po.NO_SLIP_WALL,
+                     po.PERIODIC, po.PERIODIC],
+            "periodic": [po.PERIODIC] * 6}
+    vel = [(0.25, 0.3, -0.2), (0.4, 0.2, -0.3), None, (0.7, -0.5, 0.1), None, None]
+    bc = po.bc_from(sets[types], [None] * 6 if types == "periodic" else vel)
+    rhs = _rhs(g, 5)
+    with sb.Context(to_gpu_grid(g), to_gpu_bc(bc)) as ctx:
+        got, _ = ctx.solve_predictor_adi(rhs, 0.0)
+    exp, _ = oracle.predictor_adi(g, bc, 0.0, *rhs)
+    for a, b in zip(got, exp):
+        assert np.array_equal(a, b)
