@@ -4,10 +4,10 @@
 // Dirichlet/ghost-relation end rows on walls, cyclic with Sherman-Morrison on
 // periodic axes -- so the Thomas factors (modified upper diagonal and inverse
 // pivots) and the Sherman-Morrison correction vector are computed once on the
-// host in FP64 and shared.  Lines whose coupling decays within a few dozen cells
-// (every projection step here: alpha / h^2 is well below one) are solved in
-// independent chunks (k_adi_lines, k_adi_rows); the others by one warp per line
-// (k_adi_scan) or one thread per line (k_adi_tile).
+// host in FP64 and shared.  Lines with a moderate coupling (every projection step
+// here: alpha / h^2 is well below one) are solved in chunks by sums with constant
+// weights (k_adi_lines, k_adi_rows); the others by one warp per line (k_adi_scan)
+// or one thread per line (k_adi_tile).
 #include "kernels.hpp"
 
 #include <algorithm>
@@ -30,17 +30,15 @@ struct AdiAxis {
   double uc_over_gamma = 0.0;
   double inv_den = 0.0;
   size_t off = 0;           // offset of cu/ip/z in the coefficient buffer
+  // chunked solver (see solve_chunk)
+  bool chunked = false;
+  double lambda = 0.0, scale = 0.0, fold = 0.0;
+  double step = 0.0, last = 0.0, all = 0.0;  // lambda to the power of a chunk, of the last one, of the line
+  double c_lo = 0.0, f_lo = 0.0, c_hi = 0.0, f_hi = 0.0, close = 0.0;  // sums beyond the ends
   // partition (warp-scan) solver, used when 64 <= n <= 1024 (n a multiple of
   // 32 on periodic axes; wall lines are padded to a multiple of 32):
   // per-lane segment factors, spikes and the interface operator, all laid
   // out [element][lane] so that a warp reads them with one coalesced load
-  // chunked solver (see k_adi_lines), used when the decay length fits
-  bool decay = false;
-  int reach = 0;            // K: cells after which the coupling is below rounding
-  double lambda = 0.0, scale = 0.0;
-  int node_lo = 0, node_hi = 0;            // the wall is a node (else half a cell off the first unknown)
-  double sign_lo = 0.0, sign_hi = 0.0;     // image of unknown x: add + sign x
-  double add_lo = 0.0, add_hi = 0.0;       // (at a node: add / 2 is the wall's value)
   bool partition = false;
   int seg = 0;              // K = ceil(n / 32)
   size_t poff = 0;          // offset: cu[K][32], ip[K][32], v[K][32], w[K][32], gl[64][32], gr[64][32]
@@ -54,16 +52,59 @@ struct AdiPlan {
 
 namespace {
 
-// When a line takes the chunked solver: its cost grows with (chunk + 2 reach),
-// so up to a reach of 64 cells (coupling alpha / h^2 up to about 2.5); shorter
-// lines than 8 unknowns go to k_adi_tile; a row must fit a block's threads.
-constexpr int kDecayMaxReach = 64, kDecayMinLine = 8, kRowMaxLine = 4096;
+// When a line takes the chunked solver.  The rounding of lambda moves the matrix
+// by (1 + lambda) / (1 - lambda) rounding errors, 3.3 at alpha / h^2 = 2.5 and
+// growing with its root: up to there the error against 64-bit exact solutions is
+// below the eliminations' (mean over lines of 8 to 1024 unknowns and alpha / h^2
+// from 1e-5 to 2.4: 2.7e-16 of the largest value, the eliminations 3.4e-16).
+// Shorter lines than 8 unknowns go to k_adi_tile; a line must fit a block's threads
+// (and a row its shared memory).
+constexpr double kChunkMaxBeta = 2.5;
+constexpr int kLineChunk = 16, kLineThreads = 1024;
+constexpr int kChunkMinLine = 8, kRowMaxLine = 4096, kLineMaxLine = kLineChunk * kLineThreads;
 
 double tangential_coef(int type) {
   return (type == kNoSlip || type == kPrescribed) ? -1.0 : (type == kSymmetry || type == kFixedPressure) ? 1.0 : 0.0;
 }
 
 void adi_attributes();
+
+// The chunked solver's constants for the line (component c, axis a), from the
+// rounded lambda in extended precision: the weights of the solution then add up
+// to one to rounding, so a sweep neither damps nor feeds a constant.  Appends
+// lambda^(distance to either end) of the chunks to `host`.
+void chunked_line(AdiAxis& A, double beta, const VBC& bc, int c, int a, std::vector<double>& host) {
+  using R = long double;
+  const int n = A.n, S = kLineChunk, chunks = (n + S - 1) / S;
+  A.chunked = true;
+  A.lambda = static_cast<double>(2.0L * beta / ((1.0L + 2.0L * beta) + std::sqrt(1.0L + 4.0L * beta)));
+  const R l = A.lambda;
+  auto power = [&](int k) { return static_cast<double>(std::pow(l, static_cast<R>(k))); };
+  A.scale = static_cast<double>((1.0L - l) * (1.0L - l));
+  A.fold = static_cast<double>(1.0L / (1.0L - l * l));
+  A.step = power(S);
+  A.last = power(n - S * (chunks - 1));
+  A.all = power(n);
+  // what lies beyond a wall: r there is the image add + sign r, or at a node
+  // the wall's value and the image about it
+  const R about_node = (1.0L + l) / (1.0L - l), about_face = 2.0L / (1.0L - l);
+  auto wall = [&](int face, double& constant, double& factor) {
+    const int type = bc.type[face];
+    const bool node = c == a && is_dirichlet_velocity(type);
+    const bool fixed = node || type == kNoSlip || type == kPrescribed;
+    constant = fixed ? static_cast<double>(bc.vel[face][c] * (node ? about_node : about_face)) : 0.0;
+    factor = node ? -A.lambda : fixed ? -1.0 : 1.0;
+  };
+  if(A.periodic) {
+    A.close = static_cast<double>(1.0L / (1.0L - std::pow(l, static_cast<R>(n))));
+  } else {
+    wall(2 * a, A.c_lo, A.f_lo);
+    wall(2 * a + 1, A.c_hi, A.f_hi);
+    A.close = static_cast<double>(1.0L / (1.0L - R(A.f_lo) * A.f_hi * std::pow(l, static_cast<R>(2 * n))));
+  }
+  for(int q = 0; q < chunks; ++q) host.push_back(power(q * S));
+  for(int q = 0; q < chunks; ++q) host.push_back(power(n - std::min(n, (q + 1) * S)));
+}
 
 }  // namespace
 
@@ -96,6 +137,11 @@ AdiPlan* adi_plan_create(const Grid& g, const VBC& bc, double alpha) {
       A.copy_duplicate = periodic && c == a;
       A.dup_index = L.n(a);  // active_end - 1
       A.lower = -beta;
+      A.off = host.size();
+      if(beta > 0.0 && beta <= kChunkMaxBeta && n >= kChunkMinLine && n <= (a == 0 ? kRowMaxLine : kLineMaxLine)) {
+        chunked_line(A, beta, bc, c, a, host);
+        continue;
+      }
       std::vector<double> di(n, 1.0 + 2.0 * beta), up(n, -beta), lo(n, -beta);
       lo[0] = 0.0;
       up[n - 1] = 0.0;
@@ -191,27 +237,6 @@ AdiPlan* adi_plan_create(const Grid& g, const VBC& bc, double alpha) {
           ip[q] = 1.0 / pivot;
         }
       }
-      // The infinite line's inverse is (lambda / beta) / (1 - lambda^2) times
-      // lambda^|distance|; reach is where its tail drops below 2^-56.
-      if(beta > 0.0) {
-        const double root = (1.0 + 2.0 * beta) + std::sqrt(1.0 + 4.0 * beta);
-        A.lambda = 2.0 * beta / root;
-        A.scale = 2.0 / root;
-        // (as a double: past beta = 1e15 it exceeds every int, and lambda = 1 has none)
-        const double reach = std::ceil((std::log(1.0 - A.lambda) - 56.0 * std::log(2.0)) / std::log(A.lambda));
-        A.decay = n >= kDecayMinLine && reach >= 0.0 && reach <= kDecayMaxReach && (a != 0 || n <= kRowMaxLine);
-        A.reach = A.decay ? static_cast<int>(reach) : 0;
-        auto wall = [&](int type, int face, int& node, double& sign, double& add) {
-          node = c == a && is_dirichlet_velocity(type);
-          const double v = bc.vel[face][c];
-          const bool fixed = node || type == kNoSlip || type == kPrescribed;
-          sign = fixed ? -1.0 : 1.0;
-          add = fixed ? 2.0 * v : 0.0;
-        };
-        wall(bc.type[2 * a], 2 * a, A.node_lo, A.sign_lo, A.add_lo);
-        wall(bc.type[2 * a + 1], 2 * a + 1, A.node_hi, A.sign_hi, A.add_hi);
-      }
-      A.off = host.size();
       host.insert(host.end(), cu.begin(), cu.end());
       host.insert(host.end(), ip.begin(), ip.end());
       host.insert(host.end(), z.begin(), z.end());
@@ -599,25 +624,33 @@ void launch_scan(const SweepArgs& a, const ScanArgs& sa, int axis, int a1, int a
 }
 
 // ---------------------------------------------------------------------------
-// Chunked line solver.  Away from the ends the Thomas factors of
-// (1 + 2 beta) x_q - beta (x_{q-1} + x_{q+1}) = r_q are constants: with lambda
-// the smaller root of beta l^2 - (1 + 2 beta) l + beta = 0,
-//   m_q = r_q + lambda m_{q-1},  y_q = m_q + lambda y_{q+1},  x = (lambda / beta) y,
-// and the influence of r fades as lambda^distance.  A chunk started K cells
-// before its first unknown and ended K cells after its last, with lambda^K
-// below the rounding, so gives the line's solution without the rest of the
-// line.  The ends are images: periodic wrap, or the reflection a wall row
-// stands for (its ghost relation x_{-1} = add + sign x_0, or x_{-1} = the wall's
-// value at a node and x_{-1-q} = add - x_{-1+q} beyond it), which r obeys too.
-// Replaces the per-line scans (k_adi_scan 116-127 us per sweep at 256^3 against
-// 42 us of traffic; k_adi_tile 61-98 us at 144 x 80 x 112).
+// Chunked line solver.  (1 + 2 beta) x_q - beta (x_{q-1} + x_{q+1}) = r_q on an
+// infinite line has the solution x_q = (1 - lambda) / (1 + lambda) sum over p of
+// lambda^|q - p| r_p, with lambda the smaller root of beta l^2 - (1 + 2 beta) l +
+// beta = 0.  A line's ends are images that r obeys as x does: periodic wrap, or
+// the reflection a wall row stands for (its ghost relation x_{-1} = add + sign
+// x_0, or x_{-1} = the wall's value at a node and x_{-1-q} = add - x_{-1+q}
+// beyond it).  So with the sums up to each end of a chunk,
+//   m_q = r_q + lambda m_{q-1}  (all r below),   b_q = r_q + lambda b_{q+1}  (all above),
+// the chunk is solved by m_q and y_q = m_q + lambda y_{q+1}, x = (1 - lambda)^2 y.
+// A thread holds a chunk of kLineChunk unknowns; the sums of the chunks below and
+// above it, and of the images (geometric series of the line's own two sums),
+// meet in shared memory.  Every term counts, however far: weights are positive, so
+// a small unknown far from a large r keeps its relative accuracy.
+//
+// Bound: one read and one write of each field (42 us per component and sweep at
+// 256^3).  Three components take 190 us; starting a chunk as many cells early as
+// lambda^cells needs to vanish took 219 (2 x 7 redundant reads per 16 unknowns,
+// and the terms beyond dropped), one scan per line (k_adi_scan) 366.  At 128^3
+// 30 instead of 39 us, at 128^2 8.6 instead of 10.2 (sweeps of y, z and x).
 // ---------------------------------------------------------------------------
 struct LineArgs {
   Lay L;
-  int n, begin, dup_index, periodic, copy_duplicate, reach;
-  double lambda, scale;
-  int node_lo, node_hi;
-  double sign_lo, sign_hi, add_lo, add_hi;
+  int n, begin, dup_index, periodic, copy_duplicate, chunks;
+  double lambda, scale, fold, step, last, all;
+  double c_lo, f_lo, c_hi, f_hi, close;
+  const double* from_lo;  // [chunks] lambda^(unknowns below the chunk)
+  const double* from_hi;  // [chunks] lambda^(unknowns above the chunk)
   const double* in;
   double* out;
 };
@@ -626,93 +659,96 @@ struct Lines3 {
   LineArgs c[3];  // the components of this launch
 };
 
-// r at unknown index q of a line (st apart from base), images included.
-__device__ __forceinline__ double line_at(const LineArgs& a, const double* base, int st, int q) {
-  if(q >= 0 && q < a.n) return base[q * st];
-  double add = 0.0, sign = 1.0;
-  while(q < 0 || q >= a.n) {
-    if(a.periodic) {
-      q += q < 0 ? a.n : -a.n;
-    } else if(q < 0) {
-      if(a.node_lo && q == -1) return add + sign * 0.5 * a.add_lo;
-      add += sign * a.add_lo;
-      sign *= a.sign_lo;
-      q = a.node_lo ? -2 - q : -1 - q;
-    } else {
-      if(a.node_hi && q == a.n) return add + sign * 0.5 * a.add_hi;
-      add += sign * a.add_hi;
-      sign *= a.sign_hi;
-      q = a.node_hi ? 2 * a.n - q : 2 * a.n - 1 - q;
+// Exclusive sums over the chunks of a line, in place; the whole line's sum goes
+// behind them.  Four loads at a time: a chain of single ones would wait for
+// shared memory at every chunk.
+__device__ __forceinline__ void sum_chunks(const LineArgs& a, double* v, int lanes, bool up) {
+  double s = 0.0;
+  for(int q0 = 0; q0 < a.chunks; q0 += 4) {
+    double t[4];
+#pragma unroll
+    for(int u = 0; u < 4; ++u) t[u] = q0 + u < a.chunks ? v[(up ? q0 + u : a.chunks - 1 - q0 - u) * lanes] : 0.0;
+#pragma unroll
+    for(int u = 0; u < 4; ++u) {
+      if(q0 + u >= a.chunks) break;
+      const int q = up ? q0 + u : a.chunks - 1 - q0 - u;
+      v[q * lanes] = s;
+      s = (q == a.chunks - 1 ? a.last : a.step) * s + t[u];
     }
   }
-  return add + sign * base[q * st];
+  v[a.chunks * lanes] = s;
 }
 
-// Unknowns [q0, q0 + S) of a line into y (y[t] valid for q0 + t < n).
-template <int S>
-__device__ __forceinline__ void solve_chunk(const LineArgs& a, const double* base, int st, int q0, double (&y)[S]) {
+// r of chunk c of the block's line `lane` (zero past the line's end) to x.  F and
+// B have (chunks + 1) x lanes entries.  All threads of the block call it.
+__device__ __forceinline__ void solve_chunk(const LineArgs& a, double (&y)[kLineChunk], int c, int lane, int lanes,
+                                            double* F, double* B) {
+  constexpr int S = kLineChunk;
+  const bool own = c < a.chunks;
+  const int count = own ? min(S, a.n - c * S) : 0;
   const double l = a.lambda;
-  const int K = a.reach;
-  double m = 0.0;
-  if(q0 - K >= 0 && q0 + S + K <= a.n) {  // no images
-    const double* r = base + (q0 - K) * st;
-#pragma unroll 4
-    for(int t = 0; t < K; ++t, r += st) m = *r + l * m;
+  double m = 0.0, b = 0.0;
 #pragma unroll
-    for(int t = 0; t < S; ++t, r += st) {
-      m = *r + l * m;
-      y[t] = m;
-    }
-    double z = 0.0, w = l;
-#pragma unroll 4
-    for(int t = 0; t < K; ++t, r += st) {
-      m = *r + l * m;
-      z += w * m;
-      w *= l;
-    }
-    y[S - 1] += z;
-  } else {
-    for(int t = -K; t < 0; ++t) m = line_at(a, base, st, q0 + t) + l * m;
+  for(int t = 0; t < S; ++t)
+    if(t < count) m = l * m + y[t];
 #pragma unroll
-    for(int t = 0; t < S; ++t) {
-      m = line_at(a, base, st, q0 + t) + l * m;
-      y[t] = m;
-    }
-    double z = 0.0, w = l;
-    for(int t = S; t < S + K; ++t) {
-      m = line_at(a, base, st, q0 + t) + l * m;
-      z += w * m;
-      w *= l;
-    }
-    y[S - 1] += z;
+  for(int t = S - 1; t >= 0; --t) b = l * b + y[t];
+  if(own) {
+    F[c * lanes + lane] = m;
+    B[c * lanes + lane] = b;
   }
+  __syncthreads();
+  if(c == 0) sum_chunks(a, F + lane, lanes, true);
+  if(c == (a.chunks > 1 ? 1 : 0)) sum_chunks(a, B + lane, lanes, false);
+  __syncthreads();
+  if(!own) return;
+  const double up = F[a.chunks * lanes + lane], down = B[a.chunks * lanes + lane];
+  double below, above;  // sums of the images beyond the line's ends
+  if(a.periodic) {
+    below = up * a.close;
+    above = down * a.close;
+  } else {
+    below = (a.c_lo + a.f_lo * (down + a.all * (a.c_hi + a.f_hi * up))) * a.close;
+    above = a.c_hi + a.f_hi * (up + a.all * below);
+  }
+  m = F[c * lanes + lane] + a.from_lo[c] * below;
+  b = B[c * lanes + lane] + a.from_hi[c] * above;
 #pragma unroll
-  for(int t = S - 2; t >= 0; --t) y[t] += l * y[t + 1];
+  for(int t = 0; t < S; ++t)
+    if(t < count) {
+      m = l * m + y[t];
+      y[t] = m;
+    }
+  double v = (l * m + b) * a.fold;
 #pragma unroll
-  for(int t = 0; t < S; ++t) y[t] *= a.scale;
+  for(int t = S - 1; t >= 0; --t)
+    if(t < count) {
+      v = l * v + y[t];
+      y[t] = a.scale * v;
+    }
 }
 
-// y and z sweeps: a thread solves kLineChunk unknowns of a line, a warp's
-// lines are adjacent in x (coalesced rows).  The chunk's redundant reads
-// (2 K of chunk + 2 K) come from L2: 32 unknowns per thread took 245 us per axis
-// for the three components at 256^3 (reach 7), 16 take 210 (more loads in flight).
-constexpr int kLineChunk = 16, kLineThreads = 128;
-
-__global__ void __launch_bounds__(kLineThreads) k_adi_lines(Lines3 s, int axis) {
+// y and z sweeps: a block solves `lanes` lines adjacent in x (coalesced rows), a
+// thread one chunk of one of them; reads and writes the field once.
+__global__ void __launch_bounds__(kLineThreads, 1) k_adi_lines(Lines3 s, int axis, int lanes) {
+  extern __shared__ double line_sm[];
   const LineArgs& a = s.c[blockIdx.y];
   const Lay& L = a.L;
-  const int iblocks = (L.nx + kLineThreads - 1) / kLineThreads;
-  const int chunks = (a.n + kLineChunk - 1) / kLineChunk;
+  const int iblocks = (L.nx + lanes - 1) / lanes;
   const int other = axis == 1 ? 2 : 1;
-  int b = blockIdx.x;
-  const int i = (b % iblocks) * kLineThreads + threadIdx.x;
-  b /= iblocks;
-  const int q0 = (b % chunks) * kLineChunk, o = b / chunks;
-  if(i >= L.nx || o >= L.n(other)) return;
+  const int lane = threadIdx.x % lanes, c = threadIdx.x / lanes;
+  const int i = (blockIdx.x % iblocks) * lanes + lane, o = blockIdx.x / iblocks;
+  if(o >= L.n(other)) return;
+  const int q0 = c * kLineChunk;
+  const bool work = i < L.nx && c < a.chunks;
   const int st = L.stride(axis);
   const int at = L.idx(i + 1, axis == 1 ? 0 : o + 1, axis == 1 ? o + 1 : 0);
+  const double* in = a.in + at + (a.begin + q0) * st;
   double y[kLineChunk];
-  solve_chunk<kLineChunk>(a, a.in + at + a.begin * st, st, q0, y);
+#pragma unroll
+  for(int t = 0; t < kLineChunk; ++t) y[t] = work && q0 + t < a.n ? in[t * st] : 0.0;
+  solve_chunk(a, y, c, lane, lanes, line_sm, line_sm + (a.chunks + 1) * lanes);
+  if(!work) return;
   double* out = a.out + at + (a.begin + q0) * st;
 #pragma unroll
   for(int t = 0; t < kLineChunk; ++t)
@@ -721,12 +757,9 @@ __global__ void __launch_bounds__(kLineThreads) k_adi_lines(Lines3 s, int axis) 
 }
 
 // x sweeps: a block stages whole rows in shared memory (odd row stride: lanes
-// on adjacent rows touch different banks), a thread solves kRowChunk unknowns
-// of one row, and the rows are stored back from shared memory (coalesced both
-// ways).
-constexpr int kRowChunk = 16;
-
-__global__ void __launch_bounds__(1024, 1) k_adi_rows(Lines3 s, int rows) {
+// on adjacent rows touch different banks), a thread solves one chunk of one row,
+// and the rows are stored back from shared memory (coalesced both ways).
+__global__ void __launch_bounds__(kLineThreads, 1) k_adi_rows(Lines3 s, int rows) {
   extern __shared__ double line_sm[];
   const LineArgs& a = s.c[blockIdx.y];
   const Lay& L = a.L;
@@ -740,15 +773,18 @@ __global__ void __launch_bounds__(1024, 1) k_adi_rows(Lines3 s, int rows) {
     for(int q = lane; q < a.n; q += 32) line_sm[l * stride + q] = a.in[at + q];
   }
   __syncthreads();
-  const int l = threadIdx.x % rows, q0 = threadIdx.x / rows * kRowChunk;
-  const bool work = q0 < a.n && first + l < total;
-  double y[kRowChunk];
-  if(work) solve_chunk<kRowChunk>(a, line_sm + l * stride, 1, q0, y);
-  __syncthreads();
+  const int l = threadIdx.x % rows, c = threadIdx.x / rows, q0 = c * kLineChunk;
+  const bool work = c < a.chunks && first + l < total;
+  double y[kLineChunk];
+  double* mine = line_sm + l * stride + q0;
+#pragma unroll
+  for(int t = 0; t < kLineChunk; ++t) y[t] = work && q0 + t < a.n ? mine[t] : 0.0;
+  double* F = line_sm + rows * stride;
+  solve_chunk(a, y, c, l, rows, F, F + (a.chunks + 1) * rows);
   if(work) {
 #pragma unroll
-    for(int t = 0; t < kRowChunk; ++t)
-      if(q0 + t < a.n) line_sm[l * stride + q0 + t] = y[t];
+    for(int t = 0; t < kLineChunk; ++t)
+      if(q0 + t < a.n) mine[t] = y[t];
   }
   __syncthreads();
   for(int w = warp; w < rows && first + w < total; w += warps) {
@@ -758,10 +794,9 @@ __global__ void __launch_bounds__(1024, 1) k_adi_rows(Lines3 s, int rows) {
   }
 }
 
-void launch_decay(const AdiPlan* p, const int* comps, int count, int axis, const double* const* in,
-                  double* const* out, cudaStream_t s) {
+void launch_chunked(const AdiPlan* p, const int* comps, int count, int axis, const double* const* in,
+                    double* const* out, cudaStream_t s) {
   Lines3 q{};
-  long long blocks = 0;
   int longest = 0, most_rows = 0;
   for(int t = 0; t < count; ++t) {
     const AdiAxis& A = p->ax[comps[t]][axis];
@@ -772,37 +807,45 @@ void launch_decay(const AdiPlan* p, const int* comps, int count, int axis, const
     a.dup_index = A.dup_index;
     a.periodic = A.periodic ? 1 : 0;
     a.copy_duplicate = A.copy_duplicate ? 1 : 0;
-    a.reach = A.reach;
+    a.chunks = (A.n + kLineChunk - 1) / kLineChunk;
     a.lambda = A.lambda;
     a.scale = A.scale;
-    a.node_lo = A.node_lo;
-    a.node_hi = A.node_hi;
-    a.sign_lo = A.sign_lo;
-    a.sign_hi = A.sign_hi;
-    a.add_lo = A.add_lo;
-    a.add_hi = A.add_hi;
+    a.fold = A.fold;
+    a.step = A.step;
+    a.last = A.last;
+    a.all = A.all;
+    a.c_lo = A.c_lo;
+    a.f_lo = A.f_lo;
+    a.c_hi = A.c_hi;
+    a.f_hi = A.f_hi;
+    a.close = A.close;
+    a.from_lo = p->coef + A.off;
+    a.from_hi = a.from_lo + a.chunks;
     a.in = in[comps[t]];
     a.out = out[comps[t]];
     longest = std::max(longest, A.n);
     most_rows = std::max(most_rows, a.L.ny * a.L.nz);
-    if(axis != 0) {
-      const long long b = static_cast<long long>((a.L.nx + kLineThreads - 1) / kLineThreads) *
-                          ((A.n + kLineChunk - 1) / kLineChunk) * a.L.n(axis == 1 ? 2 : 1);
-      blocks = std::max(blocks, b);
-    }
   }
+  const int chunks = (longest + kLineChunk - 1) / kLineChunk;
   ProfScope ps(kKAdi, s);
   if(axis != 0) {
-    k_adi_lines<<<dim3(static_cast<unsigned>(blocks), count), kLineThreads, 0, s>>>(q, axis);
+    int lanes = 32;
+    while(lanes * chunks > kLineThreads) lanes /= 2;
+    long long blocks = 0;
+    for(int t = 0; t < count; ++t) {
+      const Lay& L = q.c[t].L;
+      blocks = std::max(blocks, static_cast<long long>((L.nx + lanes - 1) / lanes) * L.n(axis == 1 ? 2 : 1));
+    }
+    const size_t smem = 2 * static_cast<size_t>(chunks + 1) * lanes * sizeof(double);
+    k_adi_lines<<<dim3(static_cast<unsigned>(blocks), count), lanes * chunks, smem, s>>>(q, axis, lanes);
     OFB_LAUNCH_CHECK("k_adi_lines");
     return;
   }
   // 16 rows per block (4 when that leaves fewer than two blocks per SM, or a
   // row so long that 16 pass the block's threads or 100 KB)
-  const int chunks = (longest + kRowChunk - 1) / kRowChunk;
-  const size_t row = static_cast<size_t>(longest | 1) * sizeof(double);
+  const size_t row = (static_cast<size_t>(longest | 1) + 2 * (chunks + 1)) * sizeof(double);
   int rows = 16;
-  if(most_rows < 2 * 148 * 16 || rows * chunks > 1024 || rows * row > 100 * 1024) rows = 4;
+  if(most_rows < 2 * 148 * 16 || rows * chunks > kLineThreads || rows * row > 100 * 1024) rows = 4;
   k_adi_rows<<<dim3((most_rows + rows - 1) / rows, count), (rows * chunks + 31) / 32 * 32, rows * row, s>>>(q, rows);
   OFB_LAUNCH_CHECK("k_adi_rows");
 }
@@ -830,20 +873,20 @@ void launch_adi_sweeps(const AdiPlan* p, int axis, const double* const* in, doub
   int together[3], count = 0;
   for(int c = 0; c < 3; ++c) {
     if(!p->ax[c][axis].active) continue;
-    if(p->ax[c][axis].decay) together[count++] = c;
+    if(p->ax[c][axis].chunked) together[count++] = c;
     else launch_adi_sweep(p, c, axis, in[c], out[c], s);
   }
-  if(count > 0) launch_decay(p, together, count, axis, in, out, s);
+  if(count > 0) launch_chunked(p, together, count, axis, in, out, s);
 }
 
 void launch_adi_sweep(const AdiPlan* p, int comp, int axis, const double* in, double* out,
                       cudaStream_t s) {
   const AdiAxis& A = p->ax[comp][axis];
   if(!A.active) return;
-  if(A.decay) {
+  if(A.chunked) {
     const double* ins[3] = {in, in, in};
     double* outs[3] = {out, out, out};
-    launch_decay(p, &comp, 1, axis, ins, outs, s);
+    launch_chunked(p, &comp, 1, axis, ins, outs, s);
     return;
   }
   SweepArgs a;

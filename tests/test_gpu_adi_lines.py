@@ -110,3 +110,49 @@ def test_no_diffusion_fills_the_boundaries_once(oracle, shape, types):
     exp, _ = oracle.predictor_adi(g, bc, 0.0, *rhs)
     for a, b in zip(got, exp):
         assert np.array_equal(a, b)
+
+
+ENDS = {
+    "periodic": ([po.PERIODIC] * 6, [None] * 6),
+    "walls": ([po.NO_SLIP_WALL, po.PRESCRIBED_VELOCITY, po.SYMMETRY, po.PRESCRIBED_VELOCITY, po.NO_SLIP_WALL,
+               po.SYMMETRY],
+              [None, (0.4, 0.2, -0.3), (0.1, 0.6, 0.0), (0.7, -0.5, 0.1), None, (0.2, 0.0, -0.8)]),
+    "open": ([po.PRESCRIBED_VELOCITY, po.FIXED_PRESSURE, po.FIXED_PRESSURE, po.NO_SLIP_WALL, po.PERIODIC,
+              po.PERIODIC],
+             [(1.0, 0.3, -0.2), None, None, None, None, None]),
+}
+
+
+# lines of one chunk (16 unknowns) and an unknown less or more, of two, and with
+# 32, 16 and 8 lines to a block; rows on both sides of the lengths where 16 and
+# 4 of them share one
+@pytest.mark.parametrize("types", list(ENDS))
+@pytest.mark.parametrize("shape", [(8, 15, 16), (17, 31, 8), (33, 9, 32), (16, 500, 3), (3, 520, 9), (5, 1030, 2),
+                                   (1030, 16, 1), (700, 70, 70)],
+                         ids=lambda s: "x".join(map(str, s)))
+def test_chunks_of_a_line(oracle, shape, types):
+    g = po.Grid(*shape, 0.5, 0.6, 0.55)
+    bc = po.bc_from(*ENDS[types])
+    for alpha in (1e-6, 0.05, 0.6):
+        _compare(oracle, g, bc, alpha, _rhs(g, sum(shape)))
+
+
+@pytest.mark.parametrize("types", ["periodic", "no_slip"])
+def test_small_unknowns_keep_their_relative_accuracy(oracle, types):
+    """The response to one large entry falls by many powers of ten along each
+    axis; every one of its values agrees with the elimination's relatively.
+    Either side multiplies one rounded factor per cell (both carry a few units
+    of 1.1e-16 each over at most 90 + 70 + 50 cells: below 1e-13), and wall images
+    of the other sign cancel less than two digits: 1e-11."""
+    g = po.Grid(90, 70, 50, 0.5, 0.5, 0.5)
+    bc = po.bc_from([po.PERIODIC] * 6 if types == "periodic" else [po.NO_SLIP_WALL] * 6)
+    rhs = [np.zeros(po.shape(g, c)) for c in "uvw"]
+    for r in rhs:
+        r[20, 30, 40] = 1.0
+    with sb.Context(to_gpu_grid(g), to_gpu_bc(bc)) as ctx:
+        got, _ = ctx.solve_predictor_adi(rhs, 0.3)
+    exp, _ = oracle.predictor_adi(g, bc, 0.3, *rhs)
+    for a, b in zip(got, exp):
+        a, b = po.active(a), po.active(b)
+        assert np.min(np.abs(b[b != 0.0])) < 1e-25
+        assert np.all(np.abs(a - b) <= 1e-11 * np.abs(b))
