@@ -1,8 +1,9 @@
-// Momentum-side stencils: the TVD/van Leer advection term (one launch per
-// component), the rest of the predictor right-hand side (diffusion, pressure
-// gradient, factorisation correction and the AB2 combination in one pass)
-// and the Taylor-Green initial state.
+// Momentum-side stencils: the TVD/van Leer advection term, the rest of the
+// predictor right-hand side (diffusion, pressure gradient, factorisation
+// correction and the AB2 combination in one pass), each one launch for the three
+// components, and the Taylor-Green initial state.
 #include "kernels.hpp"
+#include "quotient.cuh"
 
 namespace ofb {
 
@@ -10,27 +11,24 @@ namespace {
 
 constexpr double kSmallDenominator = 1.0e-14;  // solver/momentum_terms.cpp:14
 
-// n / d for 1e-14 <= |d| < 2^1022: the hardware's reciprocal approximation
-// (relative error 2^-23), one step of Halley's cubic iteration (2^-69) and
-// Markstein's residual correction of the quotient (Markstein, IBM J. Res. Dev.
-// 34, 1990), so the result is within one ulp.  The limiter's one division per
-// face in the general form was most of the advection's FP64 issue.
+// n / d as the division rounds it, within quotient_in_range (quotient.cuh).  The
+// hardware's reciprocal approximation reads the upper half of d and gives the
+// upper half of the result (20 fraction bits each: relative error below 2^-19).
 __device__ __forceinline__ double quotient(double n, double d) {
   double r;
   asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(d));
-  double e = fma(-d, r, 1.0);
-  e = fma(e, e, e);
-  r = fma(r, e, r);
-  const double q = n * r;
-  return fma(fma(-d, q, n), r, q);
+  return quotient_from(n, d, r);
 }
 
 // Branch-free form of one reconstruct_face call: every candidate value is
 // loaded before the velocity sign is known and the reference's three cases
 // (first-order upwind for |u_f| < 1e-14 or near the storage bounds, van Leer
 // MUSCL otherwise; solver/momentum_terms.cpp:42-151) are chosen by selects.
+// EXACT: with the division itself; else `past` is set where quotient() is outside
+// its range.
+template <bool EXACT>
 __device__ __forceinline__ double tvd_face(double vel, double left, double right, double far_left,
-                                           bool far_left_ok, double far_right, bool far_right_ok) {
+                                           bool far_left_ok, double far_right, bool far_right_ok, bool& past) {
   const bool up = vel >= 0.0;
   const double delta = right - left;
   const double num = up ? left - far_left : far_right - right;
@@ -42,7 +40,14 @@ __device__ __forceinline__ double tvd_face(double vel, double left, double right
   // the product num delta, whose underflow stands for a value below 1e-290).
   const double nd = num * delta;
   const bool positive = fabs(delta) >= kSmallDenominator && nd > 0.0;
-  const double half_phi_delta = positive ? quotient(nd, delta + num) : 0.0;
+  const double den = delta + num;
+  double half_phi_delta;
+  if constexpr(EXACT) {
+    half_phi_delta = positive ? nd / den : 0.0;
+  } else {
+    half_phi_delta = positive ? quotient(nd, den) : 0.0;
+    past = past || (positive && !quotient_in_range(__double2hiint(nd), __double2hiint(den), __double2loint(den)));
+  }
   const double muscl = up ? left + half_phi_delta : right - half_phi_delta;
   const bool first_order = fabs(vel) < kSmallDenominator || (up ? !far_left_ok : !far_right_ok);
   return first_order ? (up ? left : right) : muscl;
@@ -62,23 +67,30 @@ __device__ __forceinline__ Tile3 component_tile() {
 // The limited value carried by the face between storage points q - st and q
 // of f (position pd along the axis, smax its last storage index), times the
 // face's velocity (compute_{u,v,w}_advection, solver/momentum_terms.cpp:153-266).
+template <bool EXACT>
 __device__ __forceinline__ double face_flux(double vel, double fm1, double f0, double fm2, bool fm2_ok, double fp1,
-                                            bool fp1_ok) {
-  return vel * tvd_face(vel, fm1, f0, fm2, fm2_ok, fp1, fp1_ok);
+                                            bool fp1_ok, bool& past) {
+  return vel * tvd_face<EXACT>(vel, fm1, f0, fm2, fm2_ok, fp1, fp1_ok, past);
 }
 
 // Advection term of component C at the active points of a tile.  A point's
 // upper face is its neighbour's lower one: along x it comes from the next lane
 // (a warp evaluates 32 faces for 31 points), along z from the thread's next
 // plane; only y faces are evaluated twice -- four faces per point instead of
-// six, each the same operations as before (256^3: 755 -> 606 us at four blocks
-// per SM; three 690, five 616).
+// six, each the same operations as before (at 256^3 606 instead of 755 us when
+// that was changed, at four blocks per SM; three 690, five 616).
+//
+// Returns whether a limiter's quotient was outside the fast form's range; the
+// warp's points are then formed again with the division.  At 256^3 659 us; a
+// division in every face takes 735, a branch to it at every face 730, the
+// nearly always correct quotient that this replaces took 605.
 constexpr int kAdvectTile = kTX - 1;
 
-template <int C>
-__device__ __forceinline__ void advect_tile(const Grid& g, const double* __restrict__ u,
+template <int C, bool EXACT>
+__device__ __forceinline__ bool advect_tile(const Grid& g, const double* __restrict__ u,
                                             const double* __restrict__ v, const double* __restrict__ w,
                                             double* __restrict__ out, int bx, int kchunk) {
+  bool past = false;
   const double* __restrict__ vel[3] = {u, v, w};
   const double* __restrict__ f = vel[C];
   const Lay L = make_lay(g, kFaceX + C);
@@ -88,7 +100,7 @@ __device__ __forceinline__ void advect_tile(const Grid& g, const double* __restr
   const bool own = threadIdx.x < kAdvectTile && ip <= L.nx && jp <= L.ny;
   const int k0 = blockIdx.z * kchunk + 1;
   const int k1 = min(k0 + kchunk, L.nz + 1);
-  if(k0 >= k1) return;
+  if(k0 >= k1) return false;
   const double ihx = 1.0 / g.dx, ihy = 1.0 / g.dy, ihz = 1.0 / g.dz;
   int q = L.idx(i, j, k0);
   // velocity component d at this component's point: the mean of its two values
@@ -109,7 +121,7 @@ __device__ __forceinline__ void advect_tile(const Grid& g, const double* __restr
       at(2, k0, a, b);
       vz = 0.5 * (w[b] + w[a]);
     }
-    zlo = face_flux(vz, zm1, z0, f[k0 >= 2 ? q - 2 * L.sxy : q - L.sxy], k0 >= 2, zp1, k0 + 1 <= L.sz - 1);
+    zlo = face_flux<EXACT>(vz, zm1, z0, f[k0 >= 2 ? q - 2 * L.sxy : q - L.sxy], k0 >= 2, zp1, k0 + 1 <= L.sz - 1, past);
   }
   for(int k = k0; k < k1; ++k, q += L.sxy) {
     // x: this point's lower face, the upper one from the next lane
@@ -125,7 +137,7 @@ __device__ __forceinline__ void advect_tile(const Grid& g, const double* __restr
         at(0, k, a, b);
         vx = 0.5 * (u[b] + u[a]);
       }
-      const double lo = face_flux(vx, fm1, z0, fm2, i >= 2, fp1, i + 1 <= L.sx - 1);
+      const double lo = face_flux<EXACT>(vx, fm1, z0, fm2, i >= 2, fp1, i + 1 <= L.sx - 1, past);
       flux = (__shfl_down_sync(0xffffffffu, lo, 1) - lo) * ihx;
     }
     // y: both faces
@@ -143,8 +155,8 @@ __device__ __forceinline__ void advect_tile(const Grid& g, const double* __restr
         vl = 0.5 * (v[b] + v[a]);
         vh = 0.5 * (v[b + sd] + v[a + sd]);
       }
-      flux += (face_flux(vh, z0, fp1, fm1, true, fp2, j + 2 <= L.sy - 1) -
-               face_flux(vl, fm1, z0, fm2, j >= 2, fp1, true)) * ihy;
+      flux += (face_flux<EXACT>(vh, z0, fp1, fm1, true, fp2, j + 2 <= L.sy - 1, past) -
+               face_flux<EXACT>(vl, fm1, z0, fm2, j >= 2, fp1, true, past)) * ihy;
     }
     // z: the upper face, kept for the next plane
     {
@@ -157,7 +169,7 @@ __device__ __forceinline__ void advect_tile(const Grid& g, const double* __restr
         at(2, k + 1, a, b);
         vz = 0.5 * (w[b] + w[a]);
       }
-      const double zhi = face_flux(vz, z0, zp1, zm1, true, zp2, k + 2 <= L.sz - 1);
+      const double zhi = face_flux<EXACT>(vz, z0, zp1, zm1, true, zp2, k + 2 <= L.sz - 1, past);
       flux += (zhi - zlo) * ihz;
       zlo = zhi;
       zm1 = z0;
@@ -166,6 +178,7 @@ __device__ __forceinline__ void advect_tile(const Grid& g, const double* __restr
     }
     if(own) out[q] = flux;
   }
+  return past;
 }
 
 // Advection term of every component at its active points (the first half of
@@ -176,9 +189,16 @@ __global__ void __launch_bounds__(kTX* kTY, 4)
                 const double* __restrict__ w, double* __restrict__ au, double* __restrict__ av,
                 double* __restrict__ aw, int kchunk) {
   const Tile3 t = component_tile();
-  if(t.comp == 0) advect_tile<0>(g, u, v, w, au, t.bx, kchunk);
-  else if(t.comp == 1) advect_tile<1>(g, u, v, w, av, t.bx, kchunk);
-  else advect_tile<2>(g, u, v, w, aw, t.bx, kchunk);
+  if(t.comp == 0) {
+    if(__any_sync(0xffffffffu, advect_tile<0, false>(g, u, v, w, au, t.bx, kchunk)))
+      advect_tile<0, true>(g, u, v, w, au, t.bx, kchunk);
+  } else if(t.comp == 1) {
+    if(__any_sync(0xffffffffu, advect_tile<1, false>(g, u, v, w, av, t.bx, kchunk)))
+      advect_tile<1, true>(g, u, v, w, av, t.bx, kchunk);
+  } else {
+    if(__any_sync(0xffffffffu, advect_tile<2, false>(g, u, v, w, aw, t.bx, kchunk)))
+      advect_tile<2, true>(g, u, v, w, aw, t.bx, kchunk);
+  }
 }
 
 // Blocks of k_advect_bf: as launch3_components, on tiles of kAdvectTile points.
