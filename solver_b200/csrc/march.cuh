@@ -761,8 +761,8 @@ struct Direction {
 // stored -- k_advance forms it again from p, which costs its seven operations
 // instead of a vector written and read back.  The means of p and A p that the
 // reference removes are zero up to rounding (z - sz has none, A annihilates
-// constants) and are left in; the residual's, which they would move, is
-// removed every iteration.  Bound: reads z and p, writes p (3 vectors); at
+// constants) and are left in; those of x and of the residual, which they would
+// move, are removed every iteration.  Bound: reads z and p, writes p (3 vectors); at
 // 256^3 72 us in FP64, where the separate p update and A p took 71 + 66.
 template <typename T, bool SGN, bool FLAT>
 __global__ void __launch_bounds__(kMaxThreads, 1)
@@ -862,9 +862,10 @@ __global__ void __launch_bounds__(kMaxThreads, 1)
 
 // Solution and residual update (linsolve/poisson_solver.cpp:762-782):
 // x = (x - sx) + alpha p, r = (r - sr) - alpha A p (in FP64 arithmetic), the
-// residual's norm and the convergence test.  x keeps a zero mean up to
-// rounding (p has none).  Bound: reads p, x and r, writes x and r (5 vectors);
-// at 256^3 120 us in FP64, where the update from a stored A p took 142.
+// residual's norm and the convergence test, and the means of the new x and r (a
+// large mean in the initial guess leaves its rounding in the first x).  Bound:
+// reads p, x and r, writes x and r (5 vectors); at 256^3 123 us in FP64 (119
+// without the sum of x), where the update from a stored A p took 142.
 template <typename T, bool SGN, bool FLAT>
 __global__ void __launch_bounds__(kMaxThreads, 1)
     k_advance(OpInfo o, Tile t, Direction<T> d, T* __restrict__ x, T* __restrict__ r, SolveScalars* sc, RedBuf rb,
@@ -884,7 +885,7 @@ __global__ void __launch_bounds__(kMaxThreads, 1)
   const T* __restrict__ p = d.p[sc->body_runs & 1];
   const double alpha = sc->alpha, sr = sc->sr;
   const T sx = T(sc->sx), ax = T(alpha);
-  double acc[2] = {0.0, 0.0};
+  double acc[3] = {0.0, 0.0, 0.0};
   auto point = [&](int k, const Patch<T>& pv, const Patch<T>& minus_av, const Patch<T>& xv, const Patch<T>& rv) {
     Patch<T> xn, rn;
 #pragma unroll
@@ -897,6 +898,7 @@ __global__ void __launch_bounds__(kMaxThreads, 1)
         if(pl.interior(q, c)) {
           acc[0] += vr;
           acc[1] += vr * vr;
+          if constexpr(!SGN) acc[2] += double(xn.v[q][c]);
         }
       }
     pl.store(x, k * nxy, xn);
@@ -958,8 +960,8 @@ __global__ void __launch_bounds__(kMaxThreads, 1)
       __syncwarp();
     });
   }
-  const bool mx[2] = {false, false};
-  reduce_finish<2>(acc, mx, rb, [=](const Sums<2>& s) {
+  const bool mx[3] = {false, false, false};
+  reduce_finish<3>(acc, mx, rb, [=](const Sums<3>& s) {
     sc->body_runs += 1;
     if(sc->stop) {
       sc->cont = 0;
@@ -968,7 +970,7 @@ __global__ void __launch_bounds__(kMaxThreads, 1)
     }
     const int n = sc->n;
     const int zm = sc->zero_mean;
-    sc->sx = 0.0;
+    sc->sx = zm ? s.v[2] / n : 0.0;
     const double srn = zm ? s.v[0] / n : 0.0;
     sc->sr = srn;
     sc->sum_r = s.v[0];

@@ -135,3 +135,23 @@ def test_adi_chunks_at_line_ends(oracle, shape, types, alpha):
     assert lines == lines_ref
     for a, b in zip(got, exp):
         assert np.max(np.abs(a - b)) <= 1e-13 * np.max(np.abs(b))
+
+
+@pytest.mark.parametrize("precision", ["fp64", "mixed"])
+@pytest.mark.parametrize("types", [PER, NEU], ids=["periodic", "neumann"])
+@pytest.mark.parametrize("shape", [(48, 40, 32), (70, 72, 1)], ids=lambda s: "x".join(map(str, s)))
+def test_solution_has_no_mean_whatever_the_guess(shape, types, precision):
+    """Singular problems: the solution's mean is removed in every iteration, so a
+    guess far from zero leaves none of its rounding (1e6 x 1e-16) behind: the mean
+    of values of order one, rounded ones, is below 1e-15 of their size."""
+    import solver_b200 as sb
+    g = po.Grid(*shape, 0.02, 0.025, 0.03)
+    rng = np.random.default_rng(sum(shape))
+    rhs = rng.standard_normal(po.shape(g, "p"))
+    with sb.Context(to_gpu_grid(g), [sb.PERIODIC] * 6,
+                    precision=sb.OF_MIXED if precision == "mixed" else sb.OF_FP64) as ctx:
+        guess = 1e6 + rng.standard_normal(po.shape(g, "p"))
+        got, d = ctx.solve_pressure_poisson(rhs, to_gpu_pbc(po.pbc_from(types)), 400, 1e-10, pressure=guess)
+    x = po.active(got)
+    assert d["converged"] and d["iterations"] > 2
+    assert abs(np.mean(x)) <= 1e-15 * np.sqrt(np.mean(x * x))
