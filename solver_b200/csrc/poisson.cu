@@ -954,7 +954,14 @@ void plan_tile(const CLay& L, int halo_rows, int rz, int streams, int fields, in
     t.px = t.ix / W + 2;
     if(t.px > march::kPX) continue;
     t.tx = (L.nx + t.ix - 1) / t.ix;
-    const int max_rows = march::kMaxThreads / t.px * 2 - 2 * halo_rows;
+    // the most rows that a block's threads and its shared memory take (narrow
+    // grids: a row's shared memory has a fixed length)
+    auto smem_of = [&](int rows) {
+      t.ey = rows + 2 * halo_rows;
+      return march::smem_bytes<T>(t, streams, fields, flat, fields == 2);
+    };
+    int max_rows = march::kMaxThreads / t.px * 2 - 2 * halo_rows;
+    while(max_rows > 2 && smem_of(max_rows) > kMarchSmem) max_rows -= 2;
     if(max_rows < 2) continue;
     int last_iy = 0;
     const int nty0 = (L.ny + max_rows - 1) / max_rows;
@@ -962,10 +969,9 @@ void plan_tile(const CLay& L, int halo_rows, int rz, int streams, int fields, in
       t.iy = std::min(even((L.ny + nty - 1) / nty), max_rows);
       if(t.iy == last_iy) continue;
       last_iy = t.iy;
-      t.ey = t.iy + 2 * halo_rows;
-      const int threads = t.px * t.ey / 2;
-      const size_t smem = march::smem_bytes<T>(t, streams, fields, flat, fields == 2);
+      const size_t smem = smem_of(t.iy);
       if(smem > kMarchSmem) continue;
+      const int threads = t.px * t.ey / 2;
       const int resident = std::min<int>({(flat ? kFlatResident : march::kMaxThreads) / ((threads + 31) / 32 * 32),
                                           static_cast<int>(228 * 1024 / (smem + 2048)), 16});
       if(resident < 1) continue;

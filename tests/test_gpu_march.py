@@ -155,3 +155,29 @@ def test_solution_has_no_mean_whatever_the_guess(shape, types, precision):
     x = po.active(got)
     assert d["converged"] and d["iterations"] > 2
     assert abs(np.mean(x)) <= 1e-15 * np.sqrt(np.mean(x * x))
+
+
+@pytest.mark.parametrize("precision", ["fp64", "mixed"])
+@pytest.mark.parametrize("shape", [(2, 8192, 2), (4, 8192, 1), (3, 20480, 1), (8, 16384, 2)],
+                         ids=lambda s: "x".join(map(str, s)))
+def test_narrow_and_long_planes(oracle, shape, precision):
+    """Planes a few cells wide and many thousand long: a tile's rows are bounded
+    by its shared memory, not by its threads.  The residuals of the first
+    iterations as in test_pressure_solve_at_tile_edges."""
+    import solver_b200 as sb
+    g = po.Grid(*shape, 0.1, 0.12, 0.09)
+    rng = np.random.default_rng(sum(shape))
+    rhs = rng.standard_normal(po.shape(g, "p"))
+    pbc = po.pbc_from(MIX)
+    with sb.Context(to_gpu_grid(g), [sb.PERIODIC] * 6,
+                    precision=sb.OF_MIXED if precision == "mixed" else sb.OF_FP64) as ctx:
+        if precision == "mixed":
+            got, d = ctx.solve_pressure_poisson(rhs, to_gpu_pbc(pbc), 4000, 1e-10)
+            assert d["converged"] and d["relative_residual"] <= 1e-10
+            return
+        got, d = ctx.solve_pressure_poisson(rhs, to_gpu_pbc(pbc), 5, 1e-12)
+    ref = np.zeros(po.shape(g, "p"))
+    _, href = oracle.poisson_solve(g, pbc, 5, 1e-12, rhs, ref)
+    np.testing.assert_allclose(d["residual_history"], href, rtol=1e-9, atol=1e-12 * href[0])
+    a, b = po.active(got), po.active(ref)
+    assert np.max(np.abs(a - b)) <= 1e-9 * np.max(np.abs(b))
