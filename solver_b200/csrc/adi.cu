@@ -12,6 +12,7 @@
 
 #include <algorithm>
 #include <cmath>
+#include <memory>
 #include <vector>
 
 namespace ofb {
@@ -109,7 +110,8 @@ void chunked_line(AdiAxis& A, double beta, const VBC& bc, int c, int a, std::vec
 }  // namespace
 
 AdiPlan* adi_plan_create(const Grid& g, const VBC& bc, double alpha) {
-  AdiPlan* p = new AdiPlan();
+  std::unique_ptr<AdiPlan, void (*)(AdiPlan*)> plan(new AdiPlan(), adi_plan_destroy);
+  AdiPlan* const p = plan.get();
   p->g = g;
   std::vector<double> host;
   for(int c = 0; c < 3; ++c) {
@@ -152,7 +154,6 @@ AdiPlan* adi_plan_create(const Grid& g, const VBC& bc, double alpha) {
           // solve_cyclic_tridiagonal n == 1 (solver/projection.cpp:574-581)
           const double pivot = di[0] + lc + uc;
           if(std::fabs(pivot) < 1.0e-30) {
-            delete p;
             throw std::runtime_error("cyclic tridiagonal solve encountered a zero pivot");
           }
           cu[0] = 0.0;
@@ -171,7 +172,6 @@ AdiPlan* adi_plan_create(const Grid& g, const VBC& bc, double alpha) {
           for(int q = 1; q < n; ++q) {
             pivot = dm[q] - lo[q] * cu[q - 1];
             if(std::fabs(pivot) < 1.0e-30) {
-              delete p;
               throw std::runtime_error("tridiagonal solve encountered a zero pivot");
             }
             cu[q] = q + 1 < n ? up[q] / pivot : 0.0;
@@ -195,7 +195,6 @@ AdiPlan* adi_plan_create(const Grid& g, const VBC& bc, double alpha) {
           for(int q = n - 1; q-- > 0;) z[q] = mr[q] - mu[q] * z[q + 1];
           const double den = 1.0 + z[0] + uc * z[n - 1] / gamma;
           if(std::fabs(den) < 1.0e-30) {
-            delete p;
             throw std::runtime_error(
                 "cyclic tridiagonal solve encountered a singular Sherman-Morrison update");
           }
@@ -222,7 +221,6 @@ AdiPlan* adi_plan_create(const Grid& g, const VBC& bc, double alpha) {
         A.rhs_last = rn;
         double pivot = di[0];
         if(std::fabs(pivot) < 1.0e-30) {
-          delete p;
           throw std::runtime_error("tridiagonal solve encountered a zero pivot");
         }
         cu[0] = n > 1 ? up[0] / pivot : 0.0;
@@ -230,7 +228,6 @@ AdiPlan* adi_plan_create(const Grid& g, const VBC& bc, double alpha) {
         for(int q = 1; q < n; ++q) {
           pivot = di[q] - lo[q] * cu[q - 1];
           if(std::fabs(pivot) < 1.0e-30) {
-            delete p;
             throw std::runtime_error("tridiagonal solve encountered a zero pivot");
           }
           cu[q] = q + 1 < n ? up[q] / pivot : 0.0;
@@ -307,7 +304,7 @@ AdiPlan* adi_plan_create(const Grid& g, const VBC& bc, double alpha) {
     OFB_CHECK(cudaMemcpy(p->coef, host.data(), host.size() * sizeof(double), cudaMemcpyHostToDevice));
     OFB_CHECK(cudaStreamSynchronize(nullptr));  // the context's stream does not wait for the default one
   }
-  return p;
+  return plan.release();
 }
 
 void adi_plan_destroy(AdiPlan* p) {

@@ -25,6 +25,7 @@
 #include <cstdlib>
 #include <cstring>
 #include <algorithm>
+#include <memory>
 #include <type_traits>
 #include <vector>
 
@@ -1001,7 +1002,9 @@ void plan_tile(const CLay& L, int halo_rows, int rz, int streams, int fields, in
 }  // namespace
 
 PoissonPlan* poisson_plan_create(const Grid& g, const PBC& pbc_in, int precision) {
-  auto* P = new PoissonPlan();
+  // destroyed with the function's scope unless it gets to its end
+  std::unique_ptr<PoissonPlan, void (*)(PoissonPlan*)> plan(new PoissonPlan(), poisson_plan_destroy);
+  PoissonPlan* const P = plan.get();
   P->g = g;
   // homogeneous_boundary_conditions (linsolve/poisson_solver.cpp:164-173)
   P->pbc = pbc_in;
@@ -1059,7 +1062,6 @@ PoissonPlan* poisson_plan_create(const Grid& g, const PBC& pbc_in, int precision
   const Level& co = P->levels.back();
   const int n = co.L.count();
   if(n > kMaxCoarse) {
-    poisson_plan_destroy(P);
     throw std::invalid_argument("coarsest multigrid level has " + std::to_string(n) +
                                 " unknowns; at most " + std::to_string(kMaxCoarse) +
                                 " are supported");
@@ -1086,7 +1088,6 @@ PoissonPlan* poisson_plan_create(const Grid& g, const PBC& pbc_in, int precision
       }
     }
     if(best_abs < kSmallNumber) {
-      poisson_plan_destroy(P);
       throw std::runtime_error("direct coarse solve encountered a singular matrix");
     }
     swaps[piv] = best;
@@ -1154,7 +1155,7 @@ PoissonPlan* poisson_plan_create(const Grid& g, const PBC& pbc_in, int precision
   // context's stream does not synchronise: behind another thread's plan it
   // would still be on its way when the first solve runs
   OFB_CHECK(cudaStreamSynchronize(nullptr));
-  return P;
+  return plan.release();
 }
 
 void poisson_plan_destroy(PoissonPlan* P) {

@@ -181,3 +181,21 @@ def test_narrow_and_long_planes(oracle, shape, precision):
     np.testing.assert_allclose(d["residual_history"], href, rtol=1e-9, atol=1e-12 * href[0])
     a, b = po.active(got), po.active(ref)
     assert np.max(np.abs(a - b)) <= 1e-9 * np.max(np.abs(b))
+
+
+def test_refused_plans_leave_no_device_memory():
+    """A plan whose set-up fails (here: a coarsest level of 2500 unknowns) frees
+    what it had allocated: thirty of 10 MB each would show."""
+    import torch
+
+    import solver_b200 as sb
+    g = po.Grid(2, 20000, 4, 0.1, 0.1, 0.1)
+    rhs = np.zeros(po.shape(g, "p"))
+    pbc = to_gpu_pbc(po.pbc_from(PER))
+    with sb.Context(to_gpu_grid(g), [sb.PERIODIC] * 6) as ctx:
+        free = []
+        for _ in range(30):
+            with pytest.raises(ValueError, match="2500 unknowns"):
+                ctx.solve_pressure_poisson(rhs, pbc, 5, 1e-6)
+            free.append(torch.cuda.mem_get_info()[0])
+    assert free[0] - free[-1] < 32 << 20
