@@ -1,6 +1,7 @@
 #include "hostcopy.hpp"
 
 #include <cuda_runtime.h>
+#include <sched.h>
 #include <sys/mman.h>
 #include <unistd.h>
 
@@ -42,7 +43,15 @@ class Workers {
     for(std::thread& t : threads_) t.join();
   }
 
+  // In a child of fork() the threads do not exist: it must neither join them nor
+  // take a lock that one of them may have held.
+  bool forked() const { return getpid() != pid_; }
+
   void run(int parts, const std::function<void(int)>& fn) {
+    if(forked()) {
+      for(int i = 0; i < parts; ++i) fn(i);
+      return;
+    }
     auto job = std::make_shared<Job>();
     job->fn = &fn;
     job->parts = parts;
@@ -91,6 +100,7 @@ class Workers {
     }
   }
 
+  const pid_t pid_ = getpid();
   std::vector<std::thread> threads_;
   std::mutex mutex_;
   std::condition_variable wake_;
@@ -104,7 +114,7 @@ std::mutex g_mutex;  // guards the three below
 int g_contexts = 0;
 bool g_leased = false;
 char* g_slots = nullptr;
-std::unique_ptr<Workers> g_workers;
+Workers* g_workers = nullptr;  // not destroyed at exit: the threads end with the process
 
 }  // namespace
 
@@ -124,10 +134,11 @@ void staging_retain() {
 }
 
 void staging_release() {
-  std::unique_ptr<Workers> workers;
+  std::unique_ptr<Workers> workers;  // joined after the lock is gone
   std::lock_guard<std::mutex> lock(g_mutex);
   if(--g_contexts > 0 || g_leased) return;
-  workers = std::move(g_workers);
+  if(g_workers != nullptr && !g_workers->forked()) workers.reset(g_workers);
+  g_workers = nullptr;
   if(g_slots != nullptr) cudaFreeHost(g_slots);
   g_slots = nullptr;
 }
@@ -145,7 +156,7 @@ StagingLease::StagingLease() {
   }
   if(g_workers == nullptr) {
     const int cores = static_cast<int>(std::thread::hardware_concurrency());
-    g_workers = std::make_unique<Workers>(std::min(7, std::max(0, cores - 1)));
+    g_workers = new Workers(std::min(7, std::max(0, cores - 1)));
   }
   g_leased = held_ = true;
 }

@@ -7,6 +7,9 @@ the advection term and of the pressure fields -- must come back as passed in.
 The sizes give fields below and above one slot (2 MiB) and storage rows that
 straddle its chunks.
 """
+import os
+import subprocess
+import sys
 import threading
 
 import numpy as np
@@ -73,3 +76,51 @@ def test_staged_transfers_equal_plain_ones(size):
     for k in range(2):
         for a, b in zip(plain, got[k]):
             assert np.array_equal(a, b)
+
+
+ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+CHILD = """
+import os, sys, time
+sys.path.insert(0, {root!r})
+import numpy as np
+import solver_b200 as sb
+g = sb.Grid(96, 96, 96, 0.1, 0.1, 0.1)
+ctx = sb.Context(g, [sb.PERIODIC] * 6)
+v = [np.ones(g.shape(c)) for c in "uvw"]
+{body}
+"""
+
+
+def _run(body):
+    r = subprocess.run([sys.executable, "-W", "ignore", "-c", CHILD.format(root=ROOT, body=body)],
+                       capture_output=True, text=True, timeout=60)
+    assert r.returncode == 0, r.stderr
+    return r.stdout.split()
+
+
+@pytest.mark.parametrize("close", [False, True])
+def test_forked_child_ends_normally(close):
+    """The workers do not exist in a child of fork(): closing its copy of the
+    context or leaving must not wait for them (nor crash)."""
+    out = _run(f"""
+ctx.compute_advection_term(*v)
+time.sleep(0.05)
+pid = os.fork()
+if pid == 0:
+    if {close}:
+        ctx.close()
+    sys.exit(0)
+end = time.time() + 20
+while time.time() < end:
+    done, status = os.waitpid(pid, os.WNOHANG)
+    if done:
+        break
+    time.sleep(0.02)
+else:
+    os.kill(pid, 9)
+    status = "hangs"
+ctx.compute_advection_term(*v)
+ctx.close()
+print(status)
+""")
+    assert out == ["0"]
