@@ -110,6 +110,13 @@ class Workers {
   bool quit_ = false;
 };
 
+// CPUs that this process may use.
+int usable_cpus() {
+  cpu_set_t set;
+  if(sched_getaffinity(0, sizeof(set), &set) == 0) return CPU_COUNT(&set);
+  return static_cast<int>(std::thread::hardware_concurrency());
+}
+
 std::mutex g_mutex;  // guards the three below
 int g_contexts = 0;
 bool g_leased = false;
@@ -155,8 +162,7 @@ StagingLease::StagingLease() {
     g_slots = static_cast<char*>(p);
   }
   if(g_workers == nullptr) {
-    const int cores = static_cast<int>(std::thread::hardware_concurrency());
-    g_workers = new Workers(std::min(7, std::max(0, cores - 1)));
+    g_workers = new Workers(std::min(7, std::max(0, usable_cpus() - 1)));
   }
   g_leased = held_ = true;
 }

@@ -124,3 +124,21 @@ ctx.close()
 print(status)
 """)
     assert out == ["0"]
+
+
+@pytest.mark.parametrize("cpus", [1, 2])
+def test_workers_fit_the_cpus_of_the_process(cpus):
+    """A process held to few CPUs gets a worker less than it has CPUs, not one for
+    every core of the machine."""
+    if len(os.sched_getaffinity(0)) <= cpus:
+        pytest.skip("too few CPUs to tell")
+    out = _run(f"""
+ctx.solve_predictor_adi([x[:] for x in v], 0.0)
+ctx.close()  # ends the workers
+ctx = sb.Context(g, [sb.PERIODIC] * 6)
+os.sched_setaffinity(0, set(sorted(os.sched_getaffinity(0))[:{cpus}]))
+before = len(os.listdir("/proc/self/task"))
+ctx.compute_advection_term(*v)
+print(len(os.listdir("/proc/self/task")) - before)
+""")
+    assert int(out[0]) <= cpus - 1
