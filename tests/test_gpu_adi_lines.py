@@ -156,3 +156,18 @@ def test_small_unknowns_keep_their_relative_accuracy(oracle, types):
         a, b = po.active(a), po.active(b)
         assert np.min(np.abs(b[b != 0.0])) < 1e-25
         assert np.all(np.abs(a - b) <= 1e-11 * np.abs(b))
+
+
+@pytest.mark.parametrize("beta", [2.45, 2.55, 30.0])
+@pytest.mark.parametrize("types", ["walls", "periodic"])
+@pytest.mark.parametrize("shape", [(200, 130, 1), (1000, 40, 1), (96, 70, 12), (128, 64, 10)],
+                         ids=lambda s: "x".join(map(str, s)))
+def test_both_sides_of_the_coupling_limit(oracle, shape, types, beta):
+    """alpha / h^2 just below the chunked solver's limit (2.5) and above it, where
+    lines of 64 to 1024 unknowns take the warp scan: wall lines whose length is not
+    a multiple of 32 (199, 999, 95, 69 unknowns) padded to one, few long lines (2D)
+    four to a block, periodic ones that do not divide one thread each.  The
+    matrices' condition is at most 1 + 4 beta = 121: 1e-13 still holds."""
+    g = po.Grid(*shape, 0.5, 0.5, 0.5)
+    bc = po.bc_from(*ENDS[types])
+    _compare(oracle, g, bc, beta * 0.25, _rhs(g, sum(shape)))

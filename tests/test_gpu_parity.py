@@ -346,3 +346,44 @@ def test_step_host_failure_leaves_host_state_unchanged(sb, oracle):
         assert np.array_equal(host[name], a), name
     assert host["has_previous_advection"] == 1
     assert host["metrics"]["step"] == 1
+
+
+@pytest.mark.parametrize("precision", ["fp64", "mixed"])
+@pytest.mark.parametrize("on_device", [True, False], ids=["graph", "host_loop"])
+@pytest.mark.parametrize("case", ["taylor_green", "cavity"])
+def test_failed_step_leaves_the_resident_state_alone(sb, oracle, monkeypatch, case, on_device, precision):
+    """A solve that does not converge (one iteration at tolerance 1e-30) is only
+    noticed when the rest of the step has run behind it: none of that may have
+    touched the state, total pressure and history included, and the next step
+    goes on from it as if nothing had been tried."""
+    if not on_device:
+        monkeypatch.setenv("ORCHARD_B200_NO_GRAPH", "1")
+    if case == "cavity":
+        cfg = po.cavity_config(24, 24)
+        g, bc = oracle.cavity_grid(cfg), oracle.cavity_bc(cfg)
+        s0, nu, dt, variant = oracle.cavity_init(cfg), 0.01, oracle.cavity_dt(cfg), sb.OF_CORRECTION_CAVITY
+    else:
+        cfg = po.steps_config(32, 32, 16, 0.01, 0.5, 2, 1e-12)
+        g, bc = oracle.tg_grid(cfg), oracle.tg_bc(cfg)
+        s0, nu, dt, variant = oracle.tg_init(cfg, 0), 0.01, oracle.tg_dt(cfg), sb.OF_CORRECTION_TAYLOR_GREEN
+    prec = sb.OF_MIXED if precision == "mixed" else sb.OF_FP64
+    good, bad = sb.step_params(nu, dt, 400, 1e-10, variant), sb.step_params(nu, dt, 1, 1e-30, variant)
+    names = ("u", "v", "w", "adv_u", "adv_v", "adv_w", "p")
+    ends = []
+    for fail in (False, True):
+        with sb.Context(to_gpu_grid(g), to_gpu_bc(bc), precision=prec) as ctx:
+            ctx.upload_state(s0.u, s0.v, s0.w, s0.adv_u, s0.adv_v, s0.adv_w, s0.p, 0, s0.metrics)
+            ctx.run_steps(good, 2)
+            if fail:
+                before = ctx.download_state()
+                for _ in range(2):
+                    with pytest.raises(sb.NotConvergedError, match="at step 3"):
+                        ctx.run_steps(bad, 1)
+                after = ctx.download_state()
+                for n in names:
+                    assert np.array_equal(before[n], after[n]), n
+                assert after["metrics"]["step"] == 2
+            ctx.run_steps(good, 1)
+            ends.append(ctx.download_state())
+    for n in names:
+        assert np.array_equal(ends[0][n], ends[1][n]), n
