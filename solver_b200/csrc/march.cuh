@@ -240,12 +240,22 @@ __device__ __forceinline__ void publish(T* me, const Patch<T>& q) {
     for(int c = 0; c < kW<T>; ++c) me[r * kRow<T> + c * kPX] = q.v[r][c];
 }
 
-// Sums of the x and of the y neighbours of a published patch.  At the rim of
-// the extended tile the words read are not the true neighbours (another run's
-// end, a guard row); the cells they spoil are never used: the halo shrinks by
-// one cell per sweep.
+// Second differences along x and y of a published patch, each as the reference
+// forms it (linsolve/poisson_solver.cpp:244-262): high - 2 centre + low.  For a
+// smooth field the two operations are exact (what remains is a multiple of the
+// values' last bit and small), so the operator's error is that of its value; as
+// a multiple of the centre less the sums of the neighbours it would be that of
+// the centre's term, larger by the square of the cells across the field, and A of
+// a constant would not vanish.  At the rim of the extended tile the words read are
+// not the true neighbours (another run's end, a guard row); the cells they spoil
+// are never used: the halo shrinks by one cell per sweep.
 template <typename T>
-__device__ __forceinline__ void neighbour_sums(const T* me, const Patch<T>& q, Patch<T>& xs, Patch<T>& ys) {
+__device__ __forceinline__ T second_difference(T low, T centre, T high) {
+  return (high - T(2) * centre) + low;
+}
+
+template <typename T>
+__device__ __forceinline__ void differences(const T* me, const Patch<T>& q, Patch<T>& xs, Patch<T>& ys) {
   constexpr int W = kW<T>;
 #pragma unroll
   for(int r = 0; r < 2; ++r)
@@ -253,28 +263,26 @@ __device__ __forceinline__ void neighbour_sums(const T* me, const Patch<T>& q, P
     for(int c = 0; c < W; ++c) {
       const T l = c > 0 ? q.v[r][c > 0 ? c - 1 : 0] : me[r * kRow<T> + (W - 1) * kPX - 1];
       const T h = c < W - 1 ? q.v[r][c < W - 1 ? c + 1 : 0] : me[r * kRow<T> + 1];
-      xs.v[r][c] = l + h;
+      xs.v[r][c] = second_difference(l, q.v[r][c], h);
     }
 #pragma unroll
   for(int c = 0; c < W; ++c) {
-    ys.v[0][c] = me[c * kPX - kRow<T>] + q.v[1][c];
-    ys.v[1][c] = q.v[0][c] + me[c * kPX + 2 * kRow<T>];
+    ys.v[0][c] = second_difference(me[c * kPX - kRow<T>], q.v[0][c], q.v[1][c]);
+    ys.v[1][c] = second_difference(q.v[0][c], q.v[1][c], me[c * kPX + 2 * kRow<T>]);
   }
 }
 
-// Operator coefficients: A u = dd u - ix (x neighbours) - iy (y) - iz (z).  A
-// grid one cell deep (FLAT) folds its z images into dd.
+// Operator coefficients: A u = - ix (second difference along x) - iy (y) - iz (z).
+// On a grid one cell deep (FLAT) the z term is zz u: its images are u itself, or
+// -u at a Dirichlet face.
 template <typename T>
 struct Coef {
-  T ix, iy, iz, dd;
-  __device__ __forceinline__ Coef(const OpInfo& o, bool flat) {
-    double d = 2.0 * (o.inv2[0] + o.inv2[1]);
-    if(!flat) d += 2.0 * o.inv2[2];
-    else if(!o.periodic[2]) d += (o.dir_lo[2] ? 2.0 * o.inv2[2] : 0.0) + (o.dir_hi[2] ? 2.0 * o.inv2[2] : 0.0);
+  T ix, iy, iz, zz;
+  __device__ __forceinline__ explicit Coef(const OpInfo& o) {
     ix = T(o.inv2[0]);
     iy = T(o.inv2[1]);
     iz = T(o.inv2[2]);
-    dd = T(d);
+    zz = T(o.periodic[2] ? 0.0 : 2.0 * o.inv2[2] * (o.dir_lo[2] + o.dir_hi[2]));
   }
 };
 
@@ -288,10 +296,10 @@ __device__ __forceinline__ Patch<T> residual(const Coef<T>& a, const Patch<T>& b
   for(int r = 0; r < 2; ++r)
 #pragma unroll
     for(int c = 0; c < kW<T>; ++c) {
-      T t = b.v[r][c] - a.dd * u.v[r][c];
-      t += a.ix * xs.v[r][c];
+      T t = b.v[r][c] + a.ix * xs.v[r][c];
       t += a.iy * ys.v[r][c];
-      if constexpr(!FLAT) t += a.iz * (below.v[r][c] + above.v[r][c]);
+      if constexpr(FLAT) t -= a.zz * u.v[r][c];
+      else t += a.iz * second_difference(below.v[r][c], u.v[r][c], above.v[r][c]);
       o.v[r][c] = t;
     }
   return o;
@@ -443,7 +451,7 @@ __device__ __forceinline__ void ring4(int s0, int s1, Step step) {
 //
 // Bound: one read of b, one write of x and of bc (2.125 vectors); in FP64 at
 // 256^3 the arithmetic and the shared-memory traffic are each near the DRAM time:
-// 81 us (FP32 54), where the pre-sweeps and the residual with its restriction
+// 85 us (FP32 55), where the pre-sweeps and the residual with its restriction
 // took 53 + 65 in two passes.
 template <typename T, bool SGN, bool CD, bool FLAT>
 __global__ void __launch_bounds__(kMaxThreads, 1)
@@ -460,7 +468,7 @@ __global__ void __launch_bounds__(kMaxThreads, 1)
   }
   Weights<T, CD> W(tab, T(2.0 / 3.0 * o.invd[0]));
   const Place<T, SGN> pl(o, t, 2);
-  const Coef<T> co(o, FLAT);
+  const Coef<T> co(o);
   const T inv_children = T(1.0 / double(rx * ry * rz));
   const int nxy = o.L.nxy;
   const int k0 = blockIdx.y * t.chunk, k1 = min(k0 + t.chunk, o.L.nz);
@@ -500,12 +508,12 @@ __global__ void __launch_bounds__(kMaxThreads, 1)
     const Patch<T> a = times(W.w, bq);
     publish(me, a);
     __syncthreads();
-    neighbour_sums(me, a, xs, ys);
+    differences(me, a, xs, ys);
     const Patch<T> xq = relax(a, W.w, residual<T, true>(co, bq, a, xs, ys, a, a));
     pl.store(x, 0, xq);
     publish(me + pw, xq);
     __syncthreads();
-    neighbour_sums(me + pw, xq, xs, ys);
+    differences(me + pw, xq, xs, ys);
     racc = residual<T, true>(co, bq, xq, xs, ys, xq, xq);
     restrict_out(0);
   } else {
@@ -542,11 +550,11 @@ __global__ void __launch_bounds__(kMaxThreads, 1)
       A[N] = times(W.w, B[N]);
       __syncthreads();
       W.at(o, pl.cls, s);
-      neighbour_sums(pa, A[J], xs, ys);
+      differences(pa, A[J], xs, ys);
       const Patch<T> xc = relax(A[J], W.w, residual<T, false>(co, B[J], A[J], xs, ys, A[M], A[N]));
       if(s >= k0 && s < k1) pl.store(x, s * nxy, xc);
       if(s > k0) {
-        neighbour_sums(pa + pw, X[M], xs, ys);
+        differences(pa + pw, X[M], xs, ys);
         const Patch<T> res = residual<T, false>(co, B[M], X[M], xs, ys, X[F], xc);
         const bool first = rz == 1 || ((s - 1) & 1) == 0;
 #pragma unroll
@@ -567,7 +575,7 @@ __global__ void __launch_bounds__(kMaxThreads, 1)
 // level (FINE) it also forms mean(out) and r.z for the CG; on the others no
 // mean is needed (see k_descend).  sx, sy, sz: log2 of the coarsening ratios.
 //
-// Bound: reads x, b and e, writes out (3.125 vectors); 97 us at 256^3 in FP64 (66
+// Bound: reads x, b and e, writes out (3.125 vectors); 107 us at 256^3 in FP64 (71
 // in FP32), where the prolongation with one sweep and the second sweep took 89 + 78.
 template <typename T, bool SGN, bool CD, bool FLAT, bool FINE, bool PAIRS>
 __global__ void __launch_bounds__(kMaxThreads, 1)
@@ -585,7 +593,7 @@ __global__ void __launch_bounds__(kMaxThreads, 1)
   }
   Weights<T, CD> W(tab, T(2.0 / 3.0 * o.invd[0]));
   const Place<T, SGN> pl(o, t, 2);
-  const Coef<T> co(o, FLAT);
+  const Coef<T> co(o);
   const int nxy = o.L.nxy;
   const int k0 = blockIdx.y * t.chunk, k1 = min(k0 + t.chunk, o.L.nz);
   T* me = planes + (pl.row0 + 1) * kRow<T> + pl.p;
@@ -661,11 +669,11 @@ __global__ void __launch_bounds__(kMaxThreads, 1)
     W.at(o, pl.cls, 0);
     publish(me, y);
     __syncthreads();
-    neighbour_sums(me, y, xs, ys);
+    differences(me, y, xs, ys);
     const Patch<T> y1 = relax(y, W.w, residual<T, true>(co, bq, y, xs, ys, y, y));
     publish(me + pw, y1);
     __syncthreads();
-    neighbour_sums(me + pw, y1, xs, ys);
+    differences(me + pw, y1, xs, ys);
     finish(0, relax(y1, W.w, residual<T, true>(co, bq, y1, xs, ys, y1, y1)), bq);
   } else {
     // step s: y'(s) from y(s - 1 .. s + 1), then out(s - 1)
@@ -721,11 +729,11 @@ __global__ void __launch_bounds__(kMaxThreads, 1)
       pl.settle(B[J], sb, SGN && zneg(o, s));
       __syncthreads();
       W.at(o, pl.cls, s);
-      neighbour_sums(pa, Y[J], xs, ys);
+      differences(pa, Y[J], xs, ys);
       const Patch<T> vc = relax(Y[J], W.w, residual<T, false>(co, B[J], Y[J], xs, ys, Y[M], Y[N]));
       if(s > k0) {
         W.at(o, pl.cls, s - 1);
-        neighbour_sums(pa + pw, V[M], xs, ys);
+        differences(pa + pw, V[M], xs, ys);
         finish(s - 1, relax(V[M], W.w, residual<T, false>(co, B[M], V[M], xs, ys, V[F], vc)), B[M]);
       }
       V[J] = vc;
@@ -758,7 +766,7 @@ struct Direction {
 
 // New search direction and its products (linsolve/poisson_solver.cpp:750-761):
 // p = (z - sz) + beta p (first iteration: z - sz) and p.Ap; A p itself is not
-// stored -- k_advance forms it again from p, which costs its seven operations
+// stored -- k_advance forms it again from p, which costs its nine operations
 // instead of a vector written and read back.  The means of p and A p that the
 // reference removes are zero up to rounding (z - sz has none, A annihilates
 // constants) and are left in; those of x and of the residual, which they would
@@ -773,7 +781,7 @@ __global__ void __launch_bounds__(kMaxThreads, 1)
   const int sw = slot_words<T>(t), pw = plane_words<T>(t);
   T* pring = ring + kRing * sw;
   const Place<T, SGN> pl(o, t, 1);
-  const Coef<T> co(o, FLAT);
+  const Coef<T> co(o);
   const int nxy = o.L.nxy;
   const int k0 = blockIdx.y * t.chunk, k1 = min(k0 + t.chunk, o.L.nz);
   T* me = (FLAT ? ring : ring + 2 * kRing * sw) + (pl.row0 + 1) * kRow<T> + pl.p;
@@ -812,7 +820,7 @@ __global__ void __launch_bounds__(kMaxThreads, 1)
     combine(q, first ? none : pl.load(po, 0), false);
     publish(me, q);
     __syncthreads();
-    neighbour_sums(me, q, xs, ys);
+    differences(me, q, xs, ys);
     point(0, q, residual<T, true>(co, none, q, xs, ys, q, q));
   } else {
     // step s: p(s + 1) is combined, A p(s) formed
@@ -846,7 +854,7 @@ __global__ void __launch_bounds__(kMaxThreads, 1)
       publish(pa, P[J]);
       combine(P[N], old, SGN && zneg(o, s + 1));
       __syncthreads();
-      neighbour_sums(pa, P[J], xs, ys);
+      differences(pa, P[J], xs, ys);
       point(s, P[J], residual<T, false>(co, none, P[J], xs, ys, P[M], P[N]));
       __syncwarp();
     });
@@ -875,7 +883,7 @@ __global__ void __launch_bounds__(kMaxThreads, 1)
   const int sw = slot_words<T>(t), pw = plane_words<T>(t);
   T *xring = ring + kRing * sw, *rring = xring + kRing * sw;
   const Place<T, SGN> pl(o, t, 1);
-  const Coef<T> co(o, FLAT);
+  const Coef<T> co(o);
   const int nxy = o.L.nxy;
   const int k0 = blockIdx.y * t.chunk, k1 = min(k0 + t.chunk, o.L.nz);
   T* me = (FLAT ? ring : rring + kRing * sw) + (pl.row0 + 1) * kRow<T> + pl.p;
@@ -914,7 +922,7 @@ __global__ void __launch_bounds__(kMaxThreads, 1)
     publish(me, q);
     const Patch<T> xv = pl.load(x, 0), rv = pl.load(r, 0);
     __syncthreads();
-    neighbour_sums(me, q, xs, ys);
+    differences(me, q, xs, ys);
     point(0, q, residual<T, true>(co, none, q, xs, ys, q, q), xv, rv);
   } else {
     // step s: plane s; p three planes ahead, x and r (own cells only) likewise
@@ -954,7 +962,7 @@ __global__ void __launch_bounds__(kMaxThreads, 1)
       publish(pa, P[J]);
       if constexpr(SGN) pl.settle(P[N], T(0), zneg(o, s + 1));
       __syncthreads();
-      neighbour_sums(pa, P[J], xs, ys);
+      differences(pa, P[J], xs, ys);
       point(s, P[J], residual<T, false>(co, none, P[J], xs, ys, P[M], P[N]), pl.take(xring + J * sw),
             pl.take(rring + J * sw));
       __syncwarp();
@@ -1041,7 +1049,7 @@ __global__ void __launch_bounds__(kMaxThreads, 1)
   const int sw = slot_words<T>(t), pw = plane_words<T>(t);
   T* bring = ring + kRing * sw;
   const Place<T, SGN> pl(o, t, 1);
-  const Coef<T> co(o, FLAT);
+  const Coef<T> co(o);
   const int nxy = o.L.nxy;
   const int k0 = blockIdx.y * t.chunk, k1 = min(k0 + t.chunk, o.L.nz);
   T* me = (FLAT ? ring : bring + kRing * sw) + (pl.row0 + 1) * kRow<T> + pl.p;
@@ -1075,7 +1083,7 @@ __global__ void __launch_bounds__(kMaxThreads, 1)
     publish(me, q);
     const Patch<T> bq = centred(pl.load(b, 0));
     __syncthreads();
-    neighbour_sums(me, q, xs, ys);
+    differences(me, q, xs, ys);
     point(0, residual<T, true>(co, bq, q, xs, ys, q, q));
   } else {
     Patch<T> X[4];
@@ -1108,7 +1116,7 @@ __global__ void __launch_bounds__(kMaxThreads, 1)
       publish(pa, X[J]);
       pl.settle(X[N], sx, SGN && zneg(o, s + 1));
       __syncthreads();
-      neighbour_sums(pa, X[J], xs, ys);
+      differences(pa, X[J], xs, ys);
       point(s, residual<T, false>(co, centred(pl.take(bring + J * sw)), X[J], xs, ys, X[M], X[N]));
       __syncwarp();
     });
