@@ -33,7 +33,7 @@ struct AdiAxis {
   size_t off = 0;           // offset of cu/ip/z in the coefficient buffer
   // chunked solver (see solve_chunk)
   bool chunked = false;
-  double lambda = 0.0, scale = 0.0, fold = 0.0;
+  double lambda = 0.0, scale = 0.0, scale_lo = 0.0, fold = 0.0;  // scale + scale_lo: unevaluated
   double step = 0.0, last = 0.0, all = 0.0;  // lambda to the power of a chunk, of the last one, of the line
   double c_lo = 0.0, f_lo = 0.0, c_hi = 0.0, f_hi = 0.0, close = 0.0;  // sums beyond the ends
   // partition (warp-scan) solver, used when 64 <= n <= 1024 (n a multiple of
@@ -57,7 +57,7 @@ namespace {
 // by (1 + lambda) / (1 - lambda) rounding errors, 3.3 at alpha / h^2 = 2.5 and
 // growing with its root: up to there the error against 64-bit exact solutions is
 // below the eliminations' (mean over lines of 8 to 1024 unknowns and alpha / h^2
-// from 1e-5 to 2.4: 2.7e-16 of the largest value, the eliminations 3.4e-16).
+// from 1e-5 to 2.4: 2.7e-16 of the largest value, the eliminations 3.1e-16).
 // Shorter lines than 8 unknowns go to k_adi_tile; a line must fit a block's threads
 // (and a row its shared memory).
 constexpr double kChunkMaxBeta = 2.5;
@@ -70,25 +70,31 @@ double tangential_coef(int type) {
 
 void adi_attributes();
 
-// The chunked solver's constants for the line (component c, axis a), from the
-// rounded lambda in extended precision: the weights of the solution then add up
-// to one to rounding, so a sweep neither damps nor feeds a constant.  Appends
-// lambda^(distance to either end) of the chunks to `host`.
+// The chunked solver's constants for the line (component c, axis a), in extended
+// precision from the matrix that the eliminations take -- its diagonal is 1 + 2
+// beta as rounded -- and from the rounded lambda: the weights of the solution then
+// add up to one over the row's sum, the factor that carries that kept to twice the
+// precision (its rounding would act the same way in every sweep).  Appends lambda^(distance to either end) of the chunks
+// to `host`.
 void chunked_line(AdiAxis& A, double beta, const VBC& bc, int c, int a, std::vector<double>& host) {
   using R = long double;
   const int n = A.n, S = kLineChunk, chunks = (n + S - 1) / S;
   A.chunked = true;
-  A.lambda = static_cast<double>(2.0L * beta / ((1.0L + 2.0L * beta) + std::sqrt(1.0L + 4.0L * beta)));
+  const double diagonal = 1.0 + 2.0 * beta;
+  const R row = diagonal - 2.0L * beta;  // 1 but for that rounding
+  A.lambda = static_cast<double>(2.0L * beta / (diagonal + std::sqrt(row * (diagonal + 2.0L * beta))));
   const R l = A.lambda;
   auto power = [&](int k) { return static_cast<double>(std::pow(l, static_cast<R>(k))); };
-  A.scale = static_cast<double>((1.0L - l) * (1.0L - l));
+  const R scale = (1.0L - l) * (1.0L - l) / row;
+  A.scale = static_cast<double>(scale);
+  A.scale_lo = static_cast<double>(scale - A.scale);
   A.fold = static_cast<double>(1.0L / (1.0L - l * l));
   A.step = power(S);
   A.last = power(n - S * (chunks - 1));
   A.all = power(n);
   // what lies beyond a wall: r there is the image add + sign r, or at a node
   // the wall's value and the image about it
-  const R about_node = (1.0L + l) / (1.0L - l), about_face = 2.0L / (1.0L - l);
+  const R about_node = row * (1.0L + l) / (1.0L - l), about_face = row * 2.0L / (1.0L - l);
   auto wall = [&](int face, double& constant, double& factor) {
     const int type = bc.type[face];
     const bool node = c == a && is_dirichlet_velocity(type);
@@ -629,14 +635,15 @@ void launch_scan(const SweepArgs& a, const ScanArgs& sa, int axis, int a1, int a
 // x_0, or x_{-1} = the wall's value at a node and x_{-1-q} = add - x_{-1+q}
 // beyond it).  So with the sums up to each end of a chunk,
 //   m_q = r_q + lambda m_{q-1}  (all r below),   b_q = r_q + lambda b_{q+1}  (all above),
-// the chunk is solved by m_q and y_q = m_q + lambda y_{q+1}, x = (1 - lambda)^2 y.
+// the chunk is solved by m_q and y_q = m_q + lambda y_{q+1}, x = (1 - lambda)^2 y (the
+// factor as chunked_line rounds it).
 // A thread holds a chunk of kLineChunk unknowns; the sums of the chunks below and
 // above it, and of the images (geometric series of the line's own two sums),
 // meet in shared memory.  Every term counts, however far: weights are positive, so
 // a small unknown far from a large r keeps its relative accuracy.
 //
 // Bound: one read and one write of each field (42 us per component and sweep at
-// 256^3).  Three components take 190 us; starting a chunk as many cells early as
+// 256^3).  Three components take 194 us; starting a chunk as many cells early as
 // lambda^cells needs to vanish took 219 (2 x 7 redundant reads per 16 unknowns,
 // and the terms beyond dropped), one scan per line (k_adi_scan) 366.  At 128^3
 // 30 instead of 39 us, at 128^2 8.6 instead of 10.2 (sweeps of y, z and x).
@@ -644,7 +651,7 @@ void launch_scan(const SweepArgs& a, const ScanArgs& sa, int axis, int a1, int a
 struct LineArgs {
   Lay L;
   int n, begin, dup_index, periodic, copy_duplicate, chunks;
-  double lambda, scale, fold, step, last, all;
+  double lambda, scale, scale_lo, fold, step, last, all;
   double c_lo, f_lo, c_hi, f_hi, close;
   const double* from_lo;  // [chunks] lambda^(unknowns below the chunk)
   const double* from_hi;  // [chunks] lambda^(unknowns above the chunk)
@@ -721,7 +728,7 @@ __device__ __forceinline__ void solve_chunk(const LineArgs& a, double (&y)[kLine
   for(int t = S - 1; t >= 0; --t)
     if(t < count) {
       v = l * v + y[t];
-      y[t] = a.scale * v;
+      y[t] = a.scale * v + a.scale_lo * v;
     }
 }
 
@@ -807,6 +814,7 @@ void launch_chunked(const AdiPlan* p, const int* comps, int count, int axis, con
     a.chunks = (A.n + kLineChunk - 1) / kLineChunk;
     a.lambda = A.lambda;
     a.scale = A.scale;
+    a.scale_lo = A.scale_lo;
     a.fold = A.fold;
     a.step = A.step;
     a.last = A.last;

@@ -7,6 +7,7 @@ The oracle eliminates the same matrices; both are stable, so the fields agree to
 a few rounding errors of their largest value: 1e-13 of it.
 """
 import threading
+from fractions import Fraction
 
 import numpy as np
 import pytest
@@ -171,3 +172,30 @@ def test_both_sides_of_the_coupling_limit(oracle, shape, types, beta):
     g = po.Grid(*shape, 0.5, 0.5, 0.5)
     bc = po.bc_from(*ENDS[types])
     _compare(oracle, g, bc, beta * 0.25, _rhs(g, sum(shape)))
+
+
+@pytest.mark.parametrize("beta", [0.001, 0.05, 0.13793428401297597, 0.3, 0.7, 2.2])
+def test_sweeps_neither_damp_nor_feed_the_mean(beta):
+    """The matrix's diagonal is 1 + 2 beta as rounded, so each sweep divides a
+    periodic field's mean by its row's sum, 1 but for that rounding.  A constant of
+    the solver that is rounded differently would move the mean the same way in every
+    sweep, 1.1e-16 at a time: 7e-15 in 60.  What may remain is the rounding of the
+    factor at the chunks' ends (1.1e-16 lambda / (1 - lambda) on one unknown in 16,
+    at most 8e-18 of the mean) and the average of single roundings: 1e-17 a sweep."""
+    h = 0.5
+    g = po.Grid(24, 20, 28, h, h, h)
+    bc = po.bc_from([po.PERIODIC] * 6)
+    row = float(Fraction(1.0 + 2.0 * beta) - 2 * Fraction(beta) - 1)
+
+    def means(fields):
+        own = [tuple(slice(1, -2) if 2 - d == c else slice(1, -1) for d in range(3)) for c in range(3)]
+        return [np.asarray(f[o], np.longdouble).mean() for f, o in zip(fields, own)]
+
+    with sb.Context(to_gpu_grid(g), to_gpu_bc(bc)) as ctx:
+        # alpha = 0 first: the duplicated faces are set to one value
+        got, _ = ctx.solve_predictor_adi([1.0 + 0.5 * np.abs(r) for r in _rhs(g, 6)], 0.0)
+        before = means(got)
+        for _ in range(20):
+            got, _ = ctx.solve_predictor_adi(got, beta * h * h)
+    for m, b in zip(means(got), before):
+        assert abs(float(m / b - 1) + 60 * row) <= 6e-16
