@@ -39,7 +39,8 @@ __device__ __forceinline__ double tvd_face(double vel, double left, double right
   // differs from the two-division form by rounding only (r > 0 is read off
   // the product num delta, whose underflow stands for a value below 1e-290).
   const double nd = num * delta;
-  const bool positive = fabs(delta) >= kSmallDenominator && nd > 0.0;
+  // (comparisons that let a NaN through, as the reference's formula does)
+  const bool positive = !(fabs(delta) < kSmallDenominator) && !(nd <= 0.0);
   const double den = delta + num;
   double half_phi_delta;
   if constexpr(EXACT) {

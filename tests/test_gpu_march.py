@@ -318,3 +318,20 @@ def test_constant_solves_its_own_problem():
                                                 pressure=np.full(po.shape(g, "p"), value))
         assert d["iterations"] == 0 and d["converged"]
         assert np.all(po.active(got) == value)
+
+
+@pytest.mark.parametrize("shape", [(16, 12, 10), (32, 24, 1)], ids=lambda s: "x".join(map(str, s)))
+def test_advection_passes_a_nan_on_like_the_reference(oracle, shape):
+    """Every face value that a NaN enters is NaN, the ones it enters through the
+    limiter's far neighbour included, and no other."""
+    import solver_b200 as sb
+    g = po.Grid(*shape, 0.1, 0.1, 0.1)
+    rng = np.random.default_rng(8)
+    with sb.Context(to_gpu_grid(g), [sb.PERIODIC] * 6) as ctx:
+        for _ in range(12):
+            vel = [rng.standard_normal(po.shape(g, c)) for c in "uvw"]
+            f = vel[rng.integers(3)]
+            f[tuple(int(rng.integers(1, n - 1)) for n in f.shape)] = np.nan
+            got, exp = ctx.compute_advection_term(*vel), oracle.advection(g, *vel)
+            for a, b in zip(got, exp):
+                assert np.array_equal(np.isnan(po.active(a)), np.isnan(po.active(b)))
