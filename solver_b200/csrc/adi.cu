@@ -86,7 +86,8 @@ void chunked_line(AdiAxis& A, double beta, const VBC& bc, int c, int a, std::vec
   const R l = A.lambda;
   auto power = [&](int k) { return static_cast<double>(std::pow(l, static_cast<R>(k))); };
   const R scale = (1.0L - l) * (1.0L - l) / row;
-  A.scale = static_cast<double>(scale);
+  // rounded down: the rest is positive, and an infinity is not multiplied into a NaN
+  A.scale = std::nextafter(static_cast<double>(scale), 0.0);
   A.scale_lo = static_cast<double>(scale - A.scale);
   A.fold = static_cast<double>(1.0L / (1.0L - l * l));
   A.step = power(S);
