@@ -14,9 +14,9 @@ Arms:
   --impl b200 (default)   this repository's CUDA path through its C ABI;
   --impl reference        the reference's own CPU implementation of the same
                           step (oracle/_ref, the reference's sources compiled
-                          in place; the plain-C oracle port if that build is
-                          absent): the K timed 256^3 steps run as concurrent
-                          single-thread replicas on the host cores.
+                          in place): the K timed 256^3 steps run as concurrent
+                          single-thread replicas on the host cores.  Without
+                          that build it prints an "unavailable" line.
 
 The FP64 1-GPU line also carries two measurements of the rest of the
 headline metric (skip with --no-extras): "mixed" -- the mixed path's steps/s
@@ -233,7 +233,9 @@ def cpu_baseline(n, n_sample=128):
     return {"value": scale / sec, "unit": "steps/s", "cores": 1, "kind": kind,
             "sample": f"1 FP64 step of Taylor-Green {n_sample}^3 (nu=1/1600, CFL 0.5, tol 1e-12) "
                       f"on 1 core took {sec:.2f} s; value EXTRAPOLATED to {n}^3 by cell count "
-                      f"(x{(n / n_sample) ** 3:g}); bench.py --impl reference measures {n}^3 steps",
+                      f"(x{(n / n_sample) ** 3:g})"
+                      + (f"; bench.py --impl reference measures {n}^3 steps" if kind == "reference" else
+                         "; by the plain-C port, the reference build is not present"),
             "seconds_per_sample_step": sec, "extrapolated": True}
 
 
@@ -305,6 +307,11 @@ def run_reference_arm(args, world, rank):
     time, so ms_per_step * K is the measured wall time of the K steps."""
     if rank != 0:
         return 0
+    _, kind = cpu_lib_path()
+    if kind != "reference":
+        print(json.dumps({"impl": "reference", "unavailable": "the reference's sources were not there to build "
+                          "oracle/_ref from; the plain-C port is no substitute for it"}), flush=True)
+        return 0
     import multiprocessing as mp
     cores = os.cpu_count() or 1
     n = args.n
@@ -326,7 +333,6 @@ def run_reference_arm(args, world, rank):
     t1 = max(r[1] for r in results)
     wall = t1 - t0
     value = args.steps / wall
-    _, kind = cpu_lib_path()
     sample = (f"{args.steps} FP64 steps of Taylor-Green {n}^3 (nu=1/1600, CFL 0.5, dt = "
               f"{tg_dt(n):.17g}, tol 1e-12; the reference's own run_taylor_green_steps) as {P} "
               f"concurrent single-thread replicas on {cores} host cores "

@@ -56,3 +56,18 @@ def test_single_rank_reduce_is_identity():
     import bench
     assert bench.reduce_max(3.5, None) == 3.5
     assert bench.replica_throughput(20, 1000.0, 1) == 20.0
+
+
+def test_reference_arm_without_the_reference_says_so():
+    """No reference build: one line that says why, exit 0, and no port in its place."""
+    import json
+    import subprocess
+    sys.path.insert(0, ROOT)
+    import bench
+    if bench.cpu_lib_path()[1] == "reference":
+        pytest.skip("the reference build is present")
+    r = subprocess.run([sys.executable, os.path.join(ROOT, "bench.py"), "--impl", "reference", "--steps", "1",
+                        "--warmup", "0"], capture_output=True, text=True, timeout=300)
+    assert r.returncode == 0, r.stderr
+    line = json.loads(r.stdout.strip().splitlines()[-1])
+    assert line["impl"] == "reference" and line["unavailable"] and "value" not in line
