@@ -42,9 +42,7 @@ struct SolveScalars {
 // Per-level mean shifts of the V-cycle vectors.
 struct LevelScalars {
   double sb;  // rhs
-  double sa;  // smoother output a
-  double sx;  // smoother output b (the level's correction)
-  double sum_x;
+  double sx;  // the level's correction
 };
 
 // ---- boundary conditions (bc.cu) ----
@@ -84,7 +82,7 @@ void launch_tg_init(const Grid& g, int mode, double* u, double* v, double* w, do
                     cudaStream_t s);
 
 // ---- ADI (adi.cu) ----
-struct AdiPlan;  // per-(component, axis) Thomas coefficients, built on the host
+struct AdiPlan;  // per-(component, axis) line-solver coefficients, built on the host
 AdiPlan* adi_plan_create(const Grid& g, const VBC& bc, double alpha);
 void adi_plan_destroy(AdiPlan* p);
 // One sweep of solve_component_adi (solver/projection.cpp:868-888): reads the

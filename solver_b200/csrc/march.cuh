@@ -745,7 +745,6 @@ __global__ void __launch_bounds__(kMaxThreads, 1)
     reduce_finish<2>(acc, mx, rb, [=](const Sums<2>& s) {
       const double mean = sc->zero_mean ? s.v[0] / sc->n : 0.0;
       ls->sx = mean;
-      ls->sum_x = s.v[0];
       // r.z with z = out - mean (linsolve/poisson_solver.cpp:749, :791)
       const double rz_new = s.v[1] - mean * (sc->sum_r - sc->n * sc->sr);
       if(!sc->first) sc->beta = rz_new / sc->rz;

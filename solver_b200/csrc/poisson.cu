@@ -83,7 +83,6 @@ constexpr int kTailThreads = 512;
 // so a tail phase does no index arithmetic and reads no boundary flags.
 struct TailLevel {
   OpInfo op;
-  int sx, sy, sz;  // log2 of the refinement ratio to the next coarser level
   int off;         // offset of the level's b, x, s arrays in shared memory (elements)
   int tab;         // byte offset of the level's tables in the table region
   int nch;         // children per coarser cell
@@ -441,17 +440,13 @@ __global__ void __launch_bounds__(kDenseThreads)
     acc[1] = bs[row] * double(T(v));
   }
   if(sc == nullptr) {
-    if(blockIdx.x == 0 && threadIdx.x == 0) {
-      ls->sx = 0.0;  // the mean is already removed
-      ls->sum_x = 0.0;
-    }
+    if(blockIdx.x == 0 && threadIdx.x == 0) ls->sx = 0.0;  // the mean is already removed
     return;
   }
   const bool mx[2] = {false, false};
   reduce_finish<2>(acc, mx, rb, [=](const Sums<2>& s) {
     const double mean = sc->zero_mean ? s.v[0] / n : 0.0;
     ls->sx = mean;
-    ls->sum_x = s.v[0];
     // r.z with z = x - mean, r = b - sr (linsolve/poisson_solver.cpp:749, :791)
     const double rz_new = s.v[1] - mean * (sc->sum_r - sc->n * sc->sr) - sc->sr * s.v[0];
     if(!sc->first) sc->beta = rz_new / sc->rz;
@@ -500,8 +495,8 @@ __global__ void k_loop_gate(const SolveScalars* sc, cudaGraphConditionalHandle c
 }
 
 // Mixed path: the FP64 residual scaled to unit RMS into the FP32 inner rhs,
-// the inner correction cleared, and the inner loop's scalars initialised the
-// way k_initial_residual does it for a zero initial guess.
+// the inner correction cleared, and the inner loop's scalars initialised as
+// start_solve (march.cuh) does it for a zero initial guess.
 __global__ void __launch_bounds__(kTX* kTY)
     k_dc_to_inner(CLay L, const double* __restrict__ r, const SolveScalars* sc,
                   float* __restrict__ r32, float* __restrict__ e32, SolveScalars* si, double inner_tol,
@@ -750,9 +745,6 @@ void setup_dense(PoissonPlan* P, const int* swaps, const double* factors) {
       const Level& lv = P->levels[l];
       TailLevel& tl = t.lv[l - first];
       tl.op = lv.op;
-      tl.sx = lv.rx == 2 ? 1 : 0;
-      tl.sy = lv.ry == 2 ? 1 : 0;
-      tl.sz = lv.rz == 2 ? 1 : 0;
       cursor = (cursor + align - 1) / align * align;
       tl.off = static_cast<int>(cursor);
       cursor += 3 * static_cast<size_t>(lv.L.count());

@@ -5,6 +5,9 @@
 
 namespace ofb {
 
+// The numbers and names are part of the C ABI (of_kernel_class_name); the classes
+// of kernels that others have absorbed (kKUpdateP, kKRestrictFine,
+// kKProlongFine, kKCellPass) keep their place and count nothing.
 enum KernelClass : int {
   kKPredictor = 0,
   kKAdvection,
