@@ -242,16 +242,18 @@ struct of_ctx {
     };
     std::vector<Chunk> staged;
     std::vector<const Transfer*> plain;
+    size_t staged_bytes = 0;
     for(const Transfer& t : list) {
       if(size(t.loc) * sizeof(double) < kStagedBytes || !pageable(t.host)) {
         plain.push_back(&t);
         continue;
       }
+      staged_bytes += size(t.loc) * sizeof(double);
       const size_t n = size(t.loc), step = ofb::kStagingBytes / sizeof(double);
       for(size_t f = 0; f < n; f += step) staged.push_back(Chunk{&t, f, std::min(step, n - f)});
     }
     if(!staged.empty()) {
-      ofb::StagingLease lease;
+      ofb::StagingLease lease(staged_bytes);
       if(lease) {
         for(cudaEvent_t& e : slot_done)
           if(e == nullptr) OFB_CHECK(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));

@@ -117,8 +117,9 @@ int usable_cpus() {
   return static_cast<int>(std::thread::hardware_concurrency());
 }
 
-std::mutex g_mutex;  // guards the three below
+std::mutex g_mutex;  // guards the variables below
 int g_contexts = 0;
+size_t g_plain = 0;  // bytes moved without slots since the first context
 bool g_leased = false;
 char* g_slots = nullptr;
 Workers* g_workers = nullptr;  // not destroyed at exit: the threads end with the process
@@ -144,16 +145,21 @@ void staging_release() {
   std::unique_ptr<Workers> workers;  // joined after the lock is gone
   std::lock_guard<std::mutex> lock(g_mutex);
   if(--g_contexts > 0 || g_leased) return;
+  g_plain = 0;
   if(g_workers != nullptr && !g_workers->forked()) workers.reset(g_workers);
   g_workers = nullptr;
   if(g_slots != nullptr) cudaFreeHost(g_slots);
   g_slots = nullptr;
 }
 
-StagingLease::StagingLease() {
+StagingLease::StagingLease(size_t bytes) {
   std::lock_guard<std::mutex> lock(g_mutex);
   if(g_leased) return;
   if(g_slots == nullptr) {
+    if(g_plain < kStagingPays) {
+      g_plain += bytes;
+      return;
+    }
     void* p = nullptr;
     if(cudaHostAlloc(&p, kStagingSlots * kStagingBytes, cudaHostAllocPortable) != cudaSuccess) {
       cudaGetLastError();

@@ -103,7 +103,9 @@ def test_forked_child_ends_normally(close):
     """The workers do not exist in a child of fork(): closing its copy of the
     context or leaving must not wait for them (nor crash)."""
     out = _run(f"""
-ctx.compute_advection_term(*v)
+for _ in range(3):  # 132 MB: the slots and workers exist
+    ctx.compute_advection_term(*v)
+assert len(os.listdir("/proc/self/task")) > 7
 time.sleep(0.05)
 pid = os.fork()
 if pid == 0:
@@ -134,11 +136,42 @@ def test_workers_fit_the_cpus_of_the_process(cpus):
         pytest.skip("too few CPUs to tell")
     out = _run(f"""
 ctx.solve_predictor_adi([x[:] for x in v], 0.0)
-ctx.close()  # ends the workers
-ctx = sb.Context(g, [sb.PERIODIC] * 6)
 os.sched_setaffinity(0, set(sorted(os.sched_getaffinity(0))[:{cpus}]))
 before = len(os.listdir("/proc/self/task"))
-ctx.compute_advection_term(*v)
+for _ in range(4):
+    ctx.compute_advection_term(*v)
 print(len(os.listdir("/proc/self/task")) - before)
 """)
     assert int(out[0]) <= cpus - 1
+
+
+def test_slots_and_workers_only_where_they_pay():
+    """A program that moves little is spared them; one that moves more gets them,
+    loses them with its last context, and counts anew."""
+    out = _run("""
+ctx.solve_predictor_adi([x[:] for x in v], 0.0)  # loads what is loaded once
+ctx.close()
+def workers(calls):
+    c = sb.Context(g, [sb.PERIODIC] * 6)
+    c.upload_state(*[np.zeros(g.shape(k)) for k in "uvwuvwp"], False)
+    before = len(os.listdir("/proc/self/task"))
+    for _ in range(calls):
+        c.compute_advection_term(*v)
+    n = len(os.listdir("/proc/self/task")) - before
+    c.close()
+    return n
+print(workers(0), workers(4) > 0, workers(0))
+""")
+    assert out == ["0", "True", "0"]
+
+
+@pytest.mark.parametrize("size", SIZES, ids=lambda s: "x".join(map(str, s)))
+def test_staged_transfers_equal_plain_ones_once_the_slots_exist(size):
+    """As above for every size: another context has moved enough for the slots to
+    be there from the first call on."""
+    big = sb.Grid(96, 96, 96, 0.1, 0.1, 0.1)
+    vel = [np.ones(big.shape(c)) for c in "uvw"]
+    with sb.Context(big, [sb.PERIODIC] * 6) as holder:
+        for _ in range(4):
+            holder.compute_advection_term(*vel)
+        test_staged_transfers_equal_plain_ones(size)
