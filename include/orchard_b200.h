@@ -15,7 +15,10 @@
  *  - Host arrays are borrowed for the duration of a call only.  Calls are
  *    synchronous: they return after results and diagnostics are on the host.
  *  - One context per host thread; a context owns one CUDA stream and all
- *    device memory for its grid (state, scratch, multigrid hierarchy).
+ *    device memory for its grid (state, scratch, multigrid hierarchy).  Pageable
+ *    host arrays may pass through 8 MB of pinned memory and up to seven copying
+ *    threads that serve all contexts of the process; both are made once 64 MB
+ *    have been moved and go with the last context.
  *  - Every entry point returns an of_status; of_last_error() gives the text of
  *    the last failure on the calling thread, worded as the reference's
  *    exceptions so that the C++ layer can rethrow them unchanged.

@@ -351,9 +351,10 @@ struct of_ctx {
     for(int f = 0; f < 6 && same; ++f) same = poisson_types[f] == p.type[f];
     if(!same) {
       sync();
+      ofb::SpareMatrix spare = ofb::poisson_release_matrix(poisson);
       ofb::poisson_plan_destroy(poisson);
       poisson = nullptr;
-      poisson = ofb::poisson_plan_create(g, p, precision);
+      poisson = ofb::poisson_plan_create(g, p, precision, &spare);
       for(int f = 0; f < 6; ++f) poisson_types[f] = p.type[f];
       poisson_precision = precision;
     }

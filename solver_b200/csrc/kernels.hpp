@@ -131,7 +131,15 @@ void launch_finish(const FinishArgs& a, SolveScalars* sc, RedBuf rb, cudaStream_
 
 // ---- Poisson (poisson.cu) ----
 struct PoissonPlan;  // hierarchy, coarse factorisation, work vectors
-PoissonPlan* poisson_plan_create(const Grid& g, const PBC& pbc, int precision);
+// The dense matrix's memory of a plan that is given up, for the next one on the
+// context: allocating 2 to 8 MB (360 us) is most of a small plan's set-up.
+struct SpareMatrix {
+  void* p = nullptr;
+  size_t bytes = 0;
+};
+// `spare` (may be null) is taken over where it fits and freed where it does not.
+PoissonPlan* poisson_plan_create(const Grid& g, const PBC& pbc, int precision, SpareMatrix* spare);
+SpareMatrix poisson_release_matrix(PoissonPlan* p);  // p may be null
 void poisson_plan_destroy(PoissonPlan* p);
 int poisson_levels(const PoissonPlan* p);
 int poisson_coarse_unknowns(const PoissonPlan* p);

@@ -627,6 +627,7 @@ struct PoissonPlan {
   // levels tail_first.. run as one matrix-vector product (k_dense_apply)
   int tail_first = -1;
   void* dense = nullptr;  // their V-cycle's matrix, column by column
+  size_t dense_bytes = 0;
 };
 
 namespace {
@@ -731,7 +732,7 @@ namespace {
 // more, so there is one), lays out the shared memory of its V-cycle -- per
 // level b, x, s, then the coarsest solve's vector, factors and the levels'
 // tables -- and forms the V-cycle's matrix.
-void setup_dense(PoissonPlan* P, const int* swaps, const double* factors) {
+void setup_dense(PoissonPlan* P, const int* swaps, const double* factors, SpareMatrix* spare) {
   const int nl = static_cast<int>(P->levels.size());
   constexpr size_t tsz = sizeof(double);
   constexpr size_t kSmemLimit = 200 * 1024;
@@ -841,7 +842,9 @@ void setup_dense(PoissonPlan* P, const int* swaps, const double* factors) {
       OFB_LAUNCH_CHECK("k_dense_columns");
     };
     const size_t gbytes = static_cast<size_t>(n) * n * (P->precision == 1 ? sizeof(float) : sizeof(double));
-    OFB_CHECK(cudaMalloc(&P->dense, gbytes));
+    if(spare != nullptr && spare->bytes == gbytes) std::swap(P->dense, spare->p);
+    else OFB_CHECK(cudaMalloc(&P->dense, gbytes));
+    P->dense_bytes = gbytes;
     P->bytes += gbytes;
     if(P->precision == 1) columns(static_cast<float*>(P->dense), k_dense_columns<float>);
     else columns(static_cast<double*>(P->dense), k_dense_columns<double>);
@@ -993,7 +996,13 @@ void plan_tile(const CLay& L, int halo_rows, int rz, int streams, int fields, in
 
 }  // namespace
 
-PoissonPlan* poisson_plan_create(const Grid& g, const PBC& pbc_in, int precision) {
+PoissonPlan* poisson_plan_create(const Grid& g, const PBC& pbc_in, int precision, SpareMatrix* spare) {
+  struct FreeSpare {
+    SpareMatrix* m;
+    ~FreeSpare() {
+      if(m != nullptr) cudaFree(m->p);
+    }
+  } free_spare{spare};
   // destroyed with the function's scope unless it gets to its end
   std::unique_ptr<PoissonPlan, void (*)(PoissonPlan*)> plan(new PoissonPlan(), poisson_plan_destroy);
   PoissonPlan* const P = plan.get();
@@ -1105,7 +1114,7 @@ PoissonPlan* poisson_plan_create(const Grid& g, const PBC& pbc_in, int precision
     DeviceBytes dswaps(n * sizeof(int)), dfact(static_cast<size_t>(n) * n * sizeof(double));
     OFB_CHECK(cudaMemcpy(dswaps.p, swaps.data(), n * sizeof(int), cudaMemcpyHostToDevice));
     OFB_CHECK(cudaMemcpy(dfact.p, m.data(), static_cast<size_t>(n) * n * sizeof(double), cudaMemcpyHostToDevice));
-    setup_dense(P, static_cast<const int*>(dswaps.p), static_cast<const double*>(dfact.p));
+    setup_dense(P, static_cast<const int*>(dswaps.p), static_cast<const double*>(dfact.p), spare);
   }
 
   const size_t nf = P->levels[0].L.count();
@@ -1174,6 +1183,15 @@ void poisson_plan_destroy(PoissonPlan* P) {
   cudaFree(P->sc_in);
   cudaFree(P->dense);
   delete P;
+}
+
+SpareMatrix poisson_release_matrix(PoissonPlan* P) {
+  SpareMatrix m;
+  if(P != nullptr) {
+    std::swap(m.p, P->dense);
+    m.bytes = P->dense_bytes;
+  }
+  return m;
 }
 
 int poisson_levels(const PoissonPlan* P) { return static_cast<int>(P->levels.size()); }

@@ -335,3 +335,29 @@ def test_advection_passes_a_nan_on_like_the_reference(oracle, shape):
             got, exp = ctx.compute_advection_term(*vel), oracle.advection(g, *vel)
             for a, b in zip(got, exp):
                 assert np.array_equal(np.isnan(po.active(a)), np.isnan(po.active(b)))
+
+
+@pytest.mark.parametrize("shape", [(8, 8, 8), (20, 18, 6), (32, 24, 1)], ids=lambda s: "x".join(map(str, s)))
+def test_alternating_boundary_conditions_and_precisions(shape):
+    """One context that changes its problem from call to call (each change builds a
+    plan, which takes over the last one's matrix memory where it fits) solves each
+    as a fresh context does, bit for bit."""
+    import solver_b200 as sb
+    g = po.Grid(*shape, 0.1, 0.12, 0.09)
+    rhs = np.random.default_rng(sum(shape)).standard_normal(po.shape(g, "p"))
+    problems = [(t, p) for t in (PER, DIR, NEU, MIX) for p in (sb.OF_FP64, sb.OF_MIXED)]
+
+    def solve(ctx, types, precision):
+        ctx.set_precision(precision)
+        x, d = ctx.solve_pressure_poisson(rhs, to_gpu_pbc(po.pbc_from(types)), 300, 1e-9)
+        return np.array(x), d["iterations"]
+
+    alone = []
+    for types, precision in problems:
+        with sb.Context(to_gpu_grid(g), [sb.PERIODIC] * 6) as ctx:
+            alone.append(solve(ctx, types, precision))
+    rng = np.random.default_rng(1)
+    with sb.Context(to_gpu_grid(g), [sb.PERIODIC] * 6) as ctx:
+        for k in rng.integers(0, len(problems), 40):
+            x, it = solve(ctx, *problems[k])
+            assert it == alone[k][1] and np.array_equal(x, alone[k][0])
