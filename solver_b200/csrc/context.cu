@@ -216,10 +216,11 @@ struct of_ctx {
   // size on go through the pinned staging slots (hostcopy.hpp), chunk by chunk,
   // where these exist; the rest by plain copies.  Staged downloads have arrived
   // on return, plain ones with the next sync().
-  // Fields of 0.2 / 0.3 / 0.6 / 1.0 / 2.3 MB, the seven of a state, staged against
-  // plain: up 250/162, 297/218, 380/330, 500/475, 960/1010 us (arrays that the CPU
-  // has just written), down 250/420, 345/545, 515/800-2100, 1200/2900, 2900/7200.
-  static constexpr size_t kStagedDown = size_t(128) << 10, kStagedUp = 1000000;
+  // The seven fields of a state of 0.2 / 0.3 / 0.6 / 1.0 / 2.3 MB each, staged as
+  // one list against plain: up 175/155, 210/218, 273/300, 372/470, 740/1000 us
+  // (arrays that the CPU has just read), down 170/420, 233/540, 377/810, 980/2850,
+  // 2270/7100 (fresh arrays).
+  static constexpr size_t kStagedDown = size_t(128) << 10, kStagedUp = size_t(256) << 10;
 
   void upload(const std::vector<Transfer>& list) { transfer(list, true); }
   void download(const std::vector<Transfer>& list) { transfer(list, false); }
@@ -1233,8 +1234,17 @@ of_status of_state_upload(of_ctx* ctx, const double* u, const double* v, const d
     for(int c = 0; c < 3; ++c) {
       require_ptr(vin[c], "velocity");
       require_ptr(ain[c], "previous advection");
-      ctx->upload(ctx->vel[c], vin[c], 1 + c);
-      ctx->upload(ctx->adv_prev[c], ain[c], 1 + c);
+    }
+    require_ptr(p_total, "total pressure");
+    using T = of_ctx::Transfer;
+    std::vector<T> up;
+    for(int c = 0; c < 3; ++c) {
+      up.push_back(T{ctx->vel[c], const_cast<double*>(vin[c]), 1 + c, false});
+      up.push_back(T{ctx->adv_prev[c], const_cast<double*>(ain[c]), 1 + c, false});
+    }
+    up.push_back(T{ctx->p_total, const_cast<double*>(p_total), 0, false});
+    ctx->upload(up);
+    for(int c = 0; c < 3; ++c) {
       ctx->d2d(ctx->adv_cur[c], ctx->adv_prev[c], 1 + c);
       // Edge and corner ghosts are never written by any kernel; every
       // velocity-shaped buffer carries the state's so that full-copy
@@ -1243,8 +1253,6 @@ of_status of_state_upload(of_ctx* ctx, const double* u, const double* v, const d
       ctx->d2d(ctx->adi_b[c], ctx->vel[c], 1 + c);
       ctx->d2d(ctx->corrected[c], ctx->vel[c], 1 + c);
     }
-    require_ptr(p_total, "total pressure");
-    ctx->upload(ctx->p_total, p_total, 0);
     ctx->has_prev = has_previous_advection ? 1 : 0;
     ctx->metrics = metrics ? *metrics : of_step_metrics{};
     ctx->state_clean = false;
@@ -1259,11 +1267,14 @@ of_status of_state_download(of_ctx* ctx, double* u, double* v, double* w, double
     require_ctx(ctx);
     double* vout[3] = {u, v, w};
     double* aout[3] = {adv_u, adv_v, adv_w};
+    using T = of_ctx::Transfer;
+    std::vector<T> down;
     for(int c = 0; c < 3; ++c) {
-      if(vout[c]) ctx->download(vout[c], ctx->vel[c], 1 + c);
-      if(aout[c]) ctx->download(aout[c], ctx->adv_prev[c], 1 + c);
+      if(vout[c]) down.push_back(T{ctx->vel[c], vout[c], 1 + c, false});
+      if(aout[c]) down.push_back(T{ctx->adv_prev[c], aout[c], 1 + c, false});
     }
-    if(p_total) ctx->download(p_total, ctx->p_total, 0);
+    if(p_total) down.push_back(T{ctx->p_total, p_total, 0, false});
+    ctx->download(down);
     ctx->sync();
     if(has_previous_advection) *has_previous_advection = ctx->has_prev;
     if(metrics) *metrics = ctx->metrics;
