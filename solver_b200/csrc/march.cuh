@@ -451,7 +451,7 @@ __device__ __forceinline__ void ring4(int s0, int s1, Step step) {
 //
 // Bound: one read of b, one write of x and of bc (2.125 vectors); in FP64 at
 // 256^3 the arithmetic and the shared-memory traffic are each near the DRAM time:
-// 85 us (FP32 55), where the pre-sweeps and the residual with its restriction
+// 82 us (FP32 55), where the pre-sweeps and the residual with its restriction
 // took 53 + 65 in two passes.
 template <typename T, bool SGN, bool CD, bool FLAT>
 __global__ void __launch_bounds__(kMaxThreads, 1)
@@ -575,7 +575,7 @@ __global__ void __launch_bounds__(kMaxThreads, 1)
 // level (FINE) it also forms mean(out) and r.z for the CG; on the others no
 // mean is needed (see k_descend).  sx, sy, sz: log2 of the coarsening ratios.
 //
-// Bound: reads x, b and e, writes out (3.125 vectors); 107 us at 256^3 in FP64 (71
+// Bound: reads x, b and e, writes out (3.125 vectors); 103 us at 256^3 in FP64 (71
 // in FP32), where the prolongation with one sweep and the second sweep took 89 + 78.
 template <typename T, bool SGN, bool CD, bool FLAT, bool FINE, bool PAIRS>
 __global__ void __launch_bounds__(kMaxThreads, 1)
@@ -871,8 +871,8 @@ __global__ void __launch_bounds__(kMaxThreads, 1)
 // x = (x - sx) + alpha p, r = (r - sr) - alpha A p (in FP64 arithmetic), the
 // residual's norm and the convergence test, and the means of the new x and r (a
 // large mean in the initial guess leaves its rounding in the first x).  Bound:
-// reads p, x and r, writes x and r (5 vectors); at 256^3 123 us in FP64 (119
-// without the sum of x), where the update from a stored A p took 142.
+// reads p, x and r, writes x and r (5 vectors); at 256^3 119 to 122 us in FP64,
+// where the update from a stored A p took 142.
 template <typename T, bool SGN, bool FLAT>
 __global__ void __launch_bounds__(kMaxThreads, 1)
     k_advance(OpInfo o, Tile t, Direction<T> d, T* __restrict__ x, T* __restrict__ r, SolveScalars* sc, RedBuf rb,
