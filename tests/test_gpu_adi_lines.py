@@ -199,3 +199,14 @@ def test_sweeps_neither_damp_nor_feed_the_mean(beta):
             got, _ = ctx.solve_predictor_adi(got, beta * h * h)
     for m, b in zip(means(got), before):
         assert abs(float(m / b - 1) + 60 * row) <= 6e-16
+
+
+@pytest.mark.parametrize("types", list(ENDS))
+@pytest.mark.parametrize("shape", [(4095, 3, 1), (4097, 3, 2), (2, 2050, 3), (3, 8200, 1), (2, 16384, 1), (1, 16385, 1)],
+                         ids=lambda s: "x".join(map(str, s)))
+def test_longest_lines(oracle, shape, types):
+    """Rows of up to 4096 unknowns and columns of up to 16384 are solved in chunks
+    (four rows, or as few as one column, to a block of 1024 threads), longer ones
+    by one thread each."""
+    g = po.Grid(*shape, 0.5, 0.6, 0.55)
+    _compare(oracle, g, po.bc_from(*ENDS[types]), 0.2, _rhs(g, sum(shape)))
